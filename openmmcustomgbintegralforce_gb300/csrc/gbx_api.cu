@@ -140,9 +140,12 @@ gbx_status upload_quadrature(Context* ctx) {
   std::vector<float4> qv(Q);
   std::vector<float2> qw(Q);
   double S4 = 0.0, S7 = 0.0;
+  // GBSW keeps a direction's points together (ray by ray): 32 lanes then hold
+  // neighbouring points, whose table cells share cache lines (gbsw_integral_kernel)
+  const bool rays = c.model == GBX_MODEL_GBSW;
   for (int i = 0; i < c.n_radial; ++i)
     for (int j = 0; j < nS; ++j) {
-      const int q = i * nS + j;
+      const int q = rays ? j * c.n_radial + i : i * nS + j;
       const double r = xr[i];
       for (int k = 0; k < 3; ++k) ctx->q_off[3 * q + k] = r * leb[4 * j + k];
       ctx->q_rad[q] = r;
@@ -226,6 +229,7 @@ gbx_status alloc_atom_buffers(Context* ctx) {
     GBX_TRY(dalloc(ctx, &ctx->d_sgeom, 2));
   }
   GBX_TRY(dalloc(ctx, &ctx->d_force_fx, 3 * (size_t)n));
+  GBX_TRY(dalloc(ctx, &ctx->d_f4, 4 * (size_t)n));
   GBX_TRY(dalloc(ctx, &ctx->d_energy, 1));
   GBX_TRY(dalloc(ctx, &ctx->d_dEdR_fx, n));
   GBX_TRY(dalloc(ctx, &ctx->d_dEdq_fx, n));
@@ -293,11 +297,20 @@ gbx_status alloc_records(Context* ctx, int R) {
 // per-warp regions from the largest need the device reported (read without
 // blocking; first guess half a warp's points).  Warps whose records do not
 // fit walk their lists in the chain rule instead, with the same result.
-gbx_status prepare_records(Context* ctx, bool wanted) {
+gbx_status prepare_records(Context* ctx, bool wanted, bool adjoint) {
   ctx->records = false;
+  ctx->records_self = adjoint;
+  ctx->srec_manage = ctx->srec_auto;
   if (!wanted || ctx->cfg.model != GBX_MODEL_GBSW) return GBX_OK;
+  if (adjoint) {
+    // a caller's own graph of an unchecked adjoint walks the lists: its
+    // replays must not hold record buffers that later calls resize
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GBX_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return GBX_OK;
+  }
   const long long warps = (long long)ctx->n * ctx->n_chunks;
-  if (ctx->srec_auto) {
+  if (ctx->srec_manage) {
     long long need = 0;
     if (ctx->srec_pending) {
       const cudaError_t q = cudaEventQuery(ctx->srec_ev);
@@ -468,7 +481,7 @@ gbx_status run_pipeline(Context* ctx, const float4* posq, unsigned long long* fo
   else GBX_TRY(build_table_checked(ctx, check));
   if (count_work) GBX_CUDA(cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long) * 4, ctx->stream));
   const bool chain = forces || adjoint;
-  GBX_TRY(prepare_records(ctx, chain && !adjoint && !count_work));
+  GBX_TRY(prepare_records(ctx, chain && !count_work, adjoint));
   GBX_TRY(mark());
   GBX_TRY(gbx::launch_binning(ctx, ctx->d_pos, count_work));
   GBX_TRY(mark());
@@ -481,11 +494,10 @@ gbx_status run_pipeline(Context* ctx, const float4* posq, unsigned long long* fo
     GBX_TRY(mark());
     GBX_TRY(gbx::launch_custom_chain_prep(ctx, force, stride));
     GBX_TRY(mark());
-    if (chain) GBX_TRY(gbx::launch_chain(ctx, ctx->d_pos, force, stride, false));
+    if (chain) GBX_TRY(gbx::launch_chain(ctx, ctx->d_pos, false));
     GBX_TRY(mark());
-    GBX_TRY(gbx::launch_energy_reduce(ctx, energy, false));
+    GBX_TRY(gbx::launch_finish(ctx, force, stride, energy, chain, false));
     GBX_TRY(mark());
-    GBX_TRY(gbx::launch_publish_status(ctx));
     ctx->have_result = true;
     if (check) {
       unsigned st = 0;
@@ -501,23 +513,21 @@ gbx_status run_pipeline(Context* ctx, const float4* posq, unsigned long long* fo
   GBX_TRY(gbx::launch_born(ctx));
   if (adjoint) {
     GBX_CUDA(cudaMemsetAsync(ctx->d_dEdq_fx, 0, sizeof(unsigned long long) * ctx->n, ctx->stream));
-    GBX_CUDA(cudaMemsetAsync(ctx->d_dEdR_fx, 0, sizeof(unsigned long long) * ctx->n, ctx->stream));
   }
   GBX_TRY(mark());
   GBX_TRY(gbx::launch_pair(ctx, ctx->d_pos, force, stride, adjoint));
   GBX_TRY(mark());
   GBX_TRY(gbx::launch_chain_prep(ctx, adjoint));
   GBX_TRY(mark());
-  if (chain) GBX_TRY(gbx::launch_chain(ctx, ctx->d_pos, force, stride, adjoint));
-  if (ctx->records && ctx->srec_auto && !ctx->srec_pending) {
+  if (chain) GBX_TRY(gbx::launch_chain(ctx, ctx->d_pos, adjoint));
+  if (ctx->records && ctx->srec_manage && !ctx->srec_pending) {
     GBX_CUDA(cudaMemcpyAsync(ctx->h_rmax, ctx->d_rmax, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     GBX_CUDA(cudaEventRecord(ctx->srec_ev, ctx->stream));
     ctx->srec_pending = true;
   }
   GBX_TRY(mark());
-  GBX_TRY(gbx::launch_energy_reduce(ctx, energy, adjoint));
+  GBX_TRY(gbx::launch_finish(ctx, force, stride, energy, chain, adjoint));
   GBX_TRY(mark());
-  GBX_TRY(gbx::launch_publish_status(ctx));
   ctx->have_result = true;
   if (check) {
     unsigned st = 0;
@@ -774,7 +784,7 @@ gbx_status gbx_destroy(gbx_context* handle) {
   void* ptrs[] = {ctx->d_qv, ctx->d_qw, ctx->d_qoff, ctx->d_radius, ctx->d_charge, ctx->d_par, ctx->d_wpar,
                   ctx->d_geom, ctx->d_cell_count, ctx->d_cell_start, ctx->d_cell_cursor, ctx->d_entries,
                   ctx->d_block_sums, ctx->d_reduce, ctx->d_pos, ctx->d_J, ctx->d_born, ctx->d_bornf, ctx->d_dBdJ,
-                  ctx->d_integrals, ctx->d_dEdB_fx, ctx->d_dEdJ, ctx->d_energy_part, ctx->d_force_fx,
+                  ctx->d_integrals, ctx->d_dEdB_fx, ctx->d_dEdJ, ctx->d_energy_part, ctx->d_force_fx, ctx->d_f4,
                   ctx->d_energy, ctx->d_dEdR_fx, ctx->d_dEdq_fx, ctx->d_alpha_grad, ctx->d_status, ctx->d_work,
                   ctx->d_tgeom, ctx->d_wgeom, ctx->d_tcount, ctx->d_tstart, ctx->d_tcursor, ctx->d_tburied,
                   ctx->d_tblock_sums, ctx->d_tentry, ctx->d_tindex, ctx->d_entry4, ctx->d_entry_par,

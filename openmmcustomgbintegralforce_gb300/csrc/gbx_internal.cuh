@@ -80,7 +80,7 @@ struct ModelConst {
   int cap;
   int skip_empty;
   int nq;
-  int nshell;                // points per radial shell (index = radial * nshell + angular)
+  int nrad;                  // radial points per direction (GBSW: index = direction * nrad + radial)
   int cutoff_chain_quirk;
   float sw, c1, c3;          // GBSW: u = 1/2 + c1 dr - c3 dr^3, c1 = 3/(4w), c3 = 1/(4w^3)
   float gamma0_lnlambda;     // GBMV-I gamma_j = gamma0 ln(lambda) / R^4
@@ -182,6 +182,7 @@ struct Context {
   bool gbmv_cells = false;                    // this call's GBMV passes run by cell
   CustomPlan* custom = nullptr;               // expressions outside the canonical set (gbx_custom.cu)
   unsigned long long* d_force_fx = nullptr;  // internal force buffer [3n] (host path)
+  unsigned long long* d_f4 = nullptr;  // [4n] the chain rule's force (x, y, z) and dE/dR per atom
   double* d_energy = nullptr;     // internal energy (host path)
   unsigned long long* d_dEdR_fx = nullptr;  // adjoint [n]
   unsigned long long* d_dEdq_fx = nullptr;  // adjoint [n]
@@ -193,6 +194,8 @@ struct Context {
   // other than i shapes, written by the integral pass: warp w (atom,
   // quadrature chunk) owns records [w R, (w + 1) R)
   bool records = false;          // this call writes and reads records
+  bool records_self = false;     // ... of atom i's own entries too (the adjoint)
+  bool srec_manage = false;      // this call may size the regions (automatic, not under capture)
   bool srec_auto = true;         // size R from the largest need seen
   int4* d_srec = nullptr;
   int* d_srec_st = nullptr;      // the recorded point's list start, beside each record
@@ -282,6 +285,14 @@ __device__ __forceinline__ long long float_to_fixed_split(float v) {
   return (long long)(((unsigned long long)(long long)__float2int_rz(hf) << 32) + lo);
 }
 
+// Hardware 1/sqrt(x) (PTX rsqrt.approx, relative error below 2^-22;
+// subnormal inputs flush to zero).
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __device__ __forceinline__ void red_add_fixed(unsigned long long* addr, float v) {
   atomicAdd(addr, (unsigned long long)float_to_fixed(v));
 }
@@ -311,7 +322,9 @@ void choose_table(Context* ctx);
 
 gbx_status launch_stage_positions(Context* ctx, const void* posq);
 gbx_status launch_finish_outputs(Context* ctx, unsigned long long* force, int stride, float* energy_float);
-gbx_status launch_publish_status(Context* ctx);
+// The call's last kernel: the chain rule's sums added to the force buffer
+// (and dE/dR), the energy, the published status.
+gbx_status launch_finish(Context* ctx, unsigned long long* force, int stride, double* energy, bool chain, bool adjoint);
 gbx_status launch_table_build(Context* ctx, const float4* pos);
 size_t table_geom_scratch_doubles(int n);
 gbx_status launch_tight_build(Context* ctx, const float4* pos);
@@ -327,13 +340,11 @@ int pair_energy_parts(int n, int segments);
 int pair_segments(int n, int sms);
 ModelConst make_model_const(const Context* ctx);
 gbx_status launch_chain_prep(Context* ctx, bool adjoint);
-gbx_status launch_chain(Context* ctx, const float4* pos, unsigned long long* force, int stride, bool adjoint);
+gbx_status launch_chain(Context* ctx, const float4* pos, bool adjoint);
 bool gbmv_cells_apply(const Context* ctx);
 gbx_status launch_gbmv_cells_bin(Context* ctx, const float4* pos, const ModelConst& m);
 gbx_status launch_gbmv_cells_integral(Context* ctx, const float4* pos, const ModelConst& m);
-gbx_status launch_gbmv_cells_chain(Context* ctx, const float4* pos, const ModelConst& m, unsigned long long* force,
-                                   int stride, bool adjoint);
-gbx_status launch_energy_reduce(Context* ctx, double* energy, bool adjoint);
+gbx_status launch_gbmv_cells_chain(Context* ctx, const float4* pos, const ModelConst& m, bool adjoint);
 gbx_status launch_adjoint_out(Context* ctx, double* energy, double* forces, double* dEdq, double* dEdR,
                               double* dEdalpha);
 

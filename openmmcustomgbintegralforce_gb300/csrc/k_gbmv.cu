@@ -56,7 +56,7 @@ constexpr int kSortMax = 16 * kWarp;    // cells of up to 512 points are sorted 
 constexpr int kChainPts = 4;            // points per chain sub-step
 constexpr int kChainEnt = kWarp / kChainPts;  // entry lanes per point
 constexpr int kEntPerLane = kMaxList / kChainEnt;
-static_assert(kChainPts * kChainEnt == kWarp, "chain lane split");
+static_assert(kChainPts * kChainEnt == kWarp && kChainPts == 4, "chain lane split: a point lane per pushed field");
 
 struct CellPoints {
   int* count;   // [cells] points binned into the cell
@@ -453,43 +453,44 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_reduce_kernel(int n, Quad qu
 }
 
 struct CellChainOut {
-  unsigned long long* force;
-  int stride;
-  unsigned long long* dEdR;
+  unsigned long long* f4;  // per atom: force x, y, z and dE/dR (fixed point)
 };
 
 __device__ __forceinline__ void add_fixed3(const CellChainOut& o, int k, float gx, float gy, float gz) {
   const long long fx = float_to_fixed(gx), fy = float_to_fixed(gy), fz = float_to_fixed(gz);
-  if (fx) atomicAdd(&o.force[k], (unsigned long long)fx);
-  if (fy) atomicAdd(&o.force[k + o.stride], (unsigned long long)fy);
-  if (fz) atomicAdd(&o.force[k + 2 * o.stride], (unsigned long long)fz);
+  unsigned long long* f = o.f4 + 4 * (size_t)k;
+  if (fx) atomicAdd(f, (unsigned long long)fx);
+  if (fy) atomicAdd(f + 1, (unsigned long long)fy);
+  if (fz) atomicAdd(f + 2, (unsigned long long)fz);
 }
 
-// One fixed-point reduction (skipped when the value rounds to zero).
-__device__ __forceinline__ void add_fixed_one(unsigned long long* a, int k, float v) {
+// Field c of atom k (3: dE/dR), one fixed-point reduction (skipped when the value rounds to zero).
+__device__ __forceinline__ void add_fixed_one(const CellChainOut& o, int k, int c, float v) {
   const long long r = float_to_fixed(v);
-  if (r) atomicAdd(&a[k], (unsigned long long)r);
+  if (r) atomicAdd(o.f4 + 4 * (size_t)k + c, (unsigned long long)r);
 }
 
 // One point's chain-rule factors (the point's own lanes read them from
 // shared memory): its position in the cell frame and the factors of the
-// gradient with c ds/dS folded in.  GBMV-II: with u_j = F_j / T_j and
-// vd = v . d_j, the pull on entry j is
-//   g_j = [-400 u_j (A + C vd) + B F_j (F_j - 400 u_j r_j^2)] d_j + F_j C v
-// with A = c ds/dS s0 s2 / |v|^2, B = 2 c ds/dS s0 s1 / |v|^2,
-// C = -2 c ds/dS s0 s1 s2 / |v|^4 (the d s1, d s2 and d |v|^2 factors).
-// GBMV-I: g_j = A e_j r_j^2 d_j with A = 4 c ds/dS gamma_j
-// folded per entry.
+// gradient with c ds/dS folded in.  GBMV-II: the pull on entry j is
+//   g_j = F_j [ (-400 W_j / T_j + B F_j) d_j + V ],  W_j = A + B F_j r_j^2 + V . d_j
+// with A = c ds/dS s0 s2 / |v|^2, B = 2 c ds/dS s0 s1 / |v|^2 and
+// V = -2 c ds/dS s0 s1 s2 / |v|^4 v (the d s1, d s2 and d |v|^2 factors), and
+// c ds/dS dS/dR_j = W_j dF_j/dR_j.  Written this way a pair of entries takes 27
+// packed operations, where the expanded gradient took 35.
+// GBMV-I: g_j = A e_j r_j^2 d_j with A = 4 c ds/dS, gamma_j folded per entry.
 struct __align__(16) PointChain {
   float2 npx, npy, npz;  // minus the point's position in the cell frame, in both halves
-  float2 A, B, C;        // GBMV-I: A only
-  float2 vx, vy, vz;
+  float2 A, B;           // GBMV-I: A only
+  float2 Vx, Vy, Vz;
   float cS;
   int i;
 };
 
+// Registers are capped where the occupancy measured fastest (10,000 atoms, 24 x 50:
+// GBMV-II 532, 488, 471 us with 5, 6, 7 blocks per SM; GBMV-I 467, 487, 510 with 6, 7, 8).
 template <int MODEL, bool PER, bool ADJ>
-__global__ void __launch_bounds__(kCellThreads) gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab,
+__global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBMV2 ? 7 : 6) gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab,
                                                                        Quad quad, ModelConst m, CellPoints cp,
                                                                        const float2* __restrict__ dEdJ,
                                                                        CellChainOut out) {
@@ -536,8 +537,8 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_chain_kernel(const flo
       PointChain pc;
       pc.cS = 0.0f;
       pc.i = -1;
-      pc.npx = pc.npy = pc.npz = pc.A = pc.B = pc.C = bc2(0.f);
-      pc.vx = pc.vy = pc.vz = bc2(0.f);
+      pc.npx = pc.npy = pc.npz = pc.A = pc.B = bc2(0.f);
+      pc.Vx = pc.Vy = pc.Vz = bc2(0.f);
       if (k < P) {
         const int p = order[k];
         const int i = p / m.nq, q = p - i * m.nq;
@@ -565,10 +566,9 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_chain_kernel(const flo
                       C = 2.0f * pc.cS * (-s1 * s2 * inv3 * inv3);
           pc.A = bc2(A);
           pc.B = bc2(B);
-          pc.C = bc2(C);
-          pc.vx = bc2(vx);
-          pc.vy = bc2(vy);
-          pc.vz = bc2(vz);
+          pc.Vx = bc2(C * vx);
+          pc.Vy = bc2(C * vy);
+          pc.Vz = bc2(C * vz);
         }
       }
       // only points with a nonzero factor pull on anything (a saturated
@@ -591,9 +591,10 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_chain_kernel(const flo
           float2 dx = __fadd2_rn(ex, pc.npx), dy = __fadd2_rn(ey, pc.npy), dz = __fadd2_rn(ez, pc.npz);
           img.apply2(dx, dy, dz);
           const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-          // atom i's own entry moves with the point: no force from it
-          const float2 own = make_float2(kj.x != pi ? 1.0f : 0.0f, kj.y != pi ? 1.0f : 0.0f);
-          float2 gx, gy, gz;
+          // atom i's own entry moves with the point: no force from it (its C or
+          // gamma is dropped, or in the adjoint, which needs them, the result)
+          if (!ADJ) aw = make_float2(kj.x != pi ? aw.x : 0.0f, kj.y != pi ? aw.y : 0.0f);
+          float2 f, hx, hy, hz;  // the pull: f h
           if (MODEL == GBX_MODEL_GBMV1) {
             const float2 r4 = __fmul2_rn(r2, r2);
             const float2 g = __fmul2_rn(aw, r4);
@@ -604,57 +605,52 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_chain_kernel(const flo
                                            make_float2(-4.0f * aw.x / ek.x, -4.0f * aw.y / ek.y));
               accR[e] = __fadd2_rn(accR[e], dr);
               if (!sorted) {
-                if (l < cnt) add_fixed_one(out.dEdR, kj.x, dr.x);
-                if (l + 1 < cnt) add_fixed_one(out.dEdR, kj.y, dr.y);
+                if (l < cnt) add_fixed_one(out, kj.x, 3, dr.x);
+                if (l + 1 < cnt) add_fixed_one(out, kj.y, 3, dr.y);
               }
             }
             // dS/d(delta) = 4 gamma e r^2 delta
-            const float2 gs = __fmul2_rn(__fmul2_rn(__fmul2_rn(__fmul2_rn(pc.A, aw), ex2), r2), own);
-            gx = __fmul2_rn(gs, dx);
-            gy = __fmul2_rn(gs, dy);
-            gz = __fmul2_rn(gs, dz);
+            f = __fmul2_rn(__fmul2_rn(__fmul2_rn(pc.A, aw), ex2), r2);
+            hx = dx;
+            hy = dy;
+            hz = dz;
           } else {
             const float2 T = __ffma2_rn(bc2(100.0f), r2, ek);
             const float2 rT = rcp2(T);
             const float2 CT = __fmul2_rn(aw, rT);
             const float2 F = __fmul2_rn(CT, CT);
-            const float2 u = __fmul2_rn(F, rT);  // dF/d(delta) = -400 u delta
-            const float2 vd = __ffma2_rn(pc.vx, dx, __ffma2_rn(pc.vy, dy, __fmul2_rn(pc.vz, dz)));
+            const float2 W = __ffma2_rn(
+                pc.Vx, dx, __ffma2_rn(pc.Vy, dy, __ffma2_rn(pc.Vz, dz, __ffma2_rn(pc.B, __fmul2_rn(F, r2), pc.A))));
             if (ADJ) {
-              // dF/dR_j with T = C_j + 100 (r^2 - R_j^2), C_j = 10 p1 R_j + p2 (nm -> A):
-              // c ds/dS (s2 dF + s1 d(r^2 F^2) + d|v|^2) / |v|^2 as pc.A, pc.B, pc.C carry them
+              // dF/dR_j with T = C_j + 100 (r^2 - R_j^2), C_j = 10 p1 R_j + p2 (nm -> A)
               const float2 Tp = __ffma2_rn(bc2(-200.0f), er, bc2(Cp));
               const float2 num = __ffma2_rn(bc2(Cp), T, __fmul2_rn(make_float2(-aw.x, -aw.y), Tp));
               const float2 dFdR = __fmul2_rn(__fmul2_rn(__fmul2_rn(bc2(2.0f), CT), num), __fmul2_rn(rT, rT));
-              const float2 fac = __ffma2_rn(pc.C, vd, __ffma2_rn(pc.B, __fmul2_rn(r2, F), pc.A));
-              const float2 dr = __fmul2_rn(dFdR, fac);
+              const float2 dr = __fmul2_rn(dFdR, W);
               accR[e] = __fadd2_rn(accR[e], dr);
               if (!sorted) {
-                if (l < cnt) add_fixed_one(out.dEdR, kj.x, dr.x);
-                if (l + 1 < cnt) add_fixed_one(out.dEdR, kj.y, dr.y);
+                if (l < cnt) add_fixed_one(out, kj.x, 3, dr.x);
+                if (l + 1 < cnt) add_fixed_one(out, kj.y, 3, dr.y);
               }
             }
-            // g = [-400 u (A + C vd) + B F (F - 400 u r^2)] delta + F C v
-            const float2 m400u = __fmul2_rn(bc2(-400.0f), u);
-            const float2 sc = __fmul2_rn(
-                __ffma2_rn(m400u, __ffma2_rn(pc.C, vd, pc.A), __fmul2_rn(__fmul2_rn(pc.B, F), __ffma2_rn(m400u, r2, F))),
-                own);
-            const float2 FC = __fmul2_rn(__fmul2_rn(F, own), pc.C);
-            gx = __ffma2_rn(sc, dx, __fmul2_rn(FC, pc.vx));
-            gy = __ffma2_rn(sc, dy, __fmul2_rn(FC, pc.vy));
-            gz = __ffma2_rn(sc, dz, __fmul2_rn(FC, pc.vz));
+            const float2 s = __ffma2_rn(__fmul2_rn(bc2(-400.0f), rT), W, __fmul2_rn(pc.B, F));
+            f = F;
+            hx = __ffma2_rn(s, dx, pc.Vx);
+            hy = __ffma2_rn(s, dy, pc.Vy);
+            hz = __ffma2_rn(s, dz, pc.Vz);
           }
+          if (ADJ) f = make_float2(kj.x != pi ? f.x : 0.0f, kj.y != pi ? f.y : 0.0f);
           if (sorted) {
-            acc[e][0] = __fadd2_rn(acc[e][0], gx);
-            acc[e][1] = __fadd2_rn(acc[e][1], gy);
-            acc[e][2] = __fadd2_rn(acc[e][2], gz);
+            acc[e][0] = __ffma2_rn(f, hx, acc[e][0]);
+            acc[e][1] = __ffma2_rn(f, hy, acc[e][1]);
+            acc[e][2] = __ffma2_rn(f, hz, acc[e][2]);
           } else {
-            if (l < cnt && kj.x != pi) add_fixed3(out, kj.x, -gx.x, -gy.x, -gz.x);
-            if (l + 1 < cnt && kj.y != pi) add_fixed3(out, kj.y, -gx.y, -gy.y, -gz.y);
+            if (l < cnt && kj.x != pi) add_fixed3(out, kj.x, -f.x * hx.x, -f.x * hy.x, -f.x * hz.x);
+            if (l + 1 < cnt && kj.y != pi) add_fixed3(out, kj.y, -f.y * hx.y, -f.y * hy.y, -f.y * hz.y);
           }
-          ox = __fadd2_rn(ox, gx);
-          oy = __fadd2_rn(oy, gy);
-          oz = __fadd2_rn(oz, gz);
+          ox = __ffma2_rn(f, hx, ox);
+          oy = __ffma2_rn(f, hy, oy);
+          oz = __ffma2_rn(f, hz, oz);
         };
 #pragma unroll
         for (int e = 0; e < kPairsPerLane; ++e) {
@@ -695,7 +691,8 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_chain_kernel(const flo
           }
         }
         const int kn = __shfl_down_sync(0xffffffffu, key, 1);
-        if (lane < np && (lane == np - 1 || kn != key)) add_fixed3(out, key, o.x, o.y, o.z);
+        const bool last = lane < np && (lane == np - 1 || kn != key);  // the run's sum
+        if (last) add_fixed3(out, key, o.x, o.y, o.z);
       } else if (lane < np) {
         add_fixed3(out, key, o.x, o.y, o.z);
       }
@@ -719,15 +716,14 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_chain_kernel(const flo
         accR[e].y += __shfl_xor_sync(0xffffffffu, accR[e].y, off);
       }
     }
+    // lane (ps, es) pushes component ps of the pair's entries: an atom's
+    // components leave as neighbouring fields of its sector in one instruction
     const int l = 2 * (es + e * kChainEnt);
-    if (ps == 0) {
-      for (int h = 0; h < 2; ++h) {
-        if (l + h >= cnt) break;
-        const int kj = L.idx[l + h];
-        add_fixed3(out, kj, h ? -acc[e][0].y : -acc[e][0].x, h ? -acc[e][1].y : -acc[e][1].x,
-                   h ? -acc[e][2].y : -acc[e][2].x);
-        if (ADJ) add_fixed_one(out.dEdR, kj, h ? accR[e].y : accR[e].x);
-      }
+    const float2 sum = ps == 0 ? acc[e][0] : ps == 1 ? acc[e][1] : ps == 2 ? acc[e][2] : accR[e];
+    if (ps < 3 || ADJ) {
+      const float sign = ps < 3 ? -1.0f : 1.0f;
+      if (l < cnt) add_fixed_one(out, L.idx[l], ps, sign * sum.x);
+      if (l + 1 < cnt) add_fixed_one(out, L.idx[l + 1], ps, sign * sum.y);
     }
   }
 }
@@ -802,15 +798,14 @@ gbx_status launch_gbmv_cells_integral(Context* ctx, const float4* pos, const Mod
   return GBX_OK;
 }
 
-gbx_status launch_gbmv_cells_chain(Context* ctx, const float4* pos, const ModelConst& m, unsigned long long* force,
-                                   int stride, bool adjoint) {
+gbx_status launch_gbmv_cells_chain(Context* ctx, const float4* pos, const ModelConst& m, bool adjoint) {
   cudaStream_t st = ctx->stream;
   const Entries t = gbmv_entries(ctx);
   const Quad qd{ctx->d_qv, ctx->d_qw, ctx->d_qoff};
   const long long npts = (long long)ctx->n * m.nq;
   const CellPoints cp{ctx->d_pcount, ctx->d_pstart, ctx->d_porder, ctx->d_pcell, ctx->d_prank,
                       ctx->d_sval,   ctx->d_pstate, (size_t)npts};
-  const CellChainOut o{force, stride, ctx->d_dEdR_fx};
+  const CellChainOut o{ctx->d_f4};
   const int cell_blocks = (int)((ctx->cell_cap + kCellWarps - 1) / kCellWarps);
   const bool per = ctx->cfg.periodic != 0;
   const int sel = (m.model == GBX_MODEL_GBMV1 ? 0 : 4) + (per ? 2 : 0) + (adjoint ? 1 : 0);

@@ -14,7 +14,7 @@ ModelConst make_model_const(const Context* ctx) {
   m.cap = c.table_cap;
   m.skip_empty = c.skip_empty;
   m.nq = c.n_radial * c.lebedev_order;
-  m.nshell = c.lebedev_order;
+  m.nrad = c.n_radial;
   m.cutoff_chain_quirk = c.cutoff_chain_quirk;
   const double w = c.switch_width;
   m.sw = (float)w;
@@ -44,7 +44,8 @@ namespace {
 // atom order set, internal atom i is read from the caller's slot slot_of[i].
 template <bool DBL>
 __global__ void stage_positions_kernel(const void* __restrict__ in, int n, const int* __restrict__ slot_of,
-                                       const float* __restrict__ wpar, float4* __restrict__ out) {
+                                       const float* __restrict__ wpar, float4* __restrict__ out,
+                                       ulonglong2* __restrict__ f4) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int k = slot_of ? slot_of[i] : i;
@@ -61,6 +62,7 @@ __global__ void stage_positions_kernel(const void* __restrict__ in, int n, const
     z = p.z;
   }
   out[i] = make_float4(x, y, z, wpar[i]);
+  f4[2 * i] = f4[2 * i + 1] = make_ulonglong2(0ull, 0ull);  // the chain rule's sums of this call
 }
 
 // The caller's outputs of a call that ran on internal buffers: forces added
@@ -79,8 +81,8 @@ __global__ void finish_outputs_kernel(int n, const int* __restrict__ slot_of,
 // The call's device status, published to mapped host memory so that a later
 // call can read it without synchronising: counts of table overflows and of
 // non-finite results, and the largest table seen (cells, list entries).
-__global__ void publish_status_kernel(const unsigned* __restrict__ status, const TableGeom* __restrict__ geom,
-                                      unsigned long long* __restrict__ dev, StatusRecord* host) {
+__device__ __forceinline__ void publish_status(const unsigned* __restrict__ status, const TableGeom* __restrict__ geom,
+                                               unsigned long long* __restrict__ dev, StatusRecord* host) {
   const unsigned st = *status;
   if (st & (kStatusTableCells | kStatusTableEntries | kStatusSegmentTooLong)) ++dev[1];
   if (st & kStatusNonFinite) ++dev[2];
@@ -95,6 +97,29 @@ __global__ void publish_status_kernel(const unsigned* __restrict__ status, const
   h->max_entries = dev[4];
   __threadfence_system();
   h->seq = dev[0];
+}
+
+// The call's last kernel.  The chain rule's sums join the force buffer by
+// reductions (a caller may have other forces adding to it), the fixed-point
+// pair energy joins the energy, one thread publishes the status: one launch
+// where the energy and the status took one each.
+constexpr int kFinishThreads = 256;
+__global__ void __launch_bounds__(kFinishThreads) finish_kernel(
+    int n, const ulonglong2* __restrict__ f4, unsigned long long* __restrict__ force, int stride,
+    unsigned long long* __restrict__ dEdR, const unsigned long long* __restrict__ energy_fx,
+    double* __restrict__ energy, const unsigned* __restrict__ status, const TableGeom* __restrict__ geom,
+    unsigned long long* __restrict__ pub, StatusRecord* host) {
+  const int i = blockIdx.x * kFinishThreads + threadIdx.x;
+  if (i == 0) {
+    if (energy) *energy += fixed_to_double(*energy_fx);
+    publish_status(status, geom, pub, host);
+  }
+  if (i >= n || !f4) return;
+  const ulonglong2 a = f4[2 * i], b = f4[2 * i + 1];
+  atomicAdd(force + i, a.x);
+  atomicAdd(force + stride + i, a.y);
+  atomicAdd(force + 2 * (size_t)stride + i, b.x);
+  if (dEdR) dEdR[i] = b.y;
 }
 
 __global__ void born_kernel(int n, int n_chunks, const float* __restrict__ J, double S4, double S7, double C4,
@@ -185,10 +210,11 @@ __global__ void __launch_bounds__(kRedThreads) energy_reduce_kernel(const double
 gbx_status launch_stage_positions(Context* ctx, const void* posq) {
   const int n = ctx->n;
   const int* slot_of = ctx->in_permuted ? ctx->d_slot_of : nullptr;
+  ulonglong2* f4 = reinterpret_cast<ulonglong2*>(ctx->d_f4);
   if (ctx->in_double)
-    stage_positions_kernel<true><<<(n + 255) / 256, 256, 0, ctx->stream>>>(posq, n, slot_of, ctx->d_wpar, ctx->d_pos);
+    stage_positions_kernel<true><<<(n + 255) / 256, 256, 0, ctx->stream>>>(posq, n, slot_of, ctx->d_wpar, ctx->d_pos, f4);
   else
-    stage_positions_kernel<false><<<(n + 255) / 256, 256, 0, ctx->stream>>>(posq, n, slot_of, ctx->d_wpar, ctx->d_pos);
+    stage_positions_kernel<false><<<(n + 255) / 256, 256, 0, ctx->stream>>>(posq, n, slot_of, ctx->d_wpar, ctx->d_pos, f4);
   ++ctx->launches;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -206,18 +232,6 @@ gbx_status launch_finish_outputs(Context* ctx, unsigned long long* force, int st
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     ctx->last_error = std::string("output launch: ") + cudaGetErrorString(e);
-    return GBX_ERR_CUDA;
-  }
-  return GBX_OK;
-}
-
-gbx_status launch_publish_status(Context* ctx) {
-  publish_status_kernel<<<1, 1, 0, ctx->stream>>>(ctx->d_status, ctx->use_tight ? ctx->d_tgeom : ctx->d_geom,
-                                                  ctx->d_pub, ctx->h_pub_dev);
-  ++ctx->launches;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    ctx->last_error = std::string("status launch: ") + cudaGetErrorString(e);
     return GBX_ERR_CUDA;
   }
   return GBX_OK;
@@ -290,15 +304,24 @@ gbx_status launch_adjoint_out(Context* ctx, double* energy, double* forces, doub
   return GBX_OK;
 }
 
-gbx_status launch_energy_reduce(Context* ctx, double* energy, bool adjoint) {
-  energy_reduce_kernel<<<1, kRedThreads, 0, ctx->stream>>>(ctx->d_energy_part, ctx->energy_parts, ctx->d_energy_fx,
-                                                           energy,
-                                                           adjoint ? ctx->d_dBdJ + 4 * (size_t)ctx->n : nullptr,
-                                                           ctx->n, adjoint ? ctx->d_alpha_grad : nullptr);
+gbx_status launch_finish(Context* ctx, unsigned long long* force, int stride, double* energy, bool chain, bool adjoint) {
+  const int n = ctx->n;
+  // per-block energy partials (compiled expressions) and the alpha gradient need their own reduction first
+  const bool reduce = ctx->energy_parts > 0 || adjoint;
+  if (reduce) {
+    energy_reduce_kernel<<<1, kRedThreads, 0, ctx->stream>>>(ctx->d_energy_part, ctx->energy_parts, ctx->d_energy_fx,
+                                                             energy, adjoint ? ctx->d_dBdJ + 4 * (size_t)n : nullptr,
+                                                             n, adjoint ? ctx->d_alpha_grad : nullptr);
+    ++ctx->launches;
+  }
+  finish_kernel<<<chain ? (n + kFinishThreads - 1) / kFinishThreads : 1, kFinishThreads, 0, ctx->stream>>>(
+      n, chain ? reinterpret_cast<const ulonglong2*>(ctx->d_f4) : nullptr, force, stride,
+      adjoint ? ctx->d_dEdR_fx : nullptr, ctx->d_energy_fx, reduce ? nullptr : energy, ctx->d_status,
+      ctx->use_tight ? ctx->d_tgeom : ctx->d_geom, ctx->d_pub, ctx->h_pub_dev);
   ++ctx->launches;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
-    ctx->last_error = std::string("energy reduce launch: ") + cudaGetErrorString(e);
+    ctx->last_error = std::string("finish launch: ") + cudaGetErrorString(e);
     return GBX_ERR_CUDA;
   }
   return GBX_OK;

@@ -185,18 +185,11 @@ __device__ __forceinline__ PAtom load_patom(const SymArgs& a, int k) {
   return t;
 }
 
-// Hardware 2^x and 1/sqrt(x) (PTX ex2.approx / rsqrt.approx, relative error
-// below 2^-22; subnormal results and inputs flush to zero, which e^-D and
-// 1/f never need).
+// Hardware 2^x (PTX ex2.approx, relative error below 2^-22; subnormal results
+// flush to zero, which e^-D and 1/f never need, nor rsqrt_ftz's inputs).
 __device__ __forceinline__ float ex2_ftz(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-__device__ __forceinline__ float rsqrt_ftz(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 

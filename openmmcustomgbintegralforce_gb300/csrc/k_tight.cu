@@ -196,6 +196,16 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
                                                                         const TableGeom* __restrict__ gp, float w,
                                                                         long long cell_cap, long long entry_cap,
                                                                         unsigned* __restrict__ status) {
+  // sorted entries, as pairs field by field (EntryPair, queries.cuh)
+  auto put = [entry](int at, const float4 e) {
+    float* p = reinterpret_cast<float*>(entry) + 8 * (size_t)(at >> 1) + (at & 1);
+    p[0] = e.x;
+    p[2] = e.y;
+    p[4] = e.z;
+    p[6] = -e.w;
+  };
+  // after an odd list: the pair reads of the integral pass meet a sphere no point is near
+  const float4 kPadEntry = make_float4(0.f, 0.f, 0.f, -1e6f);
   __shared__ float4 s_e[kSortWarps][kSortBuf];
   __shared__ int s_i[kSortWarps][kSortBuf];
   __shared__ float s_k[kSortWarps][kSortBuf];
@@ -259,10 +269,11 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
           const float ko = gk[o];
           r += (ko < kq) || (ko == kq && gi[o] < iq);
         }
-        entry[cs + r] = ge[q];
+        put(cs + r, ge[q]);
         index[cs + r] = iq;
         if (r == 0) first[c0 + src].first = ge[q];
       }
+      if ((ccnt & 1) && gl == 0) put(cs + ccnt, kPadEntry);
       __syncwarp();
     }
     while (todo) {
@@ -295,10 +306,11 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
           const float ko = s_k[wib][o];
           r += (ko < kq) || (ko == kq && s_i[wib][o] < iq);
         }
-        entry[cs + r] = s_e[wib][q];
+        put(cs + r, s_e[wib][q]);
         index[cs + r] = iq;
         if (r == 0) first[cc].first = s_e[wib][q];
       }
+      if ((ccnt & 1) && lane == 0) put(cs + ccnt, kPadEntry);
       __syncwarp();
     }
   }

@@ -61,11 +61,11 @@ struct Work<true> {
 // GBSW, CharmmReferenceGBSW.cpp:616-639 / GBSWIntegral.cpp:187-224: V is the
 // product of u_j over the switching shells, 0 once an atom buries the point.
 template <class Q, class W>
-__device__ __forceinline__ float gbsw_volume(const Q& qy, const ModelConst& m, const float4* __restrict__ list,
+__device__ __forceinline__ float gbsw_volume(const Q& qy, const ModelConst& m, const Entries& t, int start,
                                              int cnt, const float4 xi, const float4 v, W& wk) {
   float V = 1.0f;
   for (int l = 0; l < cnt; ++l) {
-    const float4 a = __ldg(list + l);
+    const float4 a = entry_at<Q>(t, start + l);
     const float3 d = qy.delta(a, xi, v);
     const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
     const float lo = a.w - m.sw, hi = a.w + m.sw;
@@ -142,7 +142,7 @@ __device__ __forceinline__ void count_chain_work(const Q& qy, const ModelConst& 
     wk.fs += cs.x;
   } else {
     for (int l = 0; l < cs.x; ++l) {
-      const float4 a = __ldg(t.e + cs.y + l);
+      const float4 a = entry_at<Q>(t, cs.y + l);
       const float3 d = qy.delta(a, xi, v);
       const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
       const float lo = a.w - m.sw, hi = a.w + m.sw;
@@ -161,7 +161,7 @@ __device__ __forceinline__ float solvent_fraction(const Q& qy, const ModelConst&
     if (cnt < 0) return 0.0f;  // buried cell (exact table)
     s = cs.y;
   }
-  if (MODEL == GBX_MODEL_GBSW) return cnt > 0 ? gbsw_volume(qy, m, t.e + s, cnt, xi, v, wk) : 1.0f;
+  if (MODEL == GBX_MODEL_GBSW) return cnt > 0 ? gbsw_volume(qy, m, t, s, cnt, xi, v, wk) : 1.0f;
   float p;
   if (MODEL == GBX_MODEL_GBMV1) return logistic_solvent(m.beta, m.lambda, gbmv1_sum(qy, t.e + s, cnt, xi, v, wk), p);
   if (cnt == 0) return 1.0f;  // empty list: V = 0 (GBMVIntegralTypeII.cpp:140)
@@ -379,48 +379,97 @@ __device__ __forceinline__ float shell_g(const ModelConst& m, float V, float dr)
   return __fdividef(V, u) * du;
 }
 
-// x << n with PTX semantics: a shift of 32 or more gives 0 (two 32-bit
-// halves of the 64-bit mask, each set without a branch on l).
-__device__ __forceinline__ unsigned shl_clamped(unsigned x, unsigned n) {
-  unsigned r;
-  asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(n));
-  return r;
+// The query's delta of two entries along one axis.
+template <class Q>
+__device__ __forceinline__ float2 delta2(const Q& query, int k, float2 a, float xi, float v) {
+  if constexpr (IsTight<Q>::value) {
+    return query.delta2(k, a, xi, v);
+  } else {
+    const float4 X = make_float4(xi, xi, xi, 0.f), W = make_float4(v, v, v, 0.f);
+    const float3 d0 = query.delta(make_float4(a.x, a.x, a.x, 0.f), X, W),
+                 d1 = query.delta(make_float4(a.y, a.y, a.y, 0.f), X, W);
+    return k == 0 ? make_float2(d0.x, d1.x) : k == 1 ? make_float2(d0.y, d1.y) : make_float2(d0.z, d1.z);
+  }
 }
 
-// True if list entry l is atom i itself: its inline position is bitwise
-// atom i's, and only then is the index read.
-__device__ __forceinline__ bool is_self(const float4 a, const float4 xi, const int* __restrict__ index, int l, int i) {
-  return a.x == xi.x && a.y == xi.y && a.z == xi.z && __ldg(index + l) == i;
+// Signed distance of a point from an atom's sphere, |d| - R'.  A point at an
+// atom's own place gives -R' (the tiny term keeps 0 * rsqrt(0) out; it is far
+// below the rounding of any other squared distance).
+__device__ __forceinline__ float sphere_gap(const float3 d, float Rp) {
+  const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, fmaf(d.z, d.z, 1e-30f)));
+  return fmaf(r2, rsqrt_ftz(r2), -Rp);
 }
 
-// GBSW integrals with lanes refilled from a ring queue.  A warp classifies
-// kRefill points at a time (empty cell: V = 1; buried cell or buried by the
-// list's first entry: V = 0) and queues the points that have a list whenever
-// fewer than kRefillBelow are pending;
-// every lane evaluates list entries of its own point and takes the next
-// queued point as soon as its own is finished, so a long list keeps one lane
-// busy instead of the whole warp waiting on it, and lanes idle only at the
-// end of the warp's quadrature range.  The walk per point is the sequential one of gbsw_volume
-// (same order, same early exit).  J is summed in an order fixed by the input
-// alone, so runs are bit-reproducible.
-constexpr int kStage = 256;        // ring entries per warp (a power of two)
+// The quadrature points of one (atom, chunk) item.  Radial points well inside
+// atom i's own burying sphere (r below R'_i - w by more than FP32 rounding of
+// |v|^2 can reach) have V = 0: the exact table lists atom i in every cell they
+// fall in, so the walk would end on it at the latest.  V = 0 adds nothing to J
+// and records nothing, so the leading `inner` points of every direction are
+// left out; the rest, numbered t over all directions, are split into chunks.
+struct Points {
+  int t0, t1, inner;
+  unsigned magic;  // 2^24 / (points kept per direction), rounded up
+  template <class Q>
+  __device__ __forceinline__ void init(const Quad& quad, const ModelConst& m, const float4 xi, int c, int n_chunks,
+                                       int lane) {
+    inner = 0;
+    if constexpr (IsTight<Q>::value) {
+      const float lo = xi.w - m.sw;
+      for (int r0 = 0; r0 < m.nrad; r0 += kWarp) {
+        const int ir = r0 + lane;
+        const bool in = ir < m.nrad && quad.qv[ir].w * (1.0f + 1.0f / 1024.0f) < lo;
+        const unsigned out = __ballot_sync(0xffffffffu, !in);
+        inner = r0 + (out ? __ffs(out) - 1 : kWarp);
+        if (out) break;
+      }
+      inner = min(inner, m.nrad);
+    }
+    const int kept = m.nrad - inner;
+    const int total = m.nq / m.nrad * kept, chunk = (total + n_chunks - 1) / n_chunks;
+    magic = kept > 0 ? ((1u << 24) + kept - 1) / kept : 0u;
+    t0 = min(total, c * chunk);
+    t1 = min(total, t0 + chunk);
+  }
+  // the index of point t: exact for the at most 28,160 points of a rule (256 x 110)
+  __device__ __forceinline__ int q(int t) const { return t + inner * ((int)__umulhi((unsigned)t << 8, magic) + 1); }
+};
+
+// Whether the point lies in atom i's own switching shell.  Without images its
+// distance from atom i is |v| (the radial point, to FP32 rounding).
+template <class Q>
+__device__ __forceinline__ bool in_own_shell(const Q& query, const ModelConst& m, const float4 xi, const float4 v) {
+  if (!Q::kImages && fabsf(v.w - xi.w) >= m.sw + 1e-5f) return false;
+  return fabsf(sphere_gap(query.delta(xi, xi, v), xi.w)) < m.sw;
+}
+
+// GBSW integrals.  A warp classifies kRefill points at a time (empty cell:
+// V = 1; buried cell or buried by the list's first entry: V = 0) and queues
+// the points that have a list.  Whenever 32 points are pending, the warp walks
+// their lists in step, one lane per point, two entries per step: the list
+// position is then the same for every lane, so a step is straight-line code
+// (no refill, dequeue or record bookkeeping inside the walk: that is paid
+// once per 32 points).  Lanes idle from the end of their list to the end of
+// the longest, so short and long lists are queued apart.  The walk per point
+// is the sequential one of gbsw_volume (same order).  J is summed in an order
+// fixed by the input alone, so runs are bit-reproducible.
 constexpr int kRefill = 128;       // points classified per refill
-constexpr int kRefillBelow = 64;   // refill when fewer entries are pending
-static_assert(kRefillBelow - 1 + kRefill <= kStage, "ring overwrite");
-constexpr int kEnt = 2;            // list entries per lane step, loaded one step ahead (3 and 4 measured slower)
-static_assert(kEnt == 2, "the exact table's lists are read in aligned pairs");
+constexpr int kQueue = kRefill + kWarp;  // fewer than 32 pending when a refill starts
+constexpr int kShortList = 8;      // longest list of the short queue
+// What the integral pass records: nothing; the points an atom other than i
+// shapes, with those atoms; every shaped point with all its shaping atoms (the
+// adjoint, whose dE/dR_i has atom i's own entry).
+enum { kEmitNone = 0, kEmitOthers = 1, kEmitAll = 2 };
 
 // Persistent: a grid of resident blocks whose warps take (atom, chunk) items
 // from `next_item` one at a time, so a warp that finishes a cheap item (a
 // buried or exposed atom) takes the next instead of idling until the slowest
 // warp of its block is done.  Each item's results depend on the item alone.
-template <class Q, bool EMIT>
-__global__ void __launch_bounds__(kThreads) gbsw_integral_kernel(const float4* __restrict__ pos, int n, Entries tab,
-                                                                 Quad quad, ModelConst m, int chunk, int n_chunks,
+template <class Q, int EMIT>
+__global__ void __launch_bounds__(kThreads, 12) gbsw_integral_kernel(const float4* __restrict__ pos, int n, Entries tab,
+                                                                 Quad quad, ModelConst m, int n_chunks,
                                                                  float* __restrict__ Jpart, ShellSink sink,
                                                                  unsigned* __restrict__ next_item) {
-  __shared__ int3 s_queue[kThreads / kWarp][kStage];  // (q, list start, list length)
-  __shared__ int s_long[kThreads / kWarp];  // a shaping entry beyond list position 63
+  __shared__ int2 s_queue[kThreads / kWarp][2][kQueue];  // (q | length << 16, list start): short and long lists
   // the exact table: lists start at even entries and each cell's record sits
   // beside its first entry, so both are read 32 bytes at a time
   constexpr bool kTight = IsTight<Q>::value;
@@ -428,202 +477,197 @@ __global__ void __launch_bounds__(kThreads) gbsw_integral_kernel(const float4* _
   const int wib = threadIdx.x / kWarp;
   const unsigned lt = (1u << lane) - 1u;
   for (;;) {
-  unsigned item = 0;
-  if (lane == 0) item = atomicAdd(next_item, 1u);
-  const int warp = (int)__shfl_sync(0xffffffffu, item, 0);
-  if (warp >= n * n_chunks) return;
-  if (lane == 0) s_long[wib] = 0;
-  __syncwarp();
-  int3* queue = s_queue[wib];
-  int fill = 0;  // warp-uniform: points recorded so far (may exceed R)
-  const int i = warp % n, c = warp / n;
-  int4* region = EMIT ? sink.rec + (size_t)warp * sink.R : nullptr;
-  const float4 xi = pos[i];
-  Q query;
-  query.init(tab, xi, quad.qoff);
-  const int q0 = c * chunk, q1 = min(m.nq, q0 + chunk);
-  float J4 = 0.0f, J7 = 0.0f;
-  int head = 0, tail = 0;  // warp-uniform ring positions: taken, queued
-  int next = q0;           // warp-uniform: first point not yet classified
-  if constexpr (kTight) {
-    // Radial shells well inside atom i's own burying sphere (r below
-    // R'_i - w by more than FP32 rounding of |v|^2 can reach) hold only
-    // points with V = 0: the exact table lists atom i in every cell they
-    // fall in, so the walk would end on it at the latest.  V = 0 adds
-    // nothing to J and records nothing, so they are skipped unclassified.
-    const float lo = xi.w - m.sw;
-    const int nrad = m.nq / m.nshell;
-    int inner = 0;  // the leading shells that lie inside
-    for (int r0 = 0; r0 < nrad; r0 += kWarp) {
-      const int ir = r0 + lane;
-      const bool in = ir < nrad && quad.qv[ir * m.nshell].w * (1.0f + 1.0f / 1024.0f) < lo;
-      const unsigned out = __ballot_sync(0xffffffffu, !in);
-      inner = r0 + (out ? __ffs(out) - 1 : kWarp);
-      if (out) break;
-    }
-    next = max(q0, inner * m.nshell);
-  }
-  int q = 0, s = 0, cnt = 0, l = 0;
-  float4 an[kEnt];  // the next kEnt list entries
+    unsigned item = 0;
+    if (lane == 0) item = atomicAdd(next_item, 1u);
+    const int warp = (int)__shfl_sync(0xffffffffu, item, 0);
+    if (warp >= n * n_chunks) return;
+    int fill = 0;           // warp-uniform: points recorded so far (may exceed R)
+    bool too_long = false;  // a shaping entry beyond list position 63
+    const int i = warp % n, c = warp / n;
+    const float4 xi = pos[i];
+    Q query;
+    query.init(tab, xi, quad.qoff);
+    Points pts{};
+    pts.init<Q>(quad, m, xi, c, n_chunks, lane);
+    float J4 = 0.0f, J7 = 0.0f;
+    int pending[2] = {0, 0}, head[2] = {0, 0};  // warp-uniform, per queue
+    int next = pts.t0;                          // warp-uniform: first point not yet classified
+    for (;;) {
+      // a full batch of either queue, else more points, else what is left of both
+      int take[2] = {0, 0};
+      if (pending[0] >= kWarp) {
+        take[0] = kWarp;
+      } else if (pending[1] >= kWarp) {
+        take[1] = kWarp;
+      } else if (next < pts.t1) {
 #pragma unroll
-  for (int u = 0; u < kEnt; ++u) an[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-  bool has = false;
-  unsigned sm_lo = 0u, sm_hi = 0u;  // bit l of (hi:lo): in-shell entry l is not atom i
-  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-  float2 w = make_float2(0.f, 0.f);
-  float V = 1.0f;
-  while (true) {
-    if (tail - head < kRefillBelow && next < q1) {
-      // classify the next kRefill points into the ring (at most
-      // kRefillBelow - 1 + kRefill entries are ever pending: no overwrite)
+        for (int h = 0; h < 2; ++h) {  // what is pending moves to the front
+          int2 e = make_int2(0, 0);
+          if (lane < pending[h]) e = s_queue[wib][h][head[h] + lane];
+          __syncwarp();
+          if (lane < pending[h]) s_queue[wib][h][lane] = e;
+          head[h] = 0;
+        }
 #pragma unroll 4
-      for (int k = 0; k < kRefill / kWarp; ++k) {
-        const int qc = next + k * kWarp + lane;
-        int2 cs = make_int2(-1, 0);
-        if (qc < q1) {
-          const float4 vc = quad.qv[qc];
-          const long long cell = query.cell(xi, vc, qc);
-          float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f);
-          if constexpr (kTight) {
-            // the exact table keeps each cell's first entry beside its
-            // record: one load, not one after the other
-            cs = make_int2(0, 0);
-            if (cell >= 0) {
-              const Float4x2 r = ldg_pair(tab.first + cell);
-              a0 = r.a;
-              cs = make_int2(__float_as_int(r.b.x), __float_as_int(r.b.y));
+        for (int k = 0; k < kRefill / kWarp; ++k) {
+          const int t = next + k * kWarp + lane;
+          const int qc = pts.q(t);
+          int2 cs = make_int2(-1, 0);
+          if (t < pts.t1) {
+            const float4 vc = quad.qv[qc];
+            const long long cell = query.cell(xi, vc, qc);
+            float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if constexpr (kTight) {
+              // the exact table keeps each cell's first entry beside its
+              // record: one load, not one after the other
+              cs = make_int2(0, 0);
+              if (cell >= 0) {
+                const Float4x2 r = ldg_pair(tab.first + cell);
+                a0 = r.a;
+                cs = make_int2(__float_as_int(r.b.x), __float_as_int(r.b.y));
+              }
+            } else {
+              cs = cell >= 0 ? __ldg(tab.cell + cell) : make_int2(0, 0);
             }
-          } else {
-            cs = cell >= 0 ? __ldg(tab.cell + cell) : make_int2(0, 0);
+            if (cs.x == 0) {
+              const float2 wc = quad.qw[qc];
+              J4 += wc.x;
+              J7 += wc.y;
+            } else if (cs.x > 0) {
+              // the list's first entry, the likeliest burying atom, buries most
+              // listed points: V = 0 adds nothing, the point is not queued
+              if constexpr (!kTight) a0 = __ldg(tab.e + cs.y);
+              if (sphere_gap(query.delta(a0, xi, vc), a0.w) <= -m.sw) cs.x = -1;
+            }
           }
-          if (cs.x == 0) {
-            const float2 wc = quad.qw[qc];
-            J4 += wc.x;
-            J7 += wc.y;
-          } else if (cs.x > 0) {
-            // the list's first entry, the likeliest burying atom, buries most
-            // listed points: V = 0 adds nothing, the point is not queued
-            if constexpr (!kTight) a0 = __ldg(tab.e + cs.y);
-            const float3 d = query.delta(a0, xi, vc);
-            const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-            const float lo = a0.w - m.sw;
-            if (r2 <= lo * lo) cs.x = -1;
+          const unsigned listed = __ballot_sync(0xffffffffu, cs.x > 0);
+          const unsigned longer = __ballot_sync(0xffffffffu, cs.x > kShortList);
+          const unsigned shorter = listed & ~longer;
+          if (cs.x > 0) {
+            const bool h = cs.x > kShortList;
+            s_queue[wib][h][h ? pending[1] + __popc(longer & lt) : pending[0] + __popc(shorter & lt)] =
+                make_int2(qc | cs.x << 16, cs.y);
           }
+          pending[0] += __popc(shorter);
+          pending[1] += __popc(longer);
         }
-        const unsigned qm = __ballot_sync(0xffffffffu, cs.x > 0);
-        if (cs.x > 0) queue[(tail + __popc(qm & lt)) & (kStage - 1)] = make_int3(qc, cs.y, cs.x);
-        tail += __popc(qm);
-      }
-      next += kRefill;
-      __syncwarp();
-    }
-    const unsigned need = __ballot_sync(0xffffffffu, !has);
-    if (!has) {
-      const int idx = head + __popc(need & lt);
-      if (idx < tail) {
-        const int3 e = queue[idx & (kStage - 1)];
-        q = e.x;
-        s = e.y;
-        cnt = e.z;
-        l = 0;
-        sm_lo = 0u;
-        sm_hi = 0u;
-        V = 1.0f;
-        has = true;
-        v = quad.qv[q];
-        w = quad.qw[q];
-        if constexpr (kTight) {
-          const Float4x2 p = ldg_pair(tab.e + s);
-          an[0] = p.a;
-          an[1] = p.b;
-        } else {
-#pragma unroll
-          for (int u = 0; u < kEnt; ++u)
-            if (u < cnt) an[u] = __ldg(tab.e + s + u);
-        }
-      }
-    }
-    head = min(head + __popc(need), tail);
-    if (__ballot_sync(0xffffffffu, has) == 0u) {
-      if (next >= q1) break;
-      continue;
-    }
-    bool fin = false;
-    if (has) {
-      // kEnt list entries per step (entries l .. l + kEnt - 1 were loaded one step ahead)
-      float4 cur[kEnt];
-#pragma unroll
-      for (int u = 0; u < kEnt; ++u) cur[u] = an[u];
-      if constexpr (kTight) {
-        // l is even here (a point advances kEnt entries per step until it
-        // ends); a pair past an odd list's end reads its padding entry
-        if (l + kEnt < cnt) {
-          const Float4x2 p = ldg_pair(tab.e + s + l + kEnt);
-          an[0] = p.a;
-          an[1] = p.b;
-        }
+        next += kRefill;
+        __syncwarp();
+        continue;
       } else {
-#pragma unroll
-        for (int u = 0; u < kEnt; ++u)
-          if (l + kEnt + u < cnt) an[u] = __ldg(tab.e + s + l + kEnt + u);
+        take[0] = pending[0];
+        take[1] = min(pending[1], kWarp - take[0]);
+        if (take[0] + take[1] == 0) break;
+      }
+      // one point per lane
+      int q = 0, s = 0, cnt = 0;
+      if (lane < take[0] + take[1]) {
+        const bool h = lane >= take[0];
+        const int2 e = s_queue[wib][h][h ? head[1] + lane - take[0] : head[0] + lane];
+        q = e.x & 0xffff;
+        cnt = (unsigned)e.x >> 16;
+        s = e.y;
       }
 #pragma unroll
-      for (int u = 0; u < kEnt; ++u) {
-        if (fin) break;
-        const float4 a = cur[u];
-        const float3 d = query.delta(a, xi, v);
-        const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-        const float lo = a.w - m.sw, hi = a.w + m.sw;
-        if (r2 <= lo * lo) {
-          V = 0.0f;
-          fin = true;
+      for (int h = 0; h < 2; ++h) {
+        head[h] += take[h];
+        pending[h] -= take[h];
+      }
+      const bool mine = cnt > 0;
+      const float4 v = quad.qv[q];
+      float V = mine ? 1.0f : 0.0f;
+      unsigned sm_lo = 0u, sm_hi = 0u;  // bit l of (hi:lo): entry l shapes the point
+      bool far = false;                 // a shaping entry beyond position 63
+      EntryPair pair{};
+      auto load = [&](int l) -> EntryPair {
+        EntryPair p = pair;
+        if constexpr (kTight) {  // an odd list's last pair ends in a padding entry no point is near
+          if (l < cnt) p = ldg_entries(tab.e, s + l);
         } else {
-          if (r2 < hi * hi) {
-            const float dr = r2 * rsqrtf(r2) - a.w;
-            V *= fmaf(dr, fmaf(-m.c3 * dr, dr, m.c1), 0.5f);
-            if (EMIT && !is_self(a, xi, tab.index + s, l, i)) {
-              sm_lo |= shl_clamped(1u, (unsigned)l);
-              sm_hi |= shl_clamped(1u, (unsigned)(l - 32));
-              if (l >= 64) s_long[wib] = 1;
+          const float4 none = make_float4(0.f, 0.f, 0.f, -1e6f);  // a sphere no point is near
+          const float4 a = l < cnt ? __ldg(tab.e + s + l) : none, b = l + 1 < cnt ? __ldg(tab.e + s + l + 1) : none;
+          p = EntryPair{make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), make_float2(-a.w, -b.w)};
+        }
+        return p;
+      };
+      // entries l and l + 1 of every lane that has them, in packed FP32x2
+      // arithmetic (each half rounded as sphere_gap rounds it); bits of the shaping ones
+      auto step = [&](const EntryPair& p, int l) -> unsigned {
+        const bool on = l < cnt;
+        const float2 dx = delta2(query, 0, p.x, xi.x, v.x), dy = delta2(query, 1, p.y, xi.y, v.y),
+                     dz = delta2(query, 2, p.z, xi.z, v.z);
+        const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, make_float2(1e-30f, 1e-30f))));
+        const float2 g = __ffma2_rn(r2, make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y)), p.nw);
+        const float2 u = __ffma2_rn(
+            g, __ffma2_rn(__fmul2_rn(make_float2(-m.c3, -m.c3), g), g, make_float2(m.c1, m.c1)), make_float2(0.5f, 0.5f));
+        const bool ina = on && fabsf(g.x) < m.sw, inb = on && fabsf(g.y) < m.sw;
+        if (ina) V *= u.x;
+        if (inb) V *= u.y;
+        if (on && fminf(g.x, g.y) <= -m.sw) V = 0.0f;  // buried
+        return (ina ? 1u : 0u) | (inb ? 2u : 0u);
+      };
+      // the first kShortList entries without a test between them, the next pair loaded ahead
+      pair = load(0);
+#pragma unroll
+      for (int l = 0; l < kShortList; l += 2) {
+        const EntryPair next_pair = load(l + 2);
+        sm_lo |= step(pair, l) << l;
+        pair = next_pair;
+      }
+      for (int l = kShortList; __any_sync(0xffffffffu, l < cnt && V != 0.0f); l += 2) {
+        const EntryPair next_pair = load(l + 2);
+        const unsigned in = step(pair, l);
+        if (l < 32) sm_lo |= in << l;
+        else if (l < 64) sm_hi |= in << (l - 32);
+        else far = in != 0u || far;
+        pair = next_pair;
+      }
+      if (mine) {
+        const float2 w = quad.qw[q];
+        J4 = fmaf(w.x, V, J4);
+        J7 = fmaf(w.y, V, J7);
+      }
+      if (EMIT != kEmitNone) {
+        if (EMIT == kEmitOthers && (sm_lo | sm_hi) != 0u && V != 0.0f && in_own_shell(query, m, xi, v)) {
+          // the point lies in atom i's own shell (one radial shell or two of
+          // all): its entry, found by its place and index, is not recorded
+          for (unsigned lo = sm_lo, hi = sm_hi; (lo | hi) != 0u;) {
+            const int l = lo ? __ffs((int)lo) - 1 : 31 + __ffs((int)hi);
+            if (__ldg(tab.index + s + l) == i) {
+              if (l < 32) sm_lo &= ~(1u << l);
+              else sm_hi &= ~(1u << (l - 32));
             }
+            if (lo) lo &= lo - 1;
+            else hi &= hi - 1;
           }
-          fin = ++l == cnt;
         }
+        // slots in finishing order (the chain rule's sums do not depend on it)
+        const bool emit = (sm_lo | sm_hi) != 0u && V != 0.0f;
+        const unsigned em = __ballot_sync(0xffffffffu, emit);
+        if (emit) {
+          const int slot = fill + __popc(em & lt);
+          if (slot < sink.R) {
+            __stcs(sink.rec + (size_t)warp * sink.R + slot, make_int4(q, __float_as_int(V), (int)sm_lo, (int)sm_hi));
+            __stcs(sink.st + (size_t)warp * sink.R + slot, s);
+          }
+        }
+        fill += __popc(em);
+        too_long = __any_sync(0xffffffffu, far && V != 0.0f) || too_long;
       }
     }
-    if (fin) {
-      J4 = fmaf(w.x, V, J4);
-      J7 = fmaf(w.y, V, J7);
-      has = false;
+    for (int off = 16; off > 0; off >>= 1) {
+      J4 += __shfl_xor_sync(0xffffffffu, J4, off);
+      J7 += __shfl_xor_sync(0xffffffffu, J7, off);
     }
-    if (EMIT) {
-      // slots in finishing order (the chain rule's sums do not depend on it)
-      const bool emit = fin && (sm_lo | sm_hi) != 0u && V != 0.0f;
-      const unsigned em = __ballot_sync(0xffffffffu, emit);
-      if (emit) {
-        const int slot = fill + __popc(em & lt);
-        if (slot < sink.R) {
-          __stcs(region + slot, make_int4(q, __float_as_int(V), (int)sm_lo, (int)sm_hi));
-          __stcs(sink.st + (size_t)warp * sink.R + slot, s);
-        }
+    if (lane == 0) {
+      Jpart[(size_t)c * n + i] = J4;
+      Jpart[((size_t)n_chunks + c) * n + i] = J7;
+      if (EMIT != kEmitNone) {
+        sink.count[warp] = fill <= sink.R && !too_long ? fill : -1 - fill;
+        if (fill > 0) atomicMax(sink.max_seen, (unsigned)fill);
       }
-      fill += __popc(em);
     }
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    J4 += __shfl_xor_sync(0xffffffffu, J4, off);
-    J7 += __shfl_xor_sync(0xffffffffu, J7, off);
-  }
-  __syncwarp();
-  if (lane == 0) {
-    Jpart[(size_t)c * n + i] = J4;
-    Jpart[((size_t)n_chunks + c) * n + i] = J7;
-    if (EMIT) {
-      sink.count[warp] = fill <= sink.R && !s_long[wib] ? fill : -1 - fill;
-      if (fill > 0) atomicMax(sink.max_seen, (unsigned)fill);
-    }
-  }
-  __syncwarp();  // the ring and the long-list flag are reused by the next item
+    __syncwarp();  // the queues are reused by the next item
   }
 }
 
@@ -637,70 +681,152 @@ __global__ void __launch_bounds__(kThreads) gbsw_integral_kernel(const float4* _
 // (atom i's own radius included).
 // ---------------------------------------------------------------------------
 struct ChainOut {
-  unsigned long long* force;
-  int stride;
-  unsigned long long* dEdR;
+  // the chain rule's own sums, one 32-byte sector per atom: force x, y, z and
+  // dE/dR (fixed point); zeroed by the position staging, added to the
+  // caller's buffers by the call's last kernel
+  unsigned long long* f4;
   bool quirk;  // drop F_k beyond the cutoff (CharmmReferenceGBSW.cpp:291-292)
   float cutoff2;
 };
 
-// Records of the emitting integral pass (rec == nullptr: none this call).
+// Records of the emitting integral pass (count == nullptr: none this call).
 struct ChainRecords {
   const int4* rec;  // (q, V, mask low, mask high) per recorded point
   const int* st;    // the point's list start
   const int* count;
   int R;
-  const float* state;  // GBMV point state of the integral pass (nullptr: re-sum the lists)
 };
 
 // A component whose fixed-point value is 0 (|g| < 2^-33, common for distant
 // GBMV atoms) changes nothing: its reduction is skipped, the result is the
 // same bits.
+__device__ __forceinline__ void push3(const ChainOut& o, int k, long long fx, long long fy, long long fz) {
+  unsigned long long* f = o.f4 + 4 * (size_t)k;
+  if (fx) atomicAdd(f, (unsigned long long)fx);
+  if (fy) atomicAdd(f + 1, (unsigned long long)fy);
+  if (fz) atomicAdd(f + 2, (unsigned long long)fz);
+}
 __device__ __forceinline__ void push_force(const ChainOut& o, int k, float gx, float gy, float gz) {
-  const long long fx = float_to_fixed_split(-gx), fy = float_to_fixed_split(-gy), fz = float_to_fixed_split(-gz);
-  if (fx) atomicAdd(&o.force[k], (unsigned long long)fx);
-  if (fy) atomicAdd(&o.force[k + o.stride], (unsigned long long)fy);
-  if (fz) atomicAdd(&o.force[k + 2 * o.stride], (unsigned long long)fz);
+  push3(o, k, float_to_fixed_split(-gx), float_to_fixed_split(-gy), float_to_fixed_split(-gz));
+}
+__device__ __forceinline__ void push_radius(const ChainOut& o, int k, float v) {
+  red_add_fixed(o.f4 + 4 * (size_t)k + 3, v);
 }
 
-// GBSW: the force -g on a shaping atom k (unless the cutoff quirk drops it)
-// and +g on atom i, as one fixed-point integer triple: atom i gets the
-// negation of what k gets, so the pair's momentum balances exactly and one
-// conversion serves both.  The caller loads k together with the entry, so
-// the two reads overlap instead of the index waiting on the arithmetic.
-__device__ __forceinline__ void push_shaping(const ChainOut& o, int k, bool push, float gx, float gy, float gz,
-                                             long long& fix, long long& fiy, long long& fiz) {
-  const long long fx = float_to_fixed_split(-gx), fy = float_to_fixed_split(-gy), fz = float_to_fixed_split(-gz);
-  if (push) {
-    if (fx) atomicAdd(&o.force[k], (unsigned long long)fx);
-    if (fy) atomicAdd(&o.force[k + o.stride], (unsigned long long)fy);
-    if (fz) atomicAdd(&o.force[k + 2 * o.stride], (unsigned long long)fz);
+// A shaping atom's share of one GBSW point: c dV/dR_k and the force on k as
+// fixed-point integers.  Atom i gets the negated integers, so the pair's
+// momentum balances exactly and one conversion serves both.  The record and
+// the list-walk paths share it: the same bits.
+template <class Q>
+struct Shaping {
+  float g;  // (V/u) u'
+  long long fx, fy, fz;
+  bool push;  // false: the cutoff quirk drops the force on k
+  __device__ __forceinline__ Shaping(const Q& query, const ModelConst& m, const ChainOut& out, const float4 a,
+                                     const float4 xi, const float4 v, float V, float cq) {
+    const float3 d = query.delta(a, xi, v);
+    const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, fmaf(d.z, d.z, 1e-30f)));
+    const float ir = rsqrt_ftz(r2);
+    g = shell_g(m, V, fmaf(r2, ir, -a.w));
+    const float gs = cq * g * ir;
+    fx = float_to_fixed_split(-(gs * d.x));
+    fy = float_to_fixed_split(-(gs * d.y));
+    fz = float_to_fixed_split(-(gs * d.z));
+    push = true;
+    if (out.quirk) {
+      const float3 e = query.delta(a, xi, make_float4(0.f, 0.f, 0.f, 0.f));  // x_k - x_i
+      push = fmaf(e.x, e.x, fmaf(e.y, e.y, e.z * e.z)) <= out.cutoff2;
+    }
   }
-  fix -= fx;
-  fiy -= fy;
-  fiz -= fz;
-}
+};
 
-template <int MODEL, class Q, bool ADJ>
-__global__ void __launch_bounds__(kThreads) chain_kernel(const float4* __restrict__ pos, int n, Entries tab,
-                                                         Quad quad, ModelConst m, int chunk, int n_chunks,
-                                                         const float2* __restrict__ dEdJ, ChainOut out,
-                                                         ChainRecords rr) {
-  constexpr int kWalkKeep = 4;  // GBSW: in-shell entries remembered from the volume pass
+// GBSW chain rule over the recorded points: warp = (atom i, quadrature
+// chunk).  Each lane takes one record of a batch of 32 and the warp unrolls
+// the shaping-entry masks into a ring of (record, list position) items, from
+// which 32 items at a time are evaluated, one per lane, whatever the records'
+// entry counts; items left over when a batch ends join the next batch's.
+//
+// The pushes bound this pass: a warp's 32 shaping atoms are scattered, and an
+// L2 reduction costs the same for one 8-byte lane as for a whole 32-byte
+// sector.  The warp therefore turns its 32 x (x, y, z) integers through shared
+// memory so that an atom's components leave as neighbouring lanes of one
+// instruction into the atom's own sector of f4 (with dE/dR the fourth: the
+// adjoint's pushes cost no more sectors).  89.6 M random pushes of a triple,
+// alone: 2.13 ms as three scattered reductions, 0.65 ms turned.
+//
+// The entry's position is read as pos[index]: atom i's neighbourhood of
+// positions stays in L1, where the 16-byte list entries themselves do not.
+template <class Q, bool ADJ>
+__global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* __restrict__ pos, int n, Entries tab,
+                                                                 Quad quad, ModelConst m, int n_chunks,
+                                                                 const float2* __restrict__ dEdJ, ChainOut out,
+                                                                 ChainRecords rr) {
+  constexpr int kComp = ADJ ? 4 : 3;  // integers pushed per item
+  constexpr int kWarps = kThreads / kWarp;
+  constexpr int kRing = 2 * kWarp;    // fewer than 32 items pending, plus one round of at most 32
+  __shared__ float4 s_v[kWarps][kRing];   // (v, V) of two batches' records
+  __shared__ float2 s_c[kWarps][kRing];   // (c, list start)
+  __shared__ unsigned s_item[kWarps][kRing];  // record slot << 16 | list position
+  __shared__ long long s_f[kWarps][kWarp * kComp];
+  __shared__ int s_k[kWarps][kWarp];
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
-  const int lane = threadIdx.x % kWarp;
+  const int lane = threadIdx.x % kWarp, wib = threadIdx.x / kWarp;
   if (warp >= n * n_chunks) return;
   const int i = warp % n, c = warp / n;
   const float4 xi = pos[i];
   const float2 de = dEdJ[i];
+  const unsigned lt = (1u << lane) - 1u;
   // F_i as fixed-point integers: every contribution is rounded on its own, so
   // the record and the list-walk paths give the same bits
   long long fix = 0, fiy = 0, fiz = 0;
   Q query;
   query.init(tab, xi, quad.qoff);
+  float4* sv = s_v[wib];
+  float2* sc = s_c[wib];
+  unsigned* items = s_item[wib];
+  long long* sf = s_f[wib];
+  int* sk = s_k[wib];
+  unsigned head = 0, tail = 0;  // warp-uniform ring positions
+  // the pending items (at most 32), one per lane
+  auto evaluate = [&]() {
+    __syncwarp();
+    const bool valid = head + lane < tail;
+    int k = -1;
+    long long f[4] = {0, 0, 0, 0};
+    if (valid) {
+      const unsigned it = items[(head + lane) & (kRing - 1)];
+      const float4 rv = sv[it >> 16];
+      const float2 rc = sc[it >> 16];
+      k = __ldg(tab.index + __float_as_int(rc.y) + (int)(it & 0xffffu));
+      const float4 a = __ldg(pos + k);
+      const Shaping<Q> sh(query, m, out, a, xi, rv, rv.w, rc.x);
+      if (ADJ) f[3] = float_to_fixed(rc.x * sh.g * (-0.9520f));  // dV/dR_k = -(V/u) u' dR'/dR
+      if (k != i) {  // atom i moves with the point
+        if (sh.push) {
+          f[0] = sh.fx;
+          f[1] = sh.fy;
+          f[2] = sh.fz;
+        }
+        fix -= sh.fx;
+        fiy -= sh.fy;
+        fiz -= sh.fz;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kComp; ++u) sf[kComp * lane + u] = f[u];
+    sk[lane] = k;
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kComp; ++u) {
+      const int t = u * kWarp + lane;
+      const int e = t / kComp;
+      const long long val = sf[t];
+      if (val) atomicAdd(out.f4 + 4 * (size_t)sk[e] + (t - kComp * e), (unsigned long long)val);
+    }
+    head = min(head + kWarp, tail);
+  };
   const int npts = rr.count ? rr.count[warp] : -1;
-  if (MODEL == GBX_MODEL_GBSW && !ADJ && npts >= 0) {
-    // recorded points, 32 at a time; lanes over their shaping entries
+  if (npts >= 0) {
     const int4* region = rr.rec + (size_t)warp * rr.R;
     const int* sregion = rr.st + (size_t)warp * rr.R;
     // the next batch's records and list starts, loaded one batch ahead
@@ -711,210 +837,96 @@ __global__ void __launch_bounds__(kThreads) chain_kernel(const float4* __restric
       psn = __ldcs(sregion + lane);
     }
     for (int b = 0; b < npts; b += kWarp) {
+      const unsigned carried = tail - head;
+      const unsigned base = head;
+      const int slot = (b & kWarp) + lane;  // two batches' records alternate
       unsigned mlo = 0u, mhi = 0u;
-      int st = 0;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      float V = 0.0f, cq = 0.0f;
-      const int4 pr = prn;
-      const int ps = psn;
+      if (b + lane < npts) {
+        mlo = (unsigned)prn.z;
+        mhi = (unsigned)prn.w;
+        const float4 v = quad.qv[prn.x];
+        const float2 w = quad.qw[prn.x];
+        sv[slot] = make_float4(v.x, v.y, v.z, __int_as_float(prn.y));
+        sc[slot] = make_float2(fmaf(de.x, w.x, de.y * w.y), __int_as_float(psn));
+      }
       if (b + kWarp + lane < npts) {
         prn = __ldcs(region + b + kWarp + lane);
         psn = __ldcs(sregion + b + kWarp + lane);
       }
-      if (b + lane < npts) {
-        V = __int_as_float(pr.y);
-        mlo = (unsigned)pr.z;
-        mhi = (unsigned)pr.w;
-        v = quad.qv[pr.x];
-        const float2 w = quad.qw[pr.x];
-        cq = fmaf(de.x, w.x, de.y * w.y);
-        st = ps;  // written by the integral pass beside the record
+      unsigned have;
+      while ((have = __ballot_sync(0xffffffffu, (mlo | mhi) != 0u)) != 0u) {
+        if (mlo | mhi) {
+          int l;
+          if (mlo) {
+            l = __ffs((int)mlo) - 1;
+            mlo &= mlo - 1;
+          } else {
+            l = 31 + __ffs((int)mhi);
+            mhi &= mhi - 1;
+          }
+          items[(tail + __popc(have & lt)) & (kRing - 1)] = (unsigned)(slot << 16 | l);
+        }
+        tail += __popc(have);
+        if (tail - head >= kWarp) evaluate();
       }
-      const int len = __popc(mlo) + __popc(mhi);
-      int incl = len;
-      for (int off = 1; off < kWarp; off <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += u;
-      }
-      const int total = __shfl_sync(0xffffffffu, incl, kWarp - 1);
-      for (int r = 0; r < total; r += kWarp) {
-        const int p = r + lane;
-        int o = 0;  // owner: the points whose entries end at or before p
-        for (int step = 16; step > 0; step >>= 1)
-          if (__shfl_sync(0xffffffffu, incl, o + step - 1) <= p) o += step;
-        const int oend = __shfl_sync(0xffffffffu, incl, o), olen = __shfl_sync(0xffffffffu, len, o);
-        const unsigned olo = __shfl_sync(0xffffffffu, mlo, o), ohi = __shfl_sync(0xffffffffu, mhi, o);
-        const int ost = __shfl_sync(0xffffffffu, st, o);
-        const float4 ov = make_float4(__shfl_sync(0xffffffffu, v.x, o), __shfl_sync(0xffffffffu, v.y, o),
-                                      __shfl_sync(0xffffffffu, v.z, o), 0.0f);
-        const float oV = __shfl_sync(0xffffffffu, V, o), ocq = __shfl_sync(0xffffffffu, cq, o);
-        if (p >= total) continue;
-        const int nth = p - (oend - olen);  // nth shaping entry of the owner
-        const int nlo = __popc(olo);
-        const int l = nth < nlo ? (int)__fns(olo, 0, nth + 1) : 32 + (int)__fns(ohi, 0, nth - nlo + 1);
-        const int e = ost + l;
-        const float4 a = __ldg(tab.e + e);
-        const int k = __ldg(tab.index + e);
-        const float3 d = query.delta(a, xi, ov);
-        const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-        // the same expressions as the list walk below
-        const float g = shell_g(m, oV, r2 * rsqrtf(r2) - a.w);
-        const float gs = ocq * g * rsqrtf(r2);
-        const float gx = gs * d.x, gy = gs * d.y, gz = gs * d.z;
-        const float3 dd = query.delta(a, xi, make_float4(0.f, 0.f, 0.f, 0.f));  // x_k - x_i
-        const float ex = dd.x, ey = dd.y, ez = dd.z;
-        push_shaping(out, k, !out.quirk || fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= out.cutoff2, gx, gy, gz,
-                     fix, fiy, fiz);
-      }
+      // items carried into this batch must not outlive it: the next one takes their records' slots
+      if (carried > 0 && head == base) evaluate();
     }
   } else {
-    const int q0 = c * chunk, q1 = min(m.nq, q0 + chunk);
-    for (int q = q0 + lane; q < q1; q += kWarp) {
-      const float4 v = quad.qv[q];
-      const float2 w = quad.qw[q];
-      const float cq = fmaf(de.x, w.x, de.y * w.y);
-      if (cq == 0.0f) continue;
-      const long long cell = query.cell(xi, v, q);
-      if (cell < 0) continue;
-      const int2 cs = __ldg(tab.cell + cell);
-      const int cnt = cs.x;
-      if (cnt <= 0) continue;  // buried or empty: no atom shapes the point
-      const int s = cs.y;
-      const float4* E = tab.e + s;
-      if (MODEL == GBX_MODEL_GBSW) {
-        float V = 1.0f;
-        int keep[kWalkKeep];
-        int nk = 0, nshell = 0;
+    Points pts{};
+    pts.init<Q>(quad, m, xi, c, n_chunks, lane);
+    for (int b = pts.t0; b < pts.t1; b += kWarp) {
+      const unsigned carried = tail - head;
+      const unsigned base = head;
+      const int slot = ((b - pts.t0) & kWarp) + lane;
+      const int q = pts.q(b + lane);
+      int cnt = 0, st = 0;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      float V = 1.0f;
+      if (b + lane < pts.t1) {
+        v = quad.qv[q];
+        const float2 w = quad.qw[q];
+        const long long cell = query.cell(xi, v, q);
+        if (cell >= 0) {
+          const int2 cs = __ldg(tab.cell + cell);
+          cnt = cs.x;  // buried or empty: no atom shapes the point
+          st = cs.y;
+        }
         for (int l = 0; l < cnt; ++l) {
-          const float4 a = __ldg(E + l);
-          const float3 d = query.delta(a, xi, v);
-          const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-          const float lo = a.w - m.sw, hi = a.w + m.sw;
-          if (r2 <= lo * lo) {
+          const float4 a = entry_at<Q>(tab, st + l);
+          const float dr = sphere_gap(query.delta(a, xi, v), a.w);
+          if (dr <= -m.sw) {
             V = 0.0f;
-            break;
-          }
-          if (r2 < hi * hi) {
-            const float dr = r2 * rsqrtf(r2) - a.w;
+            cnt = 0;
+          } else if (dr < m.sw) {
             V *= fmaf(dr, fmaf(-m.c3 * dr, dr, m.c1), 0.5f);
-            if (nk < kWalkKeep) keep[nk++] = l;
-            ++nshell;
           }
         }
-        if (V == 0.0f || nshell == 0) continue;
-        const int scan = nshell <= kWalkKeep ? nk : cnt;
-        for (int t = 0; t < scan; ++t) {
-          const int l = nshell <= kWalkKeep ? keep[t] : t;
-          const float4 a = __ldg(E + l);
-          const float3 d = query.delta(a, xi, v);
-          const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-          const float lo = a.w - m.sw, hi = a.w + m.sw;
-          if (!(r2 > lo * lo && r2 < hi * hi)) continue;
-          // the same expressions as the record path (shell_g, then c g / r)
-          const float g = shell_g(m, V, r2 * rsqrtf(r2) - a.w);
-          const int k = __ldg(tab.index + s + l);
-          // dV/dR_k = -(V/u) u' dR'/dR with R' = (R + 0.03) 0.952
-          if (ADJ) red_add_fixed(&out.dEdR[k], cq * g * (-0.9520f));
-          if (k == i) continue;
-          const float gs = cq * g * rsqrtf(r2);
-          const float gx = gs * d.x, gy = gs * d.y, gz = gs * d.z;
-          const float3 dd = query.delta(a, xi, make_float4(0.f, 0.f, 0.f, 0.f));  // x_k - x_i
-          const float ex = dd.x, ey = dd.y, ez = dd.z;
-          push_shaping(out, k, !out.quirk || fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= out.cutoff2, gx,
-                       gy, gz, fix, fiy, fiz);
-        }
-      } else if (MODEL == GBX_MODEL_GBMV1) {
-        Work<false> wk;
-        float p;
-        const float Ssum = rr.state ? rr.state[(size_t)i * m.nq + q] : gbmv1_sum(query, E, cnt, xi, v, wk);
-        logistic_solvent(m.beta, m.lambda, Ssum, p);
-        const float cS = cq * __fdividef(m.beta * p, (1.0f + p) * (1.0f + p));  // c ds/dS
-        if (cS == 0.0f) continue;
-        float px = 0.f, py = 0.f, pz = 0.f;
-        for (int l = 0; l < cnt; ++l) {
-          const float4 a = __ldg(E + l);
-          const float3 d = query.delta(a, xi, v);
-          const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-          const float r4 = r2 * r2;
-          const float e = __expf(a.w * r4);
-          const int k = __ldg(tab.index + s + l);
-          if (ADJ) red_add_fixed(&out.dEdR[k], cS * e * r4 * (-4.0f * a.w / __ldg(&tab.par[s + l].x)));
-          if (k == i) continue;
-          const float gs = cS * 4.0f * a.w * e * r2;  // dS/d(delta) = 4 gamma e r^2 delta
-          const float gx = gs * d.x, gy = gs * d.y, gz = gs * d.z;
-          push_force(out, k, gx, gy, gz);
-          px += gx;
-          py += gy;
-          pz += gz;
-        }
-        // the point's pull on its own atom: summed in FP32 over the list, then fixed point
-        fix += float_to_fixed(px);
-        fiy += float_to_fixed(py);
-        fiz += float_to_fixed(pz);
-      } else {
-        Work<false> wk;
-        Gbmv2State st;
-        if (rr.state) {
-          const size_t idx = (size_t)i * m.nq + q, plane = (size_t)n * m.nq;
-          st = Gbmv2State{rr.state[idx], rr.state[idx + plane], rr.state[idx + 2 * plane], rr.state[idx + 3 * plane],
-                          rr.state[idx + 4 * plane]};
-        } else {
-          st = gbmv2_sums(query, E, tab.par + s, cnt, xi, v, wk);
-        }
-        const float s3sq = fmaf(st.vx, st.vx, fmaf(st.vy, st.vy, st.vz * st.vz));
-        float p;
-        logistic_solvent(m.beta, m.lambda, m.s0 * st.s1 * st.s2 / s3sq, p);
-        const float cS = cq * __fdividef(m.beta * p, (1.0f + p) * (1.0f + p)) * m.s0;
-        if (cS == 0.0f) continue;
-        const float inv3 = 1.0f / s3sq;
-        const float t1 = st.s2 * inv3;                  // d s1 term
-        const float t2 = st.s1 * inv3;                  // d s2 term
-        const float t3 = -st.s1 * st.s2 * inv3 * inv3;  // d s3^2 term
-        float px = 0.f, py = 0.f, pz = 0.f;
-        for (int l = 0; l < cnt; ++l) {
-          const float4 a = __ldg(E + l);
-          const float2 pk = __ldg(tab.par + s + l);
-          const float3 d = query.delta(a, xi, v);
-          const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
-          const float T = fmaf(100.0f, r2, pk.x);
-          const float CT = __fdividef(a.w, T);
-          const float F = CT * CT;
-          const float dFf = -400.0f * F * __fdividef(1.0f, T);  // dF/d(delta) = dFf delta
-          const float vd = st.vx * d.x + st.vy * d.y + st.vz * d.z;
-          const int k = __ldg(tab.index + s + l);
-          if (ADJ) {
-            const float R = pk.y;
-            const float Cp = 10.0f * m.p1, Tp = Cp - 200.0f * R;
-            const float dFdR = 2.0f * CT * __fdividef(Cp * T - a.w * Tp, T * T);
-            red_add_fixed(&out.dEdR[k], cS * (t1 * dFdR + t2 * (r2 * 2.0f * F * dFdR) + t3 * (2.0f * vd * dFdR)));
-          }
-          if (k == i) continue;
-          // dS/d(delta_k) / s0 = t1 dFf d + t2 2F (F + dFf r^2) d + 2 t3 (F v + vd dFf d)
-          const float sc = t1 * dFf + t2 * 2.0f * F * fmaf(dFf, r2, F) + t3 * 2.0f * vd * dFf;
-          const float gx = cS * fmaf(sc, d.x, t3 * 2.0f * F * st.vx);
-          const float gy = cS * fmaf(sc, d.y, t3 * 2.0f * F * st.vy);
-          const float gz = cS * fmaf(sc, d.z, t3 * 2.0f * F * st.vz);
-          push_force(out, k, gx, gy, gz);
-          px += gx;
-          py += gy;
-          pz += gz;
-        }
-        fix += float_to_fixed(px);
-        fiy += float_to_fixed(py);
-        fiz += float_to_fixed(pz);
+        if (V == 0.0f) cnt = 0;
+        sv[slot] = make_float4(v.x, v.y, v.z, V);
+        sc[slot] = make_float2(fmaf(de.x, w.x, de.y * w.y), __int_as_float(st));
       }
+      for (int l = 0; __any_sync(0xffffffffu, l < cnt); ++l) {
+        bool in = false;
+        if (l < cnt) {
+          const float4 a = entry_at<Q>(tab, st + l);
+          in = fabsf(sphere_gap(query.delta(a, xi, v), a.w)) < m.sw;
+        }
+        const unsigned have = __ballot_sync(0xffffffffu, in);
+        if (in) items[(tail + __popc(have & lt)) & (kRing - 1)] = (unsigned)(slot << 16 | l);
+        tail += __popc(have);
+        if (tail - head >= kWarp) evaluate();
+      }
+      if (carried > 0 && head == base) evaluate();
     }
   }
+  if (tail != head) evaluate();
   for (int off = 16; off > 0; off >>= 1) {
     fix += __shfl_xor_sync(0xffffffffu, fix, off);
     fiy += __shfl_xor_sync(0xffffffffu, fiy, off);
     fiz += __shfl_xor_sync(0xffffffffu, fiz, off);
   }
-  if (lane == 0) {
-    atomicAdd(&out.force[i], (unsigned long long)fix);
-    atomicAdd(&out.force[i + out.stride], (unsigned long long)fiy);
-    atomicAdd(&out.force[i + 2 * out.stride], (unsigned long long)fiz);
-  }
+  if (lane == 0) push3(out, i, fix, fiy, fiz);
 }
 
 // GBMV chain rule with the warp cooperating on one point at a time: the
@@ -997,7 +1009,7 @@ __global__ void __launch_bounds__(kThreads, 6) gbmv_chain_kernel(const float4* _
           const float r4 = r2 * r2;
           const float e = __expf(a.w * r4);
           const int k = __ldg(tab.index + s + l);
-          if (ADJ) red_add_fixed(&out.dEdR[k], cS * e * r4 * (-4.0f * a.w / __ldg(&tab.par[s + l].x)));
+          if (ADJ) push_radius(out, k, cS * e * r4 * (-4.0f * a.w / __ldg(&tab.par[s + l].x)));
           if (k == i) continue;
           const float gs = cS * 4.0f * a.w * e * r2;  // dS/d(delta) = 4 gamma e r^2 delta
           const float gx = gs * d.x, gy = gs * d.y, gz = gs * d.z;
@@ -1026,7 +1038,7 @@ __global__ void __launch_bounds__(kThreads, 6) gbmv_chain_kernel(const float4* _
             const float R = pk.y;
             const float Cp = 10.0f * m.p1, Tp = Cp - 200.0f * R;
             const float dFdR = 2.0f * CT * __fdividef(Cp * T - a.w * Tp, T * T);
-            red_add_fixed(&out.dEdR[k], cS * (t1 * dFdR + t2 * (r2 * 2.0f * F * dFdR) + t3 * (2.0f * vd * dFdR)));
+            push_radius(out, k, cS * (t1 * dFdR + t2 * (r2 * 2.0f * F * dFdR) + t3 * (2.0f * vd * dFdR)));
           }
           if (k == i) continue;
           const float sc = t1 * dFf + t2 * 2.0f * F * fmaf(dFf, r2, F) + t3 * 2.0f * vd * dFf;
@@ -1049,11 +1061,7 @@ __global__ void __launch_bounds__(kThreads, 6) gbmv_chain_kernel(const float4* _
     fiy += __shfl_xor_sync(0xffffffffu, fiy, off);
     fiz += __shfl_xor_sync(0xffffffffu, fiz, off);
   }
-  if (lane == 0) {
-    atomicAdd(&out.force[i], (unsigned long long)fix);
-    atomicAdd(&out.force[i + out.stride], (unsigned long long)fiy);
-    atomicAdd(&out.force[i + 2 * out.stride], (unsigned long long)fiz);
-  }
+  if (lane == 0) push3(out, i, fix, fiy, fiz);
 }
 
 Entries entries_of(const Context* ctx) {
@@ -1084,7 +1092,7 @@ void launch_integrals_t(Context* ctx, const float4* pos, const ModelConst& m, bo
     // persistent grid: the resident blocks of every SM (or fewer, for few items)
     if (ctx->integral_grid == 0) {
       int per_sm = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gbsw_integral_kernel<Q, true>, kThreads, 0) !=
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gbsw_integral_kernel<Q, kEmitAll>, kThreads, 0) !=
               cudaSuccess ||
           per_sm < 1)
         per_sm = 1;
@@ -1092,12 +1100,11 @@ void launch_integrals_t(Context* ctx, const float4* pos, const ModelConst& m, bo
     }
     const int grid = std::min(volume_blocks(ctx), ctx->integral_grid);
     cudaMemsetAsync(ctx->d_next_item, 0, sizeof(unsigned), ctx->stream);
-    if (ctx->records)
-      gbsw_integral_kernel<Q, true><<<grid, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks,
-                                                                         ctx->d_J, sink, ctx->d_next_item);
-    else
-      gbsw_integral_kernel<Q, false><<<grid, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks,
-                                                                          ctx->d_J, sink, ctx->d_next_item);
+    auto kernel = !ctx->records       ? gbsw_integral_kernel<Q, kEmitNone>
+                  : ctx->records_self ? gbsw_integral_kernel<Q, kEmitAll>
+                                      : gbsw_integral_kernel<Q, kEmitOthers>;
+    kernel<<<grid, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, ctx->n_chunks, ctx->d_J, sink,
+                                               ctx->d_next_item);
   }
   else if (count_work)
     integral_kernel<MODEL, Q, true><<<volume_blocks(ctx), kThreads, 0, ctx->stream>>>(
@@ -1112,29 +1119,24 @@ void launch_integrals_t(Context* ctx, const float4* pos, const ModelConst& m, bo
 }
 
 template <int MODEL, class Q, bool ADJ>
-void launch_chain_t(Context* ctx, const float4* pos, const ModelConst& m, unsigned long long* force, int stride) {
+void launch_chain_t(Context* ctx, const float4* pos, const ModelConst& m) {
   if (MODEL != GBX_MODEL_GBSW && ctx->gbmv_cells) {
-    launch_gbmv_cells_chain(ctx, pos, m, force, stride, ADJ);
+    launch_gbmv_cells_chain(ctx, pos, m, ADJ);
     return;
   }
   const Entries t = entries_of(ctx);
   const Quad qd{ctx->d_qv, ctx->d_qw, ctx->d_qoff};
   const int chunk = (m.nq + ctx->n_chunks - 1) / ctx->n_chunks;
-  ChainOut o{force, stride, ctx->d_dEdR_fx, m.cutoff_chain_quirk && m.cutoff2 > 0.0f, m.cutoff2};
-  const bool records = MODEL == GBX_MODEL_GBSW && !ADJ && ctx->records;
-  const ChainRecords rr{records ? ctx->d_srec : nullptr, records ? ctx->d_srec_st : nullptr,
-                        records ? ctx->d_rcount : nullptr, ctx->srec_R,
-                        MODEL == GBX_MODEL_GBSW ? nullptr : ctx->d_pstate};
-  bool coop = false;
-  if constexpr (MODEL != GBX_MODEL_GBSW) {
-    coop = ctx->d_pstate != nullptr;
-    if (coop)
-      gbmv_chain_kernel<MODEL, Q, ADJ><<<volume_blocks(ctx), kThreads, 0, ctx->stream>>>(
-          pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, ctx->d_dEdJ, o, ctx->d_pstate);
+  const ChainOut o{ctx->d_f4, m.cutoff_chain_quirk && m.cutoff2 > 0.0f, m.cutoff2};
+  const int blocks = volume_blocks(ctx);
+  if constexpr (MODEL == GBX_MODEL_GBSW) {
+    const ChainRecords rr{ctx->d_srec, ctx->d_srec_st, ctx->records ? ctx->d_rcount : nullptr, ctx->srec_R};
+    gbsw_chain_kernel<Q, ADJ><<<blocks, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, ctx->n_chunks, ctx->d_dEdJ,
+                                                                    o, rr);
+  } else {
+    gbmv_chain_kernel<MODEL, Q, ADJ><<<blocks, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks,
+                                                                           ctx->d_dEdJ, o, ctx->d_pstate);
   }
-  if (!coop)
-    chain_kernel<MODEL, Q, ADJ><<<volume_blocks(ctx), kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, chunk,
-                                                                                  ctx->n_chunks, ctx->d_dEdJ, o, rr);
   ++ctx->launches;
 }
 
@@ -1180,34 +1182,34 @@ gbx_status launch_integrals(Context* ctx, const float4* pos, bool count_work) {
   return launch_status(ctx, "integral launch");
 }
 
-gbx_status launch_chain(Context* ctx, const float4* pos, unsigned long long* force, int stride, bool adjoint) {
+gbx_status launch_chain(Context* ctx, const float4* pos, bool adjoint) {
   const ModelConst m = make_model_const(ctx);
   if (ctx->use_tight && ctx->cfg.periodic) {
-    if (adjoint) launch_chain_t<GBX_MODEL_GBSW, PeriodicTightQuery, true>(ctx, pos, m, force, stride);
-    else launch_chain_t<GBX_MODEL_GBSW, PeriodicTightQuery, false>(ctx, pos, m, force, stride);
+    if (adjoint) launch_chain_t<GBX_MODEL_GBSW, PeriodicTightQuery, true>(ctx, pos, m);
+    else launch_chain_t<GBX_MODEL_GBSW, PeriodicTightQuery, false>(ctx, pos, m);
   } else if (ctx->use_tight) {
-    if (adjoint) launch_chain_t<GBX_MODEL_GBSW, TightQuery, true>(ctx, pos, m, force, stride);
-    else launch_chain_t<GBX_MODEL_GBSW, TightQuery, false>(ctx, pos, m, force, stride);
+    if (adjoint) launch_chain_t<GBX_MODEL_GBSW, TightQuery, true>(ctx, pos, m);
+    else launch_chain_t<GBX_MODEL_GBSW, TightQuery, false>(ctx, pos, m);
   } else if (ctx->cfg.periodic && ctx->cfg.table_mode == GBX_TABLE_STANDALONE) {
-    if (adjoint) launch_chain_t<GBX_MODEL_GBSW, PeriodicQuery, true>(ctx, pos, m, force, stride);
-    else launch_chain_t<GBX_MODEL_GBSW, PeriodicQuery, false>(ctx, pos, m, force, stride);
+    if (adjoint) launch_chain_t<GBX_MODEL_GBSW, PeriodicQuery, true>(ctx, pos, m);
+    else launch_chain_t<GBX_MODEL_GBSW, PeriodicQuery, false>(ctx, pos, m);
   } else if (ctx->cfg.periodic) {
     switch (ctx->cfg.model * 2 + (adjoint ? 1 : 0)) {
-      case 0: launch_chain_t<GBX_MODEL_GBSW, MinImageQuery, false>(ctx, pos, m, force, stride); break;
-      case 1: launch_chain_t<GBX_MODEL_GBSW, MinImageQuery, true>(ctx, pos, m, force, stride); break;
-      case 2: launch_chain_t<GBX_MODEL_GBMV1, MinImageQuery, false>(ctx, pos, m, force, stride); break;
-      case 3: launch_chain_t<GBX_MODEL_GBMV1, MinImageQuery, true>(ctx, pos, m, force, stride); break;
-      case 4: launch_chain_t<GBX_MODEL_GBMV2, MinImageQuery, false>(ctx, pos, m, force, stride); break;
-      default: launch_chain_t<GBX_MODEL_GBMV2, MinImageQuery, true>(ctx, pos, m, force, stride); break;
+      case 0: launch_chain_t<GBX_MODEL_GBSW, MinImageQuery, false>(ctx, pos, m); break;
+      case 1: launch_chain_t<GBX_MODEL_GBSW, MinImageQuery, true>(ctx, pos, m); break;
+      case 2: launch_chain_t<GBX_MODEL_GBMV1, MinImageQuery, false>(ctx, pos, m); break;
+      case 3: launch_chain_t<GBX_MODEL_GBMV1, MinImageQuery, true>(ctx, pos, m); break;
+      case 4: launch_chain_t<GBX_MODEL_GBMV2, MinImageQuery, false>(ctx, pos, m); break;
+      default: launch_chain_t<GBX_MODEL_GBMV2, MinImageQuery, true>(ctx, pos, m); break;
     }
   } else {
     switch (ctx->cfg.model * 2 + (adjoint ? 1 : 0)) {
-      case 0: launch_chain_t<GBX_MODEL_GBSW, RefQuery, false>(ctx, pos, m, force, stride); break;
-      case 1: launch_chain_t<GBX_MODEL_GBSW, RefQuery, true>(ctx, pos, m, force, stride); break;
-      case 2: launch_chain_t<GBX_MODEL_GBMV1, RefQuery, false>(ctx, pos, m, force, stride); break;
-      case 3: launch_chain_t<GBX_MODEL_GBMV1, RefQuery, true>(ctx, pos, m, force, stride); break;
-      case 4: launch_chain_t<GBX_MODEL_GBMV2, RefQuery, false>(ctx, pos, m, force, stride); break;
-      default: launch_chain_t<GBX_MODEL_GBMV2, RefQuery, true>(ctx, pos, m, force, stride); break;
+      case 0: launch_chain_t<GBX_MODEL_GBSW, RefQuery, false>(ctx, pos, m); break;
+      case 1: launch_chain_t<GBX_MODEL_GBSW, RefQuery, true>(ctx, pos, m); break;
+      case 2: launch_chain_t<GBX_MODEL_GBMV1, RefQuery, false>(ctx, pos, m); break;
+      case 3: launch_chain_t<GBX_MODEL_GBMV1, RefQuery, true>(ctx, pos, m); break;
+      case 4: launch_chain_t<GBX_MODEL_GBMV2, RefQuery, false>(ctx, pos, m); break;
+      default: launch_chain_t<GBX_MODEL_GBMV2, RefQuery, true>(ctx, pos, m); break;
     }
   }
   return launch_status(ctx, "chain launch");

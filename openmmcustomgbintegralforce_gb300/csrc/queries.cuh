@@ -20,7 +20,7 @@ struct Quad {
 struct Entries {
   const TableGeom* geom;
   const int2* cell;    // (count, start); exact table: count -1 marks a buried cell
-  const float4* e;     // (x, y, z, main model parameter)
+  const float4* e;     // (x, y, z, main model parameter); exact table: pairs (EntryPair)
   const float2* par;   // secondary model parameters (reference table only)
   const int* index;    // atom index of each entry
   long long cell_cap;  // cells allocated: a geometry with more (a table that
@@ -31,6 +31,17 @@ struct Entries {
   const TableGeom* wrap;  // exact table of a periodic system: the reference's
                           // standalone grid, whose edges decide a point's move
 };
+
+// Two consecutive entries of an exact-table list, one field after the other,
+// so that a 32-byte load gives the operands of packed FP32x2 arithmetic.
+struct EntryPair {
+  float2 x, y, z, nw;  // nw: -R'
+};
+__device__ __forceinline__ EntryPair ldg_entries(const float4* e, int first) {
+  const Float4x2 p = ldg_pair(e + first);
+  return EntryPair{make_float2(p.a.x, p.a.y), make_float2(p.a.z, p.a.w), make_float2(p.b.x, p.b.y),
+                   make_float2(p.b.z, p.b.w)};
+}
 
 // Cells a query may index: none when the table outgrew either buffer this
 // step (the build then wrote no cell record, and the records left in place
@@ -63,6 +74,7 @@ __device__ long long query_exact(const TableGeom& g, const float4 xi, const doub
 }
 
 struct RefQuery {
+  static constexpr bool kImages = false;  // distances by minimum image
   float rel[3];  // (x_i - min) / step, cell units
   float inv[3];
   float invdims[3];  // periodic table: 1 / dims, the box in cell units being dims
@@ -140,6 +152,7 @@ struct RefQuery {
 // CutoffPeriodic, GBMVIntegralTypeI.cpp:59-62, TypeII.cpp:64-67,
 // GBSWIntegral.cpp:63-68).
 struct MinImageQuery : RefQuery {
+  static constexpr bool kImages = true;
   float L[3], iL[3];
   __device__ __forceinline__ void init(const TableGeom& geom, const float4 xi, const double* qo, long long cap) {
     RefQuery::init(geom, xi, qo, cap);
@@ -181,6 +194,7 @@ __device__ long long query_exact_wrap(const TableGeom& g, const float4 xi, const
 // minimum image in the rectangular box (ReferenceForce::getDeltaRPeriodic:
 // d -= L floor(d / L + 1/2)).
 struct PeriodicQuery {
+  static constexpr bool kImages = true;
   float rel[3];   // (x_i - min) / step, cell units
   float inv[3];
   float wrap[3];  // box edge in cell units
@@ -241,6 +255,7 @@ struct PeriodicQuery {
 // Exact GBSW table: FP32 query; the table's membership margin covers a
 // point landing in a neighbouring cell.
 struct TightQuery {
+  static constexpr bool kImages = false;
   float xr[3];
   float inv_h;
   int dims[3];
@@ -260,9 +275,12 @@ struct TightQuery {
   // 32-bit arithmetic: the exact table holds fewer than 2^31 cells (checked
   // when it is sized); one unsigned compare per axis tests both bounds
   __device__ __forceinline__ int cell_at(float ox, float oy, float oz) const {
-    const int cx = (int)floorf((xr[0] + ox) * inv_h);
-    const int cy = (int)floorf((xr[1] + oy) * inv_h);
-    const int cz = (int)floorf((xr[2] + oz) * inv_h);
+    // floor by adding 2^23 rounding down: the integer is the sum's low bits
+    // (two full-rate instructions, where float-to-int runs at a quarter of the
+    // rate); a negative or huge coordinate fails the unsigned compare
+    const int cx = __float_as_int(__fmaf_rd(xr[0] + ox, inv_h, 8388608.0f)) - 0x4B000000;
+    const int cy = __float_as_int(__fmaf_rd(xr[1] + oy, inv_h, 8388608.0f)) - 0x4B000000;
+    const int cz = __float_as_int(__fmaf_rd(xr[2] + oz, inv_h, 8388608.0f)) - 0x4B000000;
     if ((unsigned)cx >= (unsigned)dims[0] || (unsigned)cy >= (unsigned)dims[1] || (unsigned)cz >= (unsigned)dims[2])
       return -1;
     return (cx * dims[1] + cy) * dims[2] + cz;
@@ -270,6 +288,10 @@ struct TightQuery {
   __device__ __forceinline__ int cell(const float4, const float4 v, int) const { return cell_at(v.x, v.y, v.z); }
   __device__ __forceinline__ float3 delta(const float4 a, const float4 xi, const float4 v) const {
     return make_float3((a.x - xi.x) - v.x, (a.y - xi.y) - v.y, (a.z - xi.z) - v.z);
+  }
+  // delta of both entries along axis k, each half rounded as delta() rounds it
+  __device__ __forceinline__ float2 delta2(int, float2 a, float xi, float v) const {
+    return __fadd2_rn(__fadd2_rn(a, make_float2(-xi, -xi)), make_float2(-v, -v));
   }
 };
 
@@ -305,6 +327,7 @@ __device__ bool wrap_shift_exact(const TableGeom& g, const float4 xi, const doub
 // decision within a guard band of the grid's edges) and looks p' up in the
 // exact table; distances are by minimum image.
 struct PeriodicTightQuery : TightQuery {
+  static constexpr bool kImages = true;
   float xw[3];    // x_i - the standalone grid's lower edge (nm)
   float span[3];  // the standalone grid's extent (nm)
   float L[3], iL[3];
@@ -360,6 +383,11 @@ struct PeriodicTightQuery : TightQuery {
     for (int k = 0; k < 3; ++k) d[k] = fmaf(-L[k], floorf(fmaf(d[k], iL[k], 0.5f)), d[k]);
     return make_float3(d[0], d[1], d[2]);
   }
+  __device__ __forceinline__ float2 delta2(int k, float2 a, float xi, float v) const {
+    const float2 d = TightQuery::delta2(k, a, xi, v);
+    return make_float2(fmaf(-L[k], floorf(fmaf(d.x, iL[k], 0.5f)), d.x),
+                       fmaf(-L[k], floorf(fmaf(d.y, iL[k], 0.5f)), d.y));
+  }
 };
 
 // The exact table's query types (cell records with the first entry, lists
@@ -376,6 +404,17 @@ template <>
 struct IsTight<PeriodicTightQuery> {
   static constexpr bool value = true;
 };
+
+// Entry `at` of either table's lists as (x, y, z, main model parameter).
+template <class Q>
+__device__ __forceinline__ float4 entry_at(const Entries& t, int at) {
+  if constexpr (IsTight<Q>::value) {
+    const float* p = reinterpret_cast<const float*>(t.e) + 8 * (size_t)(at >> 1) + (at & 1);
+    return make_float4(__ldg(p), __ldg(p + 2), __ldg(p + 4), -__ldg(p + 6));
+  } else {
+    return __ldg(t.e + at);
+  }
+}
 
 // s = p / (1 + p) with p = exp(beta (S - lambda)): the solvent fraction
 __device__ __forceinline__ float logistic_solvent(float beta, float lambda, float S, float& p) {
