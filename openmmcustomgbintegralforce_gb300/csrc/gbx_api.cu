@@ -199,7 +199,9 @@ gbx_status alloc_atom_buffers(Context* ctx) {
   GBX_TRY(dalloc(ctx, &ctx->d_par, n));
   GBX_TRY(dalloc(ctx, &ctx->d_wpar, n));
   GBX_TRY(dalloc(ctx, &ctx->d_pos, n));
-  GBX_TRY(dalloc(ctx, &ctx->d_reduce, gbx::table_geom_scratch_doubles(n)));
+  GBX_TRY(dalloc(ctx, reinterpret_cast<unsigned char**>(&ctx->d_parts), gbx::prepare_scratch_bytes(n)));
+  GBX_TRY(dalloc(ctx, &ctx->d_ticket, 1));
+  GBX_CUDA(cudaMemset(ctx->d_ticket, 0, sizeof(unsigned)));
   GBX_TRY(dalloc(ctx, &ctx->d_J, 2 * (size_t)ctx->n_chunks * n));
   GBX_TRY(dalloc(ctx, &ctx->d_born, n));
   GBX_TRY(dalloc(ctx, &ctx->d_bornf, 2 * (size_t)n));
@@ -217,7 +219,7 @@ gbx_status alloc_atom_buffers(Context* ctx) {
     GBX_TRY(dalloc(ctx, &ctx->d_prank, (size_t)n * Q));
     GBX_TRY(dalloc(ctx, &ctx->d_porder, (size_t)n * Q));
     GBX_TRY(dalloc(ctx, &ctx->d_sval, (size_t)n * Q));
-    GBX_TRY(dalloc(ctx, &ctx->d_pgeom, 1));
+    GBX_TRY(dalloc(ctx, &ctx->d_ptotal, 1));
   }
   if (ctx->cfg.cutoff > 0) {
     GBX_TRY(dalloc(ctx, &ctx->d_perm, n));
@@ -334,7 +336,6 @@ gbx_status prepare_records(Context* ctx, bool wanted, bool adjoint) {
   }
   if (ctx->srec_R == 0 || warps != ctx->srec_warps) return GBX_OK;
   ctx->records = true;
-  GBX_CUDA(cudaMemsetAsync(ctx->d_rmax, 0, sizeof(unsigned), ctx->stream));
   return GBX_OK;
 }
 
@@ -345,11 +346,9 @@ gbx_status grow_table(Context* ctx, long long cells, long long entries) {
     GBX_TRY(dalloc(ctx, &ctx->d_cell_start, cap + 1));
     GBX_TRY(dalloc(ctx, &ctx->d_cell_cursor, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_cell2, cap));
-    GBX_TRY(dalloc(ctx, &ctx->d_block_sums, cap / (1024 * 8) + 2));
     if (ctx->cfg.model != GBX_MODEL_GBSW) {
       GBX_TRY(dalloc(ctx, &ctx->d_pcount, cap));
       GBX_TRY(dalloc(ctx, &ctx->d_pstart, cap + 1));
-      GBX_TRY(dalloc(ctx, &ctx->d_pblock_sums, cap / (1024 * 8) + 2));
     }
     ctx->cell_cap = cap;
   }
@@ -369,9 +368,10 @@ gbx_status grow_table(Context* ctx, long long cells, long long entries) {
 
 // Build the table; on a capacity miss read the needed sizes back, grow and
 // rebuild.  Synchronises the stream when `check` is set.
-gbx_status build_table_checked(Context* ctx, bool check) {
+// Starts with the call's first kernel, from `posq` (call: see launch_prepare).
+gbx_status build_table_checked(Context* ctx, const void* posq, bool check, bool call) {
   for (int attempt = 0; attempt < 3; ++attempt) {
-    GBX_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned), ctx->stream));
+    GBX_TRY(gbx::launch_prepare(ctx, posq, false, true, call));
     GBX_TRY(gbx::launch_table_build(ctx, ctx->d_pos));
     if (!check && ctx->cell_cap > 0 && ctx->entry_cap > 0) {
       ctx->table_valid = true;
@@ -417,7 +417,6 @@ gbx_status grow_tight(Context* ctx, long long cells, long long entries) {
     GBX_TRY(dalloc(ctx, &ctx->d_tburied, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_tcell, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_tfirst, cap));
-    GBX_TRY(dalloc(ctx, &ctx->d_tblock_sums, cap / (1024 * 8) + 2));
     ctx->tcell_cap = cap;
   }
   if (entries > ctx->tentry_cap) {
@@ -434,9 +433,9 @@ gbx_status grow_tight(Context* ctx, long long cells, long long entries) {
 }
 
 // Exact-table counterpart of build_table_checked.
-gbx_status build_tight_checked(Context* ctx, bool check) {
+gbx_status build_tight_checked(Context* ctx, const void* posq, bool check) {
   for (int attempt = 0; attempt < 3; ++attempt) {
-    GBX_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(unsigned), ctx->stream));
+    GBX_TRY(gbx::launch_prepare(ctx, posq, true, false, true));
     GBX_TRY(gbx::launch_tight_build(ctx, ctx->d_pos));
     if (!check && ctx->tcell_cap > 0 && ctx->tentry_cap > 0) return GBX_OK;
     unsigned st = 0;
@@ -473,12 +472,11 @@ gbx_status run_pipeline(Context* ctx, const float4* posq, unsigned long long* fo
     ++stage;
     return GBX_OK;
   };
-  GBX_TRY(mark());
-  GBX_TRY(gbx::launch_stage_positions(ctx, posq));
+  GBX_TRY(mark());  // staging is the first kernel of the table stage
   GBX_TRY(mark());
   ctx->table_valid = false;
-  if (ctx->use_tight) GBX_TRY(build_tight_checked(ctx, check || !ctx->tight_valid));
-  else GBX_TRY(build_table_checked(ctx, check));
+  if (ctx->use_tight) GBX_TRY(build_tight_checked(ctx, posq, check || !ctx->tight_valid));
+  else GBX_TRY(build_table_checked(ctx, posq, check, true));
   if (count_work) GBX_CUDA(cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long) * 4, ctx->stream));
   const bool chain = forces || adjoint;
   GBX_TRY(prepare_records(ctx, chain && !count_work, adjoint));
@@ -783,15 +781,15 @@ gbx_status gbx_destroy(gbx_context* handle) {
   gbx::custom_destroy(ctx);
   void* ptrs[] = {ctx->d_qv, ctx->d_qw, ctx->d_qoff, ctx->d_radius, ctx->d_charge, ctx->d_par, ctx->d_wpar,
                   ctx->d_geom, ctx->d_cell_count, ctx->d_cell_start, ctx->d_cell_cursor, ctx->d_entries,
-                  ctx->d_block_sums, ctx->d_reduce, ctx->d_pos, ctx->d_J, ctx->d_born, ctx->d_bornf, ctx->d_dBdJ,
+                  ctx->d_parts, ctx->d_ticket, ctx->d_pos, ctx->d_J, ctx->d_born, ctx->d_bornf, ctx->d_dBdJ,
                   ctx->d_integrals, ctx->d_dEdB_fx, ctx->d_dEdJ, ctx->d_energy_part, ctx->d_force_fx, ctx->d_f4,
                   ctx->d_energy, ctx->d_dEdR_fx, ctx->d_dEdq_fx, ctx->d_alpha_grad, ctx->d_status, ctx->d_work,
                   ctx->d_tgeom, ctx->d_wgeom, ctx->d_tcount, ctx->d_tstart, ctx->d_tcursor, ctx->d_tburied,
-                  ctx->d_tblock_sums, ctx->d_tentry, ctx->d_tindex, ctx->d_entry4, ctx->d_entry_par,
+                  ctx->d_tentry, ctx->d_tindex, ctx->d_entry4, ctx->d_entry_par,
                   ctx->d_cell2, ctx->d_tcell, ctx->d_tfirst, ctx->d_srec, ctx->d_srec_st, ctx->d_rcount, ctx->d_rmax, ctx->d_next_item, ctx->d_energy_fx, ctx->d_tile_box, ctx->d_perm,
                   ctx->d_perm_tmp, ctx->d_cell_of, ctx->d_scount, ctx->d_sstart, ctx->d_scursor, ctx->d_sgeom, ctx->d_pstate,
                   ctx->d_pcell, ctx->d_prank, ctx->d_porder, ctx->d_sval, ctx->d_pcount, ctx->d_pstart,
-                  ctx->d_pblock_sums, ctx->d_pgeom, ctx->d_slot_of, ctx->d_pub};
+                  ctx->d_ptotal, ctx->d_slot_of, ctx->d_pub};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int k = 0; k <= Context::kStages; ++k)
@@ -1368,8 +1366,7 @@ gbx_status gbx_build_lookup_table(gbx_context* handle, const void* posq, void* s
   Context* ctx = reinterpret_cast<Context*>(handle);
   if (!ctx || !posq) return GBX_ERR_INVALID_ARGUMENT;
   ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;
-  GBX_TRY(gbx::launch_stage_positions(ctx, reinterpret_cast<const float4*>(posq)));
-  return build_table_checked(ctx, true);
+  return build_table_checked(ctx, posq, true, false);
 }
 
 gbx_status gbx_get_lookup_table(gbx_context* handle, int dims[3], double mn[3], double step[3], int64_t* ncell,
@@ -1380,7 +1377,7 @@ gbx_status gbx_get_lookup_table(gbx_context* handle, int dims[3], double mn[3], 
     // the last execute integrated on the exact table: build the reference
     // table from the positions it staged
     if (!ctx->have_result) return GBX_ERR_NOT_READY;
-    GBX_TRY(build_table_checked(ctx, true));
+    GBX_TRY(build_table_checked(ctx, ctx->d_pos, true, false));
   }
   gbx::TableGeom g;
   GBX_CUDA(cudaStreamSynchronize(ctx->stream));

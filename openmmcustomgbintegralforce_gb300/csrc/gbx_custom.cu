@@ -988,7 +988,6 @@ gbx_status launch_custom_energy(Context* ctx, const float4* pos, unsigned long l
     void* bargs[] = {&b};
     e = cudaLaunchKernel((const void*)p->k_pair, dim3(p->pair_blocks), dim3(kPairThreads), bargs, 0, st);
   }
-  if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_energy_fx, 0, sizeof(unsigned long long), st);
   ctx->launches += 2;
   if (e != cudaSuccess) {
     ctx->last_error = std::string("custom energy launch: ") + cudaGetErrorString(e);

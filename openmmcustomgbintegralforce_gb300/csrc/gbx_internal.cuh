@@ -125,8 +125,8 @@ struct Context {
   int* d_entries = nullptr;      // [entry_cap] atom indices, ascending per cell
   float4* d_entry4 = nullptr;    // [entry_cap] inline copies (x, y, z, main parameter)
   float2* d_entry_par = nullptr; // [entry_cap] inline secondary parameters
-  int* d_block_sums = nullptr;
-  double* d_reduce = nullptr;    // geometry reduction scratch
+  void* d_parts = nullptr;       // partial extents of the call's first kernel
+  unsigned* d_ticket = nullptr;  // its count of finished blocks (0 between calls)
   bool table_valid = false;
 
   // exact GBSW table (GBX_TABLE_POLICY_AUTO on a standalone table):
@@ -143,7 +143,6 @@ struct Context {
   int* d_tburied = nullptr;
   int2* d_tcell = nullptr;       // (count or -1 if buried, start)
   TightCell* d_tfirst = nullptr; // per cell: first entry and (count, start)
-  int* d_tblock_sums = nullptr;
   float4* d_tentry = nullptr;    // (x, y, z, R') per list entry; lists start at even entries
   int* d_tindex = nullptr;       // atom index per list entry
   bool tight_valid = false;
@@ -177,8 +176,7 @@ struct Context {
   float* d_sval = nullptr;                    // [n Q] solvent fraction by point id
   int* d_pcount = nullptr;                    // [cell_cap] points per cell
   int* d_pstart = nullptr;                    // [cell_cap + 1] first slot per cell
-  int* d_pblock_sums = nullptr;               // scan scratch
-  TableGeom* d_pgeom = nullptr;               // the point scan's cell count and total
+  unsigned long long* d_ptotal = nullptr;     // [1] points binned
   bool gbmv_cells = false;                    // this call's GBMV passes run by cell
   CustomPlan* custom = nullptr;               // expressions outside the canonical set (gbx_custom.cu)
   unsigned long long* d_force_fx = nullptr;  // internal force buffer [3n] (host path)
@@ -320,16 +318,17 @@ gbx_status fix_chain_records(Context* ctx);
 // the shortest box edge); switching drops graphs and tables.
 void choose_table(Context* ctx);
 
-gbx_status launch_stage_positions(Context* ctx, const void* posq);
+// The call's first kernel: positions staged, the accumulators cleared, the
+// grids of the exact and / or the reference table.  call: false builds a
+// table alone, outside an evaluation (the last call's results stay).
+gbx_status launch_prepare(Context* ctx, const void* posq, bool tight, bool reference, bool call);
+size_t prepare_scratch_bytes(int n);
 gbx_status launch_finish_outputs(Context* ctx, unsigned long long* force, int stride, float* energy_float);
 // The call's last kernel: the chain rule's sums added to the force buffer
 // (and dE/dR), the energy, the published status.
 gbx_status launch_finish(Context* ctx, unsigned long long* force, int stride, double* energy, bool chain, bool adjoint);
 gbx_status launch_table_build(Context* ctx, const float4* pos);
-size_t table_geom_scratch_doubles(int n);
 gbx_status launch_tight_build(Context* ctx, const float4* pos);
-// The standalone (reference) table's grid geometry alone, into out.
-void launch_standalone_geom(Context* ctx, const float4* pos, TableGeom* out);
 // GBMV on a table the cell passes serve: bins the quadrature points by
 // cell (the cell passes' data layout); nothing otherwise.
 gbx_status launch_binning(Context* ctx, const float4* pos, bool count_work);

@@ -219,13 +219,6 @@ __global__ void gbmv_fill_kernel(long long npts, CellPoints cp) {
   if (c >= 0) cp.order[cp.start[c] + cp.rank[p]] = (int)p;
 }
 
-// The table's cell count for the point scan (which writes its total into
-// its own geometry record, not the table's).
-__global__ void copy_ncell_kernel(const TableGeom* __restrict__ table, TableGeom* __restrict__ pg, long long cap) {
-  pg->ncell = table->ncell <= cap ? table->ncell : 0;
-  pg->total = 0;
-}
-
 // Bitonic sort of 32 E keys held E per lane, element lane E + r in key[r].
 template <int E>
 __device__ __forceinline__ void warp_bitonic_sort(int (&key)[E], int lane) {
@@ -756,7 +749,6 @@ gbx_status launch_gbmv_cells_bin(Context* ctx, const float4* pos, const ModelCon
   const long long warps = (long long)ctx->n * ctx->n_chunks;
   const int bin_blocks = (int)((warps * kWarp + kBinThreads - 1) / kBinThreads);
   const long long cells = ctx->cell_cap;
-  cudaMemsetAsync(ctx->d_pcount, 0, sizeof(int) * cells, st);
   const bool per = ctx->cfg.periodic != 0;
   if (m.model == GBX_MODEL_GBMV1) {
     if (per) gbmv_bin_kernel<GBX_MODEL_GBMV1, MinImageQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
@@ -765,11 +757,10 @@ gbx_status launch_gbmv_cells_bin(Context* ctx, const float4* pos, const ModelCon
     if (per) gbmv_bin_kernel<GBX_MODEL_GBMV2, MinImageQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
     else gbmv_bin_kernel<GBX_MODEL_GBMV2, RefQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
   }
-  copy_ncell_kernel<<<1, 1, 0, st>>>(ctx->d_geom, ctx->d_pgeom, cells);
-  launch_scan<false>(ctx->d_pcount, ctx->d_pgeom, ctx->d_pblock_sums, ctx->d_pstart, nullptr, cells, 0x7fffffffffffLL,
+  launch_scan<false>(ctx->d_pcount, ctx->d_geom, ctx->d_pstart, nullptr, cells, 0x7fffffffffffLL, ctx->d_ptotal,
                      ctx->d_status, st);
   gbmv_fill_kernel<<<(int)((npts + 255) / 256), 256, 0, st>>>(npts, cp);
-  ctx->launches += 6;  // bin, ncell copy, three scan phases, fill
+  ctx->launches += 3;  // bin, scan, fill
   return GBX_OK;
 }
 

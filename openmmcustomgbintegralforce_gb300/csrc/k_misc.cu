@@ -1,4 +1,4 @@
-// Small per-atom kernels: model constants, position staging, FP64 Born-radius
+// Small per-atom kernels: model constants, FP64 Born-radius
 // assembly, dE/dB -> dE/dJ conversion and the deterministic energy reduction.
 #include <math.h>
 
@@ -35,35 +35,6 @@ ModelConst make_model_const(const Context* ctx) {
 }
 
 namespace {
-
-// Internal positions: x, y, z and the model's main per-atom parameter in .w
-// (GBSW: R' = (R + 0.03) 0.952, CharmmReferenceGBSW.cpp:625; GBMV-I:
-// gamma_j = gamma0 ln(lambda) / R^4, GBMVIntegralTypeI.cpp:168; GBMV-II:
-// C_j = 10 P1 R + P2, GBMVIntegralTypeII.cpp:179), from the caller's float4
-// or double4 positions (OpenMM's single / double precision posq).  With an
-// atom order set, internal atom i is read from the caller's slot slot_of[i].
-template <bool DBL>
-__global__ void stage_positions_kernel(const void* __restrict__ in, int n, const int* __restrict__ slot_of,
-                                       const float* __restrict__ wpar, float4* __restrict__ out,
-                                       ulonglong2* __restrict__ f4) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int k = slot_of ? slot_of[i] : i;
-  float x, y, z;
-  if (DBL) {
-    const double4 p = static_cast<const double4*>(in)[k];
-    x = (float)p.x;
-    y = (float)p.y;
-    z = (float)p.z;
-  } else {
-    const float4 p = static_cast<const float4*>(in)[k];
-    x = p.x;
-    y = p.y;
-    z = p.z;
-  }
-  out[i] = make_float4(x, y, z, wpar[i]);
-  f4[2 * i] = f4[2 * i + 1] = make_ulonglong2(0ull, 0ull);  // the chain rule's sums of this call
-}
 
 // The caller's outputs of a call that ran on internal buffers: forces added
 // to the caller's slots (each slot written by one thread), the energy added
@@ -207,23 +178,6 @@ __global__ void __launch_bounds__(kRedThreads) energy_reduce_kernel(const double
 
 }  // namespace
 
-gbx_status launch_stage_positions(Context* ctx, const void* posq) {
-  const int n = ctx->n;
-  const int* slot_of = ctx->in_permuted ? ctx->d_slot_of : nullptr;
-  ulonglong2* f4 = reinterpret_cast<ulonglong2*>(ctx->d_f4);
-  if (ctx->in_double)
-    stage_positions_kernel<true><<<(n + 255) / 256, 256, 0, ctx->stream>>>(posq, n, slot_of, ctx->d_wpar, ctx->d_pos, f4);
-  else
-    stage_positions_kernel<false><<<(n + 255) / 256, 256, 0, ctx->stream>>>(posq, n, slot_of, ctx->d_wpar, ctx->d_pos, f4);
-  ++ctx->launches;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    ctx->last_error = std::string("stage launch: ") + cudaGetErrorString(e);
-    return GBX_ERR_CUDA;
-  }
-  return GBX_OK;
-}
-
 gbx_status launch_finish_outputs(Context* ctx, unsigned long long* force, int stride, float* energy_float) {
   const int n = ctx->n;
   finish_outputs_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(
@@ -244,7 +198,6 @@ gbx_status launch_born(Context* ctx) {
       reinterpret_cast<float2*>(ctx->d_bornf), ctx->d_dBdJ, ctx->d_dBdJ + 2 * (size_t)n, ctx->d_integrals,
       ctx->d_status);
   ++ctx->launches;
-  cudaMemsetAsync(ctx->d_dEdB_fx, 0, sizeof(unsigned long long) * n, ctx->stream);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     ctx->last_error = std::string("born launch: ") + cudaGetErrorString(e);

@@ -749,7 +749,6 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
   const int wpb = kSymThreads / kWarp;
   const int gu = (a.nblocks * a.chunks + wpb - 1) / wpb, gb = (a.nblocks * kNI * kBlockSplit + wpb - 1) / wpb;
   cudaStream_t st = ctx->stream;
-  cudaMemsetAsync(ctx->d_energy_fx, 0, sizeof(unsigned long long), st);
   if (ctx->cfg.periodic) {
     // minimum image, every tile pair evaluated (bounding boxes do not wrap)
     a.L = make_float3((float)ctx->cfg.box[0], (float)ctx->cfg.box[1], (float)ctx->cfg.box[2]);

@@ -1,11 +1,11 @@
 // Lookup-table build: bins atoms into per-cell lists that are bit-identical
 // to the reference's tables.
 //
-//   geometry  one block reduces the bounding box / centre of geometry and
-//             derives the grid exactly as the reference does (FP64);
+//   geometry  the grid exactly as the reference derives it (FP64), by the
+//             call's first kernel (k_prepare.cu);
 //   count     one warp per atom enumerates its candidate cells (or samples)
 //             and counts members with atomics;
-//   scan      exclusive prefix sum of the counts -> CSR offsets;
+//   scan      counts -> list starts;
 //   fill      second enumeration writes members at atomic cursors;
 //   sort      one warp per cell ranks its entries, restoring the reference's
 //             ascending-atom insertion order, then applies the per-cell cap.
@@ -21,7 +21,6 @@
 namespace gbx {
 namespace {
 
-constexpr int kGeomThreads = 1024;
 constexpr int kMaxSamples = 96;  // samples per axis in the periodic branch
 
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
@@ -31,167 +30,6 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 
 // sqrt(3.0)/2.0 as the reference computes it in double.
 __device__ __forceinline__ double half_sqrt3() { return ddiv(__dsqrt_rn(3.0), 2.0); }
-
-// --------------------------------------------------------------------------
-// Geometry: CharmmReferenceGBSW.cpp:444-466, CustomGBIntegral.cpp:53-113,163-193
-// --------------------------------------------------------------------------
-// Per-block partial extents and sums over a fixed range of atoms (FP64 on
-// every SM instead of one: the GPU's FP64 rate per SM is low), reduced by
-// a fixed-shape tree, so the centre of geometry is the same bits every call.
-constexpr int kPartThreads = 256;
-
-struct GeomPart {
-  double mn[3], mx[3], sum[3], rmax;
-};
-
-__global__ void __launch_bounds__(kPartThreads) table_geom_partial_kernel(const float4* __restrict__ pos,
-                                                                          const double* __restrict__ radius, int n,
-                                                                          GeomPart* __restrict__ parts) {
-  __shared__ double s[10][kPartThreads];
-  const int t = threadIdx.x, a = blockIdx.x * kPartThreads + t;
-  double v[10];
-  if (a < n) {
-    const float4 p = pos[a];
-    const double c[3] = {(double)p.x, (double)p.y, (double)p.z};
-    for (int k = 0; k < 3; ++k) {
-      v[k] = c[k];
-      v[3 + k] = c[k];
-      v[6 + k] = c[k];
-    }
-    v[9] = radius[a];
-  } else {
-    const float4 p = pos[blockIdx.x * kPartThreads];  // an atom of this block: neutral for min / max
-    for (int k = 0; k < 3; ++k) {
-      v[k] = v[3 + k] = (&p.x)[k];
-      v[6 + k] = 0.0;
-    }
-    v[9] = 0.0;
-  }
-  for (int k = 0; k < 10; ++k) s[k][t] = v[k];
-  __syncthreads();
-  for (int stride = kPartThreads / 2; stride > 0; stride >>= 1) {
-    if (t < stride) {
-      for (int k = 0; k < 3; ++k) {
-        s[k][t] = fmin(s[k][t], s[k][t + stride]);
-        s[3 + k][t] = fmax(s[3 + k][t], s[3 + k][t + stride]);
-        s[6 + k][t] = dadd(s[6 + k][t], s[6 + k][t + stride]);
-      }
-      s[9][t] = fmax(s[9][t], s[9][t + stride]);
-    }
-    __syncthreads();
-  }
-  if (t == 0) {
-    GeomPart g;
-    for (int k = 0; k < 3; ++k) {
-      g.mn[k] = s[k][0];
-      g.mx[k] = s[3 + k][0];
-      g.sum[k] = s[6 + k][0];
-    }
-    g.rmax = s[9][0];
-    parts[blockIdx.x] = g;
-  }
-}
-
-// CharmmReferenceGBSW.cpp:444-466, CustomGBIntegral.cpp:53-113,163-193: the
-// grid from the partial extents (combined in block order).
-__global__ void __launch_bounds__(kGeomThreads) table_geom_kernel(const GeomPart* __restrict__ parts, int nparts,
-                                                                  int n, int mode, double h, double buffer,
-                                                                  double sw, double bx, double by, double bz,
-                                                                  TableGeom* __restrict__ g, long long cell_cap,
-                                                                  unsigned* __restrict__ status) {
-  __shared__ double s[10][kGeomThreads];
-  const int t = threadIdx.x;
-  double v[10];
-  const GeomPart p0 = parts[0];
-  for (int k = 0; k < 3; ++k) {
-    v[k] = p0.mn[k];
-    v[3 + k] = p0.mx[k];
-    v[6 + k] = 0.0;
-  }
-  v[9] = 0.0;
-  for (int b = t; b < nparts; b += kGeomThreads) {  // each thread's parts in block order
-    const GeomPart p = parts[b];
-    for (int k = 0; k < 3; ++k) {
-      v[k] = fmin(v[k], p.mn[k]);
-      v[3 + k] = fmax(v[3 + k], p.mx[k]);
-      v[6 + k] = dadd(v[6 + k], p.sum[k]);
-    }
-    v[9] = fmax(v[9], p.rmax);
-  }
-  for (int k = 0; k < 10; ++k) s[k][t] = v[k];
-  __syncthreads();
-  for (int stride = kGeomThreads / 2; stride > 0; stride >>= 1) {
-    if (t < stride) {
-      for (int k = 0; k < 3; ++k) {
-        s[k][t] = fmin(s[k][t], s[k][t + stride]);
-        s[3 + k][t] = fmax(s[3 + k][t], s[3 + k][t + stride]);
-        s[6 + k][t] = dadd(s[6 + k][t], s[6 + k][t + stride]);
-      }
-      s[9][t] = fmax(s[9][t], s[9][t + stride]);
-    }
-    __syncthreads();
-  }
-  if (t != 0) return;
-  double mn[3], mx[3], sm[3];
-  for (int k = 0; k < 3; ++k) {
-    mn[k] = s[k][0];
-    mx[k] = s[3 + k][0];
-    sm[k] = s[6 + k][0];
-  }
-  const double rmax = s[9][0];
-  TableGeom G;
-  G.mode = mode;
-  G.total = 0;
-  G.L = h;
-  long long ncell = 1;
-  if (mode == GBX_TABLE_STANDALONE || mode == GBX_TABLE_GRID) {
-    double pad;
-    if (mode == GBX_TABLE_STANDALONE)
-      pad = dadd(dadd(dadd(dadd(buffer, rmax), sw), dmul(half_sqrt3(), h)), 1e-6);
-    else
-      pad = dadd(dadd(0.03, dmul(half_sqrt3(), h)), buffer);
-    G.pad = pad;
-    for (int k = 0; k < 3; ++k) {
-      double lo = dsub(mn[k], pad), hi = dadd(mx[k], pad);
-      double length = dsub(hi, lo);
-      if (mode == GBX_TABLE_GRID && length > 1000.0) {
-        atomicOr(status, kStatusTableCells);
-        G.dims[k] = 1;
-      } else {
-        G.dims[k] = (int)ceil(ddiv(length, h)) + 1;
-      }
-      G.min[k] = lo;
-      G.max[k] = dadd(lo, dmul((double)(G.dims[k] - 1), h));
-      G.step[k] = h;
-      G.box[k] = k == 0 ? bx : (k == 1 ? by : bz);  // read only by a periodic system's wrapped query
-      ncell *= G.dims[k];
-    }
-  } else {
-    double box[3] = {bx, by, bz};
-    double cog[3];
-    for (int k = 0; k < 3; ++k) cog[k] = ddiv(sm[k], (double)n);
-    double L = 0.0;
-    for (int k = 0; k < 3; ++k) {
-      double d = box[k];
-      G.box[k] = d;
-      G.min[k] = dsub(cog[k], ddiv(d, 2.0));
-      G.max[k] = dadd(cog[k], ddiv(d, 2.0));
-      G.dims[k] = (int)ceil(ddiv(d, h)) + 1;
-      G.step[k] = ddiv(d, (double)G.dims[k]);
-      ncell *= G.dims[k];
-    }
-    L = fmax(fmax(G.step[0], G.step[1]), G.step[2]);
-    G.L = L;
-    G.pad = 0.0;
-  }
-  for (int k = 0; k < 3; ++k) {
-    G.inv_step[k] = 1.0 / G.step[k];
-    G.inv_box[k] = G.box[k] > 0.0 ? 1.0 / G.box[k] : 0.0;
-  }
-  G.ncell = ncell;
-  if (ncell > cell_cap) atomicOr(status, kStatusTableCells);
-  *g = G;
-}
 
 // --------------------------------------------------------------------------
 // Membership enumeration (count / fill)
@@ -438,11 +276,6 @@ __global__ void denormalize_kernel(const int* __restrict__ entries, const TableG
 
 }  // namespace
 
-// Scratch the geometry pass needs: one GeomPart per 256 atoms, in doubles.
-size_t table_geom_scratch_doubles(int n) {
-  return ((size_t)(n + kPartThreads - 1) / kPartThreads) * (sizeof(GeomPart) / sizeof(double));
-}
-
 namespace {
 
 int grid_for(long long work, int per_block) {
@@ -454,48 +287,19 @@ int grid_for(long long work, int per_block) {
 
 }  // namespace
 
-void launch_standalone_geom(Context* ctx, const float4* pos, TableGeom* out) {
-  const gbx_config& c = ctx->cfg;
-  cudaStream_t st = ctx->stream;
-  const int nparts = (ctx->n + kPartThreads - 1) / kPartThreads;
-  GeomPart* parts = reinterpret_cast<GeomPart*>(ctx->d_reduce);
-  table_geom_partial_kernel<<<nparts, kPartThreads, 0, st>>>(pos, ctx->d_radius, ctx->n, parts);
-  // no cell of this grid is ever allocated or indexed: no capacity to check
-  table_geom_kernel<<<1, kGeomThreads, 0, st>>>(parts, nparts, ctx->n, GBX_TABLE_STANDALONE, c.grid_length,
-                                                c.table_buffer, c.switch_width, c.box[0], c.box[1], c.box[2], out,
-                                                0x7fffffffffffffffLL, ctx->d_status);
-  ctx->launches += 2;
-}
-
 gbx_status launch_table_build(Context* ctx, const float4* pos) {
   const gbx_config& c = ctx->cfg;
   cudaStream_t st = ctx->stream;
-  const int nparts = (ctx->n + kPartThreads - 1) / kPartThreads;
-  GeomPart* parts = reinterpret_cast<GeomPart*>(ctx->d_reduce);
-  table_geom_partial_kernel<<<nparts, kPartThreads, 0, st>>>(pos, ctx->d_radius, ctx->n, parts);
-  table_geom_kernel<<<1, kGeomThreads, 0, st>>>(parts, nparts, ctx->n, c.table_mode, c.grid_length, c.table_buffer,
-                                                c.switch_width, c.box[0], c.box[1], c.box[2], ctx->d_geom,
-                                                ctx->cell_cap, ctx->d_status);
-  ctx->launches += 2;
   const long long cells = ctx->cell_cap;
-  if (cells == 0) {
-    // sizing call: geometry only; the caller reads it back and allocates
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) {
-      ctx->last_error = std::string("table geometry launch: ") + cudaGetErrorString(e);
-      return GBX_ERR_CUDA;
-    }
-    return GBX_OK;
-  }
-  cudaMemsetAsync(ctx->d_cell_count, 0, sizeof(int) * cells, st);
+  if (cells == 0) return GBX_OK;  // sizing call: the grid alone; the caller reads it back and allocates
   Emit em{ctx->d_cell_count, ctx->d_cell_start, ctx->d_cell_cursor, ctx->d_entries, ctx->entry_cap, ctx->d_status};
   const int threads = 256;
   const int blocks = grid_for((long long)ctx->n * kWarp, threads);
   for (int pass = 0; pass < 2; ++pass) {
     if (pass == 1) {
-      launch_scan(ctx->d_cell_count, ctx->d_geom, ctx->d_block_sums, ctx->d_cell_start, ctx->d_cell_cursor, cells,
-                  ctx->entry_cap, ctx->d_status, st);
-      ctx->launches += 3;  // the scan's three kernels
+      launch_scan(ctx->d_cell_count, ctx->d_geom, ctx->d_cell_start, ctx->d_cell_cursor, cells, ctx->entry_cap,
+                  reinterpret_cast<unsigned long long*>(&ctx->d_geom->total), ctx->d_status, st);
+      ++ctx->launches;
     }
     const bool fill = pass == 1;
     switch (c.table_mode) {

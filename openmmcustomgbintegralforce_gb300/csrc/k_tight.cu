@@ -29,82 +29,10 @@
 namespace gbx {
 namespace {
 
-constexpr int kGeomThreads = 1024;
 constexpr int kSortWarps = 4;
 constexpr int kSortBuf = 256;
 constexpr int kSortLanes = 8;                                   // lanes per short list
 constexpr int kSortSmall = kSortBuf / (kWarp / kSortLanes);     // longest short list (64)
-
-__global__ void __launch_bounds__(kGeomThreads) tight_geom_kernel(const float4* __restrict__ pos, int n, double h,
-                                                                  double w, double extent, TableGeom* __restrict__ g,
-                                                                  long long cell_cap, unsigned* __restrict__ status) {
-  __shared__ float s_min[3][kGeomThreads / kWarp], s_max[3][kGeomThreads / kWarp], s_r[kGeomThreads / kWarp];
-  const int t = threadIdx.x;
-  float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY}, rmax = 0.f;
-  for (int a = t; a < n; a += blockDim.x) {
-    const float4 p = pos[a];
-    mn[0] = fminf(mn[0], p.x);
-    mn[1] = fminf(mn[1], p.y);
-    mn[2] = fminf(mn[2], p.z);
-    mx[0] = fmaxf(mx[0], p.x);
-    mx[1] = fmaxf(mx[1], p.y);
-    mx[2] = fmaxf(mx[2], p.z);
-    rmax = fmaxf(rmax, p.w);
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    for (int k = 0; k < 3; ++k) {
-      mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], off));
-      mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], off));
-    }
-    rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
-  }
-  if (t % kWarp == 0) {
-    for (int k = 0; k < 3; ++k) {
-      s_min[k][t / kWarp] = mn[k];
-      s_max[k][t / kWarp] = mx[k];
-    }
-    s_r[t / kWarp] = rmax;
-  }
-  __syncthreads();
-  if (t != 0) return;
-  for (int ww = 0; ww < kGeomThreads / kWarp; ++ww) {
-    for (int k = 0; k < 3; ++k) {
-      mn[k] = fminf(mn[k], s_min[k][ww]);
-      mx[k] = fmaxf(mx[k], s_max[k][ww]);
-    }
-    rmax = fmaxf(rmax, s_r[ww]);
-  }
-  TableGeom G;
-  const double margin = (double)rmax + w + h;
-  long long ncell = 1;
-  double amax = 0.0;
-  for (int k = 0; k < 3; ++k) {
-    G.min[k] = (double)mn[k] - margin;
-    G.dims[k] = (int)ceil(((double)mx[k] - (double)mn[k] + 2.0 * margin) / h) + 1;
-    if (!(G.dims[k] >= 1 && G.dims[k] <= 65536)) {
-      atomicOr(status, kStatusTableCells);
-      G.dims[k] = 1;
-    }
-    G.max[k] = G.min[k] + G.dims[k] * h;
-    G.step[k] = h;
-    G.box[k] = 0.0;
-    ncell *= G.dims[k];
-    amax = fmax(amax, fmax(fabs((double)mn[k]), fabs((double)mx[k])));
-  }
-  G.mode = -1;
-  G.L = h;
-  // membership margin: FP32 rounding of cell coordinates and distances
-  // (extent: a periodic system's longest box edge, by which a point may be moved)
-  G.pad = 2e-5 + 4.0 * 1.1920929e-7 * (amax + 2.0 * margin + extent);
-  G.total = 0;
-  for (int k = 0; k < 3; ++k) {
-    G.inv_step[k] = 1.0 / h;
-    G.inv_box[k] = 0.0;
-  }
-  G.ncell = ncell;
-  if (ncell > cell_cap) atomicOr(status, kStatusTableCells);
-  *g = G;
-}
 
 struct TightArgs {
   const float4* pos;  // x, y, z, R'
@@ -320,17 +248,8 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
 
 gbx_status launch_tight_build(Context* ctx, const float4* pos) {
   cudaStream_t st = ctx->stream;
-  const double h = ctx->tight_h;
-  const gbx_config& c = ctx->cfg;
-  const double extent = c.periodic ? fmax(c.box[0], fmax(c.box[1], c.box[2])) : 0.0;
-  if (c.periodic) launch_standalone_geom(ctx, pos, ctx->d_wgeom);
-  tight_geom_kernel<<<1, kGeomThreads, 0, st>>>(pos, ctx->n, h, c.switch_width, extent, ctx->d_tgeom, ctx->tcell_cap,
-                                                ctx->d_status);
-  ++ctx->launches;
   const long long cells = ctx->tcell_cap;
   if (cells > 0) {
-    cudaMemsetAsync(ctx->d_tcount, 0, sizeof(int) * cells, st);
-    cudaMemsetAsync(ctx->d_tburied, 0, sizeof(int) * cells, st);
     TightArgs a{pos,           ctx->n,          ctx->d_tgeom,   (float)ctx->cfg.switch_width,
                 ctx->d_tcount, ctx->d_tstart,   ctx->d_tcursor, ctx->d_tburied,
                 ctx->d_tentry, ctx->d_tindex,   cells,          ctx->tentry_cap,
@@ -340,9 +259,9 @@ gbx_status launch_tight_build(Context* ctx, const float4* pos) {
     if (blocks > 65535) blocks = 65535;
     tight_members_kernel<false><<<(int)blocks, threads, 0, st>>>(a);
     ++ctx->launches;
-    launch_scan<true>(ctx->d_tcount, ctx->d_tgeom, ctx->d_tblock_sums, ctx->d_tstart, ctx->d_tcursor, cells,
-                ctx->tentry_cap, ctx->d_status, st);
-    ctx->launches += 3;  // the scan's three kernels
+    launch_scan<true>(ctx->d_tcount, ctx->d_tgeom, ctx->d_tstart, ctx->d_tcursor, cells, ctx->tentry_cap,
+                      reinterpret_cast<unsigned long long*>(&ctx->d_tgeom->total), ctx->d_status, st);
+    ++ctx->launches;
     tight_members_kernel<true><<<(int)blocks, threads, 0, st>>>(a);
     ++ctx->launches;
     long long sb = (cells + kSortWarps * kWarp - 1) / (kSortWarps * kWarp);

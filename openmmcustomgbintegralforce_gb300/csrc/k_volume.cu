@@ -1099,7 +1099,6 @@ void launch_integrals_t(Context* ctx, const float4* pos, const ModelConst& m, bo
       ctx->integral_grid = per_sm * ctx->sms;
     }
     const int grid = std::min(volume_blocks(ctx), ctx->integral_grid);
-    cudaMemsetAsync(ctx->d_next_item, 0, sizeof(unsigned), ctx->stream);
     auto kernel = !ctx->records       ? gbsw_integral_kernel<Q, kEmitNone>
                   : ctx->records_self ? gbsw_integral_kernel<Q, kEmitAll>
                                       : gbsw_integral_kernel<Q, kEmitOthers>;
