@@ -41,6 +41,7 @@
 // FP32 difference is within a few tenths of a nanometre of the cell.
 #include <math.h>
 
+#include "bitonic.cuh"
 #include "gbx_internal.cuh"
 #include "queries.cuh"
 #include "scan.cuh"
@@ -217,38 +218,6 @@ __global__ void gbmv_fill_kernel(long long npts, CellPoints cp) {
   if (p >= npts) return;
   const int c = cp.cell[p];
   if (c >= 0) cp.order[cp.start[c] + cp.rank[p]] = (int)p;
-}
-
-// Bitonic sort of 32 E keys held E per lane, element lane E + r in key[r].
-template <int E>
-__device__ __forceinline__ void warp_bitonic_sort(int (&key)[E], int lane) {
-#pragma unroll
-  for (int k = 2; k <= kWarp * E; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j < E) {
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-          const int rp = r ^ j;
-          if (rp > r) {
-            const bool up = ((lane * E + r) & k) == 0;
-            const int a = key[r], b = key[rp];
-            key[r] = up ? min(a, b) : max(a, b);
-            key[rp] = up ? max(a, b) : min(a, b);
-          }
-        }
-      } else {
-        const int lj = j / E;
-        const bool lower = (lane & lj) == 0;
-#pragma unroll
-        for (int r = 0; r < E; ++r) {
-          const bool up = ((lane * E + r) & k) == 0;
-          const int o = __shfl_xor_sync(0xffffffffu, key[r], lj);
-          key[r] = (up == lower) ? min(key[r], o) : max(key[r], o);
-        }
-      }
-    }
-  }
 }
 
 template <int E>

@@ -7,21 +7,25 @@
 //             and counts members with atomics;
 //   scan      counts -> list starts;
 //   fill      second enumeration writes members at atomic cursors;
-//   sort      one warp per cell ranks its entries, restoring the reference's
-//             ascending-atom insertion order, then applies the per-cell cap.
+//   sort      one warp per cell sorts its entries, restoring the reference's
+//             ascending-atom insertion order, applies the per-cell cap and
+//             writes the atoms' positions and parameters inline.
 //
 // Every FP64 operation that decides membership is written with explicit
 // round-to-nearest intrinsics so that no multiply-add is contracted: the
 // decisions match the reference's separately rounded C++ arithmetic.
 #include <math.h>
 
+#include "bitonic.cuh"
 #include "gbx_internal.cuh"
 #include "scan.cuh"
 
 namespace gbx {
 namespace {
 
-constexpr int kMaxSamples = 96;  // samples per axis in the periodic branch
+constexpr int kMaxSamples = 96;  // grid values or samples per axis kept in shared memory
+constexpr int kMemberThreads = 256;
+constexpr int kMemberWarps = kMemberThreads / kWarp;
 
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
@@ -56,49 +60,102 @@ struct Emit {
   }
 };
 
+// Column `col` of an axis-0 x axis-1 rectangle of n1 columns per row, by FP32
+// division (exact for the at most 2^20 columns an atom reaches).
+__device__ __forceinline__ int2 column(int col, int n1, float inv_n1) {
+  int i = (int)(((float)col + 0.5f) * inv_n1);
+  i -= i * n1 > col;
+  return make_int2(i, col - i * n1);
+}
+
 // CharmmReferenceGBSW.cpp:472-496 (STANDALONE) and CustomGBIntegral.cpp:198-227 (GRID).
+// A warp per atom, a lane per column of grid points.  The offset from the atom
+// depends on one axis only, so each axis value's is formed once, in the
+// reference's FP64; the membership of a point is decided by the FP32 sum of
+// their squares wherever that is clear of the boundary by a margin that covers
+// its rounding, and by the reference's FP64 operations otherwise (FP64 for
+// every point took 98 us of a count pass at 6,007 atoms).
 template <int MODE, bool FILL>
 __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const double* __restrict__ radius, int n,
                                           const TableGeom* __restrict__ gp, double h, double buffer, Emit em,
                                           long long cell_cap) {
+  __shared__ double s_d[kMemberWarps][3][kMaxSamples];
+  __shared__ float s_sq[kMemberWarps][3][kMaxSamples];
+  const int wib = threadIdx.x / kWarp;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   const int lane = threadIdx.x % kWarp;
   const TableGeom& g = *gp;
   if (g.ncell > cell_cap) return;
   const long long ncell = g.ncell;
+  const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
+  double (*ds)[kMaxSamples] = s_d[wib];
+  float (*sq)[kMaxSamples] = s_sq[wib];
   for (int a = warp; a < n; a += (gridDim.x * blockDim.x) / kWarp) {
-    float4 p = pos[a];
-    const double c[3] = {(double)p.x, (double)p.y, (double)p.z};
+    const float4 p = pos[a];
     double pad;
     if (MODE == GBX_TABLE_STANDALONE) pad = g.pad;
     else pad = dadd(dadd(radius[a], dmul(half_sqrt3(), h)), buffer);
     const double pad2 = dmul(pad, pad);
-    int b[3], e[3];
-    for (int k = 0; k < 3; ++k) {
-      b[k] = (int)floor(ddiv(dsub(dsub(c[k], pad), g.min[k]), h));
-      e[k] = (int)ceil(ddiv(dsub(dadd(c[k], pad), g.min[k]), h));
+    int b_ = 0, n_ = 0;
+    if (lane < 3) {  // an axis per lane
+      const double c = lane == 0 ? p.x : (lane == 1 ? p.y : p.z);
+      b_ = (int)floor(ddiv(dsub(dsub(c, pad), g.min[lane]), h));
+      n_ = (int)ceil(ddiv(dsub(dadd(c, pad), g.min[lane]), h)) - b_ + 1;
     }
-    const int nx = e[0] - b[0] + 1, ny = e[1] - b[1] + 1, nz = e[2] - b[2] + 1;
+    int b[3], nn[3];
+    bool ok = true, fits = true;
+    for (int k = 0; k < 3; ++k) {
+      b[k] = __shfl_sync(0xffffffffu, b_, k);
+      nn[k] = __shfl_sync(0xffffffffu, n_, k);
+      ok = ok && nn[k] >= 1 && nn[k] <= 1024;
+      fits = fits && nn[k] <= kMaxSamples;
+    }
     // non-finite or absurd inputs: skip the atom instead of looping on garbage bounds
-    if (!(nx >= 1 && ny >= 1 && nz >= 1 && nx <= 1024 && ny <= 1024 && nz <= 1024)) {
+    if (!ok) {
       if (lane == 0) atomicOr(em.status, kStatusTableCells);
       continue;
     }
-    const int total = nx * ny * nz;
-    const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
-    for (int t = lane; t < total; t += kWarp) {
-      const int i = b[0] + t / (ny * nz);
-      const int j = b[1] + (t / nz) % ny;
-      const int k = b[2] + t % nz;
-      const double d0 = dsub(dadd(g.min[0], dmul((double)i, h)), c[0]);
-      const double d1 = dsub(dadd(g.min[1], dmul((double)j, h)), c[1]);
-      const double d2 = dsub(dadd(g.min[2], dmul((double)k, h)), c[2]);
+    // the reference's offset of grid value m of axis k from the atom, and its test of a sum of squares
+    auto offset = [&](int k, int m) {
+      return dsub(dadd(g.min[k], dmul((double)(b[k] + m), h)), (double)(k == 0 ? p.x : (k == 1 ? p.y : p.z)));
+    };
+    auto inside = [&](double d0, double d1, double d2) {
       const double s = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
-      bool member;
-      if (MODE == GBX_TABLE_STANDALONE) member = __dsqrt_rn(s) < pad;
-      else member = s < pad2;
-      if (member) em.put<FILL>((long long)i * sx + (long long)j * sy + k, a, ncell);
+      return MODE == GBX_TABLE_STANDALONE ? __dsqrt_rn(s) < pad : s < pad2;
+    };
+    const int cols = nn[0] * nn[1];
+    const float inv_n1 = 1.0f / (float)nn[1];
+    if (!fits) {  // a grid finer than a hundredth of the pad: FP64 throughout
+      for (int col = lane; col < cols; col += kWarp) {
+        const int2 ij = column(col, nn[1], inv_n1);
+        const double d0 = offset(0, ij.x), d1 = offset(1, ij.y);
+        for (int k = 0; k < nn[2]; ++k)
+          if (inside(d0, d1, offset(2, k)))
+            em.put<FILL>((long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2] + k, a, ncell);
+      }
+      continue;
     }
+    for (int t = lane; t < nn[0] + nn[1] + nn[2]; t += kWarp) {
+      const int k = t < nn[0] ? 0 : (t < nn[0] + nn[1] ? 1 : 2);
+      const int m = t - (k == 0 ? 0 : (k == 1 ? nn[0] : nn[0] + nn[1]));
+      const double d = offset(k, m);
+      ds[k][m] = d;
+      sq[k][m] = (float)d * (float)d;
+    }
+    __syncwarp();
+    // FP32 squared distances carry a relative error below 4 2^-24
+    const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
+    for (int col = lane; col < cols; col += kWarp) {
+      const int2 ij = column(col, nn[1], inv_n1);
+      const float sxy = sq[0][ij.x] + sq[1][ij.y];
+      if (sxy > out2) continue;
+      const long long row = (long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2];
+      for (int k = 0; k < nn[2]; ++k) {
+        const float s = sxy + sq[2][k];
+        if (s < in2 || (s <= out2 && inside(ds[0][ij.x], ds[1][ij.y], ds[2][k]))) em.put<FILL>(row + k, a, ncell);
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -115,9 +172,9 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
   // per warp and axis: the samples, their cell index (-1 outside) and the
   // squared offset from the atom in FP32 -- each depends on one axis only,
   // so it is computed once per axis value
-  __shared__ double s_samp[8][3][kMaxSamples];
-  __shared__ float s_sq[8][3][kMaxSamples];
-  __shared__ int s_id[8][3][kMaxSamples];
+  __shared__ double s_samp[kMemberWarps][3][kMaxSamples];
+  __shared__ float s_sq[kMemberWarps][3][kMaxSamples];
+  __shared__ int s_id[kMemberWarps][3][kMaxSamples];
   const int wib = threadIdx.x / kWarp;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   const int lane = threadIdx.x % kWarp;
@@ -178,55 +235,95 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
       sq[k][m] = e * e;
     }
     __syncwarp();
-    const int total = cnt[0] * cnt[1] * cnt[2];
+    const int cols = cnt[0] * cnt[1];
+    const float inv_n1 = 1.0f / (float)cnt[1];
     const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
     // FP32 squared distances carry a relative error below 4 2^-24
     const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
-    for (int t = lane; t < total; t += kWarp) {
-      const int kx = t / (cnt[1] * cnt[2]);
-      const int ky = (t / cnt[2]) % cnt[1];
-      const int kz = t % cnt[2];
-      const int i0 = idx[0][kx], i1 = idx[1][ky], i2 = idx[2][kz];
-      if (i0 < 0 || i1 < 0 || i2 < 0) continue;
-      const float sf = (sq[0][kx] + sq[1][ky]) + sq[2][kz];
-      bool member = sf < in2;
-      if (!member && sf <= out2) {
-        // the reference's FP64 test
-        const double e0 = dsub(samp[0][kx], c[0]), e1 = dsub(samp[1][ky], c[1]), e2 = dsub(samp[2][kz], c[2]);
-        member = dadd(dadd(dmul(e0, e0), dmul(e1, e1)), dmul(e2, e2)) < pad2;
+    for (int col = lane; col < cols; col += kWarp) {  // a lane per column of samples
+      const int2 ij = column(col, cnt[1], inv_n1);
+      const int i0 = idx[0][ij.x], i1 = idx[1][ij.y];
+      const float sxy = sq[0][ij.x] + sq[1][ij.y];
+      if (i0 < 0 || i1 < 0 || sxy > out2) continue;
+      const long long row = (long long)i0 * sx + (long long)i1 * sy;
+      for (int kz = 0; kz < cnt[2]; ++kz) {
+        const float sf = sxy + sq[2][kz];
+        bool member = sf < in2;
+        if (!member && sf <= out2) {
+          // the reference's FP64 test
+          const double e0 = dsub(samp[0][ij.x], c[0]), e1 = dsub(samp[1][ij.y], c[1]), e2 = dsub(samp[2][kz], c[2]);
+          member = dadd(dadd(dmul(e0, e0), dmul(e1, e1)), dmul(e2, e2)) < pad2;
+        }
+        const int i2 = idx[2][kz];
+        if (member && i2 >= 0) em.put<FILL>(row + i2, a, ncell);
       }
-      if (member) em.put<FILL>((long long)i0 * sx + (long long)i1 * sy + i2, a, ncell);
     }
     __syncwarp();
   }
 }
 
 // --------------------------------------------------------------------------
-// Per-cell rank sort (ascending atom index) and cap.
+// Per-cell sort (ascending atom index) and cap, and inline copies of each
+// listed atom's position and parameters, so the volume kernels stream a
+// cell's list without a dependent gather.
 // --------------------------------------------------------------------------
 constexpr int kSortWarps = 4;
-constexpr int kSortBuf = 512;  // per-warp shared staging; longer lists rank from global
+
+struct Inline {
+  const float4* pos;
+  const float2* par;
+  float4* entry4;
+  float2* entry_par;
+  __device__ __forceinline__ void put(long long e, int atom) const {
+    entry4[e] = __ldg(pos + atom);
+    entry_par[e] = __ldg(par + atom);
+  }
+};
+
+// Lists of up to 32 E entries, in registers.
+template <int E>
+__device__ __forceinline__ void sort_list(int* __restrict__ entries, const Inline& in, long long s, int cnt, int kept,
+                                          int lane) {
+  int key[E];
+#pragma unroll
+  for (int r = 0; r < E; ++r) {
+    const int e = lane * E + r;
+    key[r] = e < cnt ? entries[s + e] : 0x7fffffff;
+  }
+  warp_bitonic_sort<E>(key, lane);
+#pragma unroll
+  for (int r = 0; r < E; ++r) {
+    const int e = lane * E + r;
+    if (e < cnt) entries[s + e] = key[r];
+    if (e < kept) in.put(s + e, key[r]);
+  }
+}
 
 __global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(int* __restrict__ count,
                                                                         const int* __restrict__ start,
                                                                         int* __restrict__ entries,
-                                                                        int2* __restrict__ cell,
+                                                                        int2* __restrict__ cell, Inline in,
                                                                         const TableGeom* __restrict__ gp, int cap,
                                                                         long long cell_cap, long long entry_cap,
                                                                         unsigned* __restrict__ status) {
-  __shared__ int s_buf[kSortWarps][kSortBuf];
   const int wib = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
   const long long ncell = gp->ncell <= cell_cap ? gp->ncell : 0;
   if (gp->total > entry_cap) return;
-  int* buf = s_buf[wib];
   for (long long c = (long long)blockIdx.x * kSortWarps + wib; c < ncell; c += (long long)gridDim.x * kSortWarps) {
     const int cnt = count[c];
     const int s = start[c];
-    if (lane == 0) cell[c] = make_int2(cap > 0 && cnt > cap ? cap : cnt, s);
+    const int kept = cap > 0 && cnt > cap ? cap : cnt;
+    if (lane == 0) cell[c] = make_int2(kept, s);
     if (cnt == 0) continue;
-    if (cnt > kSortBuf) {
-      if (cnt > kMaxSortSegment && lane == 0) atomicOr(status, kStatusSegmentTooLong);
-      if (cnt > kMaxSortSegment) continue;
+    if (cnt <= kWarp) sort_list<1>(entries, in, s, cnt, kept, lane);
+    else if (cnt <= 2 * kWarp) sort_list<2>(entries, in, s, cnt, kept, lane);
+    else if (cnt <= 4 * kWarp) sort_list<4>(entries, in, s, cnt, kept, lane);
+    else if (cnt <= 8 * kWarp) sort_list<8>(entries, in, s, cnt, kept, lane);
+    else if (cnt <= 16 * kWarp) sort_list<16>(entries, in, s, cnt, kept, lane);
+    else if (cnt > kMaxSortSegment) {
+      if (lane == 0) atomicOr(status, kStatusSegmentTooLong);
+      continue;
+    } else {
       // long list: ranks from global memory, results staged per lane
       int vals[kMaxSortSegment / kWarp], ranks[kMaxSortSegment / kWarp];
       int m = 0;
@@ -241,36 +338,13 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(int* __r
         ranks[m] = r;
       }
       __syncwarp();
-      for (int k = 0; k < m; ++k) entries[s + ranks[k]] = vals[k];
-    } else {
-      for (int p = lane; p < cnt; p += kWarp) buf[p] = entries[s + p];
-      __syncwarp();
-      for (int p = lane; p < cnt; p += kWarp) {
-        const int v = buf[p];
-        int r = 0;
-        for (int q = 0; q < cnt; ++q) {
-          const int u = buf[q];
-          r += (u < v) || (u == v && q < p);
-        }
-        entries[s + r] = v;
+      for (int k = 0; k < m; ++k) {
+        entries[s + ranks[k]] = vals[k];
+        if (ranks[k] < kept) in.put(s + ranks[k], vals[k]);
       }
     }
     __syncwarp();
-    if (lane == 0 && cap > 0 && cnt > cap) count[c] = cap;
-  }
-}
-
-// Inline copies of each listed atom's position and parameters, so the
-// volume kernels stream a cell's list without a dependent gather.
-__global__ void denormalize_kernel(const int* __restrict__ entries, const TableGeom* __restrict__ gp,
-                                   const float4* __restrict__ pos, const float2* __restrict__ par,
-                                   float4* __restrict__ entry4, float2* __restrict__ entry_par, long long entry_cap) {
-  const long long total = gp->total <= entry_cap ? gp->total : 0;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int j = entries[e];
-    entry4[e] = pos[j];
-    entry_par[e] = par[j];
+    if (lane == 0 && kept < cnt) count[c] = kept;
   }
 }
 
@@ -293,7 +367,7 @@ gbx_status launch_table_build(Context* ctx, const float4* pos) {
   const long long cells = ctx->cell_cap;
   if (cells == 0) return GBX_OK;  // sizing call: the grid alone; the caller reads it back and allocates
   Emit em{ctx->d_cell_count, ctx->d_cell_start, ctx->d_cell_cursor, ctx->d_entries, ctx->entry_cap, ctx->d_status};
-  const int threads = 256;
+  const int threads = kMemberThreads;
   const int blocks = grid_for((long long)ctx->n * kWarp, threads);
   for (int pass = 0; pass < 2; ++pass) {
     if (pass == 1) {
@@ -330,12 +404,10 @@ gbx_status launch_table_build(Context* ctx, const float4* pos) {
     }
     ++ctx->launches;
   }
+  const Inline in{pos, ctx->d_par, ctx->d_entry4, ctx->d_entry_par};
   sort_cells_kernel<<<grid_for(cells, kSortWarps), kSortWarps * kWarp, 0, st>>>(
-      ctx->d_cell_count, ctx->d_cell_start, ctx->d_entries, ctx->d_cell2, ctx->d_geom, c.table_cap, cells, ctx->entry_cap,
-      ctx->d_status);
-  ++ctx->launches;
-  denormalize_kernel<<<grid_for(ctx->entry_cap, 256), 256, 0, st>>>(ctx->d_entries, ctx->d_geom, pos, ctx->d_par,
-                                                                    ctx->d_entry4, ctx->d_entry_par, ctx->entry_cap);
+      ctx->d_cell_count, ctx->d_cell_start, ctx->d_entries, ctx->d_cell2, in, ctx->d_geom, c.table_cap, cells,
+      ctx->entry_cap, ctx->d_status);
   ++ctx->launches;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

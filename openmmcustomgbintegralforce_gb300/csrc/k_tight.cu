@@ -32,7 +32,8 @@ namespace {
 constexpr int kSortWarps = 4;
 constexpr int kSortBuf = 256;
 constexpr int kSortLanes = 8;                                   // lanes per short list
-constexpr int kSortSmall = kSortBuf / (kWarp / kSortLanes);     // longest short list (64)
+constexpr int kSortGroups = kWarp / kSortLanes;
+constexpr int kSortSmall = kSortBuf / kSortGroups;              // longest short list (64)
 
 struct TightArgs {
   const float4* pos;  // x, y, z, R'
@@ -80,31 +81,48 @@ __global__ void tight_members_kernel(TightArgs a) {
       if (lane == 0) atomicOr(a.status, kStatusTableCells);
       continue;
     }
-    const int ny = e[1] - b[1] + 1, nz = e[2] - b[2] + 1;
-    const int total = (e[0] - b[0] + 1) * ny * nz;
-    for (int t = lane; t < total; t += kWarp) {
-      const int c[3] = {b[0] + t / (ny * nz), b[1] + (t / nz) % ny, b[2] + t % nz};
-      float near2 = 0.f, far2 = 0.f;
-      for (int k = 0; k < 3; ++k) {
-        const float lo = c[k] * h, hi = lo + h;
-        const float dn = fmaxf(fmaxf(lo - x[k], x[k] - hi), 0.f);
-        const float df = fmaxf(x[k] - lo, hi - x[k]);
-        near2 = fmaf(dn, dn, near2);
-        far2 = fmaf(df, df, far2);
+    // the offsets of cell c's lower and upper face along one axis, every
+    // operation rounded on its own: the count and the fill pass, compiled
+    // apart, must decide alike
+    auto faces = [h](int c, float at) {
+      const float lo = __fmul_rn((float)c, h);
+      return make_float2(__fsub_rn(lo, at), __fsub_rn(__fadd_rn(lo, h), at));
+    };
+    // a lane per column of cells
+    const int ny = e[1] - b[1] + 1, cols = (e[0] - b[0] + 1) * ny;
+    const float inv_ny = 1.0f / (float)ny;
+    for (int col = lane; col < cols; col += kWarp) {
+      int cx = (int)(((float)col + 0.5f) * inv_ny);
+      cx -= cx * ny > col;
+      const int c[2] = {b[0] + cx, b[1] + col - cx * ny};
+      float near_xy = 0.f, far_xy = 0.f;
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float2 f = faces(c[k], x[k]);
+        const float dn = fmaxf(fmaxf(f.x, -f.y), 0.f), df = fmaxf(-f.x, f.y);
+        near_xy = fmaf(dn, dn, near_xy);
+        far_xy = fmaf(df, df, far_xy);
       }
-      if (!(near2 < reach * reach)) continue;
-      const long long cell = c[0] * sx + c[1] * sy + c[2];
-      if (!FILL) {
-        atomicAdd(&a.count[cell], 1);
-        if (bury > 0.f && far2 <= bury * bury) atomicOr(&a.buried[cell], 1);
-      } else {
-        const int slot = atomicAdd(&a.cursor[cell], 1);
-        const long long o = (long long)a.start[cell] + slot;
-        if (o < a.entry_cap) {
-          a.entry[o] = p;
-          a.index[o] = at;
+      if (!(near_xy < reach * reach)) continue;
+      const long long row = c[0] * sx + c[1] * sy;
+      for (int cz = b[2]; cz <= e[2]; ++cz) {
+        const float2 f = faces(cz, x[2]);
+        const float dn = fmaxf(fmaxf(f.x, -f.y), 0.f);
+        if (!(fmaf(dn, dn, near_xy) < reach * reach)) continue;
+        const long long cell = row + cz;
+        if (!FILL) {
+          atomicAdd(&a.count[cell], 1);
+          const float df = fmaxf(-f.x, f.y);
+          if (bury > 0.f && fmaf(df, df, far_xy) <= bury * bury) atomicOr(&a.buried[cell], 1);
         } else {
-          atomicOr(a.status, kStatusTableEntries);
+          const int slot = atomicAdd(&a.cursor[cell], 1);
+          const long long o = (long long)a.start[cell] + slot;
+          if (o < a.entry_cap) {
+            a.entry[o] = p;
+            a.index[o] = at;
+          } else {
+            atomicOr(a.status, kStatusTableEntries);
+          }
         }
       }
     }
@@ -141,81 +159,96 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
   const TableGeom& g = *gp;
   if (g.ncell > cell_cap || g.total > entry_cap) return;
   const long long ncell = g.ncell;
-  const long long sx = (long long)g.dims[1] * g.dims[2];
+  const int isx = g.dims[1] * g.dims[2];  // fewer than 2^31 cells
   const float cmin[3] = {(float)g.min[0], (float)g.min[1], (float)g.min[2]};
   const float step = (float)g.step[0];
-  // lanes classify 32 consecutive cells (coalesced); the warp then sorts the
-  // listed, unburied ones one at a time
-  for (long long c0 = ((long long)blockIdx.x * kSortWarps + wib) * kWarp; c0 < ncell;
-       c0 += (long long)gridDim.x * kSortWarps * kWarp) {
-    const long long c = c0 + lane;
+  // eight lanes per cell, four consecutive cells at a time: lists of up to
+  // eight entries (most) are ranked in registers, up to kSortSmall in the
+  // group's quarter of the warp's buffer; longer lists take the whole warp
+  const int grp = lane / kSortLanes, gl = lane % kSortLanes;
+  const unsigned gmask = ((1u << kSortLanes) - 1u) << (grp * kSortLanes);
+  for (long long c0 = ((long long)blockIdx.x * kSortWarps + wib) * kSortGroups; c0 < ncell;
+       c0 += (long long)gridDim.x * kSortWarps * kSortGroups) {
+    const long long c = c0 + grp;
     int cnt = 0, s = 0, bur = 0;
     if (c < ncell) {
       cnt = count[c];
       s = start[c];
       bur = cnt > 0 ? buried[c] : 0;
-      cell[c] = make_int2(bur ? -1 : cnt, s);
-      first[c].cs = make_int2(bur ? -1 : cnt, s);
-      if (bur) count[c] = -1;
-    }
-    // lists of up to kSortSmall entries: four cells at a time, eight lanes
-    // per cell, each group in its own quarter of the warp's buffer; longer
-    // lists: the whole warp on one cell
-    unsigned small = __ballot_sync(0xffffffffu, cnt > 0 && !bur && cnt <= kSortSmall);
-    unsigned todo = __ballot_sync(0xffffffffu, cnt > kSortSmall && !bur);
-    const int grp = lane / kSortLanes, gl = lane % kSortLanes;
-    while (small) {
-      unsigned t = small;
-      for (int k = 0; k < grp; ++k) t &= t - 1;  // the grp-th listed cell left
-      const int src = t ? __ffs(t) - 1 : -1;
-      for (int k = 0; k < kWarp / kSortLanes; ++k) small &= small - 1;
-      const int ccnt0 = __shfl_sync(0xffffffffu, cnt, src >= 0 ? src : 0);
-      const int cs = __shfl_sync(0xffffffffu, s, src >= 0 ? src : 0);
-      const int ccnt = src >= 0 ? ccnt0 : 0;
-      float4* ge = s_e[wib] + grp * kSortSmall;
-      int* gi = s_i[wib] + grp * kSortSmall;
-      float* gk = s_k[wib] + grp * kSortSmall;
-      if (ccnt > 0) {
-        const long long cc = c0 + src;
-        const int cx = (int)(cc / sx), cy = (int)((cc / g.dims[2]) % g.dims[1]), cz = (int)(cc % g.dims[2]);
-        const float ctr[3] = {cmin[0] + ((float)cx + 0.5f) * step, cmin[1] + ((float)cy + 0.5f) * step,
-                              cmin[2] + ((float)cz + 0.5f) * step};
-        for (int q = gl; q < ccnt; q += kSortLanes) {
-          const float4 e = entry[cs + q];
-          ge[q] = e;
-          gi[q] = index[cs + q];
-          const float dx = e.x - ctr[0], dy = e.y - ctr[1], dz = e.z - ctr[2];
-          gk[q] = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (e.w - w);
-        }
+      if (gl == 0) {
+        cell[c] = make_int2(bur ? -1 : cnt, s);
+        first[c].cs = make_int2(bur ? -1 : cnt, s);
       }
-      __syncwarp();
-      for (int q = gl; q < ccnt; q += kSortLanes) {
-        const float kq = gk[q];
-        const int iq = gi[q];
+    }
+    if (cnt > 0 && !bur && cnt <= kSortSmall) {
+      const int cx = (int)c / isx, rem = (int)c - cx * isx, cy = rem / g.dims[2], cz = rem - cy * g.dims[2];
+      const float ctr[3] = {cmin[0] + ((float)cx + 0.5f) * step, cmin[1] + ((float)cy + 0.5f) * step,
+                            cmin[2] + ((float)cz + 0.5f) * step};
+      // key: distance to the cell centre less R' - w (atoms likely to bury
+      // the cell's points first); FP32, any fixed order is exact
+      auto key = [&](const float4 e) {
+        const float dx = e.x - ctr[0], dy = e.y - ctr[1], dz = e.z - ctr[2];
+        return sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (e.w - w);
+      };
+      if (cnt <= kSortLanes) {
+        float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
+        int i = 0x7fffffff;
+        float k = INFINITY;
+        if (gl < cnt) {
+          e = entry[s + gl];
+          i = index[s + gl];
+          k = key(e);
+        }
         int r = 0;
-        for (int o = 0; o < ccnt; ++o) {
-          const float ko = gk[o];
-          r += (ko < kq) || (ko == kq && gi[o] < iq);
+#pragma unroll
+        for (int o = 0; o < kSortLanes; ++o) {
+          const float ko = __shfl_sync(gmask, k, o, kSortLanes);
+          const int io = __shfl_sync(gmask, i, o, kSortLanes);
+          r += (ko < k) || (ko == k && io < i);
         }
-        put(cs + r, ge[q]);
-        index[cs + r] = iq;
-        if (r == 0) first[c0 + src].first = ge[q];
+        if (gl < cnt) {
+          put(s + r, e);
+          index[s + r] = i;
+          if (r == 0) first[c].first = e;
+        }
+      } else {
+        float4* ge = s_e[wib] + grp * kSortSmall;
+        int* gi = s_i[wib] + grp * kSortSmall;
+        float* gk = s_k[wib] + grp * kSortSmall;
+        for (int q = gl; q < cnt; q += kSortLanes) {
+          const float4 e = entry[s + q];
+          ge[q] = e;
+          gi[q] = index[s + q];
+          gk[q] = key(e);
+        }
+        __syncwarp(gmask);
+        for (int q = gl; q < cnt; q += kSortLanes) {
+          const float kq = gk[q];
+          const int iq = gi[q];
+          int r = 0;
+          for (int o = 0; o < cnt; ++o) {
+            const float ko = gk[o];
+            r += (ko < kq) || (ko == kq && gi[o] < iq);
+          }
+          put(s + r, ge[q]);
+          index[s + r] = iq;
+          if (r == 0) first[c].first = ge[q];
+        }
       }
-      if ((ccnt & 1) && gl == 0) put(cs + ccnt, kPadEntry);
-      __syncwarp();
+      if ((cnt & 1) && gl == 0) put(s + cnt, kPadEntry);
     }
+    __syncwarp();
+    unsigned todo = __ballot_sync(0xffffffffu, gl == 0 && cnt > kSortSmall && !bur);
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1;
-      const long long cc = c0 + src;
+      const long long cc = c0 + src / kSortLanes;
       const int ccnt = __shfl_sync(0xffffffffu, cnt, src), cs = __shfl_sync(0xffffffffu, s, src);
       if (ccnt > kSortBuf) {
         if (lane == 0) atomicOr(status, kStatusSegmentTooLong);
         continue;
       }
-      // key: distance to the cell centre less R' - w (atoms likely to bury
-      // the cell's points first); FP32, any fixed order is exact
-      const int cx = (int)(cc / sx), cy = (int)((cc / g.dims[2]) % g.dims[1]), cz = (int)(cc % g.dims[2]);
+      const int cx = (int)cc / isx, rem = (int)cc - cx * isx, cy = rem / g.dims[2], cz = rem - cy * g.dims[2];
       const float ctr[3] = {cmin[0] + ((float)cx + 0.5f) * step, cmin[1] + ((float)cy + 0.5f) * step,
                             cmin[2] + ((float)cz + 0.5f) * step};
       for (int q = lane; q < ccnt; q += kWarp) {
@@ -264,7 +297,7 @@ gbx_status launch_tight_build(Context* ctx, const float4* pos) {
     ++ctx->launches;
     tight_members_kernel<true><<<(int)blocks, threads, 0, st>>>(a);
     ++ctx->launches;
-    long long sb = (cells + kSortWarps * kWarp - 1) / (kSortWarps * kWarp);
+    long long sb = (cells + kSortWarps * kSortGroups - 1) / (kSortWarps * kSortGroups);
     if (sb > (long long)ctx->sms * 64) sb = (long long)ctx->sms * 64;
     tight_sort_kernel<<<(int)sb, kSortWarps * kWarp, 0, st>>>(ctx->d_tcount, ctx->d_tstart, ctx->d_tburied,
                                                                ctx->d_tentry, ctx->d_tindex, ctx->d_tcell, ctx->d_tfirst,
