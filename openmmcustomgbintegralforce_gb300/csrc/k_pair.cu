@@ -134,11 +134,11 @@ __global__ void __launch_bounds__(kPairThreads) pair_kernel(PairArgs a) {
 // ---------------------------------------------------------------------------
 // Symmetric scheme (the context path): every unordered pair once.  A warp
 // owns an i-block of 128 atoms (four per lane: 128 b + 32 u + lane)
-// and a run of 32-atom j-tiles above the block.  A j-tile's atoms and their
-// force / dE/dB accumulators rotate one lane per step through shuffles, so
+// and a run of 32-atom j-tiles above the block.  A j-tile's force / dE/dB
+// accumulators rotate one lane per step through shuffles, so
 // after 32 steps every (i, j) pair of the tile was evaluated once and each
 // lane again holds the complete j-side sums of its own j atom.  Pairs inside
-// an i-block, and the self terms, are done by pair_block_kernel.  Every sum
+// an i-block, and the self terms, are done by pair_block_unit.  Every sum
 // runs in a fixed order; i- and j-side sums are rounded to fixed point once
 // per tile and added as integers.
 // ---------------------------------------------------------------------------
@@ -242,7 +242,7 @@ __device__ __forceinline__ void gb_pair(const PAtom& I, float pqi, float kDi, fl
 // turns every one of its terms into a zero that leaves the sums unchanged.
 struct PAtom2 {
   float2 nx, ny, nz;  // -x, -y, -z
-  float2 B, pq, kD, kB;
+  float2 B, pq, kD;
 };
 
 struct PAcc2 {
@@ -250,7 +250,7 @@ struct PAcc2 {
 };
 
 struct PJ2 {  // one j atom, broadcast to both halves
-  float2 x, y, z, q, B, invB, kB, pq;
+  float2 x, y, z, q, B, invB, pq;
 };
 
 __device__ __forceinline__ float2 bcast2(float v) { return make_float2(v, v); }
@@ -267,7 +267,8 @@ __device__ __forceinline__ void gb_pair2(const PAtom2& I, const PJ2& J, float cu
   const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
   const float2 arg = __fmul2_rn(r2, __fmul2_rn(I.kD, J.invB));
   const float2 ex = make_float2(ex2_ftz(arg.x), ex2_ftz(arg.y));
-  const float2 f2 = __ffma2_rn(__fmul2_rn(I.B, J.B), ex, r2);
+  const float2 BB = __fmul2_rn(I.B, J.B);
+  const float2 f2 = __ffma2_rn(BB, ex, r2);
   float2 invf = make_float2(rsqrt_ftz(f2.x), rsqrt_ftz(f2.y));
   if (CUTOFF) {
     if (r2.x > cutoff2) invf.x = 0.0f;
@@ -275,18 +276,21 @@ __device__ __forceinline__ void gb_pair2(const PAtom2& I, const PJ2& J, float cu
   }
   const float2 e = __fmul2_rn(__fmul2_rn(I.pq, J.q), invf);
   esum = __fadd2_rn(esum, e);
-  const float2 c = __fmul2_rn(__fmul2_rn(e, invf), invf);
+  const float2 c = __fmul2_rn(e, __fmul2_rn(invf, invf));
   const float2 cex = __fmul2_rn(c, ex);
   const float2 gn = __ffma2_rn(bcast2(-0.25f), cex, c);  // -g = c (1 - e^-D / 4)
+  // dG/dB_i / (-1/2) = c e^-D (r^2 / (4 B_i) + B_j) = db / B_i, dG/dB_j likewise
+  // db / B_j: one term for both sides, divided once per tile
+  const float2 db = __ffma2_rn(bcast2(0.25f), r2, BB);
   ai.fx = __ffma2_rn(gn, dx, ai.fx);
   ai.fy = __ffma2_rn(gn, dy, ai.fy);
   ai.fz = __ffma2_rn(gn, dz, ai.fz);
-  ai.db = __ffma2_rn(cex, __ffma2_rn(r2, I.kB, J.B), ai.db);
+  ai.db = __ffma2_rn(cex, db, ai.db);
   if (ADJ) ai.dq = __ffma2_rn(J.pq, invf, ai.dq);
   aj.fx = __ffma2_rn(gn, dx, aj.fx);
   aj.fy = __ffma2_rn(gn, dy, aj.fy);
   aj.fz = __ffma2_rn(gn, dz, aj.fz);
-  aj.db = __ffma2_rn(cex, __ffma2_rn(r2, J.kB, I.B), aj.db);
+  aj.db = __ffma2_rn(cex, db, aj.db);
   if (ADJ) aj.dq = __ffma2_rn(I.pq, invf, aj.dq);
 }
 
@@ -361,24 +365,20 @@ __device__ __forceinline__ float2 shfl2(float2 v, int src) {
   return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
-// The plain form is capped at 96 registers (five blocks per SM); the cutoff
-// and adjoint forms keep their wider register sets.  PER: minimum image in a
-// periodic box, every tile pair evaluated.
-template <bool CUTOFF, bool ADJ, bool PER = false>
-__global__ void __launch_bounds__(kSymThreads, (CUTOFF || ADJ) ? 1 : 5) pair_sym_kernel(SymArgs a) {
+// Units of the symmetric scheme: one warp, an i-block against a run of j-tiles
+// above it.  PER: minimum image in a periodic box, every tile pair evaluated.
+// Returns the lane's share of the energy.
+template <bool CUTOFF, bool ADJ, bool PER>
+__device__ __forceinline__ double pair_sym_unit(const SymArgs& a, int unit, int lane, long long (*si)[kWarp],
+                                                float4* sj4, float2* sj2) {
   static_assert(kNI % 2 == 0, "i atoms are paired into float2 halves");
   constexpr int kNH = kNI / 2;
-  const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
-  const int lane = threadIdx.x % kWarp;
-  if (unit >= a.nblocks * a.chunks) return;
   const int b = unit / a.chunks, ch = unit % a.chunks;
   const int jt0 = kNI * b + kNI + ch * a.chunk;
   const int jt1 = min(a.ntiles, jt0 + a.chunk);
   // the i atoms' fixed-point sums, lane-private in shared memory (touched
   // once per tile; in registers they would cost a quarter of the occupancy)
   constexpr int kNF = ADJ ? 5 : 4;
-  __shared__ long long s_si[kSymThreads / kWarp][kNI * kNF][kWarp];
-  long long(*si)[kWarp] = s_si[threadIdx.x / kWarp];
   double E = 0.0;
   if (jt0 < jt1) {
 #pragma unroll
@@ -394,7 +394,6 @@ __global__ void __launch_bounds__(kSymThreads, (CUTOFF || ADJ) ? 1 : 5) pair_sym
       I[h].B = make_float2(p0.B, p1.B);
       I[h].pq = make_float2(a.pref * p0.q, a.pref * p1.q);
       I[h].kD = make_float2(-0.25f * kLog2e * p0.invB, -0.25f * kLog2e * p1.invB);
-      I[h].kB = make_float2(0.25f * p0.invB, 0.25f * p1.invB);
     }
     const int src = (lane + 1) % kWarp;
     float4 ilo = make_float4(0.f, 0.f, 0.f, 0.f), ihi = ilo;
@@ -411,23 +410,27 @@ __global__ void __launch_bounds__(kSymThreads, (CUTOFF || ADJ) ? 1 : 5) pair_sym
     for (int jt = jt0; jt < jt1; ++jt) {
       if (CUTOFF && !PER && box_gap2(ilo, ihi, a.tile_box[2 * jt], a.tile_box[2 * jt + 1]) > a.cutoff2) continue;
       PAtom J = load_patom(a, kWarp * jt + lane);
+      __syncwarp();
+      sj4[lane] = make_float4(J.x, J.y, J.z, J.q);
+      sj2[lane] = make_float2(J.B, J.invB);
+      __syncwarp();
       const float2 z2 = make_float2(0.f, 0.f);
       PAcc2 ai[kNH], aj{z2, z2, z2, z2, z2};
 #pragma unroll
       for (int h = 0; h < kNH; ++h) ai[h] = PAcc2{z2, z2, z2, z2, z2};
       float2 et = z2;
-#pragma unroll 2
+#pragma unroll 8
       for (int t = 0; t < kWarp; ++t) {
         const PJ2 J2{bcast2(J.x), bcast2(J.y), bcast2(J.z), bcast2(J.q), bcast2(J.B), bcast2(J.invB),
-                     bcast2(0.25f * J.invB), bcast2(a.pref * J.q)};
+                     bcast2(a.pref * J.q)};
 #pragma unroll
         for (int h = 0; h < kNH; ++h) gb_pair2<CUTOFF, ADJ, PER>(I[h], J2, a.cutoff2, ai[h], aj, et, a.L, a.iL);
-        J.x = __shfl_sync(0xffffffffu, J.x, src);
-        J.y = __shfl_sync(0xffffffffu, J.y, src);
-        J.z = __shfl_sync(0xffffffffu, J.z, src);
-        J.q = __shfl_sync(0xffffffffu, J.q, src);
-        J.B = __shfl_sync(0xffffffffu, J.B, src);
-        J.invB = __shfl_sync(0xffffffffu, J.invB, src);
+        // the next step's j atom: the tile's copy in shared memory (two loads
+        // where rotating it took six shuffles)
+        const int nl = (lane + t + 1) % kWarp;
+        const float4 jp = sj4[nl];
+        const float2 jb = sj2[nl];
+        J = PAtom{jp.x, jp.y, jp.z, jp.w, jb.x, jb.y};
         aj.fx = shfl2(aj.fx, src);
         aj.fy = shfl2(aj.fy, src);
         aj.fz = shfl2(aj.fz, src);
@@ -435,16 +438,19 @@ __global__ void __launch_bounds__(kSymThreads, (CUTOFF || ADJ) ? 1 : 5) pair_sym
         if (ADJ) aj.dq = shfl2(aj.dq, src);
       }
       PFixed sj;
-      sj.add(PAcc{aj.fx.x + aj.fx.y, aj.fy.x + aj.fy.y, aj.fz.x + aj.fz.y, aj.db.x + aj.db.y, aj.dq.x + aj.dq.y});
+      sj.add(PAcc{aj.fx.x + aj.fx.y, aj.fy.x + aj.fy.y, aj.fz.x + aj.fz.y, (aj.db.x + aj.db.y) * J.invB,
+                  aj.dq.x + aj.dq.y});
       push_atom<ADJ>(a, kWarp * jt + lane, sj);
 #pragma unroll
       for (int h = 0; h < kNH; ++h) {
         const float2 v[5] = {ai[h].fx, ai[h].fy, ai[h].fz, ai[h].db, ai[h].dq};
 #pragma unroll
         for (int f = 0; f < kNF; ++f) {
-          const float sc = f < 3 ? -1.0f : f == 3 ? -0.5f : 1.0f;  // force: negated sums; dE/dB: -1/2 db
-          si[(2 * h) * kNF + f][lane] += float_to_fixed(sc * v[f].x);
-          si[(2 * h + 1) * kNF + f][lane] += float_to_fixed(sc * v[f].y);
+          // force: negated sums; dE/dB: -1/2 db / B_i (k_D = -log2(e) / (4 B_i))
+          const float2 sc = f < 3 ? bcast2(-1.0f)
+                            : f == 3 ? make_float2(2.0f / kLog2e * I[h].kD.x, 2.0f / kLog2e * I[h].kD.y) : bcast2(1.0f);
+          si[(2 * h) * kNF + f][lane] += float_to_fixed(sc.x * v[f].x);
+          si[(2 * h + 1) * kNF + f][lane] += float_to_fixed(sc.y * v[f].y);
         }
       }
       E += (double)et.x + (double)et.y;
@@ -460,8 +466,7 @@ __global__ void __launch_bounds__(kSymThreads, (CUTOFF || ADJ) ? 1 : 5) pair_sym
       push_atom<ADJ>(a, kSymI * b + kWarp * u + lane, su);
     }
   }
-  E = warp_sum(E);
-  if (lane == 0 && E != 0.0) atomicAdd(a.energy, (unsigned long long)__double2ll_rn(E * kFixedScale));
+  return E;
 }
 
 // Pairs inside each i-block (i side only, each ordered pair once: lane t of
@@ -470,12 +475,9 @@ __global__ void __launch_bounds__(kSymThreads, (CUTOFF || ADJ) ? 1 : 5) pair_sym
 // are separate fixed-point reductions, so small systems get eight times the
 // warps.
 constexpr int kBlockSplit = 2;  // warps per broadcast slot
-template <bool CUTOFF, bool ADJ, bool PER = false>
-__global__ void __launch_bounds__(kSymThreads) pair_block_kernel(SymArgs a) {
-  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
+template <bool CUTOFF, bool ADJ, bool PER>
+__device__ __forceinline__ double pair_block_unit(const SymArgs& a, int wid, int lane) {
   const int b = wid / (kNI * kBlockSplit), h = (wid / kBlockSplit) % kNI, part = wid % kBlockSplit;
-  const int lane = threadIdx.x % kWarp;
-  if (b >= a.nblocks) return;
   PAtom I[kNI];
   float pq[kNI], kD[kNI], kB[kNI], e[kNI];
   PAcc ai[kNI], dummy{0.f, 0.f, 0.f, 0.f, 0.f};
@@ -515,6 +517,28 @@ __global__ void __launch_bounds__(kSymThreads) pair_block_kernel(SymArgs a) {
     push_atom<ADJ>(a, kSymI * b + kWarp * u + lane, su);
     E += 0.5 * (double)e[u] + (h == 0 && part == 0 ? 0.5 * (double)pq[u] * I[u].q * I[u].invB : 0.0);
   }
+  return E;
+}
+
+// One launch for both: warps past the symmetric units take the i-blocks' inner
+// pairs, which fill the last wave (and at 1,000 atoms, where neither fills the
+// GPU, run beside the units instead of after them: 27 -> 18 us).  Four blocks
+// per SM (128 registers) with eight steps unrolled measured fastest; the pass
+// is then bound by the FP32 pipe's operand bandwidth: its time follows the
+// packed multiply-adds (3.1 cycles each, a packed add or multiply 2), not the
+// MUFU operations (removing every one saved 3 %).  50,000 atoms: 1.36 -> 1.25
+// ms; with a 2.0 nm cutoff 0.59 -> 0.50 ms.
+template <bool CUTOFF, bool ADJ, bool PER = false>
+__global__ void __launch_bounds__(kSymThreads, ADJ ? 3 : 4) pair_sym_kernel(SymArgs a) {
+  constexpr int kWarps = kSymThreads / kWarp;
+  __shared__ long long s_si[kWarps][kNI * (ADJ ? 5 : 4)][kWarp];
+  __shared__ float4 s_j4[kWarps][kWarp];
+  __shared__ float2 s_j2[kWarps][kWarp];
+  const int w = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+  const int unit = blockIdx.x * kWarps + w, units = a.nblocks * a.chunks;
+  double E = 0.0;
+  if (unit < units) E = pair_sym_unit<CUTOFF, ADJ, PER>(a, unit, lane, s_si[w], s_j4[w], s_j2[w]);
+  else if (unit - units < a.nblocks * kNI * kBlockSplit) E = pair_block_unit<CUTOFF, ADJ, PER>(a, unit - units, lane);
   E = warp_sum(E);
   if (lane == 0 && E != 0.0) atomicAdd(a.energy, (unsigned long long)__double2ll_rn(E * kFixedScale));
 }
@@ -688,7 +712,8 @@ SymArgs sym_args(int n) {
   // j-tiles per unit: long runs amortise the i-block setup, but small
   // systems need short ones to give ~8k working warps
   const long long visits = (long long)a.nblocks * a.ntiles / 2;
-  a.chunk = (int)std::max(2LL, std::min((long long)kSymChunkMax, visits / 8192));
+  // (one tile below 2,048 visits, about 4,000 atoms, where even two leave SMs idle)
+  a.chunk = visits < 2048 ? 1 : (int)std::max(2LL, std::min((long long)kSymChunkMax, visits / 8192));
   a.chunks = (a.ntiles + a.chunk - 1) / a.chunk;
   return a;
 }
@@ -747,7 +772,7 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
   a.tile_box = ctx->d_tile_box;
   a.perm = nullptr;
   const int wpb = kSymThreads / kWarp;
-  const int gu = (a.nblocks * a.chunks + wpb - 1) / wpb, gb = (a.nblocks * kNI * kBlockSplit + wpb - 1) / wpb;
+  const int gu = (a.nblocks * (a.chunks + kNI * kBlockSplit) + wpb - 1) / wpb;
   cudaStream_t st = ctx->stream;
   if (ctx->cfg.periodic) {
     // minimum image, every tile pair evaluated (bounding boxes do not wrap)
@@ -755,12 +780,10 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
     a.iL = make_float3((float)(1.0 / ctx->cfg.box[0]), (float)(1.0 / ctx->cfg.box[1]), (float)(1.0 / ctx->cfg.box[2]));
     if (adjoint) {
       pair_sym_kernel<true, true, true><<<gu, kSymThreads, 0, st>>>(a);
-      pair_block_kernel<true, true, true><<<gb, kSymThreads, 0, st>>>(a);
     } else {
       pair_sym_kernel<true, false, true><<<gu, kSymThreads, 0, st>>>(a);
-      pair_block_kernel<true, false, true><<<gb, kSymThreads, 0, st>>>(a);
     }
-    ctx->launches += 2;
+    ++ctx->launches;
   } else if (a.cutoff2 > 0) {
     // spatial order, then tile boxes over it
     const int n = a.n, nb = (n + 255) / 256;
@@ -780,24 +803,16 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
     if (adjoint) {
       pair_sym_kernel<true, true><<<gu, kSymThreads, 0, st>>>(a);
       ++ctx->launches;
-      pair_block_kernel<true, true><<<gb, kSymThreads, 0, st>>>(a);
-      ++ctx->launches;
     } else {
       pair_sym_kernel<true, false><<<gu, kSymThreads, 0, st>>>(a);
-      ++ctx->launches;
-      pair_block_kernel<true, false><<<gb, kSymThreads, 0, st>>>(a);
       ++ctx->launches;
     }
   } else {
     if (adjoint) {
       pair_sym_kernel<false, true><<<gu, kSymThreads, 0, st>>>(a);
       ++ctx->launches;
-      pair_block_kernel<false, true><<<gb, kSymThreads, 0, st>>>(a);
-      ++ctx->launches;
     } else {
       pair_sym_kernel<false, false><<<gu, kSymThreads, 0, st>>>(a);
-      ++ctx->launches;
-      pair_block_kernel<false, false><<<gb, kSymThreads, 0, st>>>(a);
       ++ctx->launches;
     }
   }
