@@ -140,12 +140,11 @@ gbx_status upload_quadrature(Context* ctx) {
   std::vector<float4> qv(Q);
   std::vector<float2> qw(Q);
   double S4 = 0.0, S7 = 0.0;
-  // GBSW keeps a direction's points together (ray by ray): 32 lanes then hold
-  // neighbouring points, whose table cells share cache lines (gbsw_integral_kernel)
-  const bool rays = c.model == GBX_MODEL_GBSW;
+  // a direction's points together (ray by ray): 32 lanes then hold neighbouring
+  // points, whose table cells share cache lines (gbsw_integral_kernel)
   for (int i = 0; i < c.n_radial; ++i)
     for (int j = 0; j < nS; ++j) {
-      const int q = rays ? j * c.n_radial + i : i * nS + j;
+      const int q = j * c.n_radial + i;
       const double r = xr[i];
       for (int k = 0; k < 3; ++k) ctx->q_off[3 * q + k] = r * leb[4 * j + k];
       ctx->q_rad[q] = r;

@@ -93,7 +93,8 @@ __global__ void __launch_bounds__(kFinishThreads) finish_kernel(
   if (dEdR) dEdR[i] = b.y;
 }
 
-__global__ void born_kernel(int n, int n_chunks, const float* __restrict__ J, double S4, double S7, double C4,
+constexpr int kBornThreads = 64;
+__global__ void __launch_bounds__(kBornThreads) born_kernel(int n, int n_chunks, const float* __restrict__ J, double S4, double S7, double C4,
                             double C7, double alpha0, double alpha1, double* __restrict__ born,
                             float2* __restrict__ bornf, double* __restrict__ dBdJ, double* __restrict__ dBda,
                             double* __restrict__ integrals, unsigned* __restrict__ status) {
@@ -193,7 +194,8 @@ gbx_status launch_finish_outputs(Context* ctx, unsigned long long* force, int st
 
 gbx_status launch_born(Context* ctx) {
   const int n = ctx->n;
-  born_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(
+  // small blocks: the FP64 chains of a few thousand atoms spread over every SM
+  born_kernel<<<(n + kBornThreads - 1) / kBornThreads, kBornThreads, 0, ctx->stream>>>(
       n, ctx->n_chunks, ctx->d_J, ctx->S4, ctx->S7, ctx->C4, ctx->C7, ctx->alpha0, ctx->alpha1, ctx->d_born,
       reinterpret_cast<float2*>(ctx->d_bornf), ctx->d_dBdJ, ctx->d_dBdJ + 2 * (size_t)n, ctx->d_integrals,
       ctx->d_status);

@@ -24,6 +24,7 @@ namespace gbx {
 namespace {
 
 constexpr int kMaxSamples = 96;  // grid values or samples per axis kept in shared memory
+constexpr int kColumnLanes = 8;  // lanes per column of grid points or samples
 constexpr int kMemberThreads = 256;
 constexpr int kMemberWarps = kMemberThreads / kWarp;
 
@@ -69,7 +70,8 @@ __device__ __forceinline__ int2 column(int col, int n1, float inv_n1) {
 }
 
 // CharmmReferenceGBSW.cpp:472-496 (STANDALONE) and CustomGBIntegral.cpp:198-227 (GRID).
-// A warp per atom, a lane per column of grid points.  The offset from the atom
+// A warp per atom, eight lanes per column of grid points (a column's counters
+// share sectors, so its atomics leave together).  The offset from the atom
 // depends on one axis only, so each axis value's is formed once, in the
 // reference's FP64; the membership of a point is decided by the FP32 sum of
 // their squares wherever that is clear of the boundary by a margin that covers
@@ -145,12 +147,12 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
     __syncwarp();
     // FP32 squared distances carry a relative error below 4 2^-24
     const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
-    for (int col = lane; col < cols; col += kWarp) {
+    for (int col = lane / kColumnLanes; col < cols; col += kWarp / kColumnLanes) {
       const int2 ij = column(col, nn[1], inv_n1);
       const float sxy = sq[0][ij.x] + sq[1][ij.y];
       if (sxy > out2) continue;
       const long long row = (long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2];
-      for (int k = 0; k < nn[2]; ++k) {
+      for (int k = lane % kColumnLanes; k < nn[2]; k += kColumnLanes) {
         const float s = sxy + sq[2][k];
         if (s < in2 || (s <= out2 && inside(ds[0][ij.x], ds[1][ij.y], ds[2][k]))) em.put<FILL>(row + k, a, ncell);
       }
@@ -240,13 +242,13 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
     const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
     // FP32 squared distances carry a relative error below 4 2^-24
     const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
-    for (int col = lane; col < cols; col += kWarp) {  // a lane per column of samples
+    for (int col = lane / kColumnLanes; col < cols; col += kWarp / kColumnLanes) {
       const int2 ij = column(col, cnt[1], inv_n1);
       const int i0 = idx[0][ij.x], i1 = idx[1][ij.y];
       const float sxy = sq[0][ij.x] + sq[1][ij.y];
       if (i0 < 0 || i1 < 0 || sxy > out2) continue;
       const long long row = (long long)i0 * sx + (long long)i1 * sy;
-      for (int kz = 0; kz < cnt[2]; ++kz) {
+      for (int kz = lane % kColumnLanes; kz < cnt[2]; kz += kColumnLanes) {
         const float sf = sxy + sq[2][kz];
         bool member = sf < in2;
         if (!member && sf <= out2) {
@@ -318,8 +320,6 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(int* __r
     if (cnt <= kWarp) sort_list<1>(entries, in, s, cnt, kept, lane);
     else if (cnt <= 2 * kWarp) sort_list<2>(entries, in, s, cnt, kept, lane);
     else if (cnt <= 4 * kWarp) sort_list<4>(entries, in, s, cnt, kept, lane);
-    else if (cnt <= 8 * kWarp) sort_list<8>(entries, in, s, cnt, kept, lane);
-    else if (cnt <= 16 * kWarp) sort_list<16>(entries, in, s, cnt, kept, lane);
     else if (cnt > kMaxSortSegment) {
       if (lane == 0) atomicOr(status, kStatusSegmentTooLong);
       continue;

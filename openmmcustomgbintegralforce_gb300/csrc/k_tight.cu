@@ -29,6 +29,7 @@
 namespace gbx {
 namespace {
 
+constexpr int kColumnLanes = 8;
 constexpr int kSortWarps = 4;
 constexpr int kSortBuf = 256;
 constexpr int kSortLanes = 8;                                   // lanes per short list
@@ -44,7 +45,6 @@ struct TightArgs {
   const int* start;
   int* cursor;
   int* buried;
-  float4* entry;
   int* index;
   long long cell_cap, entry_cap;
   unsigned* status;
@@ -88,10 +88,11 @@ __global__ void tight_members_kernel(TightArgs a) {
       const float lo = __fmul_rn((float)c, h);
       return make_float2(__fsub_rn(lo, at), __fsub_rn(__fadd_rn(lo, h), at));
     };
-    // a lane per column of cells
+    // eight lanes per column of cells: a column's counters share a sector, so
+    // its atomics leave together
     const int ny = e[1] - b[1] + 1, cols = (e[0] - b[0] + 1) * ny;
     const float inv_ny = 1.0f / (float)ny;
-    for (int col = lane; col < cols; col += kWarp) {
+    for (int col = lane / kColumnLanes; col < cols; col += kWarp / kColumnLanes) {
       int cx = (int)(((float)col + 0.5f) * inv_ny);
       cx -= cx * ny > col;
       const int c[2] = {b[0] + cx, b[1] + col - cx * ny};
@@ -105,7 +106,7 @@ __global__ void tight_members_kernel(TightArgs a) {
       }
       if (!(near_xy < reach * reach)) continue;
       const long long row = c[0] * sx + c[1] * sy;
-      for (int cz = b[2]; cz <= e[2]; ++cz) {
+      for (int cz = b[2] + lane % kColumnLanes; cz <= e[2]; cz += kColumnLanes) {
         const float2 f = faces(cz, x[2]);
         const float dn = fmaxf(fmaxf(f.x, -f.y), 0.f);
         if (!(fmaf(dn, dn, near_xy) < reach * reach)) continue;
@@ -118,7 +119,6 @@ __global__ void tight_members_kernel(TightArgs a) {
           const int slot = atomicAdd(&a.cursor[cell], 1);
           const long long o = (long long)a.start[cell] + slot;
           if (o < a.entry_cap) {
-            a.entry[o] = p;
             a.index[o] = at;
           } else {
             atomicOr(a.status, kStatusTableEntries);
@@ -129,10 +129,12 @@ __global__ void tight_members_kernel(TightArgs a) {
   }
 }
 
-// Sort each list by (distance from the cell centre to the atom's burying
+// Sort each list of atom indices, and write the entries (positions and radii)
+// in that order: by (distance from the cell centre to the atom's burying
 // sphere, atom index) -- a deterministic order whatever the fill order was --
 // and mark buried cells with count -1.
-__global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __restrict__ count,
+__global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const float4* __restrict__ pos,
+                                                                        const int* __restrict__ count,
                                                                         const int* __restrict__ start,
                                                                         const int* __restrict__ buried,
                                                                         float4* __restrict__ entry,
@@ -195,8 +197,8 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
         int i = 0x7fffffff;
         float k = INFINITY;
         if (gl < cnt) {
-          e = entry[s + gl];
           i = index[s + gl];
+          e = __ldg(pos + i);
           k = key(e);
         }
         int r = 0;
@@ -216,9 +218,10 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
         int* gi = s_i[wib] + grp * kSortSmall;
         float* gk = s_k[wib] + grp * kSortSmall;
         for (int q = gl; q < cnt; q += kSortLanes) {
-          const float4 e = entry[s + q];
+          const int i = index[s + q];
+          const float4 e = __ldg(pos + i);
           ge[q] = e;
-          gi[q] = index[s + q];
+          gi[q] = i;
           gk[q] = key(e);
         }
         __syncwarp(gmask);
@@ -252,9 +255,10 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(int* __r
       const float ctr[3] = {cmin[0] + ((float)cx + 0.5f) * step, cmin[1] + ((float)cy + 0.5f) * step,
                             cmin[2] + ((float)cz + 0.5f) * step};
       for (int q = lane; q < ccnt; q += kWarp) {
-        const float4 e = entry[cs + q];
+        const int i = index[cs + q];
+        const float4 e = __ldg(pos + i);
         s_e[wib][q] = e;
-        s_i[wib][q] = index[cs + q];
+        s_i[wib][q] = i;
         const float dx = e.x - ctr[0], dy = e.y - ctr[1], dz = e.z - ctr[2];
         s_k[wib][q] = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (e.w - w);
       }
@@ -285,7 +289,7 @@ gbx_status launch_tight_build(Context* ctx, const float4* pos) {
   if (cells > 0) {
     TightArgs a{pos,           ctx->n,          ctx->d_tgeom,   (float)ctx->cfg.switch_width,
                 ctx->d_tcount, ctx->d_tstart,   ctx->d_tcursor, ctx->d_tburied,
-                ctx->d_tentry, ctx->d_tindex,   cells,          ctx->tentry_cap,
+                ctx->d_tindex, cells,           ctx->tentry_cap,
                 ctx->d_status};
     const int threads = 256;
     long long blocks = ((long long)ctx->n * kWarp + threads - 1) / threads;
@@ -299,7 +303,7 @@ gbx_status launch_tight_build(Context* ctx, const float4* pos) {
     ++ctx->launches;
     long long sb = (cells + kSortWarps * kSortGroups - 1) / (kSortWarps * kSortGroups);
     if (sb > (long long)ctx->sms * 64) sb = (long long)ctx->sms * 64;
-    tight_sort_kernel<<<(int)sb, kSortWarps * kWarp, 0, st>>>(ctx->d_tcount, ctx->d_tstart, ctx->d_tburied,
+    tight_sort_kernel<<<(int)sb, kSortWarps * kWarp, 0, st>>>(pos, ctx->d_tcount, ctx->d_tstart, ctx->d_tburied,
                                                                ctx->d_tentry, ctx->d_tindex, ctx->d_tcell, ctx->d_tfirst,
                                                                ctx->d_tgeom,
                                                                (float)ctx->cfg.switch_width, cells, ctx->tentry_cap,
