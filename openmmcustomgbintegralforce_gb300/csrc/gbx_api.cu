@@ -214,8 +214,7 @@ gbx_status alloc_atom_buffers(Context* ctx) {
   GBX_TRY(dalloc(ctx, &ctx->d_tile_box, 2 * (((size_t)n + 31) / 32)));
   if (ctx->cfg.model != GBX_MODEL_GBSW) {
     GBX_TRY(dalloc(ctx, &ctx->d_pstate, (size_t)n * Q * (ctx->cfg.model == GBX_MODEL_GBMV1 ? 1 : 5)));
-    GBX_TRY(dalloc(ctx, &ctx->d_pcell, (size_t)n * Q));
-    GBX_TRY(dalloc(ctx, &ctx->d_prank, (size_t)n * Q));
+    GBX_TRY(dalloc(ctx, &ctx->d_pat, (size_t)n * Q));
     GBX_TRY(dalloc(ctx, &ctx->d_porder, (size_t)n * Q));
     GBX_TRY(dalloc(ctx, &ctx->d_sval, (size_t)n * Q));
     GBX_TRY(dalloc(ctx, &ctx->d_ptotal, 1));
@@ -347,6 +346,7 @@ gbx_status grow_table(Context* ctx, long long cells, long long entries) {
     GBX_TRY(dalloc(ctx, &ctx->d_cell2, cap));
     if (ctx->cfg.model != GBX_MODEL_GBSW) {
       GBX_TRY(dalloc(ctx, &ctx->d_pcount, cap));
+      GBX_TRY(dalloc(ctx, &ctx->d_plive, cap));
       GBX_TRY(dalloc(ctx, &ctx->d_pstart, cap + 1));
     }
     ctx->cell_cap = cap;
@@ -787,7 +787,7 @@ gbx_status gbx_destroy(gbx_context* handle) {
                   ctx->d_tentry, ctx->d_tindex, ctx->d_entry4, ctx->d_entry_par,
                   ctx->d_cell2, ctx->d_tcell, ctx->d_tfirst, ctx->d_srec, ctx->d_srec_st, ctx->d_rcount, ctx->d_rmax, ctx->d_next_item, ctx->d_energy_fx, ctx->d_tile_box, ctx->d_perm,
                   ctx->d_perm_tmp, ctx->d_cell_of, ctx->d_scount, ctx->d_sstart, ctx->d_scursor, ctx->d_sgeom, ctx->d_pstate,
-                  ctx->d_pcell, ctx->d_prank, ctx->d_porder, ctx->d_sval, ctx->d_pcount, ctx->d_pstart,
+                  ctx->d_pat, ctx->d_porder, ctx->d_sval, ctx->d_pcount, ctx->d_plive, ctx->d_pstart,
                   ctx->d_ptotal, ctx->d_slot_of, ctx->d_pub};
   for (void* p : ptrs)
     if (p) cudaFree(p);

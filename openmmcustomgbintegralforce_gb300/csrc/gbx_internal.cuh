@@ -80,6 +80,8 @@ struct ModelConst {
   int cap;
   int skip_empty;
   int nq;
+  unsigned nq_magic;         // point_atom: ceil(2^(31 + L) / nq) with 2^(L - 1) < nq <= 2^L
+  int nq_shift;              // L - 1
   int nrad;                  // radial points per direction (index = direction * nrad + radial)
   int cutoff_chain_quirk;
   float sw, c1, c3;          // GBSW: u = 1/2 + c1 dr - c3 dr^3, c1 = 3/(4w), c3 = 1/(4w^3)
@@ -89,6 +91,10 @@ struct ModelConst {
   float cutoff2;             // pair cutoff squared (<= 0: none)
   float pref;                // pair prefactor
   double h, buffer, cutoff;
+  // p / nq for a point id below 2^31 (exact: the magic's excess times p stays below 2^(31 + L))
+  __device__ __forceinline__ int point_atom(int p) const {
+    return nq > 1 ? (int)(__umulhi((unsigned)p, nq_magic) >> nq_shift) : p;
+  }
 };
 
 // One evaluation context (one force instance).
@@ -170,11 +176,11 @@ struct Context {
   int4* d_sgeom = nullptr;                    // cutoff: spatial grid geometry
   float* d_pstate = nullptr;                  // GBMV: per-point sums kept for the chain rule
   // GBMV points binned by lookup-table cell (k_gbmv.cu)
-  int* d_pcell = nullptr;                     // [n Q] the point's cell or -1
-  int* d_prank = nullptr;                     // [n Q] slot within the cell
+  int2* d_pat = nullptr;                      // [n Q] (the point's cell or -1, slot within the cell)
   int* d_porder = nullptr;                    // [n Q] point id per slot
   float* d_sval = nullptr;                    // [n Q] solvent fraction by point id
   int* d_pcount = nullptr;                    // [cell_cap] points per cell
+  int* d_plive = nullptr;                     // [cell_cap] of those, the chain rule's
   int* d_pstart = nullptr;                    // [cell_cap + 1] first slot per cell
   unsigned long long* d_ptotal = nullptr;     // [1] points binned
   bool gbmv_cells = false;                    // this call's GBMV passes run by cell

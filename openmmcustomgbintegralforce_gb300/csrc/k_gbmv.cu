@@ -41,6 +41,8 @@
 // FP32 difference is within a few tenths of a nanometre of the cell.
 #include <math.h>
 
+#include <type_traits>
+
 #include "bitonic.cuh"
 #include "gbx_internal.cuh"
 #include "queries.cuh"
@@ -61,10 +63,10 @@ static_assert(kChainPts * kChainEnt == kWarp && kChainPts == 4, "chain lane spli
 
 struct CellPoints {
   int* count;   // [cells] points binned into the cell
+  int* live;    // [cells] of those, the points the chain rule visits: first in the cell's slots
   int* start;   // [cells + 1] first slot
   int* order;   // [points] point id per slot, sorted within each cell by the integral pass
-  int* cell;    // [points] the point's cell or -1
-  int* rank;    // [points] the point's slot within its cell (atomic order)
+  int2* at;     // [points] (the point's cell or -1, its slot within the cell in atomic order)
   float* sval;  // [points] solvent fraction by point id
   float* state; // [planes][points] the point's sums by slot (GBMV-I: S; GBMV-II: s1, s2, vx, vy, vz)
   size_t plane;
@@ -127,10 +129,9 @@ __device__ __forceinline__ void bin_point(const CellPoints& cp, const Entries& t
                                           long long cell) {
   const int cnt = cell >= 0 ? __ldg(&tab.cell[cell].x) : 0;
   if (cnt > 0) {
-    cp.cell[p] = (int)cell;
-    cp.rank[p] = atomicAdd(&cp.count[cell], 1);
+    cp.at[p] = make_int2((int)cell, atomicAdd(&cp.count[cell], 1));
   } else {
-    cp.cell[p] = -1;
+    cp.at[p].x = -1;
     cp.sval[p] = empty_list_fraction<MODEL>(m);
   }
 }
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
   const float4 xi = pos[i];
   Q query;
   query.init(tab, xi, quad.qoff);
+  if constexpr (std::is_same<Q, BoxQuery>::value) query.set_reach(quad.qv[m.nrad - 1].w);  // the outermost point
   const int q0 = c * chunk, q1 = min(m.nq, q0 + chunk);
   const unsigned lt = (1u << lane) - 1u;
   int* defer = s_defer[wib];
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
     ndef = 0;
   };
   for (int base = q0; base < q1; base += kBinBatch * kWarp) {
-    long long cell[kBinBatch];
+    int cell[kBinBatch];
     int cnt[kBinBatch];
     bool late[kBinBatch];
 #pragma unroll
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
       cell[u] = -1;
       cnt[u] = 0;
       late[u] = false;
-      if (q < q1) cell[u] = query.cell_fast(quad.qv[q], late[u]);
+      if (q < q1) cell[u] = (int)query.cell_fast(quad.qv[q], late[u]);
       const unsigned dm = __ballot_sync(0xffffffffu, late[u]);
       if (late[u]) defer[ndef + __popc(dm & lt)] = q;
       ndef += __popc(dm);
@@ -201,10 +203,9 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
       const int q = base + u * kWarp + lane;
       const size_t p = (size_t)i * m.nq + q;
       if (cell[u] >= 0 && cnt[u] > 0) {
-        cp.cell[p] = (int)cell[u];
-        cp.rank[p] = slot[u];
+        cp.at[p] = make_int2(cell[u], slot[u]);
       } else if (q < q1 && !late[u]) {
-        cp.cell[p] = -1;
+        cp.at[p].x = -1;
         cp.sval[p] = empty_list_fraction<MODEL>(m);
       }
     }
@@ -213,11 +214,24 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
   if (ndef > 0) flush();
 }
 
-__global__ void gbmv_fill_kernel(long long npts, CellPoints cp) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= npts) return;
-  const int c = cp.cell[p];
-  if (c >= 0) cp.order[cp.start[c] + cp.rank[p]] = (int)p;
+// Two points per 16-byte load, kFillLoads loads in flight per thread.
+constexpr int kFillLoads = 4;
+__global__ void __launch_bounds__(256) gbmv_fill_kernel(long long npts, CellPoints cp) {
+  const long long pair0 = (long long)blockIdx.x * blockDim.x * kFillLoads + threadIdx.x;
+  int4 v[kFillLoads];
+#pragma unroll
+  for (int u = 0; u < kFillLoads; ++u) {
+    const long long p = 2 * (pair0 + (long long)u * blockDim.x);
+    v[u] = make_int4(-1, 0, -1, 0);
+    if (p + 1 < npts) v[u] = __ldcs(reinterpret_cast<const int4*>(cp.at + p));
+    else if (p < npts) v[u].x = cp.at[p].x, v[u].y = cp.at[p].y;
+  }
+#pragma unroll
+  for (int u = 0; u < kFillLoads; ++u) {
+    const long long p = 2 * (pair0 + (long long)u * blockDim.x);
+    if (v[u].x >= 0) cp.order[cp.start[v[u].x] + v[u].y] = (int)p;
+    if (v[u].z >= 0) cp.order[cp.start[v[u].z] + v[u].w] = (int)p + 1;
+  }
 }
 
 template <int E>
@@ -261,17 +275,22 @@ __device__ __forceinline__ float2 rcp2(float2 t) { return make_float2(rcp_ftz(t.
 // packed FP32x2 arithmetic (__ffma2_rn and friends: one instruction for two
 // entries, each half rounded as its scalar form).  A list whose length is
 // not a multiple of four is padded with entries whose every contribution is
-// exactly zero (C = 0 for GBMV-II, gamma = 0 for GBMV-I's chain;
-// T = 100 r^2 + 1 >= 1), index -1.
+// exactly zero (C = 0 for GBMV-II; T = 100 r^2 + 1 >= 1).
 struct __align__(16) CellList {
   float x[kMaxList], y[kMaxList], z[kMaxList];  // x_j - c0
   float w[kMaxList];    // GBMV-II C_j | GBMV-I gamma_j
   float k[kMaxList];    // GBMV-II C_j - 100 R_j^2 | GBMV-I R_j
-  float r[kMaxList];    // GBMV-II R_j
-  int idx[kMaxList];    // atom index
 };
 
-__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+// The chain rule's copy: pairs of entries, read as three 16-byte words per
+// pair (five fields and the indices read one by one held the load pipe).
+struct __align__(16) ChainPair {
+  float2 x, y, z;  // x_j - c0
+  float2 w;        // GBMV-II C_j | GBMV-I gamma_j
+  float2 k;        // GBMV-II C_j - 100 R_j^2 | GBMV-I R_j
+  int2 idx;        // atom index
+};
+
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
@@ -288,20 +307,16 @@ __device__ __forceinline__ void stage_list(CellList& L, const Entries& tab, int2
       L.z[l] = a.z - c0.z;
       L.w[l] = a.w;
       L.k[l] = pk.x;
-      L.r[l] = pk.y;
-      L.idx[l] = __ldg(tab.index + cs.y + l);
     } else {
       L.x[l] = L.y[l] = L.z[l] = 0.0f;
       L.w[l] = 0.0f;
       L.k[l] = 1.0f;
-      L.r[l] = 1.0f;
-      L.idx[l] = -1;
     }
   }
 }
 
 template <int MODEL, bool PER>
-__global__ void __launch_bounds__(kCellThreads) gbmv_cell_integral_kernel(const float4* __restrict__ pos, Entries tab,
+__global__ void __launch_bounds__(kCellThreads, 8) gbmv_cell_integral_kernel(const float4* __restrict__ pos, Entries tab,
                                                                           Quad quad, ModelConst m, CellPoints cp) {
   __shared__ CellList s_list[kCellWarps];
   const int w = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
@@ -324,11 +339,12 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_integral_kernel(const 
   // GBMV-II's padding entries add exactly zero; GBMV-I's (e^0 = 1) do not,
   // so its last (cnt mod 4) entries are taken one at a time
   const int nquad = MODEL == GBX_MODEL_GBMV2 ? (cnt + 3) >> 2 : cnt >> 2;
+  int kept = 0;  // warp-uniform: points of the cell the chain rule visits
   for (int base = 0; base < P; base += kWarp) {
     const int k = base + lane;
     const bool valid = k < P;
     const int p = valid ? order[k] : 0;
-    const int i = p / m.nq, q = p - i * m.nq;
+    const int i = m.point_atom(p), q = p - i * m.nq;
     const float4 xi = __ldg(pos + i), v = __ldg(quad.qv + q);
     const float px = (xi.x - c0.x) + v.x, py = (xi.y - c0.y) + v.y, pz = (xi.z - c0.z) + v.z;
     const float2 npx = bc2(-px), npy = bc2(-py), npz = bc2(-pz);
@@ -366,6 +382,11 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_integral_kernel(const 
         s.s1 += __expf(L.w[l] * (r2 * r2));
       }
     }
+    // Only a point whose solvent fraction still varies pulls on anything (a
+    // saturated one, 57 in 100 at 10,000 atoms, has an exactly zero
+    // derivative): the chain rule's points and their sums are packed to those,
+    // in order, over the slots already read.
+    bool live = false;
     if (valid) {
       float pl, S;
       if (MODEL == GBX_MODEL_GBMV1) {
@@ -375,7 +396,13 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_integral_kernel(const 
         S = m.s0 * s.s1 * s.s2 / s3sq;
       }
       cp.sval[p] = logistic_solvent(m.beta, m.lambda, S, pl);
-      float* st = cp.state + start + k;
+      live = logistic_slope(m.beta, pl) != 0.0f;
+    }
+    const unsigned lm = __ballot_sync(0xffffffffu, live);
+    if (live) {
+      const int slot = kept + __popc(lm & ((1u << lane) - 1u));
+      order[slot] = p;
+      float* st = cp.state + start + slot;
       st[0] = s.s1;
       if (MODEL == GBX_MODEL_GBMV2) {
         st[cp.plane] = s.s2;
@@ -384,7 +411,10 @@ __global__ void __launch_bounds__(kCellThreads) gbmv_cell_integral_kernel(const 
         st[4 * cp.plane] = s.vz;
       }
     }
+    kept += __popc(lm);
+    __syncwarp();
   }
+  if (lane == 0) cp.live[cell] = kept;
 }
 
 // J4, J7 per (atom, chunk) over the solvent fractions, in quadrature order.
@@ -449,35 +479,61 @@ struct __align__(16) PointChain {
   int i;
 };
 
-// Registers are capped where the occupancy measured fastest (10,000 atoms, 24 x 50:
-// GBMV-II 532, 488, 471 us with 5, 6, 7 blocks per SM; GBMV-I 467, 487, 510 with 6, 7, 8).
+// One warp (cell) per block: cells differ several-fold in points, and a block of
+// four held its registers until its slowest warp was done.  Registers are
+// capped where the occupancy measured fastest (10,000 atoms, 24 x 50, with 24,
+// 28, 32 blocks per SM: GBMV-II 381, 360, 369 us; GBMV-I 453, 416, 406 us;
+// four-warp blocks 405 and 446 us).
+constexpr int kChainWarps = 1;
 template <int MODEL, bool PER, bool ADJ>
-__global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBMV2 ? 7 : 6) gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab,
+__global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 16 : MODEL == GBX_MODEL_GBMV2 ? 28 : 32)
+    gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab,
                                                                        Quad quad, ModelConst m, CellPoints cp,
                                                                        const float2* __restrict__ dEdJ,
                                                                        CellChainOut out) {
-  __shared__ CellList s_list[kCellWarps];
-  __shared__ PointChain s_pt[kCellWarps][kWarp];
-  __shared__ float3 s_own[kCellWarps][kWarp];
+  __shared__ ChainPair s_list[kChainWarps][kMaxList / 2];
+  __shared__ float2 s_r[ADJ ? kChainWarps : 1][ADJ ? kMaxList / 2 : 1];  // R_j of the pairs
+  __shared__ PointChain s_pt[kChainWarps][kWarp];
+  __shared__ float3 s_own[kChainWarps][kWarp];
   const int w = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-  const long long cell = (long long)blockIdx.x * kCellWarps + w;
+  const long long cell = (long long)blockIdx.x * kChainWarps + w;
   const TableGeom& G = *tab.geom;
   if (cell >= G.ncell || cell >= tab.cell_cap) return;
-  const int P = cp.count[cell];
+  const int binned = cp.count[cell];
+  if (binned == 0) return;
+  const int P = cp.live[cell];
   if (P == 0) return;
   const int2 cs = __ldg(tab.cell + cell);
   const int cnt = min(cs.x, kMaxList);
   const float3 c0 = cell_corner(G, (int)cell);
   Image<PER> img;
   img.init(G);
-  CellList& L = s_list[w];
-  stage_list<PER>(L, tab, cs, cnt, c0, lane);
+  ChainPair* L = s_list[w];
+  for (int l = lane; l < ((cnt + 1) & ~1); l += kWarp) {
+    float4 a = make_float4(c0.x, c0.y, c0.z, 0.0f);  // padding: every contribution exactly zero
+    float2 pk = make_float2(1.0f, 1.0f);
+    int k = -1;
+    if (l < cnt) {
+      a = __ldg(tab.e + cs.y + l);
+      pk = __ldg(tab.par + cs.y + l);
+      k = __ldg(tab.index + cs.y + l);
+    }
+    float* f = reinterpret_cast<float*>(L + l / 2) + (l & 1);
+    f[0] = a.x - c0.x;
+    f[2] = a.y - c0.y;
+    f[4] = a.z - c0.z;
+    f[6] = a.w;
+    f[8] = pk.x;
+    f[10] = __int_as_float(k);
+    if (ADJ) reinterpret_cast<float*>(s_r[w] + l / 2)[l & 1] = pk.y;
+  }
+  __syncwarp();
   const int start = cp.start[cell];
   const int* order = cp.order + start;
   const float* state = cp.state + start;
   // cells too dense to sort keep the atomic slot order: every contribution
   // is then reduced on its own (integer sums, independent of the order)
-  const bool sorted = P <= kSortMax;
+  const bool sorted = binned <= kSortMax;
   // lane (ps, es): point ps of each group of kChainPts, entry pairs es, es +
   // kChainEnt, ... (entries 2 j and 2 j + 1 of pair j)
   const int ps = lane / kChainEnt, es = lane % kChainEnt;
@@ -503,7 +559,7 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
       pc.Vx = pc.Vy = pc.Vz = bc2(0.f);
       if (k < P) {
         const int p = order[k];
-        const int i = p / m.nq, q = p - i * m.nq;
+        const int i = m.point_atom(p), q = p - i * m.nq;
         const float4 xi = __ldg(pos + i), v = __ldg(quad.qv + q);
         const float2 wq = __ldg(quad.qw + q);
         const float2 de = __ldg(dEdJ + i);
@@ -515,14 +571,14 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
         float pl;
         if (MODEL == GBX_MODEL_GBMV1) {
           logistic_solvent(m.beta, m.lambda, state[k], pl);
-          pc.cS = cq * __fdividef(m.beta * pl, (1.0f + pl) * (1.0f + pl));
+          pc.cS = cq * logistic_slope(m.beta, pl);
           pc.A = bc2(4.0f * pc.cS);
         } else {
           const float s1 = state[k], s2 = state[k + cp.plane], vx = state[k + 2 * cp.plane],
                       vy = state[k + 3 * cp.plane], vz = state[k + 4 * cp.plane];
           const float s3sq = fmaf(vx, vx, fmaf(vy, vy, vz * vz));
           logistic_solvent(m.beta, m.lambda, m.s0 * s1 * s2 / s3sq, pl);
-          pc.cS = cq * __fdividef(m.beta * pl, (1.0f + pl) * (1.0f + pl)) * m.s0;
+          pc.cS = cq * logistic_slope(m.beta, pl) * m.s0;
           const float inv3 = 1.0f / s3sq;
           const float A = pc.cS * (s2 * inv3), B = 2.0f * pc.cS * (s1 * inv3),
                       C = 2.0f * pc.cS * (-s1 * s2 * inv3 * inv3);
@@ -533,9 +589,8 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
           pc.Vz = bc2(C * vz);
         }
       }
-      // only points with a nonzero factor pull on anything (a saturated
-      // solvent fraction gives exact zeros): they are packed in order, so
-      // the sums see the same nonzero terms in the same order
+      // a point whose factor came out zero after all (c = 0, an underflow) is
+      // left out, the rest keep their order
       const unsigned lm = __ballot_sync(0xffffffffu, pc.cS != 0.0f);
       if (pc.cS != 0.0f) pts[__popc(lm & ((1u << lane) - 1u))] = pc;
       np = __popc(lm);
@@ -543,8 +598,8 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
     __syncwarp();
     for (int sub = 0; sub < np; sub += kChainPts) {
       const int t = sub + ps;
-      const PointChain& pc = pts[t < np ? t : 0];
-      const bool live = t < np && pc.cS != 0.0f;
+      const PointChain pc = pts[t < np ? t : 0];
+      const bool live = t < np;
       float2 ox = bc2(0.f), oy = bc2(0.f), oz = bc2(0.f);
       if (live) {
         const int pi = pc.i;
@@ -616,11 +671,10 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
         };
 #pragma unroll
         for (int e = 0; e < kPairsPerLane; ++e) {
-          const int l = 2 * (es + e * kChainEnt);
+          const int j = es + e * kChainEnt, l = 2 * j;
           if (l < cnt) {
-            const float2 R2 = ADJ && MODEL == GBX_MODEL_GBMV2 ? ld2(L.r + l) : bc2(0.f);
-            pair(e, l, ld2(L.x + l), ld2(L.y + l), ld2(L.z + l), ld2(L.w + l), ld2(L.k + l), R2,
-                 *reinterpret_cast<const int2*>(L.idx + l));
+            const ChainPair c = L[j];
+            pair(e, l, c.x, c.y, c.z, c.w, c.k, ADJ ? s_r[w][j] : bc2(0.f), c.idx);
           }
         }
       }
@@ -666,6 +720,7 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
   // lanes, one fixed-point reduction per entry
 #pragma unroll
   for (int e = 0; e < kPairsPerLane; ++e) {
+    if (2 * e * kChainEnt >= cnt) break;
 #pragma unroll
     for (int off = kChainEnt; off < kWarp; off <<= 1) {
 #pragma unroll
@@ -684,8 +739,9 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
     const float2 sum = ps == 0 ? acc[e][0] : ps == 1 ? acc[e][1] : ps == 2 ? acc[e][2] : accR[e];
     if (ps < 3 || ADJ) {
       const float sign = ps < 3 ? -1.0f : 1.0f;
-      if (l < cnt) add_fixed_one(out, L.idx[l], ps, sign * sum.x);
-      if (l + 1 < cnt) add_fixed_one(out, L.idx[l + 1], ps, sign * sum.y);
+      const int2 k = L[es + e * kChainEnt].idx;
+      if (l < cnt) add_fixed_one(out, k.x, ps, sign * sum.x);
+      if (l + 1 < cnt) add_fixed_one(out, k.y, ps, sign * sum.y);
     }
   }
 }
@@ -695,7 +751,7 @@ __global__ void __launch_bounds__(kCellThreads, ADJ ? 4 : MODEL == GBX_MODEL_GBM
 // The cell passes apply to the GBMV models on a table capped at kMaxList.
 bool gbmv_cells_apply(const Context* ctx) {
   const gbx_config& c = ctx->cfg;
-  return c.model != GBX_MODEL_GBSW && c.table_cap >= 1 && c.table_cap <= kMaxList && ctx->d_pcell != nullptr &&
+  return c.model != GBX_MODEL_GBSW && c.table_cap >= 1 && c.table_cap <= kMaxList && ctx->d_pat != nullptr &&
          ctx->d_pcount != nullptr &&
          (long long)ctx->n * (c.n_radial * c.lebedev_order) < 0x7fffffffLL;
 }
@@ -713,22 +769,23 @@ gbx_status launch_gbmv_cells_bin(Context* ctx, const float4* pos, const ModelCon
   const Quad qd{ctx->d_qv, ctx->d_qw, ctx->d_qoff};
   const int chunk = (m.nq + ctx->n_chunks - 1) / ctx->n_chunks;
   const long long npts = (long long)ctx->n * m.nq;
-  const CellPoints cp{ctx->d_pcount, ctx->d_pstart, ctx->d_porder, ctx->d_pcell, ctx->d_prank,
+  const CellPoints cp{ctx->d_pcount, ctx->d_plive, ctx->d_pstart, ctx->d_porder, ctx->d_pat,
                       ctx->d_sval,   ctx->d_pstate, (size_t)npts};
   const long long warps = (long long)ctx->n * ctx->n_chunks;
   const int bin_blocks = (int)((warps * kWarp + kBinThreads - 1) / kBinThreads);
   const long long cells = ctx->cell_cap;
-  const bool per = ctx->cfg.periodic != 0;
+  const bool box = m.table_mode == GBX_TABLE_PERIODIC;  // a point's cell does not depend on minimum images
   if (m.model == GBX_MODEL_GBMV1) {
-    if (per) gbmv_bin_kernel<GBX_MODEL_GBMV1, MinImageQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
+    if (box) gbmv_bin_kernel<GBX_MODEL_GBMV1, BoxQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
     else gbmv_bin_kernel<GBX_MODEL_GBMV1, RefQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
   } else {
-    if (per) gbmv_bin_kernel<GBX_MODEL_GBMV2, MinImageQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
+    if (box) gbmv_bin_kernel<GBX_MODEL_GBMV2, BoxQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
     else gbmv_bin_kernel<GBX_MODEL_GBMV2, RefQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
   }
   launch_scan<false>(ctx->d_pcount, ctx->d_geom, ctx->d_pstart, nullptr, cells, 0x7fffffffffffLL, ctx->d_ptotal,
                      ctx->d_status, st);
-  gbmv_fill_kernel<<<(int)((npts + 255) / 256), 256, 0, st>>>(npts, cp);
+  constexpr int per_block = 2 * kFillLoads * 256;
+  gbmv_fill_kernel<<<(int)((npts + per_block - 1) / per_block), 256, 0, st>>>(npts, cp);
   ctx->launches += 3;  // bin, scan, fill
   return GBX_OK;
 }
@@ -739,7 +796,7 @@ gbx_status launch_gbmv_cells_integral(Context* ctx, const float4* pos, const Mod
   const Quad qd{ctx->d_qv, ctx->d_qw, ctx->d_qoff};
   const int chunk = (m.nq + ctx->n_chunks - 1) / ctx->n_chunks;
   const long long npts = (long long)ctx->n * m.nq;
-  const CellPoints cp{ctx->d_pcount, ctx->d_pstart, ctx->d_porder, ctx->d_pcell, ctx->d_prank,
+  const CellPoints cp{ctx->d_pcount, ctx->d_plive, ctx->d_pstart, ctx->d_porder, ctx->d_pat,
                       ctx->d_sval,   ctx->d_pstate, (size_t)npts};
   const long long warps = (long long)ctx->n * ctx->n_chunks;
   const int bin_blocks = (int)((warps * kWarp + kBinThreads - 1) / kBinThreads);
@@ -763,21 +820,21 @@ gbx_status launch_gbmv_cells_chain(Context* ctx, const float4* pos, const ModelC
   const Entries t = gbmv_entries(ctx);
   const Quad qd{ctx->d_qv, ctx->d_qw, ctx->d_qoff};
   const long long npts = (long long)ctx->n * m.nq;
-  const CellPoints cp{ctx->d_pcount, ctx->d_pstart, ctx->d_porder, ctx->d_pcell, ctx->d_prank,
+  const CellPoints cp{ctx->d_pcount, ctx->d_plive, ctx->d_pstart, ctx->d_porder, ctx->d_pat,
                       ctx->d_sval,   ctx->d_pstate, (size_t)npts};
   const CellChainOut o{ctx->d_f4};
-  const int cell_blocks = (int)((ctx->cell_cap + kCellWarps - 1) / kCellWarps);
+  const int cell_blocks = (int)((ctx->cell_cap + kChainWarps - 1) / kChainWarps);
   const bool per = ctx->cfg.periodic != 0;
   const int sel = (m.model == GBX_MODEL_GBMV1 ? 0 : 4) + (per ? 2 : 0) + (adjoint ? 1 : 0);
   switch (sel) {
-    case 0: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, false><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 1: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, true><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 2: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, false><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 3: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, true><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 4: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, false><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 5: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, true><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 6: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, false><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    default: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, true><<<cell_blocks, kCellThreads, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    case 0: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    case 1: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    case 2: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    case 3: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    case 4: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    case 5: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    case 6: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+    default: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
   }
   ++ctx->launches;
   return GBX_OK;

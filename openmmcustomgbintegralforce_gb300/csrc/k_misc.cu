@@ -15,6 +15,10 @@ ModelConst make_model_const(const Context* ctx) {
   m.skip_empty = c.skip_empty;
   m.nq = c.n_radial * c.lebedev_order;
   m.nrad = c.n_radial;
+  int bits = 1;
+  while ((1LL << bits) < m.nq) ++bits;
+  m.nq_magic = (unsigned)(((1ULL << (31 + bits)) + m.nq - 1) / m.nq);
+  m.nq_shift = bits - 1;
   m.cutoff_chain_quirk = c.cutoff_chain_quirk;
   const double w = c.switch_width;
   m.sw = (float)w;

@@ -147,6 +147,50 @@ struct RefQuery {
   }
 };
 
+// The same query of a box-sampled table (GBX_TABLE_PERIODIC), for passes that
+// only look cells up: an atom whose every point stays inside the box needs no
+// move; a cell face is detected by one compare over the axes (the box edges
+// are cell faces too); floor by adding 1.5 2^23 rounding down, at full rate
+// (the general form's rounding and conversion instructions run at a quarter).
+struct BoxQuery : RefQuery {
+  bool inside;  // no point of the atom leaves the box
+  __device__ __forceinline__ void init(const Entries& t, const float4 xi, const double* qo) {
+    RefQuery::init(t, xi, qo);
+    inside = false;
+  }
+  // reach: the largest radius of the rule's points (nm)
+  __device__ __forceinline__ void set_reach(float reach) {
+    inside = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float r = fmaf(reach, inv[k], 0.01f);
+      inside = inside && rel[k] - r > 0.0f && rel[k] + r < (float)g->dims[k];
+    }
+  }
+  __device__ __forceinline__ int cell_fast(const float4 v, bool& unsafe) const {
+    unsafe = false;
+    if (off) return -1;
+    float t[3] = {fmaf(v.x, inv[0], rel[0]), fmaf(v.y, inv[1], rel[1]), fmaf(v.z, inv[2], rel[2])};
+    const int d[3] = {g->dims[0], g->dims[1], g->dims[2]};
+    if (!inside) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) t[k] = fmaf(-floorf(t[k] * invdims[k]), (float)d[k], t[k]);
+    }
+    int id[3];
+    float face = 0.0f;  // the largest distance from a cell's middle along an axis
+    bool in = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float m = __fadd_rd(t[k], 12582912.0f);
+      id[k] = __float_as_int(m) - 0x4B400000;
+      face = fmaxf(face, fabsf((t[k] - (m - 12582912.0f)) - 0.5f));
+      in = in && (unsigned)id[k] < (unsigned)d[k];
+    }
+    unsafe = !in || face > 0.5f - eps;
+    return unsafe ? -1 : (id[0] * d[1] + id[1]) * d[2] + id[2];
+  }
+};
+
 // A box-sampled (periodic-branch) table of a CutoffPeriodic system: the
 // reference query, distances by minimum image (the integral classes with
 // CutoffPeriodic, GBMVIntegralTypeI.cpp:59-62, TypeII.cpp:64-67,
@@ -414,6 +458,11 @@ __device__ __forceinline__ float4 entry_at(const Entries& t, int at) {
   } else {
     return __ldg(t.e + at);
   }
+}
+
+// ds/dS of the logistic below, from its p
+__device__ __forceinline__ float logistic_slope(float beta, float p) {
+  return __fdividef(beta * p, (1.0f + p) * (1.0f + p));
 }
 
 // s = p / (1 + p) with p = exp(beta (S - lambda)): the solvent fraction
