@@ -20,6 +20,8 @@ import torch
 from ._lib import EXEC_CHECK, Context
 from .spec import GBModel
 
+_LEGACY_STREAM = 1  # cudaStreamLegacy: torch's default stream
+
 
 class GBEnergyFunction(torch.autograd.Function):
     """E = GB(positions [n,3], charges [n], radii [n], alpha [2]) on one context."""
@@ -31,31 +33,41 @@ class GBEnergyFunction(torch.autograd.Function):
         n = gb.n
         if positions.shape != (n, 3) or charges.shape != (n,) or radii.shape != (n,) or alpha.shape != (2,):
             raise ValueError("GBEnergyFunction: expected positions [n,3], charges [n], radii [n], alpha [2]")
-        gb.set_particle_parameters(charges.detach().double().cpu().numpy(), radii.detach().double().cpu().numpy())
-        a = alpha.detach().double().cpu().numpy()
-        gb.set_global_parameters(float(a[0]), float(a[1]))
+        # one transfer for the three parameter tensors, one allocation for every
+        # output, one product for every gradient: the call's host work is
+        # torch operations, each of them 5 to 30 us
+        parts = [t.detach() for t in (charges, radii, alpha)]
+        if len({(t.dtype, t.device) for t in parts}) > 1:
+            parts = [t.to(positions.device, torch.float64) for t in parts]
+        p = torch.cat(parts).to("cpu", torch.float64).numpy()
+        gb.set_particle_parameters(p[:n], p[n:2 * n])
+        gb.set_global_parameters(float(p[2 * n]), float(p[2 * n + 1]))
         dev = positions.device
-        posq = torch.zeros((n, 4), dtype=torch.float32, device=dev)
-        posq[:, :3] = positions.detach().to(torch.float32)
-        f64 = dict(dtype=torch.float64, device=dev)
-        energy = torch.zeros(1, **f64)
-        forces = torch.zeros((n, 3), **f64)
-        dq = torch.zeros(n, **f64)
-        dR = torch.zeros(n, **f64)
-        da = torch.zeros(2, **f64)
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        gb.adjoint_device(posq.data_ptr(), energy.data_ptr(), forces.data_ptr(), dq.data_ptr(), dR.data_ptr(),
-                          da.data_ptr(), EXEC_CHECK if check else 0, stream)
-        ctx.save_for_backward(forces, dq, dR, da)
+        posq = torch.empty((n, 4), dtype=torch.float32, device=dev)  # w is not read
+        posq[:, :3] = positions.detach()
+        # energy | forces [n, 3] | dE/dq [n] | dE/dR [n] | dE/dalpha [2]
+        out = torch.empty(3 + 5 * n, dtype=torch.float64, device=dev)
+        at = out.data_ptr()
+        # the default stream by its own handle: 0 would be the context's stream,
+        # which nothing orders after the copy into posq
+        stream = torch.cuda.current_stream(dev).cuda_stream or _LEGACY_STREAM
+        gb.adjoint_device(posq.data_ptr(), at, at + 8, at + 8 * (1 + 3 * n), at + 8 * (1 + 4 * n),
+                          at + 8 * (1 + 5 * n), EXEC_CHECK if check else 0, stream)
+        ctx.save_for_backward(out)
+        ctx.n = n
         ctx.dtypes = (positions.dtype, charges.dtype, radii.dtype, alpha.dtype)
-        return energy[0].to(positions.dtype)
+        return out[0].to(positions.dtype)
 
     @staticmethod
     def backward(ctx, grad):
-        forces, dq, dR, da = ctx.saved_tensors
-        g = grad.to(torch.float64)
+        (out,) = ctx.saved_tensors
+        n = ctx.n
+        g = out * grad.to(torch.float64)
         tp, tq, tr, ta = ctx.dtypes
-        return (-forces * g).to(tp), (dq * g).to(tq), (dR * g).to(tr), (da * g).to(ta), None, None
+        if tp == tq == tr == ta:
+            g = g.to(tp)
+        dx, dq, dR, da = g[1:].split((3 * n, n, n, 2))
+        return (-dx).view(n, 3).to(tp), dq.to(tq), dR.to(tr), da.to(ta), None, None
 
 
 class GBEnergy(torch.nn.Module):

@@ -189,14 +189,18 @@ int choose_chunks(int n, int Q, int sms) {
   return c;
 }
 
+constexpr size_t kParamBytes = sizeof(double) + sizeof(float2) + 2 * sizeof(float);
+
 gbx_status alloc_atom_buffers(Context* ctx) {
   const int n = ctx->n;
   const int Q = ctx->cfg.n_radial * ctx->cfg.lebedev_order;
   ctx->n_chunks = choose_chunks(n, Q, ctx->sms);
-  GBX_TRY(dalloc(ctx, &ctx->d_radius, n));
-  GBX_TRY(dalloc(ctx, &ctx->d_charge, n));
-  GBX_TRY(dalloc(ctx, &ctx->d_par, n));
-  GBX_TRY(dalloc(ctx, &ctx->d_wpar, n));
+  // the per-atom parameters in one block, uploaded by one copy
+  GBX_TRY(dalloc(ctx, &ctx->d_params, kParamBytes * (size_t)n));
+  ctx->d_radius = reinterpret_cast<double*>(ctx->d_params);
+  ctx->d_par = reinterpret_cast<float2*>(ctx->d_radius + n);
+  ctx->d_wpar = reinterpret_cast<float*>(ctx->d_par + n);
+  ctx->d_charge = ctx->d_wpar + n;
   GBX_TRY(dalloc(ctx, &ctx->d_pos, n));
   GBX_TRY(dalloc(ctx, reinterpret_cast<unsigned char**>(&ctx->d_parts), gbx::prepare_scratch_bytes(n)));
   GBX_TRY(dalloc(ctx, &ctx->d_ticket, 1));
@@ -538,11 +542,9 @@ gbx_status run_pipeline(Context* ctx, const float4* posq, unsigned long long* fo
   return GBX_OK;
 }
 
-void set_model_params(Context* ctx, std::vector<float>& wpar, std::vector<float2>& par) {
+void set_model_params(const Context* ctx, float* wpar, float2* par) {
   const gbx_config& c = ctx->cfg;
   const int n = ctx->n;
-  wpar.resize(n);
-  par.resize(n);
   for (int i = 0; i < n; ++i) {
     const double R = ctx->radius[i];
     if (c.model == GBX_MODEL_GBSW) {
@@ -778,7 +780,7 @@ gbx_status gbx_destroy(gbx_context* handle) {
   if (!ctx) return GBX_ERR_INVALID_ARGUMENT;
   drop_graph(ctx);
   gbx::custom_destroy(ctx);
-  void* ptrs[] = {ctx->d_qv, ctx->d_qw, ctx->d_qoff, ctx->d_radius, ctx->d_charge, ctx->d_par, ctx->d_wpar,
+  void* ptrs[] = {ctx->d_qv, ctx->d_qw, ctx->d_qoff, ctx->d_params,
                   ctx->d_geom, ctx->d_cell_count, ctx->d_cell_start, ctx->d_cell_cursor, ctx->d_entries,
                   ctx->d_parts, ctx->d_ticket, ctx->d_pos, ctx->d_J, ctx->d_born, ctx->d_bornf, ctx->d_dBdJ,
                   ctx->d_integrals, ctx->d_dEdB_fx, ctx->d_dEdJ, ctx->d_energy_part, ctx->d_force_fx, ctx->d_f4,
@@ -826,14 +828,15 @@ gbx_status gbx_set_particle_parameters(gbx_context* handle, const double* charge
   }
   ctx->charge.assign(charge, charge + n);
   ctx->radius.assign(radius, radius + n);
-  std::vector<float> qf(n), wpar;
-  std::vector<float2> par;
+  std::vector<unsigned char> block(kParamBytes * (size_t)n);
+  double* r = reinterpret_cast<double*>(block.data());
+  float2* par = reinterpret_cast<float2*>(r + n);
+  float* wpar = reinterpret_cast<float*>(par + n);
+  float* qf = wpar + n;
+  memcpy(r, radius, sizeof(double) * n);
   for (int i = 0; i < n; ++i) qf[i] = (float)charge[i];
   set_model_params(ctx, wpar, par);
-  GBX_CUDA(cudaMemcpy(ctx->d_radius, radius, sizeof(double) * n, cudaMemcpyHostToDevice));
-  GBX_CUDA(cudaMemcpy(ctx->d_charge, qf.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-  GBX_CUDA(cudaMemcpy(ctx->d_wpar, wpar.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-  GBX_CUDA(cudaMemcpy(ctx->d_par, par.data(), sizeof(float2) * n, cudaMemcpyHostToDevice));
+  GBX_CUDA(cudaMemcpy(ctx->d_params, block.data(), block.size(), cudaMemcpyHostToDevice));
   gbx::choose_table(ctx);
   return GBX_OK;
 }
@@ -1324,11 +1327,28 @@ gbx_status gbx_adjoint(gbx_context* handle, const void* posq, double* energy, do
   }
   ctx->stream = stream ? (cudaStream_t)stream : ctx->own_stream;
   const int n = ctx->n;
-  GBX_CUDA(cudaMemsetAsync(ctx->d_force_fx, 0, sizeof(unsigned long long) * 3 * n, ctx->stream));
-  GBX_CUDA(cudaMemsetAsync(ctx->d_energy, 0, sizeof(double), ctx->stream));
-  const bool check = (flags & GBX_EXEC_CHECK) || (ctx->use_tight ? ctx->tcell_cap == 0 : ctx->cell_cap == 0);
-  GBX_TRY(run_pipeline(ctx, reinterpret_cast<const float4*>(posq), ctx->d_force_fx, n, ctx->d_energy, check, true,
-                       false));
+  auto evaluate = [&](bool check) -> gbx_status {
+    GBX_CUDA(cudaMemsetAsync(ctx->d_force_fx, 0, sizeof(unsigned long long) * 3 * n, ctx->stream));
+    GBX_CUDA(cudaMemsetAsync(ctx->d_energy, 0, sizeof(double), ctx->stream));
+    return run_pipeline(ctx, reinterpret_cast<const float4*>(posq), ctx->d_force_fx, n, ctx->d_energy, check, true,
+                        false);
+  };
+  if ((flags & GBX_EXEC_CHECK) && tables_sized(ctx)) {
+    // checked, but with one wait at the end instead of one more for the table:
+    // a table that outgrew its buffers is evaluated again
+    GBX_TRY(evaluate(false));
+    GBX_CUDA(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    GBX_CUDA(cudaStreamSynchronize(ctx->stream));
+    const unsigned st = *ctx->h_status;
+    if (st & (gbx::kStatusTableCells | gbx::kStatusTableEntries | gbx::kStatusSegmentTooLong)) {
+      GBX_TRY(evaluate(true));
+    } else if (st & gbx::kStatusNonFinite) {
+      ctx->last_error = "non-finite Born radius";
+      return GBX_ERR_NONFINITE;
+    }
+  } else {
+    GBX_TRY(evaluate((flags & GBX_EXEC_CHECK) || (ctx->use_tight ? ctx->tcell_cap == 0 : ctx->cell_cap == 0)));
+  }
   return gbx::launch_adjoint_out(ctx, energy, forces, dEdq, dEdR, dEdalpha);
 }
 

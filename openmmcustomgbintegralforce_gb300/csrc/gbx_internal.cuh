@@ -115,6 +115,7 @@ struct Context {
 
   // particle data
   std::vector<double> charge, radius;
+  unsigned char* d_params = nullptr;  // one block: the four arrays below
   double* d_radius = nullptr;  // FP64 radii (table geometry)
   float* d_charge = nullptr;
   float2* d_par = nullptr;     // secondary model parameters per atom
