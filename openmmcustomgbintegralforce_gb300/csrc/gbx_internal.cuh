@@ -46,6 +46,7 @@ struct TableGeom {
   double inv_box[3];   // queries: formed once here, not per lane in FP64
   double pad;       // standalone uniform pad
   double L;         // periodic: max(step)
+  double reach;     // the quadrature's outer radius: no point is farther from its atom
   int dims[3];
   int mode;
   long long ncell;

@@ -41,8 +41,6 @@
 // FP32 difference is within a few tenths of a nanometre of the cell.
 #include <math.h>
 
-#include <type_traits>
-
 #include "bitonic.cuh"
 #include "gbx_internal.cuh"
 #include "queries.cuh"
@@ -158,7 +156,6 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
   const float4 xi = pos[i];
   Q query;
   query.init(tab, xi, quad.qoff);
-  if constexpr (std::is_same<Q, BoxQuery>::value) query.set_reach(quad.qv[m.nrad - 1].w);  // the outermost point
   const int q0 = c * chunk, q1 = min(m.nq, q0 + chunk);
   const unsigned lt = (1u << lane) - 1u;
   int* defer = s_defer[wib];
@@ -190,14 +187,22 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
 #pragma unroll
     for (int u = 0; u < kBinBatch; ++u)
       if (cell[u] >= 0) cnt[u] = __ldg(&tab.cell[cell[u]].x);
-    // one slot atomic per listed point (the warp's points mostly fall in
-    // distinct cells: aggregating them by __match_any_sync measured slower)
+    // Neighbouring lanes hold neighbouring points of a ray: a run of lanes in one
+    // cell takes its slots with one atomic, as consecutive slots
     int slot[kBinBatch];
+    int run[kBinBatch];  // the lane that starts this lane's run
 #pragma unroll
     for (int u = 0; u < kBinBatch; ++u) {
+      const int before = __shfl_up_sync(0xffffffffu, cell[u], 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || cell[u] != before);
+      run[u] = 31 - __clz((int)(heads & (lt | (1u << lane))));
+      const unsigned later = heads & ~(lt | (1u << lane));
+      const int len = (later ? __ffs((int)later) - 1 : kWarp) - lane;  // of a run's first lane
       slot[u] = 0;
-      if (cell[u] >= 0 && cnt[u] > 0) slot[u] = atomicAdd(&cp.count[cell[u]], 1);
+      if (run[u] == lane && cell[u] >= 0 && cnt[u] > 0) slot[u] = atomicAdd(&cp.count[cell[u]], len);
     }
+#pragma unroll
+    for (int u = 0; u < kBinBatch; ++u) slot[u] = __shfl_sync(0xffffffffu, slot[u], run[u]) + lane - run[u];
 #pragma unroll
     for (int u = 0; u < kBinBatch; ++u) {
       const int q = base + u * kWarp + lane;
@@ -214,24 +219,24 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
   if (ndef > 0) flush();
 }
 
-// Two points per 16-byte load, kFillLoads loads in flight per thread.
+// kFillLoads points in flight per thread; a warp's points are consecutive, so
+// a run's slots are written together.
 constexpr int kFillLoads = 4;
-__global__ void __launch_bounds__(256) gbmv_fill_kernel(long long npts, CellPoints cp) {
-  const long long pair0 = (long long)blockIdx.x * blockDim.x * kFillLoads + threadIdx.x;
-  int4 v[kFillLoads];
+constexpr int kFillThreads = 256;
+__global__ void __launch_bounds__(kFillThreads) gbmv_fill_kernel(long long npts, CellPoints cp) {
+  const long long p0 = (long long)blockIdx.x * (kFillThreads * kFillLoads) + threadIdx.x;
+  int2 v[kFillLoads];
+  int start[kFillLoads];
 #pragma unroll
   for (int u = 0; u < kFillLoads; ++u) {
-    const long long p = 2 * (pair0 + (long long)u * blockDim.x);
-    v[u] = make_int4(-1, 0, -1, 0);
-    if (p + 1 < npts) v[u] = __ldcs(reinterpret_cast<const int4*>(cp.at + p));
-    else if (p < npts) v[u].x = cp.at[p].x, v[u].y = cp.at[p].y;
+    const long long p = p0 + u * kFillThreads;
+    v[u] = p < npts ? __ldcs(cp.at + p) : make_int2(-1, 0);
   }
 #pragma unroll
-  for (int u = 0; u < kFillLoads; ++u) {
-    const long long p = 2 * (pair0 + (long long)u * blockDim.x);
-    if (v[u].x >= 0) cp.order[cp.start[v[u].x] + v[u].y] = (int)p;
-    if (v[u].z >= 0) cp.order[cp.start[v[u].z] + v[u].w] = (int)p + 1;
-  }
+  for (int u = 0; u < kFillLoads; ++u) start[u] = v[u].x >= 0 ? __ldg(cp.start + v[u].x) : 0;
+#pragma unroll
+  for (int u = 0; u < kFillLoads; ++u)
+    if (v[u].x >= 0) cp.order[start[u] + v[u].y] = (int)(p0 + u * kFillThreads);
 }
 
 template <int E>
@@ -287,7 +292,7 @@ struct __align__(16) CellList {
 struct __align__(16) ChainPair {
   float2 x, y, z;  // x_j - c0
   float2 w;        // GBMV-II C_j | GBMV-I gamma_j
-  float2 k;        // GBMV-II C_j - 100 R_j^2 | GBMV-I R_j
+  float2 k;        // GBMV-II C_j - 100 R_j^2 | GBMV-I's adjoint -4 gamma_j / R_j
   int2 idx;        // atom index
 };
 
@@ -486,7 +491,7 @@ struct __align__(16) PointChain {
 // four-warp blocks 405 and 446 us).
 constexpr int kChainWarps = 1;
 template <int MODEL, bool PER, bool ADJ>
-__global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 16 : MODEL == GBX_MODEL_GBMV2 ? 28 : 32)
+__global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MODEL_GBMV2 ? 28 : 32)
     gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab,
                                                                        Quad quad, ModelConst m, CellPoints cp,
                                                                        const float2* __restrict__ dEdJ,
@@ -523,7 +528,8 @@ __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 16 : MODEL == GBX_MO
     f[2] = a.y - c0.y;
     f[4] = a.z - c0.z;
     f[6] = a.w;
-    f[8] = pk.x;
+    // GBMV-I's adjoint: dS/dR_j = -4 gamma_j e_j r^4 / R_j (gamma ~ R^-4), the division once per entry
+    f[8] = ADJ && MODEL == GBX_MODEL_GBMV1 ? -4.0f * a.w / pk.x : pk.x;
     f[10] = __int_as_float(k);
     if (ADJ) reinterpret_cast<float*>(s_r[w] + l / 2)[l & 1] = pk.y;
   }
@@ -617,9 +623,7 @@ __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 16 : MODEL == GBX_MO
             const float2 g = __fmul2_rn(aw, r4);
             const float2 ex2 = make_float2(__expf(g.x), __expf(g.y));
             if (ADJ) {
-              // dS/dR_j = -4 gamma_j e_j r^4 / R_j (gamma ~ R^-4); padding: gamma = 0
-              const float2 dr = __fmul2_rn(__fmul2_rn(__fmul2_rn(bc2(pc.cS), ex2), r4),
-                                           make_float2(-4.0f * aw.x / ek.x, -4.0f * aw.y / ek.y));
+              const float2 dr = __fmul2_rn(__fmul2_rn(__fmul2_rn(bc2(pc.cS), ex2), r4), ek);  // padding: 0
               accR[e] = __fadd2_rn(accR[e], dr);
               if (!sorted) {
                 if (l < cnt) add_fixed_one(out, kj.x, 3, dr.x);
@@ -784,8 +788,8 @@ gbx_status launch_gbmv_cells_bin(Context* ctx, const float4* pos, const ModelCon
   }
   launch_scan<false>(ctx->d_pcount, ctx->d_geom, ctx->d_pstart, nullptr, cells, 0x7fffffffffffLL, ctx->d_ptotal,
                      ctx->d_status, st);
-  constexpr int per_block = 2 * kFillLoads * 256;
-  gbmv_fill_kernel<<<(int)((npts + per_block - 1) / per_block), 256, 0, st>>>(npts, cp);
+  constexpr int per_block = kFillLoads * kFillThreads;
+  gbmv_fill_kernel<<<(int)((npts + per_block - 1) / per_block), kFillThreads, 0, st>>>(npts, cp);
   ctx->launches += 3;  // bin, scan, fill
   return GBX_OK;
 }

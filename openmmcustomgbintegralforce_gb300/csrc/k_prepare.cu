@@ -53,7 +53,7 @@ struct PrepareArgs {
   long long tight_cap;
   TableGeom* ref;
   int mode;
-  double h, buffer, box[3];
+  double h, buffer, box[3], reach;
   long long ref_cap;
 };
 
@@ -112,6 +112,7 @@ __device__ __forceinline__ void tight_rest(const PrepareArgs& a, const GeomPart&
   double amax = 0.0;
   for (int k = 0; k < 3; ++k) amax = fmax(amax, fmax(fabs((double)e.mn[k]), fabs((double)e.mx[k])));
   g.mode = -1;
+  g.reach = a.reach;
   g.L = a.tight_h;
   // membership margin: FP32 rounding of cell coordinates and distances
   // (extent: a periodic system's longest box edge, by which a point may be moved)
@@ -159,6 +160,7 @@ __device__ __forceinline__ void ref_axis(const PrepareArgs& a, const GeomPart& e
 
 __device__ __forceinline__ void ref_rest(const PrepareArgs& a, TableGeom& g, unsigned& status) {
   g.mode = a.mode;
+  g.reach = a.reach;
   g.total = 0;
   g.L = a.mode == GBX_TABLE_PERIODIC ? fmax(fmax(g.step[0], g.step[1]), g.step[2]) : a.h;
   if (a.mode == GBX_TABLE_PERIODIC) g.pad = 0.0;
@@ -384,6 +386,7 @@ gbx_status launch_prepare(Context* ctx, const void* posq, bool tight, bool refer
   a.mode = wrapped ? GBX_TABLE_STANDALONE : c.table_mode;
   a.h = c.grid_length;
   a.buffer = c.table_buffer;
+  a.reach = c.r1;
   for (int k = 0; k < 3; ++k) a.box[k] = c.box[k];
   a.ref_cap = wrapped ? 0x7fffffffffffffffLL : ctx->cell_cap;  // no cell of the wrapping grid is ever indexed
   // a block per 256 atoms; more where the clears are longer than the atoms

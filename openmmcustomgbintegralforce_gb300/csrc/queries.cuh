@@ -87,13 +87,19 @@ struct RefQuery {
     qoff = qo;
     off = geom.ncell > cap;
     const double x[3] = {(double)xi.x, (double)xi.y, (double)xi.z};
-    const int dmax = max(geom.dims[0], max(geom.dims[1], geom.dims[2]));
+    // A coordinate t = v / step + rel in cell units carries the FP32 rounding of
+    // rel, of v and 1 / step, of the sum and of a move by whole boxes: at most
+    // 2^-24 (3 |rel| + 4 |v| / step).  The guard band is twice 4 (|rel| + reach /
+    // step) 2^-24 (a band of 3e-4 cells, ten times this, cost 21 of the 108 us of
+    // a 6,007-atom integral pass in FP64 queries).
+    float mag = 0.0f;
     for (int k = 0; k < 3; ++k) {
       rel[k] = (float)((x[k] - geom.min[k]) * geom.inv_step[k]);
       inv[k] = (float)geom.inv_step[k];
       invdims[k] = 1.0f / (float)geom.dims[k];
+      mag = fmaxf(mag, fmaf((float)geom.reach, inv[k], fabsf(rel[k])));
     }
-    eps = 1e-4f + 64.0f * (float)dmax * 5.96e-8f;
+    eps = 1e-6f + 8.0f * mag * 5.96e-8f;
   }
   __device__ __forceinline__ void init(const Entries& t, const float4 xi, const double* qo) {
     init(*t.geom, xi, qo, usable_cells(t));
@@ -156,14 +162,10 @@ struct BoxQuery : RefQuery {
   bool inside;  // no point of the atom leaves the box
   __device__ __forceinline__ void init(const Entries& t, const float4 xi, const double* qo) {
     RefQuery::init(t, xi, qo);
-    inside = false;
-  }
-  // reach: the largest radius of the rule's points (nm)
-  __device__ __forceinline__ void set_reach(float reach) {
     inside = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float r = fmaf(reach, inv[k], 0.01f);
+      const float r = fmaf((float)g->reach, inv[k], 0.01f);
       inside = inside && rel[k] - r > 0.0f && rel[k] + r < (float)g->dims[k];
     }
   }
