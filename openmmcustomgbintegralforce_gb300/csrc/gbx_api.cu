@@ -348,7 +348,9 @@ gbx_status grow_table(Context* ctx, long long cells, long long entries) {
     GBX_TRY(dalloc(ctx, &ctx->d_cell_start, cap + 1));
     GBX_TRY(dalloc(ctx, &ctx->d_cell_cursor, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_cell2, cap));
-    if (ctx->cfg.model != GBX_MODEL_GBSW) {
+    if (ctx->cfg.model == GBX_MODEL_GBSW) {
+      GBX_TRY(dalloc(ctx, &ctx->d_rfirst, cap));
+    } else {
       GBX_TRY(dalloc(ctx, &ctx->d_pcount, cap));
       GBX_TRY(dalloc(ctx, &ctx->d_plive, cap));
       GBX_TRY(dalloc(ctx, &ctx->d_pstart, cap + 1));
@@ -363,7 +365,8 @@ gbx_status grow_table(Context* ctx, long long cells, long long entries) {
     }
     GBX_TRY(dalloc(ctx, &ctx->d_entries, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_entry4, cap));
-    GBX_TRY(dalloc(ctx, &ctx->d_entry_par, cap));
+    if (ctx->cfg.model == GBX_MODEL_GBSW) GBX_TRY(dalloc(ctx, &ctx->d_entry_index, cap));
+    else GBX_TRY(dalloc(ctx, &ctx->d_entry_par, cap));
     ctx->entry_cap = cap;
   }
   return GBX_OK;
@@ -786,7 +789,7 @@ gbx_status gbx_destroy(gbx_context* handle) {
                   ctx->d_integrals, ctx->d_dEdB_fx, ctx->d_dEdJ, ctx->d_energy_part, ctx->d_force_fx, ctx->d_f4,
                   ctx->d_energy, ctx->d_dEdR_fx, ctx->d_dEdq_fx, ctx->d_alpha_grad, ctx->d_status, ctx->d_work,
                   ctx->d_tgeom, ctx->d_wgeom, ctx->d_tcount, ctx->d_tstart, ctx->d_tcursor, ctx->d_tburied,
-                  ctx->d_tentry, ctx->d_tindex, ctx->d_entry4, ctx->d_entry_par,
+                  ctx->d_tentry, ctx->d_tindex, ctx->d_entry4, ctx->d_entry_par, ctx->d_entry_index, ctx->d_rfirst,
                   ctx->d_cell2, ctx->d_tcell, ctx->d_tfirst, ctx->d_srec, ctx->d_srec_st, ctx->d_rcount, ctx->d_rmax, ctx->d_next_item, ctx->d_energy_fx, ctx->d_tile_box, ctx->d_perm,
                   ctx->d_perm_tmp, ctx->d_cell_of, ctx->d_scount, ctx->d_sstart, ctx->d_scursor, ctx->d_sgeom, ctx->d_pstate,
                   ctx->d_pat, ctx->d_porder, ctx->d_sval, ctx->d_pcount, ctx->d_plive, ctx->d_pstart,

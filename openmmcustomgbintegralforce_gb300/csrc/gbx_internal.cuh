@@ -53,7 +53,7 @@ struct TableGeom {
   long long total;  // list entries before capping
 };
 
-// Exact GBSW table, per cell: the list's first (sorted) entry and the cell's
+// GBSW tables, per cell: the list's first (sorted) entry and the cell's
 // (count or -1 if buried, start) record, read together by one 32-byte load.
 struct __align__(32) TightCell {
   float4 first;
@@ -131,8 +131,10 @@ struct Context {
   int* d_cell_cursor = nullptr;
   int2* d_cell2 = nullptr;       // [cell_cap] (capped count, start) for the volume kernels
   int* d_entries = nullptr;      // [entry_cap] atom indices, ascending per cell
-  float4* d_entry4 = nullptr;    // [entry_cap] inline copies (x, y, z, main parameter)
-  float2* d_entry_par = nullptr; // [entry_cap] inline secondary parameters
+  float4* d_entry4 = nullptr;    // [entry_cap] inline copies (x, y, z, main parameter; GBSW: as pairs)
+  float2* d_entry_par = nullptr; // GBMV: [entry_cap] inline secondary parameters
+  int* d_entry_index = nullptr;  // GBSW: [entry_cap] atom of each inline entry (likeliest burying atom first)
+  TightCell* d_rfirst = nullptr; // GBSW: [cell_cap] the cell's first inline entry and record
   void* d_parts = nullptr;       // partial extents of the call's first kernel
   unsigned* d_ticket = nullptr;  // its count of finished blocks (0 between calls)
   bool table_valid = false;

@@ -65,7 +65,7 @@ __device__ __forceinline__ float gbsw_volume(const Q& qy, const ModelConst& m, c
                                              int cnt, const float4 xi, const float4 v, W& wk) {
   float V = 1.0f;
   for (int l = 0; l < cnt; ++l) {
-    const float4 a = entry_at<Q>(t, start + l);
+    const float4 a = entry_at(t, start + l);
     const float3 d = qy.delta(a, xi, v);
     const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
     const float lo = a.w - m.sw, hi = a.w + m.sw;
@@ -142,7 +142,7 @@ __device__ __forceinline__ void count_chain_work(const Q& qy, const ModelConst& 
     wk.fs += cs.x;
   } else {
     for (int l = 0; l < cs.x; ++l) {
-      const float4 a = entry_at<Q>(t, cs.y + l);
+      const float4 a = entry_at(t, cs.y + l);
       const float3 d = qy.delta(a, xi, v);
       const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
       const float lo = a.w - m.sw, hi = a.w + m.sw;
@@ -379,19 +379,6 @@ __device__ __forceinline__ float shell_g(const ModelConst& m, float V, float dr)
   return __fdividef(V, u) * du;
 }
 
-// The query's delta of two entries along one axis.
-template <class Q>
-__device__ __forceinline__ float2 delta2(const Q& query, int k, float2 a, float xi, float v) {
-  if constexpr (IsTight<Q>::value) {
-    return query.delta2(k, a, xi, v);
-  } else {
-    const float4 X = make_float4(xi, xi, xi, 0.f), W = make_float4(v, v, v, 0.f);
-    const float3 d0 = query.delta(make_float4(a.x, a.x, a.x, 0.f), X, W),
-                 d1 = query.delta(make_float4(a.y, a.y, a.y, 0.f), X, W);
-    return k == 0 ? make_float2(d0.x, d1.x) : k == 1 ? make_float2(d0.y, d1.y) : make_float2(d0.z, d1.z);
-  }
-}
-
 // Signed distance of a point from an atom's sphere, |d| - R'.  A point at an
 // atom's own place gives -R' (the tiny term keeps 0 * rsqrt(0) out; it is far
 // below the rounding of any other squared distance).
@@ -470,9 +457,8 @@ __global__ void __launch_bounds__(kThreads, 12) gbsw_integral_kernel(const float
                                                                  float* __restrict__ Jpart, ShellSink sink,
                                                                  unsigned* __restrict__ next_item) {
   __shared__ int2 s_queue[kThreads / kWarp][2][kQueue];  // (q | length << 16, list start): short and long lists
-  // the exact table: lists start at even entries and each cell's record sits
-  // beside its first entry, so both are read 32 bytes at a time
-  constexpr bool kTight = IsTight<Q>::value;
+  // lists start at even entries and each cell's record sits beside its first
+  // entry, so both are read 32 bytes at a time
   const int lane = threadIdx.x % kWarp;
   const int wib = threadIdx.x / kWarp;
   const unsigned lt = (1u << lane) - 1u;
@@ -517,17 +503,12 @@ __global__ void __launch_bounds__(kThreads, 12) gbsw_integral_kernel(const float
             const float4 vc = quad.qv[qc];
             const long long cell = query.cell(xi, vc, qc);
             float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if constexpr (kTight) {
-              // the exact table keeps each cell's first entry beside its
-              // record: one load, not one after the other
-              cs = make_int2(0, 0);
-              if (cell >= 0) {
-                const Float4x2 r = ldg_pair(tab.first + cell);
-                a0 = r.a;
-                cs = make_int2(__float_as_int(r.b.x), __float_as_int(r.b.y));
-              }
-            } else {
-              cs = cell >= 0 ? __ldg(tab.cell + cell) : make_int2(0, 0);
+            // the cell's first entry beside its record: one load, not one after the other
+            cs = make_int2(0, 0);
+            if (cell >= 0) {
+              const Float4x2 r = ldg_pair(tab.first + cell);
+              a0 = r.a;
+              cs = make_int2(__float_as_int(r.b.x), __float_as_int(r.b.y));
             }
             if (cs.x == 0) {
               const float2 wc = quad.qw[qc];
@@ -536,7 +517,6 @@ __global__ void __launch_bounds__(kThreads, 12) gbsw_integral_kernel(const float
             } else if (cs.x > 0) {
               // the list's first entry, the likeliest burying atom, buries most
               // listed points: V = 0 adds nothing, the point is not queued
-              if constexpr (!kTight) a0 = __ldg(tab.e + cs.y);
               if (sphere_gap(query.delta(a0, xi, vc), a0.w) <= -m.sw) cs.x = -1;
             }
           }
@@ -581,21 +561,15 @@ __global__ void __launch_bounds__(kThreads, 12) gbsw_integral_kernel(const float
       EntryPair pair{};
       auto load = [&](int l) -> EntryPair {
         EntryPair p = pair;
-        if constexpr (kTight) {  // an odd list's last pair ends in a padding entry no point is near
-          if (l < cnt) p = ldg_entries(tab.e, s + l);
-        } else {
-          const float4 none = make_float4(0.f, 0.f, 0.f, -1e6f);  // a sphere no point is near
-          const float4 a = l < cnt ? __ldg(tab.e + s + l) : none, b = l + 1 < cnt ? __ldg(tab.e + s + l + 1) : none;
-          p = EntryPair{make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), make_float2(-a.w, -b.w)};
-        }
+        if (l < cnt) p = ldg_entries(tab.e, s + l);  // an odd list ends in a padding entry no point is near
         return p;
       };
       // entries l and l + 1 of every lane that has them, in packed FP32x2
       // arithmetic (each half rounded as sphere_gap rounds it); bits of the shaping ones
       auto step = [&](const EntryPair& p, int l) -> unsigned {
         const bool on = l < cnt;
-        const float2 dx = delta2(query, 0, p.x, xi.x, v.x), dy = delta2(query, 1, p.y, xi.y, v.y),
-                     dz = delta2(query, 2, p.z, xi.z, v.z);
+        const float2 dx = query.delta2(0, p.x, xi.x, v.x), dy = query.delta2(1, p.y, xi.y, v.y),
+                     dz = query.delta2(2, p.z, xi.z, v.z);
         const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, make_float2(1e-30f, 1e-30f))));
         const float2 g = __ffma2_rn(r2, make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y)), p.nw);
         const float2 u = __ffma2_rn(
@@ -893,7 +867,7 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
           st = cs.y;
         }
         for (int l = 0; l < cnt; ++l) {
-          const float4 a = entry_at<Q>(tab, st + l);
+          const float4 a = entry_at(tab, st + l);
           const float dr = sphere_gap(query.delta(a, xi, v), a.w);
           if (dr <= -m.sw) {
             V = 0.0f;
@@ -909,7 +883,7 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
       for (int l = 0; __any_sync(0xffffffffu, l < cnt); ++l) {
         bool in = false;
         if (l < cnt) {
-          const float4 a = entry_at<Q>(tab, st + l);
+          const float4 a = entry_at(tab, st + l);
           in = fabsf(sphere_gap(query.delta(a, xi, v), a.w)) < m.sw;
         }
         const unsigned have = __ballot_sync(0xffffffffu, in);
@@ -1069,6 +1043,9 @@ Entries entries_of(const Context* ctx) {
     return Entries{ctx->d_tgeom,     ctx->d_tcell,   ctx->d_tentry,
                    nullptr,          ctx->d_tindex,  ctx->tcell_cap,
                    ctx->d_tfirst,    ctx->tentry_cap, ctx->cfg.periodic ? ctx->d_wgeom : nullptr};
+  if (ctx->cfg.model == GBX_MODEL_GBSW)
+    return Entries{ctx->d_geom,   ctx->d_cell2, ctx->d_entry4, nullptr, ctx->d_entry_index, ctx->cell_cap,
+                   ctx->d_rfirst, ctx->entry_cap};
   return Entries{ctx->d_geom,    ctx->d_cell2,    ctx->d_entry4, ctx->d_entry_par, ctx->d_entries, ctx->cell_cap,
                  nullptr,        ctx->entry_cap};
 }

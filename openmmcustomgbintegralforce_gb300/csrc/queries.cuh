@@ -20,19 +20,19 @@ struct Quad {
 struct Entries {
   const TableGeom* geom;
   const int2* cell;    // (count, start); exact table: count -1 marks a buried cell
-  const float4* e;     // (x, y, z, main model parameter); exact table: pairs (EntryPair)
+  const float4* e;     // GBMV: (x, y, z, main model parameter); GBSW: pairs of entries (EntryPair)
   const float2* par;   // secondary model parameters (reference table only)
   const int* index;    // atom index of each entry
   long long cell_cap;  // cells allocated: a geometry with more (a table that
                        // outgrew its buffers, not yet resized) is never indexed
-  const TightCell* first; // exact table: each cell's first list entry and record (else nullptr)
+  const TightCell* first; // GBSW: each cell's first list entry and record (else nullptr)
   long long entry_cap;    // entries allocated: a table with more was not sorted
                           // this step, its cell records are an earlier step's
   const TableGeom* wrap;  // exact table of a periodic system: the reference's
                           // standalone grid, whose edges decide a point's move
 };
 
-// Two consecutive entries of an exact-table list, one field after the other,
+// Two consecutive entries of a GBSW list (either table), one field after the other,
 // so that a 32-byte load gives the operands of packed FP32x2 arithmetic.
 struct EntryPair {
   float2 x, y, z, nw;  // nw: -R'
@@ -151,6 +151,10 @@ struct RefQuery {
   __device__ __forceinline__ float3 delta(const float4 a, const float4 xi, const float4 v) const {
     return make_float3((a.x - xi.x) - v.x, (a.y - xi.y) - v.y, (a.z - xi.z) - v.z);
   }
+  // delta of both entries along axis k, each half rounded as delta() rounds it
+  __device__ __forceinline__ float2 delta2(int, float2 a, float xi, float v) const {
+    return __fadd2_rn(__fadd2_rn(a, make_float2(-xi, -xi)), make_float2(-v, -v));
+  }
 };
 
 // The same query of a box-sampled table (GBX_TABLE_PERIODIC), for passes that
@@ -215,6 +219,11 @@ struct MinImageQuery : RefQuery {
 #pragma unroll
     for (int k = 0; k < 3; ++k) d[k] = fmaf(-L[k], floorf(fmaf(d[k], iL[k], 0.5f)), d[k]);
     return make_float3(d[0], d[1], d[2]);
+  }
+  __device__ __forceinline__ float2 delta2(int k, float2 a, float xi, float v) const {
+    const float2 d = __fadd2_rn(__fadd2_rn(a, make_float2(-xi, -xi)), make_float2(-v, -v));
+    return make_float2(fmaf(-L[k], floorf(fmaf(d.x, iL[k], 0.5f)), d.x),
+                       fmaf(-L[k], floorf(fmaf(d.y, iL[k], 0.5f)), d.y));
   }
 };
 
@@ -295,6 +304,11 @@ struct PeriodicQuery {
 #pragma unroll
     for (int k = 0; k < 3; ++k) d[k] = fmaf(-L[k], floorf(fmaf(d[k], iL[k], 0.5f)), d[k]);
     return make_float3(d[0], d[1], d[2]);
+  }
+  __device__ __forceinline__ float2 delta2(int k, float2 a, float xi, float v) const {
+    const float2 d = __fadd2_rn(__fadd2_rn(a, make_float2(-xi, -xi)), make_float2(-v, -v));
+    return make_float2(fmaf(-L[k], floorf(fmaf(d.x, iL[k], 0.5f)), d.x),
+                       fmaf(-L[k], floorf(fmaf(d.y, iL[k], 0.5f)), d.y));
   }
 };
 
@@ -436,8 +450,7 @@ struct PeriodicTightQuery : TightQuery {
   }
 };
 
-// The exact table's query types (cell records with the first entry, lists
-// in aligned pairs, buried cells).
+// The exact table's query types (buried cells; every atom that a point needs is listed).
 template <class Q>
 struct IsTight {
   static constexpr bool value = false;
@@ -451,15 +464,10 @@ struct IsTight<PeriodicTightQuery> {
   static constexpr bool value = true;
 };
 
-// Entry `at` of either table's lists as (x, y, z, main model parameter).
-template <class Q>
+// Entry `at` of a GBSW list as (x, y, z, R').
 __device__ __forceinline__ float4 entry_at(const Entries& t, int at) {
-  if constexpr (IsTight<Q>::value) {
-    const float* p = reinterpret_cast<const float*>(t.e) + 8 * (size_t)(at >> 1) + (at & 1);
-    return make_float4(__ldg(p), __ldg(p + 2), __ldg(p + 4), -__ldg(p + 6));
-  } else {
-    return __ldg(t.e + at);
-  }
+  const float* p = reinterpret_cast<const float*>(t.e) + 8 * (size_t)(at >> 1) + (at & 1);
+  return make_float4(__ldg(p), __ldg(p + 2), __ldg(p + 4), -__ldg(p + 6));
 }
 
 // ds/dS of the logistic below, from its p
