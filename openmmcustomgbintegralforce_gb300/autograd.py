@@ -56,7 +56,7 @@ class GBEnergyFunction(torch.autograd.Function):
         ctx.save_for_backward(out)
         ctx.n = n
         ctx.dtypes = (positions.dtype, charges.dtype, radii.dtype, alpha.dtype)
-        return out[0].to(positions.dtype)
+        return out[0].to(positions.dtype, copy=True)  # its own memory: a caller may write to it before backward
 
     @staticmethod
     def backward(ctx, grad):
