@@ -83,8 +83,9 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
                                           long long cell_cap) {
   __shared__ double s_d[kMemberWarps][3][kMaxSamples];
   __shared__ float s_sq[kMemberWarps][3][kMaxSamples];
+  __shared__ int2 s_range[kMemberWarps][3];  // first grid index and their number
+  __shared__ double s_pad[kMemberWarps];
   const int wib = threadIdx.x / kWarp;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   const int lane = threadIdx.x % kWarp;
   const TableGeom& g = *gp;
   if (g.ncell > cell_cap) return;
@@ -92,23 +93,27 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
   const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
   double (*ds)[kMaxSamples] = s_d[wib];
   float (*sq)[kMaxSamples] = s_sq[wib];
-  for (int a = warp; a < n; a += (gridDim.x * blockDim.x) / kWarp) {
-    const float4 p = pos[a];
-    double pad;
-    if (MODE == GBX_TABLE_STANDALONE) pad = g.pad;
-    else pad = dadd(dadd(radius[a], dmul(half_sqrt3(), h)), buffer);
-    const double pad2 = dmul(pad, pad);
-    int b_ = 0, n_ = 0;
-    if (lane < 3) {  // an axis per lane
-      const double c = lane == 0 ? p.x : (lane == 1 ? p.y : p.z);
-      b_ = (int)floor(ddiv(dsub(dsub(c, pad), g.min[lane]), h));
-      n_ = (int)ceil(ddiv(dsub(dadd(c, pad), g.min[lane]), h)) - b_ + 1;
+  for (int base = blockIdx.x * kMemberWarps; base < n; base += gridDim.x * kMemberWarps) {
+    __syncthreads();  // the previous atoms' values are read
+    if (threadIdx.x < 3 * kMemberWarps && base + threadIdx.x / 3 < n) {  // an axis of an atom per thread
+      const int w = threadIdx.x / 3, k = threadIdx.x % 3;
+      double pad;
+      if (MODE == GBX_TABLE_STANDALONE) pad = g.pad;
+      else pad = dadd(dadd(radius[base + w], dmul(half_sqrt3(), h)), buffer);
+      const double c = reinterpret_cast<const float*>(pos + base + w)[k];
+      const int first = (int)floor(ddiv(dsub(dsub(c, pad), g.min[k]), h));
+      s_range[w][k] = make_int2(first, (int)ceil(ddiv(dsub(dadd(c, pad), g.min[k]), h)) - first + 1);
+      if (k == 0) s_pad[w] = pad;
     }
+    __syncthreads();
+    const int a = base + wib;
+    if (a >= n) continue;
+    const double pad = s_pad[wib], pad2 = dmul(pad, pad);
     int b[3], nn[3];
     bool ok = true, fits = true;
     for (int k = 0; k < 3; ++k) {
-      b[k] = __shfl_sync(0xffffffffu, b_, k);
-      nn[k] = __shfl_sync(0xffffffffu, n_, k);
+      b[k] = s_range[wib][k].x;
+      nn[k] = s_range[wib][k].y;
       ok = ok && nn[k] >= 1 && nn[k] <= 1024;
       fits = fits && nn[k] <= kMaxSamples;
     }
@@ -119,7 +124,8 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
     }
     // the reference's offset of grid value m of axis k from the atom, and its test of a sum of squares
     auto offset = [&](int k, int m) {
-      return dsub(dadd(g.min[k], dmul((double)(b[k] + m), h)), (double)(k == 0 ? p.x : (k == 1 ? p.y : p.z)));
+      return dsub(dadd(g.min[k], dmul((double)(s_range[wib][k].x + m), h)),
+                  (double)reinterpret_cast<const float*>(pos + a)[k]);
     };
     auto inside = [&](double d0, double d1, double d2) {
       const double s = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
@@ -157,7 +163,6 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
         if (s < in2 || (s <= out2 && inside(ds[0][ij.x], ds[1][ij.y], ds[2][k]))) em.put<FILL>(row + k, a, ncell);
       }
     }
-    __syncwarp();
   }
 }
 
@@ -177,8 +182,10 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
   __shared__ double s_samp[kMemberWarps][3][kMaxSamples];
   __shared__ float s_sq[kMemberWarps][3][kMaxSamples];
   __shared__ int s_id[kMemberWarps][3][kMaxSamples];
+  __shared__ int s_cnt[kMemberWarps][3];
+  __shared__ double s_pad2[kMemberWarps];
+  __shared__ float s_axis[3][3];  // 1 / box, box, 1 / step
   const int wib = threadIdx.x / kWarp;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   const int lane = threadIdx.x % kWarp;
   const TableGeom& g = *gp;
   if (g.ncell > cell_cap) return;
@@ -187,42 +194,54 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
   float (*sq)[kMaxSamples] = s_sq[wib];
   int (*idx)[kMaxSamples] = s_id[wib];
   constexpr float kEpsCell = 1e-4f;  // cell units: far above the FP32 rounding of a sample's position
-  for (int a = warp; a < n; a += (gridDim.x * blockDim.x) / kWarp) {
-    float4 p = pos[a];
-    const double c[3] = {(double)p.x, (double)p.y, (double)p.z};
-    const double L = g.L;
-    const double pad = dadd(dadd(radius[a], dmul(half_sqrt3(), L)), buffer);
-    const double pad2 = dmul(pad, pad);
-    int cnt0 = 0;
-    // lanes 0..2 walk one axis each (samples by repeated addition, as the reference)
-    if (lane < 3) {
-      const int k = lane;
-      double x = dsub(dsub(c[k], pad), L);
-      const double end = dadd(dadd(c[k], pad), L);
+  if (threadIdx.x < 3) {
+    s_axis[0][threadIdx.x] = (float)g.inv_box[threadIdx.x];
+    s_axis[1][threadIdx.x] = (float)g.box[threadIdx.x];
+    s_axis[2][threadIdx.x] = (float)g.inv_step[threadIdx.x];
+  }
+  for (int base = blockIdx.x * kMemberWarps; base < n; base += gridDim.x * kMemberWarps) {
+    __syncthreads();  // the previous atoms' samples are read
+    // an axis of an atom per thread: samples by repeated addition, as the reference
+    if (threadIdx.x < 3 * kMemberWarps && base + threadIdx.x / 3 < n) {
+      const int w = threadIdx.x / 3, k = threadIdx.x % 3;
+      const double c = reinterpret_cast<const float*>(pos + base + w)[k];
+      const double L = g.L, step = g.step[k];
+      const double pad = dadd(dadd(radius[base + w], dmul(half_sqrt3(), L)), buffer);
+      double x = dsub(dsub(c, pad), L);
+      const double end = dadd(dadd(c, pad), L);
+      // samples certainly below the end, added without a compare: one fewer
+      // than fit (half a step covers the additions' rounding many times over)
+      const float fit = (float)(end - x) * (float)g.inv_step[k];
+      const int sure = fit > 1.0f ? (fit < (float)kMaxSamples ? (int)fit - 1 : kMaxSamples) : 0;
       int m = 0;
+      for (; m < sure; ++m) {
+        s_samp[w][k][m] = x;
+        x = dadd(x, step);
+      }
       while (x < end && m <= kMaxSamples) {
-        if (m < kMaxSamples) samp[k][m] = x;
+        if (m < kMaxSamples) s_samp[w][k][m] = x;
         ++m;
-        x = dadd(x, g.step[k]);
+        x = dadd(x, step);
       }
       if (m > kMaxSamples) atomicOr(status, kStatusTableEntries);
-      cnt0 = m;
+      s_cnt[w][k] = m < kMaxSamples ? m : kMaxSamples;
+      if (k == 0) s_pad2[w] = dmul(pad, pad);
     }
-    int cnt[3];
-    for (int k = 0; k < 3; ++k) {
-      const int v = __shfl_sync(0xffffffffu, cnt0, k);
-      cnt[k] = v < kMaxSamples ? v : kMaxSamples;
-    }
-    __syncwarp();
+    __syncthreads();
+    const int a = base + wib;
+    if (a >= n) continue;
+    const float* c = reinterpret_cast<const float*>(pos + a);
+    const double pad2 = s_pad2[wib];
+    const int cnt[3] = {s_cnt[wib][0], s_cnt[wib][1], s_cnt[wib][2]};
     for (int t = lane; t < cnt[0] + cnt[1] + cnt[2]; t += kWarp) {
       const int k = t < cnt[0] ? 0 : (t < cnt[0] + cnt[1] ? 1 : 2);
       const int m = t - (k == 0 ? 0 : (k == 1 ? cnt[0] : cnt[0] + cnt[1]));
       const double xk = samp[k][m];
       // the sample moved into the box by whole box edges, then its cell
       const float rel = (float)(xk - g.min[k]);
-      const float tb = rel * (float)g.inv_box[k];
+      const float tb = rel * s_axis[0][k];
       const float nb = floorf(tb);
-      const float u = fmaf(-nb, (float)g.box[k], rel) * (float)g.inv_step[k];
+      const float u = fmaf(-nb, s_axis[1][k], rel) * s_axis[2][k];
       const float fu = floorf(u);
       int id;
       if (tb - nb > kEpsCell && tb - nb < 1.0f - kEpsCell && u - fu > kEpsCell && u - fu < 1.0f - kEpsCell) {
@@ -233,7 +252,7 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
         id = (int)floor(ddiv(dsub(x0, g.min[k]), g.step[k]));
       }
       idx[k][m] = (id < 0 || id >= g.dims[k]) ? -1 : id;
-      const float e = (float)(xk - c[k]);
+      const float e = (float)(xk - (double)c[k]);
       sq[k][m] = e * e;
     }
     __syncwarp();
@@ -253,14 +272,14 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
         bool member = sf < in2;
         if (!member && sf <= out2) {
           // the reference's FP64 test
-          const double e0 = dsub(samp[0][ij.x], c[0]), e1 = dsub(samp[1][ij.y], c[1]), e2 = dsub(samp[2][kz], c[2]);
+          const double e0 = dsub(samp[0][ij.x], (double)c[0]), e1 = dsub(samp[1][ij.y], (double)c[1]),
+                       e2 = dsub(samp[2][kz], (double)c[2]);
           member = dadd(dadd(dmul(e0, e0), dmul(e1, e1)), dmul(e2, e2)) < pad2;
         }
         const int i2 = idx[2][kz];
         if (member && i2 >= 0) em.put<FILL>(row + i2, a, ncell);
       }
     }
-    __syncwarp();
   }
 }
 
