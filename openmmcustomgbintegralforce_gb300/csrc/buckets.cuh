@@ -1,0 +1,58 @@
+// The members of a lookup table in one pass: every cell has a bucket of `size`
+// slots, an atom takes the next slot of each cell it belongs to, and members
+// past the bucket are chained to their cell, so the table is complete whatever
+// the bucket's size.  A scan of the counts then places the final lists
+// (scan.cuh), and the sort reads bucket and chain and writes them there.
+// Enumerating the members twice, to count and to fill, had cost more than the
+// bucket's scattered slots do: table stage of 50,000 GBSW atoms 240 -> 220 us,
+// of 1,001 40 -> 37, of 6,001 on a grid table 78 -> 60.  (Slots of a number
+// side by side, for neighbouring cells' sake, measured the same or worse;
+// starts taken inside the sort, by groups of 32 cells, saved the scan's 4 us
+// and cost 40 in the sort and 20 in the integrals of 50,000 atoms.)
+// The host sizes the buckets from the longest list of the sizing call, with a
+// quarter to spare.
+// Included by the table translation units; internal linkage in each.
+#pragma once
+
+#include "gbx_internal.cuh"
+
+namespace gbx {
+namespace {
+
+struct Members {
+  int* count;   // [cells] members per cell (0 on entry)
+  int* slots;   // [cells][size]
+  int* chain;   // [cells] 1 + the cell's last chained member (0 on entry)
+  int2* node;   // [node_cap] (atom, chain before it)
+  int size;
+  long long node_cap;
+  unsigned* chained;  // members in nodes (0 on entry)
+  unsigned* status;
+  __device__ __forceinline__ void put(long long cell, int atom) const {
+    const int slot = atomicAdd(&count[cell], 1);
+    if (slot < size) {
+      slots[cell * size + slot] = atom;
+      return;
+    }
+    const unsigned o = atomicAdd(chained, 1u);
+    if (o < node_cap) node[o] = make_int2(atom, atomicExch(&chain[cell], (int)o + 1));
+    else atomicOr(status, kStatusTableEntries);
+  }
+  // The members of a cell whose list is longer than its bucket, into out[0 .. cnt):
+  // `width` lanes, lane 0 .. width - 1.  (Atom 0 stands for members that found no
+  // node; the status then says so.)
+  __device__ __forceinline__ void gather(long long cell, int cnt, int* out, int lane, int width) const {
+    for (int q = lane; q < size; q += width) out[q] = slots[cell * size + q];
+    if (lane != 0) return;
+    int k = size;
+    for (int o = chain[cell]; o > 0 && k < cnt;) {
+      const int2 v = node[o - 1];
+      out[k++] = v.x;
+      o = v.y;
+    }
+    while (k < cnt) out[k++] = 0;
+  }
+};
+
+}  // namespace
+}  // namespace gbx

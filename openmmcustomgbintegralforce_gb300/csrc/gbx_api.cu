@@ -341,13 +341,32 @@ gbx_status prepare_records(Context* ctx, bool wanted, bool adjoint) {
   return GBX_OK;
 }
 
+// Buckets of `want` slots per cell: at most 256 and, so that a sparse grid does
+// not pay for empty cells, four times the entries in all; list members past
+// them are chained.  Never shrinks.
+gbx_status grow_buckets(Context* ctx, gbx::TableBuckets& b, long long want, long long cells, long long entries) {
+  const long long room = std::max(4 * entries, 1LL << 22) / std::max(cells, 1LL);
+  const int size = (int)std::min(std::min(want, 256LL), room);
+  if (size <= b.size) return GBX_OK;
+  b.size = 0;
+  GBX_TRY(dalloc(ctx, &b.slots, (size_t)cells * size));
+  b.size = size;
+  return GBX_OK;
+}
+
+// Slots for the longest list seen and a quarter more.
+long long bucket_for(int longest) { return ((long long)longest * 5 / 4 + 7) / 8 * 8; }
+constexpr long long kFirstBucket = 32;  // before any list is known
+
 gbx_status grow_table(Context* ctx, long long cells, long long entries) {
+  const long long slots = std::max(kFirstBucket, (long long)ctx->buckets.size);
   if (cells > ctx->cell_cap) {
     const long long cap = cells + cells / 4 + 1024;
     GBX_TRY(dalloc(ctx, &ctx->d_cell_count, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_cell_start, cap + 1));
-    GBX_TRY(dalloc(ctx, &ctx->d_cell_cursor, cap));
+    GBX_TRY(dalloc(ctx, &ctx->buckets.chain, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_cell2, cap));
+    ctx->buckets.size = 0;
     if (ctx->cfg.model == GBX_MODEL_GBSW) {
       GBX_TRY(dalloc(ctx, &ctx->d_rfirst, cap));
     } else {
@@ -363,13 +382,14 @@ gbx_status grow_table(Context* ctx, long long cells, long long entries) {
       ctx->last_error = "lookup table would exceed 2^31 entries";
       return GBX_ERR_TABLE_TOO_LARGE;
     }
+    GBX_TRY(dalloc(ctx, &ctx->buckets.node, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_entries, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_entry4, cap));
     if (ctx->cfg.model == GBX_MODEL_GBSW) GBX_TRY(dalloc(ctx, &ctx->d_entry_index, cap));
     else GBX_TRY(dalloc(ctx, &ctx->d_entry_par, cap));
     ctx->entry_cap = cap;
   }
-  return GBX_OK;
+  return grow_buckets(ctx, ctx->buckets, slots, ctx->cell_cap, ctx->entry_cap);
 }
 
 // Build the table; on a capacity miss read the needed sizes back, grow and
@@ -396,7 +416,8 @@ gbx_status build_table_checked(Context* ctx, const void* posq, bool check, bool 
     const bool entries_short = (st & gbx::kStatusTableEntries) != 0;
     if (!cells_short && !entries_short) {
       ctx->table_valid = true;
-      return GBX_OK;
+      // sized in this call: the next one finds buckets for its longest list
+      return attempt > 0 ? grow_buckets(ctx, ctx->buckets, bucket_for(g.longest), ctx->cell_cap, ctx->entry_cap) : GBX_OK;
     }
     if (cells_short && g.ncell <= 1) {
       ctx->last_error = "lookup table dimension is too large, check atom positions";
@@ -415,11 +436,13 @@ gbx_status build_table_checked(Context* ctx, const void* posq, bool check, bool 
 }
 
 gbx_status grow_tight(Context* ctx, long long cells, long long entries) {
+  const long long slots = std::max(kFirstBucket, (long long)ctx->tbuckets.size);
   if (cells > ctx->tcell_cap) {
     const long long cap = cells + cells / 4 + 1024;
     GBX_TRY(dalloc(ctx, &ctx->d_tcount, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_tstart, cap + 1));
-    GBX_TRY(dalloc(ctx, &ctx->d_tcursor, cap));
+    GBX_TRY(dalloc(ctx, &ctx->tbuckets.chain, cap));
+    ctx->tbuckets.size = 0;
     GBX_TRY(dalloc(ctx, &ctx->d_tburied, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_tcell, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_tfirst, cap));
@@ -431,11 +454,12 @@ gbx_status grow_tight(Context* ctx, long long cells, long long entries) {
       ctx->last_error = "exact table would exceed 2^31 entries";
       return GBX_ERR_TABLE_TOO_LARGE;
     }
+    GBX_TRY(dalloc(ctx, &ctx->tbuckets.node, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_tentry, cap));
     GBX_TRY(dalloc(ctx, &ctx->d_tindex, cap));
     ctx->tentry_cap = cap;
   }
-  return GBX_OK;
+  return grow_buckets(ctx, ctx->tbuckets, slots, ctx->tcell_cap, ctx->tentry_cap);
 }
 
 // Exact-table counterpart of build_table_checked.
@@ -457,7 +481,7 @@ gbx_status build_tight_checked(Context* ctx, const void* posq, bool check) {
     const bool entries_short = (st & gbx::kStatusTableEntries) != 0;
     if (!cells_short && !entries_short) {
       ctx->tight_valid = true;
-      return GBX_OK;
+      return attempt > 0 ? grow_buckets(ctx, ctx->tbuckets, bucket_for(g.longest), ctx->tcell_cap, ctx->tentry_cap) : GBX_OK;
     }
     if (cells_short && (g.ncell <= ctx->tcell_cap || g.ncell > ((long long)1 << 31))) {
       ctx->last_error = "exact table geometry out of range, check atom positions";
@@ -784,11 +808,11 @@ gbx_status gbx_destroy(gbx_context* handle) {
   drop_graph(ctx);
   gbx::custom_destroy(ctx);
   void* ptrs[] = {ctx->d_qv, ctx->d_qw, ctx->d_qoff, ctx->d_params,
-                  ctx->d_geom, ctx->d_cell_count, ctx->d_cell_start, ctx->d_cell_cursor, ctx->d_entries,
+                  ctx->d_geom, ctx->d_cell_count, ctx->d_cell_start, ctx->buckets.slots, ctx->buckets.chain, ctx->buckets.node, ctx->d_entries,
                   ctx->d_parts, ctx->d_ticket, ctx->d_pos, ctx->d_J, ctx->d_born, ctx->d_bornf, ctx->d_dBdJ,
                   ctx->d_integrals, ctx->d_dEdB_fx, ctx->d_dEdJ, ctx->d_energy_part, ctx->d_force_fx, ctx->d_f4,
                   ctx->d_energy, ctx->d_dEdR_fx, ctx->d_dEdq_fx, ctx->d_alpha_grad, ctx->d_status, ctx->d_work,
-                  ctx->d_tgeom, ctx->d_wgeom, ctx->d_tcount, ctx->d_tstart, ctx->d_tcursor, ctx->d_tburied,
+                  ctx->d_tgeom, ctx->d_wgeom, ctx->d_tcount, ctx->d_tstart, ctx->tbuckets.slots, ctx->tbuckets.chain, ctx->tbuckets.node, ctx->d_tburied,
                   ctx->d_tentry, ctx->d_tindex, ctx->d_entry4, ctx->d_entry_par, ctx->d_entry_index, ctx->d_rfirst,
                   ctx->d_cell2, ctx->d_tcell, ctx->d_tfirst, ctx->d_srec, ctx->d_srec_st, ctx->d_rcount, ctx->d_rmax, ctx->d_next_item, ctx->d_energy_fx, ctx->d_tile_box, ctx->d_perm,
                   ctx->d_perm_tmp, ctx->d_cell_of, ctx->d_scount, ctx->d_sstart, ctx->d_scursor, ctx->d_sgeom, ctx->d_pstate,

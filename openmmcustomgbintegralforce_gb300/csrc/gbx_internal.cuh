@@ -50,7 +50,17 @@ struct TableGeom {
   int dims[3];
   int mode;
   long long ncell;
-  long long total;  // list entries before capping
+  long long total;  // list entries before capping (even per list where lists are read in pairs)
+  int longest;       // longest list, where one is longer than its bucket (else 0)
+  unsigned chained;  // list members outside their cell's bucket
+};
+
+// Where a table's members are collected (buckets.cuh).
+struct TableBuckets {
+  int* slots = nullptr;   // [cell_cap][size]
+  int size = 0;
+  int* chain = nullptr;   // [cell_cap] members past the bucket, as a list of nodes
+  int2* node = nullptr;   // [entry_cap]
 };
 
 // GBSW tables, per cell: the list's first (sorted) entry and the cell's
@@ -128,7 +138,7 @@ struct Context {
   long long cell_cap = 0, entry_cap = 0;
   int* d_cell_count = nullptr;   // uncapped count -> final (capped) count
   int* d_cell_start = nullptr;   // [cell_cap+1]
-  int* d_cell_cursor = nullptr;
+  TableBuckets buckets;
   int2* d_cell2 = nullptr;       // [cell_cap] (capped count, start) for the volume kernels
   int* d_entries = nullptr;      // [entry_cap] atom indices, ascending per cell
   float4* d_entry4 = nullptr;    // [entry_cap] inline copies (x, y, z, main parameter; GBSW: as pairs)
@@ -149,7 +159,7 @@ struct Context {
   long long tcell_cap = 0, tentry_cap = 0;
   int* d_tcount = nullptr;
   int* d_tstart = nullptr;
-  int* d_tcursor = nullptr;
+  TableBuckets tbuckets;
   int* d_tburied = nullptr;
   int2* d_tcell = nullptr;       // (count or -1 if buried, start)
   TightCell* d_tfirst = nullptr; // per cell: first entry and (count, start)

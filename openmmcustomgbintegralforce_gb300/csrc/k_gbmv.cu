@@ -786,8 +786,8 @@ gbx_status launch_gbmv_cells_bin(Context* ctx, const float4* pos, const ModelCon
     if (box) gbmv_bin_kernel<GBX_MODEL_GBMV2, BoxQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
     else gbmv_bin_kernel<GBX_MODEL_GBMV2, RefQuery><<<bin_blocks, kBinThreads, 0, st>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, cp);
   }
-  launch_scan<false>(ctx->d_pcount, ctx->d_geom, ctx->d_pstart, nullptr, cells, 0x7fffffffffffLL, ctx->d_ptotal,
-                     ctx->d_status, st);
+  launch_scan(ctx->d_pcount, ctx->d_geom, ctx->d_pstart, cells, 0x7fffffffffffLL, ctx->d_ptotal, nullptr, 0,
+              ctx->d_status, st);
   constexpr int per_block = kFillLoads * kFillThreads;
   gbmv_fill_kernel<<<(int)((npts + per_block - 1) / per_block), kFillThreads, 0, st>>>(npts, cp);
   ctx->launches += 3;  // bin, scan, fill

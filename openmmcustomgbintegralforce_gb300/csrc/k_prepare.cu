@@ -118,6 +118,8 @@ __device__ __forceinline__ void tight_rest(const PrepareArgs& a, const GeomPart&
   // (extent: a periodic system's longest box edge, by which a point may be moved)
   g.pad = 2e-5 + 4.0 * 1.1920929e-7 * (amax + 2.0 * margin + a.extent);
   g.total = 0;
+  g.longest = 0;
+  g.chained = 0u;
   g.ncell = (long long)g.dims[0] * g.dims[1] * g.dims[2];
   if (g.ncell > a.tight_cap) status |= kStatusTableCells;
 }
@@ -162,6 +164,8 @@ __device__ __forceinline__ void ref_rest(const PrepareArgs& a, TableGeom& g, uns
   g.mode = a.mode;
   g.reach = a.reach;
   g.total = 0;
+  g.longest = 0;
+  g.chained = 0u;
   g.L = a.mode == GBX_TABLE_PERIODIC ? fmax(fmax(g.step[0], g.step[1]), g.step[2]) : a.h;
   if (a.mode == GBX_TABLE_PERIODIC) g.pad = 0.0;
   g.ncell = (long long)g.dims[0] * g.dims[1] * g.dims[2];
@@ -375,9 +379,11 @@ gbx_status launch_prepare(Context* ctx, const void* posq, bool tight, bool refer
     a.tight_cap = ctx->tcell_cap;
     clear(ctx->d_tcount, (size_t)ctx->tcell_cap);
     clear(ctx->d_tburied, (size_t)ctx->tcell_cap);
+    clear(ctx->tbuckets.chain, (size_t)ctx->tcell_cap);
   }
   if (reference) {
     clear(ctx->d_cell_count, (size_t)ctx->cell_cap);
+    clear(ctx->buckets.chain, (size_t)ctx->cell_cap);
     clear(ctx->d_pcount, (size_t)ctx->cell_cap);
     clear(ctx->d_ptotal, 2);
   }

@@ -18,6 +18,7 @@
 
 #include "bitonic.cuh"
 #include "gbx_internal.cuh"
+#include "buckets.cuh"
 #include "scan.cuh"
 
 namespace gbx {
@@ -40,27 +41,6 @@ __device__ __forceinline__ double half_sqrt3() { return ddiv(__dsqrt_rn(3.0), 2.
 // Membership enumeration (count / fill)
 // --------------------------------------------------------------------------
 
-struct Emit {
-  int* count;
-  const int* start;
-  int* cursor;
-  int* entries;
-  long long entry_cap;
-  unsigned* status;
-  template <bool FILL>
-  __device__ __forceinline__ void put(long long idx, int atom, long long ncell) const {
-    if (idx < 0 || idx >= ncell) return;
-    if (!FILL) {
-      atomicAdd(&count[idx], 1);
-    } else {
-      int slot = atomicAdd(&cursor[idx], 1);
-      long long p = (long long)start[idx] + slot;
-      if (p < entry_cap) entries[p] = atom;
-      else atomicOr(status, kStatusTableEntries);
-    }
-  }
-};
-
 // Column `col` of an axis-0 x axis-1 rectangle of n1 columns per row, by FP32
 // division (exact for the at most 2^20 columns an atom reaches).
 __device__ __forceinline__ int2 column(int col, int n1, float inv_n1) {
@@ -77,9 +57,9 @@ __device__ __forceinline__ int2 column(int col, int n1, float inv_n1) {
 // their squares wherever that is clear of the boundary by a margin that covers
 // its rounding, and by the reference's FP64 operations otherwise (FP64 for
 // every point took 98 us of a count pass at 6,007 atoms).
-template <int MODE, bool FILL>
+template <int MODE>
 __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const double* __restrict__ radius, int n,
-                                          const TableGeom* __restrict__ gp, double h, double buffer, Emit em,
+                                          const TableGeom* __restrict__ gp, double h, double buffer, Members mem,
                                           long long cell_cap) {
   __shared__ double s_d[kMemberWarps][3][kMaxSamples];
   __shared__ float s_sq[kMemberWarps][3][kMaxSamples];
@@ -119,7 +99,7 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
     }
     // non-finite or absurd inputs: skip the atom instead of looping on garbage bounds
     if (!ok) {
-      if (lane == 0) atomicOr(em.status, kStatusTableCells);
+      if (lane == 0) atomicOr(mem.status, kStatusTableCells);
       continue;
     }
     // the reference's offset of grid value m of axis k from the atom, and its test of a sum of squares
@@ -131,6 +111,9 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
       const double s = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
       return MODE == GBX_TABLE_STANDALONE ? __dsqrt_rn(s) < pad : s < pad2;
     };
+    auto put = [&](long long cell) {
+      if (cell >= 0 && cell < ncell) mem.put(cell, a);
+    };
     const int cols = nn[0] * nn[1];
     const float inv_n1 = 1.0f / (float)nn[1];
     if (!fits) {  // a grid finer than a hundredth of the pad: FP64 throughout
@@ -139,7 +122,7 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
         const double d0 = offset(0, ij.x), d1 = offset(1, ij.y);
         for (int k = 0; k < nn[2]; ++k)
           if (inside(d0, d1, offset(2, k)))
-            em.put<FILL>((long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2] + k, a, ncell);
+            put((long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2] + k);
       }
       continue;
     }
@@ -160,7 +143,7 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
       const long long row = (long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2];
       for (int k = lane % kColumnLanes; k < nn[2]; k += kColumnLanes) {
         const float s = sxy + sq[2][k];
-        if (s < in2 || (s <= out2 && inside(ds[0][ij.x], ds[1][ij.y], ds[2][k]))) em.put<FILL>(row + k, a, ncell);
+        if (s < in2 || (s <= out2 && inside(ds[0][ij.x], ds[1][ij.y], ds[2][k]))) put(row + k);
       }
     }
   }
@@ -172,9 +155,8 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
 // FP32 value is clear of the decision's boundary by a margin that covers its
 // rounding, and in the reference's FP64 operations otherwise (FP64 runs at a
 // small fraction of the FP32 rate on this part).
-template <bool FILL>
 __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, const double* __restrict__ radius,
-                                              int n, const TableGeom* __restrict__ gp, double buffer, Emit em,
+                                              int n, const TableGeom* __restrict__ gp, double buffer, Members mem,
                                               long long cell_cap, unsigned* __restrict__ status) {
   // per warp and axis: the samples, their cell index (-1 outside) and the
   // squared offset from the atom in FP32 -- each depends on one axis only,
@@ -256,6 +238,9 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
       sq[k][m] = e * e;
     }
     __syncwarp();
+    auto put = [&](long long cell) {
+      if (cell >= 0 && cell < ncell) mem.put(cell, a);
+    };
     const int cols = cnt[0] * cnt[1];
     const float inv_n1 = 1.0f / (float)cnt[1];
     const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
@@ -277,7 +262,7 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
           member = dadd(dadd(dmul(e0, e0), dmul(e1, e1)), dmul(e2, e2)) < pad2;
         }
         const int i2 = idx[2][kz];
-        if (member && i2 >= 0) em.put<FILL>(row + i2, a, ncell);
+        if (member && i2 >= 0) put(row + i2);
       }
     }
   }
@@ -322,13 +307,13 @@ struct Inline {
 
 // Lists of up to 32 E entries, in registers.
 template <bool GBSW, int E>
-__device__ __forceinline__ void sort_list(int* __restrict__ entries, const Inline& in, const TableGeom& g, long long c,
-                                          long long s, int cnt, int kept, int lane) {
+__device__ __forceinline__ void sort_list(const int* src, int* entries, const Inline& in, const TableGeom& g,
+                                          long long c, long long s, int cnt, int kept, int lane) {
   int key[E];
 #pragma unroll
   for (int r = 0; r < E; ++r) {
     const int e = lane * E + r;
-    key[r] = e < cnt ? entries[s + e] : 0x7fffffff;
+    key[r] = e < cnt ? src[e] : 0x7fffffff;
   }
   warp_bitonic_sort<E>(key, lane);
 #pragma unroll
@@ -374,20 +359,28 @@ __device__ __forceinline__ void sort_list(int* __restrict__ entries, const Inlin
 }
 
 template <bool GBSW>
-__global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(int* __restrict__ count,
-                                                                        const int* __restrict__ start,
-                                                                        int* __restrict__ entries,
-                                                                        int2* __restrict__ cell, Inline in,
-                                                                        const TableGeom* __restrict__ gp, int cap,
-                                                                        long long cell_cap, long long entry_cap,
-                                                                        unsigned* __restrict__ status) {
+__global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(Members mem, const int* __restrict__ start,
+                                                                        int* entries, int2* __restrict__ cell,
+                                                                        Inline in, const TableGeom* __restrict__ gp,
+                                                                        int cap, long long cell_cap,
+                                                                        long long entry_cap) {
   const int wib = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
   const long long ncell = gp->ncell <= cell_cap ? gp->ncell : 0;
   if (gp->total > entry_cap) return;
   for (long long c = (long long)blockIdx.x * kSortWarps + wib; c < ncell; c += (long long)gridDim.x * kSortWarps) {
-    const int cnt = count[c];
+    int cnt = mem.count[c];
     const int s = start[c];
+    if (cnt > kMaxSortSegment) {  // no list: no record may say there is one
+      if (lane == 0) atomicOr(mem.status, kStatusSegmentTooLong);
+      cnt = 0;
+    }
     const int kept = cap > 0 && cnt > cap ? cap : cnt;
+    const int* src = mem.slots + c * mem.size;
+    if (cnt > mem.size) {
+      mem.gather(c, cnt, entries + s, lane, kWarp);
+      src = entries + s;
+      __syncwarp();
+    }
     if (lane == 0) {
       cell[c] = make_int2(kept, s);
       if (GBSW) {
@@ -397,21 +390,18 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(int* __r
       }
     }
     if (cnt == 0) continue;
-    if (cnt <= kWarp) sort_list<GBSW, 1>(entries, in, *gp, c, s, cnt, kept, lane);
-    else if (cnt <= 2 * kWarp) sort_list<GBSW, 2>(entries, in, *gp, c, s, cnt, kept, lane);
-    else if (cnt <= 4 * kWarp) sort_list<GBSW, 4>(entries, in, *gp, c, s, cnt, kept, lane);
-    else if (cnt > kMaxSortSegment) {
-      if (lane == 0) atomicOr(status, kStatusSegmentTooLong);
-      continue;
-    } else {
+    if (cnt <= kWarp) sort_list<GBSW, 1>(src, entries, in, *gp, c, s, cnt, kept, lane);
+    else if (cnt <= 2 * kWarp) sort_list<GBSW, 2>(src, entries, in, *gp, c, s, cnt, kept, lane);
+    else if (cnt <= 4 * kWarp) sort_list<GBSW, 4>(src, entries, in, *gp, c, s, cnt, kept, lane);
+    else {
       // long list: ranks from global memory, results staged per lane
       int vals[kMaxSortSegment / kWarp], ranks[kMaxSortSegment / kWarp];
       int m = 0;
       for (int p = lane; p < cnt; p += kWarp, ++m) {
-        const int v = entries[s + p];
+        const int v = src[p];
         int r = 0;
         for (int q = 0; q < cnt; ++q) {
-          const int u = entries[s + q];
+          const int u = src[q];
           r += (u < v) || (u == v && q < p);
         }
         vals[m] = v;
@@ -427,7 +417,7 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(int* __r
       }
     }
     __syncwarp();
-    if (lane == 0 && kept < cnt) count[c] = kept;
+    if (lane == 0 && kept < cnt) mem.count[c] = kept;
   }
 }
 
@@ -449,55 +439,39 @@ gbx_status launch_table_build(Context* ctx, const float4* pos) {
   cudaStream_t st = ctx->stream;
   const long long cells = ctx->cell_cap;
   if (cells == 0) return GBX_OK;  // sizing call: the grid alone; the caller reads it back and allocates
-  Emit em{ctx->d_cell_count, ctx->d_cell_start, ctx->d_cell_cursor, ctx->d_entries, ctx->entry_cap, ctx->d_status};
+  const TableBuckets& bk = ctx->buckets;
+  const Members mem{ctx->d_cell_count,     bk.slots, bk.chain, bk.node, bk.size, ctx->entry_cap,
+                    &ctx->d_geom->chained, ctx->d_status};
   const int threads = kMemberThreads;
   const int blocks = grid_for((long long)ctx->n * kWarp, threads);
-  for (int pass = 0; pass < 2; ++pass) {
-    if (pass == 1) {
-      auto* total = reinterpret_cast<unsigned long long*>(&ctx->d_geom->total);
-      if (c.model == GBX_MODEL_GBSW)  // lists in aligned pairs
-        launch_scan<true>(ctx->d_cell_count, ctx->d_geom, ctx->d_cell_start, ctx->d_cell_cursor, cells, ctx->entry_cap,
-                          total, ctx->d_status, st);
-      else
-        launch_scan<false>(ctx->d_cell_count, ctx->d_geom, ctx->d_cell_start, ctx->d_cell_cursor, cells,
-                           ctx->entry_cap, total, ctx->d_status, st);
-      ++ctx->launches;
-    }
-    const bool fill = pass == 1;
-    switch (c.table_mode) {
-      case GBX_TABLE_STANDALONE:
-        if (fill)
-          table_members_grid_kernel<GBX_TABLE_STANDALONE, true><<<blocks, threads, 0, st>>>(
-              pos, ctx->d_radius, ctx->n, ctx->d_geom, c.grid_length, c.table_buffer, em, cells);
-        else
-          table_members_grid_kernel<GBX_TABLE_STANDALONE, false><<<blocks, threads, 0, st>>>(
-              pos, ctx->d_radius, ctx->n, ctx->d_geom, c.grid_length, c.table_buffer, em, cells);
-        break;
-      case GBX_TABLE_GRID:
-        if (fill)
-          table_members_grid_kernel<GBX_TABLE_GRID, true><<<blocks, threads, 0, st>>>(
-              pos, ctx->d_radius, ctx->n, ctx->d_geom, c.grid_length, c.table_buffer, em, cells);
-        else
-          table_members_grid_kernel<GBX_TABLE_GRID, false><<<blocks, threads, 0, st>>>(
-              pos, ctx->d_radius, ctx->n, ctx->d_geom, c.grid_length, c.table_buffer, em, cells);
-        break;
-      default:
-        if (fill)
-          table_members_periodic_kernel<true><<<blocks, threads, 0, st>>>(pos, ctx->d_radius, ctx->n, ctx->d_geom,
-                                                                          c.table_buffer, em, cells, ctx->d_status);
-        else
-          table_members_periodic_kernel<false><<<blocks, threads, 0, st>>>(pos, ctx->d_radius, ctx->n, ctx->d_geom,
-                                                                           c.table_buffer, em, cells, ctx->d_status);
-        break;
-    }
-    ++ctx->launches;
+  switch (c.table_mode) {
+    case GBX_TABLE_STANDALONE:
+      table_members_grid_kernel<GBX_TABLE_STANDALONE>
+          <<<blocks, threads, 0, st>>>(pos, ctx->d_radius, ctx->n, ctx->d_geom, c.grid_length, c.table_buffer, mem, cells);
+      break;
+    case GBX_TABLE_GRID:
+      table_members_grid_kernel<GBX_TABLE_GRID>
+          <<<blocks, threads, 0, st>>>(pos, ctx->d_radius, ctx->n, ctx->d_geom, c.grid_length, c.table_buffer, mem, cells);
+      break;
+    default:
+      table_members_periodic_kernel<<<blocks, threads, 0, st>>>(pos, ctx->d_radius, ctx->n, ctx->d_geom,
+                                                                c.table_buffer, mem, cells, ctx->d_status);
+      break;
   }
+  ++ctx->launches;
+  auto* total = reinterpret_cast<unsigned long long*>(&ctx->d_geom->total);
+  if (c.model == GBX_MODEL_GBSW)  // lists in aligned pairs
+    launch_scan<true>(ctx->d_cell_count, ctx->d_geom, ctx->d_cell_start, cells, ctx->entry_cap, total,
+                      &ctx->d_geom->longest, bk.size, ctx->d_status, st);
+  else
+    launch_scan<false>(ctx->d_cell_count, ctx->d_geom, ctx->d_cell_start, cells, ctx->entry_cap, total,
+                       &ctx->d_geom->longest, bk.size, ctx->d_status, st);
+  ++ctx->launches;
   const Inline in{pos,           ctx->d_par, ctx->d_entry4, ctx->d_entry_par, ctx->d_entry_index,
                   ctx->d_rfirst, (float)c.switch_width};
   auto sort = c.model == GBX_MODEL_GBSW ? sort_cells_kernel<true> : sort_cells_kernel<false>;
-  sort<<<grid_for(cells, kSortWarps), kSortWarps * kWarp, 0, st>>>(ctx->d_cell_count, ctx->d_cell_start,
-                                                                   ctx->d_entries, ctx->d_cell2, in, ctx->d_geom,
-                                                                   c.table_cap, cells, ctx->entry_cap, ctx->d_status);
+  sort<<<grid_for(cells, kSortWarps), kSortWarps * kWarp, 0, st>>>(
+      mem, ctx->d_cell_start, ctx->d_entries, ctx->d_cell2, in, ctx->d_geom, c.table_cap, cells, ctx->entry_cap);
   ++ctx->launches;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

@@ -24,6 +24,7 @@
 #include <math.h>
 
 #include "gbx_internal.cuh"
+#include "buckets.cuh"
 #include "scan.cuh"
 
 namespace gbx {
@@ -41,16 +42,11 @@ struct TightArgs {
   int n;
   const TableGeom* geom;
   float w;
-  int* count;
-  const int* start;
-  int* cursor;
+  Members mem;
   int* buried;
-  int* index;
-  long long cell_cap, entry_cap;
-  unsigned* status;
+  long long cell_cap;
 };
 
-template <bool FILL>
 __global__ void tight_members_kernel(TightArgs a) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   const int lane = threadIdx.x % kWarp;
@@ -78,12 +74,10 @@ __global__ void tight_members_kernel(TightArgs a) {
       if (!(e[k] >= b[k] && e[k] - b[k] < 256)) ok = false;
     }
     if (!ok) {
-      if (lane == 0) atomicOr(a.status, kStatusTableCells);
+      if (lane == 0) atomicOr(a.mem.status, kStatusTableCells);
       continue;
     }
-    // the offsets of cell c's lower and upper face along one axis, every
-    // operation rounded on its own: the count and the fill pass, compiled
-    // apart, must decide alike
+    // the offsets of cell c's lower and upper face along one axis
     auto faces = [h](int c, float at) {
       const float lo = __fmul_rn((float)c, h);
       return make_float2(__fsub_rn(lo, at), __fsub_rn(__fadd_rn(lo, h), at));
@@ -111,19 +105,9 @@ __global__ void tight_members_kernel(TightArgs a) {
         const float dn = fmaxf(fmaxf(f.x, -f.y), 0.f);
         if (!(fmaf(dn, dn, near_xy) < reach * reach)) continue;
         const long long cell = row + cz;
-        if (!FILL) {
-          atomicAdd(&a.count[cell], 1);
-          const float df = fmaxf(-f.x, f.y);
-          if (bury > 0.f && fmaf(df, df, far_xy) <= bury * bury) atomicOr(&a.buried[cell], 1);
-        } else {
-          const int slot = atomicAdd(&a.cursor[cell], 1);
-          const long long o = (long long)a.start[cell] + slot;
-          if (o < a.entry_cap) {
-            a.index[o] = at;
-          } else {
-            atomicOr(a.status, kStatusTableEntries);
-          }
-        }
+        a.mem.put(cell, at);
+        const float df = fmaxf(-f.x, f.y);
+        if (bury > 0.f && fmaf(df, df, far_xy) <= bury * bury) atomicOr(&a.buried[cell], 1);
       }
     }
   }
@@ -134,16 +118,14 @@ __global__ void tight_members_kernel(TightArgs a) {
 // sphere, atom index) -- a deterministic order whatever the fill order was --
 // and mark buried cells with count -1.
 __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const float4* __restrict__ pos,
-                                                                        const int* __restrict__ count,
-                                                                        const int* __restrict__ start,
+                                                                        Members mem, const int* __restrict__ start,
                                                                         const int* __restrict__ buried,
                                                                         float4* __restrict__ entry,
                                                                         int* __restrict__ index,
                                                                         int2* __restrict__ cell,
                                                                         TightCell* __restrict__ first,
                                                                         const TableGeom* __restrict__ gp, float w,
-                                                                        long long cell_cap, long long entry_cap,
-                                                                        unsigned* __restrict__ status) {
+                                                                        long long cell_cap, long long entry_cap) {
   // sorted entries, as pairs field by field (EntryPair, queries.cuh)
   auto put = [entry](int at, const float4 e) {
     float* p = reinterpret_cast<float*>(entry) + 8 * (size_t)(at >> 1) + (at & 1);
@@ -173,15 +155,27 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
        c0 += (long long)gridDim.x * kSortWarps * kSortGroups) {
     const long long c = c0 + grp;
     int cnt = 0, s = 0, bur = 0;
+    const int* src = index;  // the unsorted members
     if (c < ncell) {
-      cnt = count[c];
+      cnt = mem.count[c];
       s = start[c];
       bur = cnt > 0 ? buried[c] : 0;
+      if (cnt > kSortBuf && !bur) {  // no list: no record may say there is one
+        if (gl == 0) atomicOr(mem.status, kStatusSegmentTooLong);
+        cnt = 0;
+      }
+      if (cnt > mem.size && !bur) {
+        mem.gather(c, cnt, index + s, gl, kSortLanes);
+        src = index + s;
+      } else {
+        src = mem.slots + c * mem.size;
+      }
       if (gl == 0) {
         cell[c] = make_int2(bur ? -1 : cnt, s);
         first[c].cs = make_int2(bur ? -1 : cnt, s);
       }
     }
+    __syncwarp();
     if (cnt > 0 && !bur && cnt <= kSortSmall) {
       const int cx = (int)c / isx, rem = (int)c - cx * isx, cy = rem / g.dims[2], cz = rem - cy * g.dims[2];
       const float ctr[3] = {cmin[0] + ((float)cx + 0.5f) * step, cmin[1] + ((float)cy + 0.5f) * step,
@@ -197,7 +191,7 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
         int i = 0x7fffffff;
         float k = INFINITY;
         if (gl < cnt) {
-          i = index[s + gl];
+          i = src[gl];
           e = __ldg(pos + i);
           k = key(e);
         }
@@ -218,7 +212,7 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
         int* gi = s_i[wib] + grp * kSortSmall;
         float* gk = s_k[wib] + grp * kSortSmall;
         for (int q = gl; q < cnt; q += kSortLanes) {
-          const int i = index[s + q];
+          const int i = src[q];
           const float4 e = __ldg(pos + i);
           ge[q] = e;
           gi[q] = i;
@@ -243,19 +237,16 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
     __syncwarp();
     unsigned todo = __ballot_sync(0xffffffffu, gl == 0 && cnt > kSortSmall && !bur);
     while (todo) {
-      const int src = __ffs(todo) - 1;
+      const int from = __ffs(todo) - 1;
       todo &= todo - 1;
-      const long long cc = c0 + src / kSortLanes;
-      const int ccnt = __shfl_sync(0xffffffffu, cnt, src), cs = __shfl_sync(0xffffffffu, s, src);
-      if (ccnt > kSortBuf) {
-        if (lane == 0) atomicOr(status, kStatusSegmentTooLong);
-        continue;
-      }
+      const long long cc = c0 + from / kSortLanes;
+      const int ccnt = __shfl_sync(0xffffffffu, cnt, from), cs = __shfl_sync(0xffffffffu, s, from);
+      const int* csrc = ccnt > mem.size ? index + cs : mem.slots + cc * mem.size;
       const int cx = (int)cc / isx, rem = (int)cc - cx * isx, cy = rem / g.dims[2], cz = rem - cy * g.dims[2];
       const float ctr[3] = {cmin[0] + ((float)cx + 0.5f) * step, cmin[1] + ((float)cy + 0.5f) * step,
                             cmin[2] + ((float)cz + 0.5f) * step};
       for (int q = lane; q < ccnt; q += kWarp) {
-        const int i = index[cs + q];
+        const int i = csrc[q];
         const float4 e = __ldg(pos + i);
         s_e[wib][q] = e;
         s_i[wib][q] = i;
@@ -287,27 +278,25 @@ gbx_status launch_tight_build(Context* ctx, const float4* pos) {
   cudaStream_t st = ctx->stream;
   const long long cells = ctx->tcell_cap;
   if (cells > 0) {
-    TightArgs a{pos,           ctx->n,          ctx->d_tgeom,   (float)ctx->cfg.switch_width,
-                ctx->d_tcount, ctx->d_tstart,   ctx->d_tcursor, ctx->d_tburied,
-                ctx->d_tindex, cells,           ctx->tentry_cap,
-                ctx->d_status};
+    const TableBuckets& b = ctx->tbuckets;
+    const Members mem{ctx->d_tcount, b.slots,         b.chain,
+                      b.node,        b.size,          ctx->tentry_cap,
+                      &ctx->d_tgeom->chained, ctx->d_status};
+    const TightArgs a{pos, ctx->n, ctx->d_tgeom, (float)ctx->cfg.switch_width, mem, ctx->d_tburied, cells};
     const int threads = 256;
     long long blocks = ((long long)ctx->n * kWarp + threads - 1) / threads;
     if (blocks > 65535) blocks = 65535;
-    tight_members_kernel<false><<<(int)blocks, threads, 0, st>>>(a);
+    tight_members_kernel<<<(int)blocks, threads, 0, st>>>(a);
     ++ctx->launches;
-    launch_scan<true>(ctx->d_tcount, ctx->d_tgeom, ctx->d_tstart, ctx->d_tcursor, cells, ctx->tentry_cap,
-                      reinterpret_cast<unsigned long long*>(&ctx->d_tgeom->total), ctx->d_status, st);
-    ++ctx->launches;
-    tight_members_kernel<true><<<(int)blocks, threads, 0, st>>>(a);
+    launch_scan<true>(ctx->d_tcount, ctx->d_tgeom, ctx->d_tstart, cells, ctx->tentry_cap,
+                      reinterpret_cast<unsigned long long*>(&ctx->d_tgeom->total), &ctx->d_tgeom->longest, b.size,
+                      ctx->d_status, st);
     ++ctx->launches;
     long long sb = (cells + kSortWarps * kSortGroups - 1) / (kSortWarps * kSortGroups);
     if (sb > (long long)ctx->sms * 64) sb = (long long)ctx->sms * 64;
-    tight_sort_kernel<<<(int)sb, kSortWarps * kWarp, 0, st>>>(pos, ctx->d_tcount, ctx->d_tstart, ctx->d_tburied,
-                                                               ctx->d_tentry, ctx->d_tindex, ctx->d_tcell, ctx->d_tfirst,
-                                                               ctx->d_tgeom,
-                                                               (float)ctx->cfg.switch_width, cells, ctx->tentry_cap,
-                                                               ctx->d_status);
+    tight_sort_kernel<<<(int)sb, kSortWarps * kWarp, 0, st>>>(pos, mem, ctx->d_tstart, ctx->d_tburied, ctx->d_tentry,
+                                                              ctx->d_tindex, ctx->d_tcell, ctx->d_tfirst, ctx->d_tgeom,
+                                                              (float)ctx->cfg.switch_width, cells, ctx->tentry_cap);
     ++ctx->launches;
   }
   cudaError_t e = cudaGetLastError();

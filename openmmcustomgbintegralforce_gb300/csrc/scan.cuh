@@ -25,12 +25,13 @@ __device__ __forceinline__ int scan_alloc(int count) {
 
 // start[c] for the cells of `geom` (none if it has more than cell_cap);
 // *total (zero on entry) receives the sum.  Cells past the entry capacity
-// raise the status and start at the largest index, which no fill may write.
+// raise the status and start at the largest index.  *longest (if wanted)
+// receives the largest count above `bucket`.
 template <bool EVEN>
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(const int* __restrict__ count,
                                                             const TableGeom* gp, int* __restrict__ start,
-                                                            int* __restrict__ cursor, long long cell_cap,
-                                                            long long entry_cap, unsigned long long* total,
+                                                            long long cell_cap, long long entry_cap,
+                                                            unsigned long long* total, int* longest, int bucket,
                                                             unsigned* __restrict__ status) {
   __shared__ int s_warp[kScanThreads / kWarp];
   __shared__ long long s_base;
@@ -47,9 +48,10 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const int* __restric
   } else {
     for (int k = 0; k < kScanItems; ++k) v[k] = base + k < ncell ? count[base + k] : 0;
   }
-  int sum = 0;
+  int sum = 0, most = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
+    most = max(most, v[k]);
     const int c = scan_alloc<EVEN>(v[k]);
     v[k] = sum;  // exclusive within the thread
     sum += c;
@@ -60,6 +62,10 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const int* __restric
     if (lane >= off) incl += u;
   }
   if (lane == kWarp - 1) s_warp[w] = incl;
+  if (longest) {
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0 && most > bucket) atomicMax(longest, most);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     int acc = 0;
@@ -80,24 +86,17 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(const int* __restric
   if (base + kScanItems <= ncell) {
     *reinterpret_cast<int4*>(start + base) = make_int4(o[0], o[1], o[2], o[3]);
     *reinterpret_cast<int4*>(start + base + 4) = make_int4(o[4], o[5], o[6], o[7]);
-    if (cursor) {
-      *reinterpret_cast<int4*>(cursor + base) = make_int4(0, 0, 0, 0);
-      *reinterpret_cast<int4*>(cursor + base + 4) = make_int4(0, 0, 0, 0);
-    }
   } else {
-    for (int k = 0; k < kScanItems && base + k < ncell; ++k) {
-      start[base + k] = o[k];
-      if (cursor) cursor[base + k] = 0;
-    }
+    for (int k = 0; k < kScanItems && base + k < ncell; ++k) start[base + k] = o[k];
   }
 }
 
 template <bool EVEN = false>
-inline void launch_scan(const int* count, const TableGeom* geom, int* start, int* cursor, long long cell_cap,
-                        long long entry_cap, unsigned long long* total, unsigned* status, cudaStream_t st) {
+inline void launch_scan(const int* count, const TableGeom* geom, int* start, long long cell_cap, long long entry_cap,
+                        unsigned long long* total, int* longest, int bucket, unsigned* status, cudaStream_t st) {
   const long long nb = (cell_cap + kScanTile - 1) / kScanTile;
-  scan_kernel<EVEN><<<(int)(nb < 1 ? 1 : nb), kScanThreads, 0, st>>>(count, geom, start, cursor, cell_cap, entry_cap,
-                                                                     total, status);
+  scan_kernel<EVEN><<<(int)(nb < 1 ? 1 : nb), kScanThreads, 0, st>>>(count, geom, start, cell_cap, entry_cap, total,
+                                                                     longest, bucket, status);
 }
 
 }  // namespace

@@ -229,3 +229,32 @@ def test_autograd_types_and_streams(dtypes):
     for t, k in zip(plain[1:], GRADS):
         want = -ref[k] if k == "forces" else ref[k]
         assert rel_rms(t.double().cpu().numpy(), want) < F_TOL, k
+
+
+# a table sized on spread-out atoms keeps buckets for short lists: crowded, the
+# same atoms have lists far longer than their buckets and as many entries
+@pytest.mark.parametrize("n", [40, 250])
+@pytest.mark.parametrize("name", ["exact", "standalone", "grid", "gbmv1", "gbmv2"])
+def test_lists_longer_than_their_buckets(n, name):
+    rng = np.random.default_rng(n)
+    k = int(np.ceil(n ** (1 / 3)))
+    lattice = np.stack(np.meshgrid(*[np.arange(k)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    sparse = 0.6 * lattice.astype(np.float64)
+    dense = (rng.uniform(1.0, 1.3, (n, 3))).astype(np.float32).astype(np.float64)
+    r = rng.uniform(0.12, 0.2, n)
+    q = rng.normal(size=n)
+    box = box_for(sparse)
+    m = {"exact": GBModel.charmm_gbsw(), "standalone": GBModel.charmm_gbsw(reference_table=True),
+         "grid": GBModel.gbsw_integral(), "gbmv1": GBModel.gbmv1(box=box), "gbmv2": GBModel.gbmv2(box=box)}[name]
+    a, b = context(m, (q, r)), context(m, (q, r))
+    a.execute_host(sparse)
+    for _ in range(2):
+        Ea, Fa = a.execute_host(dense)
+        Eb, Fb = b.execute_host(dense)
+        assert Ea == Eb and np.array_equal(Fa, Fb)
+        assert np.array_equal(a.integrals(), b.integrals())
+    assert_table(a, m, dense, r)
+    ref = O.Oracle(m).integrals(dense, r)[0]
+    assert np.abs(a.integrals() - ref).max() < I_TOL * np.abs(ref).max()
+    a.close()
+    b.close()
