@@ -79,73 +79,72 @@ struct RefQuery {
   float inv[3];
   float invdims[3];  // periodic table: 1 / dims, the box in cell units being dims
   float eps;     // guard band in cell units
-  bool off;      // the geometry has more cells than are allocated: no cell
+  int dims[3];   // 0: the geometry has more cells than are allocated, no cell
+  bool box;      // box-sampled table: points are moved by whole boxes
   const TableGeom* g;
   const double* qoff;
+  // A coordinate t = v / step + rel in cell units carries the FP32 rounding of
+  // rel, of v and 1 / step, of the sum and of a move by whole boxes: at most
+  // 2^-24 (3 |rel| + 4 |v| / step).  The guard band is twice 4 (|rel| + reach /
+  // step) 2^-24 (a band of 3e-4 cells, ten times this, cost 21 of the 108 us of
+  // a 6,007-atom integral pass in FP64 queries).
+  static __device__ __forceinline__ float guard_band(float mag) { return 1e-6f + 8.0f * mag * 5.96e-8f; }
   __device__ __forceinline__ void init(const TableGeom& geom, const float4 xi, const double* qo, long long cap) {
     g = &geom;
     qoff = qo;
-    off = geom.ncell > cap;
+    const bool off = geom.ncell > cap;
+    box = geom.mode == GBX_TABLE_PERIODIC;
     const double x[3] = {(double)xi.x, (double)xi.y, (double)xi.z};
-    // A coordinate t = v / step + rel in cell units carries the FP32 rounding of
-    // rel, of v and 1 / step, of the sum and of a move by whole boxes: at most
-    // 2^-24 (3 |rel| + 4 |v| / step).  The guard band is twice 4 (|rel| + reach /
-    // step) 2^-24 (a band of 3e-4 cells, ten times this, cost 21 of the 108 us of
-    // a 6,007-atom integral pass in FP64 queries).
     float mag = 0.0f;
     for (int k = 0; k < 3; ++k) {
       rel[k] = (float)((x[k] - geom.min[k]) * geom.inv_step[k]);
       inv[k] = (float)geom.inv_step[k];
+      dims[k] = off ? 0 : geom.dims[k];
       invdims[k] = 1.0f / (float)geom.dims[k];
       mag = fmaxf(mag, fmaf((float)geom.reach, inv[k], fabsf(rel[k])));
     }
-    eps = 1e-6f + 8.0f * mag * 5.96e-8f;
+    eps = guard_band(mag);
   }
   __device__ __forceinline__ void init(const Entries& t, const float4 xi, const double* qo) {
     init(*t.geom, xi, qo, usable_cells(t));
   }
   __device__ __forceinline__ long long cell(const float4 xi, const float4 v, int q) const {
     bool unsafe;
-    const long long c = cell_fast(v, unsafe);
+    const int c = cell_fast(v, unsafe);
     return unsafe ? query_exact(*g, xi, qoff, q) : c;
   }
   // The FP32 query alone; unsafe: the point lies within the guard band of a
   // cell face or grid edge and needs the exact query (the result is then -1).
-  __device__ __forceinline__ long long cell_fast(const float4 v, bool& unsafe) const {
-    unsafe = false;
-    if (off) return -1;
-    const TableGeom& G = *g;
+  // The grid's edges are cell faces too, so one compare over the axes finds
+  // both; floor by adding 1.5 2^23 rounding down, at full rate (rounding and
+  // conversion instructions run at a quarter; beyond 2^22 cells the guard band
+  // covers everything).
+  __device__ __forceinline__ int cell_fast(const float4 v, bool& unsafe) const {
     float t[3] = {fmaf(v.x, inv[0], rel[0]), fmaf(v.y, inv[1], rel[1]), fmaf(v.z, inv[2], rel[2])};
+    if (box) {
+      // the box-sampled grid spans the box (step = box / dims): moving the
+      // point by whole boxes (CustomGBIntegral.cpp:284-309) is a shift by
+      // whole multiples of dims in cell units
+#pragma unroll
+      for (int k = 0; k < 3; ++k) t[k] = fmaf(-floor_fast(t[k] * invdims[k]), (float)dims[k], t[k]);
+    }
+    return cell_at(t, unsafe);
+  }
+  static __device__ __forceinline__ float floor_fast(float x) { return __fadd_rd(x, 12582912.0f) - 12582912.0f; }
+  __device__ __forceinline__ int cell_at(const float* t, bool& unsafe) const {
     int id[3];
-    bool safe = true;
+    float face = 0.0f;  // the largest distance from a cell's middle along an axis
+    bool in = true;
+    const int last = box ? 0 : 1;  // a grid's last index is a point, not a cell
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      if (G.mode == GBX_TABLE_PERIODIC) {
-        // the box-sampled grid spans the box (step = box / dims): moving the
-        // point by whole boxes (CustomGBIntegral.cpp:284-309) is a shift by
-        // whole multiples of dims in cell units; a point within the guard
-        // band of a box edge takes the exact path
-        const float W = (float)G.dims[k];
-        const float nb = floorf(t[k] * invdims[k]);
-        t[k] = fmaf(-nb, W, t[k]);
-        if (t[k] < eps || t[k] > W - eps) safe = false;
-      }
-      const float f = floorf(t[k]);
-      const float fr = t[k] - f;
-      id[k] = (int)f;
-      if (fr < eps || fr > 1.0f - eps) safe = false;
-      if (G.mode == GBX_TABLE_PERIODIC) {
-        if (id[k] < 0 || id[k] >= G.dims[k]) safe = false;
-      } else {
-        if (t[k] < -eps || t[k] > (float)(G.dims[k] - 1) + eps) return -1;
-        if (t[k] < eps || t[k] > (float)(G.dims[k] - 1) - eps) safe = false;
-      }
+      const float m = __fadd_rd(t[k], 12582912.0f);
+      id[k] = __float_as_int(m) - 0x4B400000;
+      face = fmaxf(face, fabsf((t[k] - (m - 12582912.0f)) - 0.5f));
+      in = in && (unsigned)id[k] < (unsigned)(dims[k] - last);
     }
-    if (!safe) {
-      unsafe = true;
-      return -1;
-    }
-    return (long long)id[0] * ((long long)G.dims[1] * G.dims[2]) + (long long)id[1] * G.dims[2] + id[2];
+    unsafe = dims[0] > 0 && (face > 0.5f - eps || (box && !in));
+    return in && !unsafe ? (id[0] * dims[1] + id[1]) * dims[2] + id[2] : -1;
   }
   // x_j - p formed as (x_j - x_i) - v: the FP32 difference of nearby atoms is exact
   __device__ __forceinline__ float3 delta(const float4 a, const float4 xi, const float4 v) const {
@@ -158,42 +157,44 @@ struct RefQuery {
 };
 
 // The same query of a box-sampled table (GBX_TABLE_PERIODIC), for passes that
-// only look cells up: an atom whose every point stays inside the box needs no
-// move; a cell face is detected by one compare over the axes (the box edges
-// are cell faces too); floor by adding 1.5 2^23 rounding down, at full rate
-// (the general form's rounding and conversion instructions run at a quarter).
+// only look cells up, a warp per atom: an atom whose every point stays inside
+// the box needs no move.
 struct BoxQuery : RefQuery {
   bool inside;  // no point of the atom leaves the box
+  float W[3];   // dims
   __device__ __forceinline__ void init(const Entries& t, const float4 xi, const double* qo) {
-    RefQuery::init(t, xi, qo);
+    const TableGeom& geom = *t.geom;
+    g = &geom;
+    qoff = qo;
+    box = true;
+    const bool off = geom.ncell > usable_cells(t);
+    // an axis per lane (FP64 instructions cost the same for one lane as for 32)
+    const int a = threadIdx.x % kWarp % 3;
+    const double x = a == 0 ? xi.x : (a == 1 ? xi.y : xi.z);
+    const float rel_ = (float)((x - geom.min[a]) * geom.inv_step[a]), inv_ = (float)geom.inv_step[a],
+                w_ = (float)geom.dims[a], invdims_ = 1.0f / w_, reach = (float)geom.reach;
+    float mag = 0.0f;
     inside = true;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float r = fmaf((float)g->reach, inv[k], 0.01f);
-      inside = inside && rel[k] - r > 0.0f && rel[k] + r < (float)g->dims[k];
+      rel[k] = __shfl_sync(0xffffffffu, rel_, k);
+      inv[k] = __shfl_sync(0xffffffffu, inv_, k);
+      W[k] = __shfl_sync(0xffffffffu, w_, k);
+      invdims[k] = __shfl_sync(0xffffffffu, invdims_, k);
+      dims[k] = off ? 0 : geom.dims[k];
+      mag = fmaxf(mag, fmaf(reach, inv[k], fabsf(rel[k])));
+      const float r = fmaf(reach, inv[k], 0.01f);
+      inside = inside && rel[k] - r > 0.0f && rel[k] + r < W[k];
     }
+    eps = guard_band(mag);
   }
   __device__ __forceinline__ int cell_fast(const float4 v, bool& unsafe) const {
-    unsafe = false;
-    if (off) return -1;
     float t[3] = {fmaf(v.x, inv[0], rel[0]), fmaf(v.y, inv[1], rel[1]), fmaf(v.z, inv[2], rel[2])};
-    const int d[3] = {g->dims[0], g->dims[1], g->dims[2]};
     if (!inside) {
 #pragma unroll
-      for (int k = 0; k < 3; ++k) t[k] = fmaf(-floorf(t[k] * invdims[k]), (float)d[k], t[k]);
+      for (int k = 0; k < 3; ++k) t[k] = fmaf(-floor_fast(t[k] * invdims[k]), W[k], t[k]);
     }
-    int id[3];
-    float face = 0.0f;  // the largest distance from a cell's middle along an axis
-    bool in = true;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const float m = __fadd_rd(t[k], 12582912.0f);
-      id[k] = __float_as_int(m) - 0x4B400000;
-      face = fmaxf(face, fabsf((t[k] - (m - 12582912.0f)) - 0.5f));
-      in = in && (unsigned)id[k] < (unsigned)d[k];
-    }
-    unsafe = !in || face > 0.5f - eps;
-    return unsafe ? -1 : (id[0] * d[1] + id[1]) * d[2] + id[2];
+    return cell_at(t, unsafe);
   }
 };
 
