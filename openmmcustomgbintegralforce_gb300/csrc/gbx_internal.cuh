@@ -358,6 +358,9 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
 int pair_energy_parts(int n, int segments);
 int pair_segments(int n, int sms);
 ModelConst make_model_const(const Context* ctx);
+// The GBSW chain rule forms dE/dJ itself: no launch_chain_prep (compiled
+// expressions and the adjoint, which needs more from it, go through memory).
+bool chain_forms_dEdJ(const Context* ctx, bool adjoint);
 gbx_status launch_chain_prep(Context* ctx, bool adjoint);
 gbx_status launch_chain(Context* ctx, const float4* pos, bool adjoint);
 bool gbmv_cells_apply(const Context* ctx);

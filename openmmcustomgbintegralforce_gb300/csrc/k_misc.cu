@@ -212,7 +212,12 @@ gbx_status launch_born(Context* ctx) {
   return GBX_OK;
 }
 
+bool chain_forms_dEdJ(const Context* ctx, bool adjoint) {
+  return ctx->cfg.model == GBX_MODEL_GBSW && !adjoint && !ctx->custom;
+}
+
 gbx_status launch_chain_prep(Context* ctx, bool adjoint) {
+  if (chain_forms_dEdJ(ctx, adjoint)) return GBX_OK;
   const int n = ctx->n;
   chain_prep_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(
       n, ctx->d_dEdB_fx, ctx->d_dBdJ, ctx->d_dBdJ + 2 * (size_t)n, ctx->d_dEdJ,

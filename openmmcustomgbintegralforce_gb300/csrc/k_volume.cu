@@ -714,6 +714,20 @@ struct Shaping {
   }
 };
 
+// dE/dJ of an atom: as a kernel before left it, or formed from dE/dB and dB/dJ
+// by the warp that needs it (a launch less: 98.6 -> 97.6 us at 1,001 atoms, and
+// no difference from 6,000 up).
+struct DEdJ {
+  const float2* value;  // nullptr: not formed
+  const unsigned long long* dEdB_fx;
+  const double* dBdJ;   // [2n]
+  __device__ __forceinline__ float2 of(int i, int lane) const {
+    if (value) return value[i];
+    const float part = (float)(fixed_to_double(dEdB_fx[i]) * dBdJ[2 * i + (lane & 1)]);
+    return make_float2(__shfl_sync(0xffffffffu, part, 0), __shfl_sync(0xffffffffu, part, 1));
+  }
+};
+
 // GBSW chain rule over the recorded points: warp = (atom i, quadrature
 // chunk).  Each lane takes one record of a batch of 32 and the warp unrolls
 // the shaping-entry masks into a ring of (record, list position) items, from
@@ -732,9 +746,8 @@ struct Shaping {
 // positions stays in L1, where the 16-byte list entries themselves do not.
 template <class Q, bool ADJ>
 __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* __restrict__ pos, int n, Entries tab,
-                                                                 Quad quad, ModelConst m, int n_chunks,
-                                                                 const float2* __restrict__ dEdJ, ChainOut out,
-                                                                 ChainRecords rr) {
+                                                                 Quad quad, ModelConst m, int n_chunks, DEdJ dEdJ,
+                                                                 ChainOut out, ChainRecords rr) {
   constexpr int kComp = ADJ ? 4 : 3;  // integers pushed per item
   constexpr int kWarps = kThreads / kWarp;
   constexpr int kRing = 2 * kWarp;    // fewer than 32 items pending, plus one round of at most 32
@@ -748,7 +761,7 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
   if (warp >= n * n_chunks) return;
   const int i = warp % n, c = warp / n;
   const float4 xi = pos[i];
-  const float2 de = dEdJ[i];
+  const float2 de = dEdJ.of(i, lane);
   const unsigned lt = (1u << lane) - 1u;
   // F_i as fixed-point integers: every contribution is rounded on its own, so
   // the record and the list-walk paths give the same bits
@@ -1107,8 +1120,8 @@ void launch_chain_t(Context* ctx, const float4* pos, const ModelConst& m) {
   const int blocks = volume_blocks(ctx);
   if constexpr (MODEL == GBX_MODEL_GBSW) {
     const ChainRecords rr{ctx->d_srec, ctx->d_srec_st, ctx->records ? ctx->d_rcount : nullptr, ctx->srec_R};
-    gbsw_chain_kernel<Q, ADJ><<<blocks, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, ctx->n_chunks, ctx->d_dEdJ,
-                                                                    o, rr);
+    const DEdJ de{chain_forms_dEdJ(ctx, ADJ) ? nullptr : ctx->d_dEdJ, ctx->d_dEdB_fx, ctx->d_dBdJ};
+    gbsw_chain_kernel<Q, ADJ><<<blocks, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, ctx->n_chunks, de, o, rr);
   } else {
     gbmv_chain_kernel<MODEL, Q, ADJ><<<blocks, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, chunk, ctx->n_chunks,
                                                                            ctx->d_dEdJ, o, ctx->d_pstate);
