@@ -337,14 +337,15 @@ GBX_API gbx_status gbx_get_chain_work(gbx_context* ctx, double* list_evals, doub
  * counterpart in the reference. */
 GBX_API gbx_status gbx_get_launches(gbx_context* ctx, long long* launches);
 
-/* GBSW forces: the integral pass writes one 16-byte record (q, V, mask of
- * the shaping list entries) per quadrature point that an atom other than its
- * own shapes, so that the chain rule visits only those entries instead of
- * re-walking every point's cell list.  Each warp (atom x quadrature chunk) owns per_warp records.  per_warp < 0: automatic (the default; first half a warp's points,
- * then 1.125x the largest need seen), 0: no records (the chain rule walks the
- * lists), > 0: that fixed size.  A warp whose records do not fit walks its
- * lists instead, with bit-identical results, so the size only affects speed.
- * No counterpart in the reference. */
+/* GBSW forces and adjoint: the integral pass writes one 16-byte record (q, V,
+ * mask of the shaping list entries) per quadrature point that an atom other
+ * than its own shapes (the adjoint: any atom), so that the chain rule visits
+ * only those entries instead of re-walking every point's cell list.  Each warp
+ * (atom x quadrature chunk) owns per_warp records.  per_warp < 0: automatic
+ * (the default; first half a warp's points, then 1.125x the largest need
+ * seen), 0: no records (the chain rule walks the lists), > 0: that fixed size.
+ * A warp whose records do not fit walks its lists instead, with bit-identical
+ * results, so the size only affects speed.  No counterpart in the reference. */
 GBX_API gbx_status gbx_set_chain_records(gbx_context* ctx, int per_warp);
 
 /* Records of the last execute: written (-1 if it kept none), the largest
@@ -354,10 +355,11 @@ GBX_API gbx_status gbx_get_chain_records(gbx_context* ctx, long long* written, i
                                          int* overflowed);
 
 /* Per-stage device times (ms) of the last execute, from CUDA events recorded
- * on the execute stream when timing is enabled.  Stages: 0 position staging,
- * 1 lookup table, 2 integrals, 3 Born radii, 4 pair term, 5 chain prep,
- * 6 chain rule, 7 energy reduction.  Diagnostics; no counterpart in the
- * reference. */
+ * on the execute stream when timing is enabled.  Stages: 0 (empty: staging is
+ * part of the next), 1 positions staged and lookup table, 2 point binning
+ * (GBMV), 3 integrals, 4 Born radii, 5 pair term, 6 chain prep (empty where
+ * the chain rule needs none), 7 chain rule, 8 forces, energy and status out.
+ * Diagnostics; no counterpart in the reference. */
 GBX_API gbx_status gbx_set_timing(gbx_context* ctx, int enable);
 GBX_API gbx_status gbx_get_stage_times(gbx_context* ctx, double* ms, int max_stages, int* num_stages);
 

@@ -230,7 +230,7 @@ gbx_status alloc_atom_buffers(Context* ctx) {
     GBX_TRY(dalloc(ctx, &ctx->d_scount, gbx::kMaxSortCells));
     GBX_TRY(dalloc(ctx, &ctx->d_sstart, gbx::kMaxSortCells));
     GBX_TRY(dalloc(ctx, &ctx->d_scursor, gbx::kMaxSortCells));
-    GBX_TRY(dalloc(ctx, &ctx->d_sgeom, 2));
+    GBX_TRY(dalloc(ctx, &ctx->d_sgeom, 1));
   }
   GBX_TRY(dalloc(ctx, &ctx->d_force_fx, 3 * (size_t)n));
   GBX_TRY(dalloc(ctx, &ctx->d_f4, 4 * (size_t)n));

@@ -55,6 +55,14 @@ struct TableGeom {
   unsigned chained;  // list members outside their cell's bucket
 };
 
+// Grid of the spatial order of the cutoff pair term (k_pair.cu).
+struct SortGeom {
+  float lo[3];
+  float inv_cell;
+  int dims[3];
+  int ncell;
+};
+
 // Where a table's members are collected (buckets.cuh).
 struct TableBuckets {
   int* slots = nullptr;   // [cell_cap][size]
@@ -187,7 +195,7 @@ struct Context {
   int* d_scount = nullptr;                    // cutoff: atoms per spatial cell [kMaxSortCells]
   int* d_sstart = nullptr;
   int* d_scursor = nullptr;
-  int4* d_sgeom = nullptr;                    // cutoff: spatial grid geometry
+  SortGeom* d_sgeom = nullptr;                  // cutoff: spatial grid geometry
   float* d_pstate = nullptr;                  // GBMV: per-point sums kept for the chain rule
   // GBMV points binned by lookup-table cell (k_gbmv.cu)
   int2* d_pat = nullptr;                      // [n Q] (the point's cell or -1, slot within the cell)

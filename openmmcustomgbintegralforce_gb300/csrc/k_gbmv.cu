@@ -11,9 +11,9 @@
 //
 //   bin      warp per (atom, quadrature chunk), lanes over points: the
 //            point's cell (the reference query, exact near cell faces),
-//            a slot in the cell by one atomic per point, four points per
-//            lane in flight; points whose cell has no list get their
-//            solvent fraction here
+//            a slot in the cell by one atomic per run of a ray's points in
+//            one cell, four points per lane in flight; points whose cell has
+//            no list get their solvent fraction here
 //   scan     points per cell -> each cell's first slot
 //   fill     point ids into their cell's slots
 //   integral warp per cell: sorts the cell's point ids (the slots were
@@ -26,7 +26,9 @@
 //   reduce   warp per (atom, chunk): J4, J7 over the solvent fractions in
 //            quadrature order (the integral pass's partition, so the Born
 //            radii are assembled as before)
-//   chain    warp per cell, lanes as 4 points x 8 lanes of entry pairs
+//   chain    warp per cell over the points whose solvent fraction still
+//            varies (the integral pass leaves them first), lanes as 4 points
+//            x 8 lanes of entry pairs
 //            (packed FP32x2, two entries per instruction; the integral pass
 //            likewise evaluates two entries per instruction): each lane
 //            keeps the pull of its entries in registers over all of the
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(kBinThreads) gbmv_bin_kernel(const float4* __r
                                                                CellPoints cp) {
   // kBinBatch points per lane per step: their cell queries, list-count loads
   // and slot atomics are issued back to back.  A point within the FP32
-  // query's guard band (about one in 500) needs the FP64 query; those are
+  // query's guard band (one in several thousand) needs the FP64 query; those are
   // queued per warp and resolved kBinDefer at a time with every lane busy,
   // instead of stalling the warp for each one (FP64 runs at a small fraction
   // of the FP32 rate on this part, whatever the number of active lanes).
@@ -492,10 +494,8 @@ struct __align__(16) PointChain {
 constexpr int kChainWarps = 1;
 template <int MODEL, bool PER, bool ADJ>
 __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MODEL_GBMV2 ? 28 : 32)
-    gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab,
-                                                                       Quad quad, ModelConst m, CellPoints cp,
-                                                                       const float2* __restrict__ dEdJ,
-                                                                       CellChainOut out) {
+    gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab, Quad quad, ModelConst m, CellPoints cp,
+                           const float2* __restrict__ dEdJ, CellChainOut out) {
   __shared__ ChainPair s_list[kChainWarps][kMaxList / 2];
   __shared__ float2 s_r[ADJ ? kChainWarps : 1][ADJ ? kMaxList / 2 : 1];  // R_j of the pairs
   __shared__ PointChain s_pt[kChainWarps][kWarp];

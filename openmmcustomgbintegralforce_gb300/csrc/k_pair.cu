@@ -4,8 +4,9 @@
 //   D = r^2 / (4 B_i B_j),  f = sqrt(r^2 + B_i B_j e^-D),  e_ij = pref q_i q_j / f
 //   E = sum_{i<j} e_ij + 1/2 sum_i pref q_i^2 / B_i
 //
-// Each thread owns one atom i and streams every j through shared memory
-// (warp-uniform broadcast reads).  Only i-side quantities are accumulated, so
+// The context's pair term is the symmetric scheme below (pair_sym_kernel).  The
+// allocation-free entry point's (pair_kernel): each thread owns one atom i and
+// streams every j through shared memory (warp-uniform broadcast reads).  Only i-side quantities are accumulated, so
 // every ordered pair is visited once from each end: twice the pair
 // arithmetic of a symmetric tile scheme, but no j-side accumulators, no
 // shuffles and no per-tile atomics, and every per-atom sum runs in a fixed
@@ -550,66 +551,8 @@ __global__ void __launch_bounds__(kSymThreads, ADJ ? 3 : 4) pair_sym_kernel(SymA
 // input alone.  32 consecutive slots then form a compact tile whose bounding
 // box is far from most others, and the cutoff culls those tile pairs.
 // ---------------------------------------------------------------------------
-struct SortGeom {
-  float lo[3];
-  float inv_cell;
-  int dims[3];
-  int ncell;
-};
-
 constexpr int kBoxThreads = 1024;
 constexpr int kSortSeg = 512;  // atoms per cell ranked in shared memory
-
-__global__ void __launch_bounds__(kBoxThreads) sort_geom_kernel(const float4* __restrict__ pos, int n,
-                                                                SortGeom* __restrict__ g) {
-  __shared__ float s_lo[3][kBoxThreads / kWarp], s_hi[3][kBoxThreads / kWarp];
-  float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    const float4 p = pos[k];
-    lo[0] = fminf(lo[0], p.x), hi[0] = fmaxf(hi[0], p.x);
-    lo[1] = fminf(lo[1], p.y), hi[1] = fmaxf(hi[1], p.y);
-    lo[2] = fminf(lo[2], p.z), hi[2] = fmaxf(hi[2], p.z);
-  }
-  for (int off = 16; off > 0; off >>= 1)
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], off));
-      hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], off));
-    }
-  if (threadIdx.x % kWarp == 0)
-    for (int d = 0; d < 3; ++d) {
-      s_lo[d][threadIdx.x / kWarp] = lo[d];
-      s_hi[d][threadIdx.x / kWarp] = hi[d];
-    }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x / kWarp); ++w)
-      for (int d = 0; d < 3; ++d) {
-        s_lo[d][0] = fminf(s_lo[d][0], s_lo[d][w]);
-        s_hi[d][0] = fmaxf(s_hi[d][0], s_hi[d][w]);
-      }
-    float cell = 1.0f;
-    for (;;) {
-      long long tot = 1;
-      int dims[3];
-      for (int d = 0; d < 3; ++d) {
-        const float span = (s_hi[d][0] - s_lo[d][0]) / cell;
-        // non-finite or huge spans (invalid positions) collapse to one cell row
-        dims[d] = (span >= 0.0f && span < (float)kMaxSortCells) ? (int)span + 1 : 1;
-        tot *= dims[d];
-      }
-      if (tot <= kMaxSortCells || cell > 1e6f) {
-        for (int d = 0; d < 3; ++d) {
-          g->lo[d] = s_lo[d][0];
-          g->dims[d] = dims[d];
-        }
-        g->inv_cell = 1.0f / cell;
-        g->ncell = (int)tot;
-        break;
-      }
-      cell *= 1.25f;
-    }
-  }
-}
 
 __device__ __forceinline__ int sort_cell(const SortGeom& g, const float4 p) {
   int c[3];
@@ -787,15 +730,13 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
   } else if (a.cutoff2 > 0) {
     // spatial order, then tile boxes over it
     const int n = a.n, nb = (n + 255) / 256;
-    SortGeom* sg = reinterpret_cast<SortGeom*>(ctx->d_sgeom);
-    sort_geom_kernel<<<1, kBoxThreads, 0, st>>>(pos, n, sg);
-    cudaMemsetAsync(ctx->d_scount, 0, sizeof(int) * kMaxSortCells, st);
+    const SortGeom* sg = ctx->d_sgeom;  // written, and d_scount cleared, by the call's first kernel
     sort_count_kernel<<<nb, 256, 0, st>>>(pos, n, sg, ctx->d_cell_of, ctx->d_scount);
     sort_scan_kernel<<<1, kBoxThreads, 0, st>>>(ctx->d_scount, sg, ctx->d_sstart, ctx->d_scursor);
     sort_scatter_kernel<<<nb, 256, 0, st>>>(ctx->d_cell_of, n, ctx->d_sstart, ctx->d_scursor, ctx->d_perm_tmp);
     sort_cells_by_atom_kernel<<<ctx->sms * 8, kSymThreads, 0, st>>>(ctx->d_scount, ctx->d_sstart, sg, ctx->d_perm_tmp,
                                                                ctx->d_perm);
-    ctx->launches += 5;
+    ctx->launches += 4;
     a.perm = ctx->d_perm;
     tile_box_kernel<<<(a.ntiles + wpb - 1) / wpb, kSymThreads, 0, st>>>(pos, ctx->d_perm, a.n, a.ntiles,
                                                                         ctx->d_tile_box);

@@ -55,6 +55,7 @@ struct PrepareArgs {
   int mode;
   double h, buffer, box[3], reach;
   long long ref_cap;
+  SortGeom* sort;  // cutoff pair term: the grid of its spatial order
 };
 
 // Internal positions: x, y, z and the model's main per-atom parameter in .w
@@ -170,6 +171,30 @@ __device__ __forceinline__ void ref_rest(const PrepareArgs& a, TableGeom& g, uns
   if (a.mode == GBX_TABLE_PERIODIC) g.pad = 0.0;
   g.ncell = (long long)g.dims[0] * g.dims[1] * g.dims[2];
   if (g.ncell > a.ref_cap) status |= kStatusTableCells;
+}
+
+// The grid of the cutoff pair term's spatial order: 1 nm cells, grown so that
+// there are at most kMaxSortCells.  (One block that read every position for
+// its extents took 27 us of a 50,000-atom step.)
+__device__ __forceinline__ SortGeom sort_grid(const GeomPart& e) {
+  SortGeom g;
+  float cell = 1.0f;
+  for (;;) {
+    long long tot = 1;
+    for (int d = 0; d < 3; ++d) {
+      const float span = (e.mx[d] - e.mn[d]) / cell;
+      // non-finite or huge spans (invalid positions) collapse to one cell row
+      g.dims[d] = (span >= 0.0f && span < (float)kMaxSortCells) ? (int)span + 1 : 1;
+      tot *= g.dims[d];
+    }
+    if (tot <= kMaxSortCells || cell > 1e6f) {
+      for (int d = 0; d < 3; ++d) g.lo[d] = e.mn[d];
+      g.inv_cell = 1.0f / cell;
+      g.ncell = (int)tot;
+      return g;
+    }
+    cell *= 1.25f;
+  }
 }
 
 // REF: the reference's grid is wanted (FP64 sums and radii; the exact table's
@@ -332,6 +357,7 @@ __global__ void __launch_bounds__(kPrepThreads) prepare_kernel(const __grid_cons
     __syncwarp();
     if (lane == 0) ref_rest(a, s_geom[1], status);
   }
+  if (a.sort && w == 2 && lane == 0) *a.sort = sort_grid(s_all);
   if (status) atomicOr(&s_status, status);
   __syncthreads();
   if (t == 0) {
@@ -370,6 +396,10 @@ gbx_status launch_prepare(Context* ctx, const void* posq, bool tight, bool refer
     clear(ctx->d_energy_fx, 2);
     clear(ctx->d_next_item, 1);
     clear(ctx->d_rmax, 1);
+  }
+  if (call && ctx->d_sgeom && !c.periodic && !ctx->custom) {
+    a.sort = ctx->d_sgeom;
+    clear(ctx->d_scount, kMaxSortCells);
   }
   const bool wrapped = tight && c.periodic;  // the standalone grid's edges decide where a point is moved
   if (tight) {

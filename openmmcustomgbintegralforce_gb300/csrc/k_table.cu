@@ -3,11 +3,10 @@
 //
 //   geometry  the grid exactly as the reference derives it (FP64), by the
 //             call's first kernel (k_prepare.cu);
-//   count     one warp per atom enumerates its candidate cells (or samples)
-//             and counts members with atomics;
+//   members   one warp per atom enumerates its candidate cells (or samples)
+//             and puts it in the bucket of each it belongs to (buckets.cuh);
 //   scan      counts -> list starts;
-//   fill      second enumeration writes members at atomic cursors;
-//   sort      one warp per cell sorts its entries, restoring the reference's
+//   sort      one warp per cell sorts its members, restoring the reference's
 //             ascending-atom insertion order, applies the per-cell cap and
 //             writes the atoms' positions and parameters inline.
 //
@@ -17,8 +16,8 @@
 #include <math.h>
 
 #include "bitonic.cuh"
-#include "gbx_internal.cuh"
 #include "buckets.cuh"
+#include "gbx_internal.cuh"
 #include "scan.cuh"
 
 namespace gbx {
@@ -38,7 +37,7 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 __device__ __forceinline__ double half_sqrt3() { return ddiv(__dsqrt_rn(3.0), 2.0); }
 
 // --------------------------------------------------------------------------
-// Membership enumeration (count / fill)
+// Membership enumeration
 // --------------------------------------------------------------------------
 
 // Column `col` of an axis-0 x axis-1 rectangle of n1 columns per row, by FP32
@@ -56,7 +55,11 @@ __device__ __forceinline__ int2 column(int col, int n1, float inv_n1) {
 // reference's FP64; the membership of a point is decided by the FP32 sum of
 // their squares wherever that is clear of the boundary by a margin that covers
 // its rounding, and by the reference's FP64 operations otherwise (FP64 for
-// every point took 98 us of a count pass at 6,007 atoms).
+// every point took 98 us of a pass over 6,007 atoms).  FP64 instructions cost
+// the same for three lanes as for 32 and were what bound the pass, so what an
+// axis needs of them is done for a block's eight atoms together (24 threads;
+// three lanes of each atom's own warp: 78 -> 70 us of that table, and 37 + 49
+// -> 28 + 41 us of two passes over 10,001 atoms of the periodic form).
 template <int MODE>
 __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const double* __restrict__ radius, int n,
                                           const TableGeom* __restrict__ gp, double h, double buffer, Members mem,

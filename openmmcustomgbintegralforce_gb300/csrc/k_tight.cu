@@ -23,8 +23,8 @@
 // buried point usually stops at its first entry.
 #include <math.h>
 
-#include "gbx_internal.cuh"
 #include "buckets.cuh"
+#include "gbx_internal.cuh"
 #include "scan.cuh"
 
 namespace gbx {
