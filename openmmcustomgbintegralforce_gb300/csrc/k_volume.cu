@@ -58,6 +58,12 @@ struct Work<true> {
 // and in a periodic system its minimum image.
 // ---------------------------------------------------------------------------
 
+// Entry `at` of a list as work counting walks it: a reference table's in the
+// reference's order (ascending atoms), the exact table's in its own.
+__device__ __forceinline__ float4 counted_entry(const Entries& t, int at) {
+  return t.first ? entry_at(t, at) : __ldg(t.e + __ldg(t.index + at));
+}
+
 // GBSW, CharmmReferenceGBSW.cpp:616-639 / GBSWIntegral.cpp:187-224: V is the
 // product of u_j over the switching shells, 0 once an atom buries the point.
 template <class Q, class W>
@@ -65,7 +71,7 @@ __device__ __forceinline__ float gbsw_volume(const Q& qy, const ModelConst& m, c
                                              int cnt, const float4 xi, const float4 v, W& wk) {
   float V = 1.0f;
   for (int l = 0; l < cnt; ++l) {
-    const float4 a = entry_at(t, start + l);
+    const float4 a = counted_entry(t, start + l);
     const float3 d = qy.delta(a, xi, v);
     const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
     const float lo = a.w - m.sw, hi = a.w + m.sw;
@@ -142,7 +148,7 @@ __device__ __forceinline__ void count_chain_work(const Q& qy, const ModelConst& 
     wk.fs += cs.x;
   } else {
     for (int l = 0; l < cs.x; ++l) {
-      const float4 a = entry_at(t, cs.y + l);
+      const float4 a = counted_entry(t, cs.y + l);
       const float3 d = qy.delta(a, xi, v);
       const float r2 = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
       const float lo = a.w - m.sw, hi = a.w + m.sw;
@@ -1063,6 +1069,18 @@ Entries entries_of(const Context* ctx) {
                  nullptr,        ctx->entry_cap};
 }
 
+// The same for work counting: a reference GBSW table's lists in ascending atom
+// order, through the positions.
+Entries counted_entries_of(const Context* ctx, const float4* pos) {
+  Entries t = entries_of(ctx);
+  if (ctx->cfg.model == GBX_MODEL_GBSW && !ctx->use_tight) {
+    t.e = pos;
+    t.index = ctx->d_entries;
+    t.first = nullptr;
+  }
+  return t;
+}
+
 int volume_blocks(const Context* ctx) {
   const long long warps = (long long)ctx->n * ctx->n_chunks;
   return (int)((warps * kWarp + kThreads - 1) / kThreads);
@@ -1097,13 +1115,10 @@ void launch_integrals_t(Context* ctx, const float4* pos, const ModelConst& m, bo
   }
   else if (count_work)
     integral_kernel<MODEL, Q, true><<<volume_blocks(ctx), kThreads, 0, ctx->stream>>>(
-        pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, ctx->d_J, ctx->d_work, ctx->d_pstate);
+        pos, ctx->n, counted_entries_of(ctx, pos), qd, m, chunk, ctx->n_chunks, ctx->d_J, ctx->d_work, ctx->d_pstate);
   else if constexpr (MODEL != GBX_MODEL_GBSW)
     gbmv_integral_kernel<MODEL, Q><<<volume_blocks(ctx), kThreads, 0, ctx->stream>>>(
         pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, ctx->d_J, ctx->d_pstate);
-  else
-    integral_kernel<MODEL, Q, false><<<volume_blocks(ctx), kThreads, 0, ctx->stream>>>(
-        pos, ctx->n, t, qd, m, chunk, ctx->n_chunks, ctx->d_J, nullptr, ctx->d_pstate);
   ++ctx->launches;
 }
 
