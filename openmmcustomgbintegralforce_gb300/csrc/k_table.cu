@@ -24,7 +24,6 @@ namespace gbx {
 namespace {
 
 constexpr int kMaxSamples = 96;  // grid values or samples per axis kept in shared memory
-constexpr int kColumnLanes = 8;  // lanes per column of grid points or samples
 constexpr int kMemberThreads = 256;
 constexpr int kMemberWarps = kMemberThreads / kWarp;
 
@@ -40,17 +39,9 @@ __device__ __forceinline__ double half_sqrt3() { return ddiv(__dsqrt_rn(3.0), 2.
 // Membership enumeration
 // --------------------------------------------------------------------------
 
-// Column `col` of an axis-0 x axis-1 rectangle of n1 columns per row, by FP32
-// division (exact for the at most 2^20 columns an atom reaches).
-__device__ __forceinline__ int2 column(int col, int n1, float inv_n1) {
-  int i = (int)(((float)col + 0.5f) * inv_n1);
-  i -= i * n1 > col;
-  return make_int2(i, col - i * n1);
-}
-
 // CharmmReferenceGBSW.cpp:472-496 (STANDALONE) and CustomGBIntegral.cpp:198-227 (GRID).
-// A warp per atom, eight lanes per column of grid points (a column's counters
-// share sectors, so its atomics leave together).  The offset from the atom
+// A warp per atom over the grid points of its box, neighbouring lanes on
+// neighbouring points (whose counters share sectors).  The offset from the atom
 // depends on one axis only, so each axis value's is formed once, in the
 // reference's FP64; the membership of a point is decided by the FP32 sum of
 // their squares wherever that is clear of the boundary by a margin that covers
@@ -114,18 +105,14 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
       const double s = dadd(dadd(dmul(d0, d0), dmul(d1, d1)), dmul(d2, d2));
       return MODE == GBX_TABLE_STANDALONE ? __dsqrt_rn(s) < pad : s < pad2;
     };
-    auto put = [&](long long cell) {
-      if (cell >= 0 && cell < ncell) mem.put(cell, a);
-    };
-    const int cols = nn[0] * nn[1];
-    const float inv_n1 = 1.0f / (float)nn[1];
-    if (!fits) {  // a grid finer than a hundredth of the pad: FP64 throughout
-      for (int col = lane; col < cols; col += kWarp) {
-        const int2 ij = column(col, nn[1], inv_n1);
-        const double d0 = offset(0, ij.x), d1 = offset(1, ij.y);
-        for (int k = 0; k < nn[2]; ++k)
-          if (inside(d0, d1, offset(2, k)))
-            put((long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2] + k);
+    if (!fits) {  // a grid finer than a hundredth of the pad: FP64 throughout, a column of points per lane
+      for (int col = lane; col < nn[0] * nn[1]; col += kWarp) {
+        const int i = col / nn[1], j = col - i * nn[1];
+        const double d0 = offset(0, i), d1 = offset(1, j);
+        for (int k = 0; k < nn[2]; ++k) {
+          const long long cell = (long long)(b[0] + i) * sx + (long long)(b[1] + j) * sy + b[2] + k;
+          if (cell >= 0 && cell < ncell && inside(d0, d1, offset(2, k))) mem.put(cell, a);
+        }
       }
       continue;
     }
@@ -139,15 +126,22 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
     __syncwarp();
     // FP32 squared distances carry a relative error below 4 2^-24
     const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
-    for (int col = lane / kColumnLanes; col < cols; col += kWarp / kColumnLanes) {
-      const int2 ij = column(col, nn[1], inv_n1);
-      const float sxy = sq[0][ij.x] + sq[1][ij.y];
-      if (sxy > out2) continue;
-      const long long row = (long long)(b[0] + ij.x) * sx + (long long)(b[1] + ij.y) * sy + b[2];
-      for (int k = lane % kColumnLanes; k < nn[2]; k += kColumnLanes) {
-        const float s = sxy + sq[2][k];
-        if (s < in2 || (s <= out2 && inside(ds[0][ij.x], ds[1][ij.y], ds[2][k]))) put(row + k);
+    const int total = nn[0] * nn[1] * nn[2];
+    const BoxIndex box(nn[1], nn[2]);
+    for (int t0 = lane; t0 < total; t0 += kPutBatch * kWarp) {
+      long long cell[kPutBatch];
+#pragma unroll
+      for (int u = 0; u < kPutBatch; ++u) {
+        const int t = t0 + u * kWarp;
+        cell[u] = -1;
+        if (t >= total) continue;
+        const int3 o = box(t);
+        const float r2 = (sq[0][o.x] + sq[1][o.y]) + sq[2][o.z];
+        if (!(r2 < in2 || (r2 <= out2 && inside(ds[0][o.x], ds[1][o.y], ds[2][o.z])))) continue;
+        const long long c = (long long)(b[0] + o.x) * sx + (long long)(b[1] + o.y) * sy + b[2] + o.z;
+        if (c < ncell) cell[u] = c;  // negative: outside, none
       }
+      mem.put(cell, a);
     }
   }
 }
@@ -241,32 +235,33 @@ __global__ void table_members_periodic_kernel(const float4* __restrict__ pos, co
       sq[k][m] = e * e;
     }
     __syncwarp();
-    auto put = [&](long long cell) {
-      if (cell >= 0 && cell < ncell) mem.put(cell, a);
-    };
-    const int cols = cnt[0] * cnt[1];
-    const float inv_n1 = 1.0f / (float)cnt[1];
     const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
     // FP32 squared distances carry a relative error below 4 2^-24
     const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
-    for (int col = lane / kColumnLanes; col < cols; col += kWarp / kColumnLanes) {
-      const int2 ij = column(col, cnt[1], inv_n1);
-      const int i0 = idx[0][ij.x], i1 = idx[1][ij.y];
-      const float sxy = sq[0][ij.x] + sq[1][ij.y];
-      if (i0 < 0 || i1 < 0 || sxy > out2) continue;
-      const long long row = (long long)i0 * sx + (long long)i1 * sy;
-      for (int kz = lane % kColumnLanes; kz < cnt[2]; kz += kColumnLanes) {
-        const float sf = sxy + sq[2][kz];
+    const int total = cnt[0] * cnt[1] * cnt[2];
+    const BoxIndex box(cnt[1], cnt[2]);
+    for (int t0 = lane; t0 < total; t0 += kPutBatch * kWarp) {
+      long long cell[kPutBatch];
+#pragma unroll
+      for (int u = 0; u < kPutBatch; ++u) {
+        const int t = t0 + u * kWarp;
+        cell[u] = -1;
+        if (t >= total) continue;
+        const int3 o = box(t);
+        const float sf = (sq[0][o.x] + sq[1][o.y]) + sq[2][o.z];
         bool member = sf < in2;
         if (!member && sf <= out2) {
           // the reference's FP64 test
-          const double e0 = dsub(samp[0][ij.x], (double)c[0]), e1 = dsub(samp[1][ij.y], (double)c[1]),
-                       e2 = dsub(samp[2][kz], (double)c[2]);
+          const double e0 = dsub(samp[0][o.x], (double)c[0]), e1 = dsub(samp[1][o.y], (double)c[1]),
+                       e2 = dsub(samp[2][o.z], (double)c[2]);
           member = dadd(dadd(dmul(e0, e0), dmul(e1, e1)), dmul(e2, e2)) < pad2;
         }
-        const int i2 = idx[2][kz];
-        if (member && i2 >= 0) put(row + i2);
+        const int i0 = idx[0][o.x], i1 = idx[1][o.y], i2 = idx[2][o.z];
+        if (!member || i0 < 0 || i1 < 0 || i2 < 0) continue;
+        const long long at = (long long)i0 * sx + (long long)i1 * sy + i2;
+        if (at < ncell) cell[u] = at;
       }
+      mem.put(cell, a);
     }
   }
 }

@@ -30,7 +30,6 @@
 namespace gbx {
 namespace {
 
-constexpr int kColumnLanes = 8;
 constexpr int kSortWarps = 4;
 constexpr int kSortBuf = 256;
 constexpr int kSortLanes = 8;                                   // lanes per short list
@@ -82,33 +81,30 @@ __global__ void tight_members_kernel(TightArgs a) {
       const float lo = __fmul_rn((float)c, h);
       return make_float2(__fsub_rn(lo, at), __fsub_rn(__fadd_rn(lo, h), at));
     };
-    // eight lanes per column of cells: a column's counters share a sector, so
-    // its atomics leave together
-    const int ny = e[1] - b[1] + 1, cols = (e[0] - b[0] + 1) * ny;
-    const float inv_ny = 1.0f / (float)ny;
-    for (int col = lane / kColumnLanes; col < cols; col += kWarp / kColumnLanes) {
-      int cx = (int)(((float)col + 0.5f) * inv_ny);
-      cx -= cx * ny > col;
-      const int c[2] = {b[0] + cx, b[1] + col - cx * ny};
-      float near_xy = 0.f, far_xy = 0.f;
+    const int ny = e[1] - b[1] + 1, nz = e[2] - b[2] + 1, total = (e[0] - b[0] + 1) * ny * nz;
+    const BoxIndex box(ny, nz);
+    for (int t0 = lane; t0 < total; t0 += kPutBatch * kWarp) {
+      long long cell[kPutBatch];
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const float2 f = faces(c[k], x[k]);
-        const float dn = fmaxf(fmaxf(f.x, -f.y), 0.f), df = fmaxf(-f.x, f.y);
-        near_xy = fmaf(dn, dn, near_xy);
-        far_xy = fmaf(df, df, far_xy);
+      for (int u = 0; u < kPutBatch; ++u) {
+        const int t = t0 + u * kWarp;
+        cell[u] = -1;
+        if (t >= total) continue;
+        const int3 o = box(t);
+        const int c[3] = {b[0] + o.x, b[1] + o.y, b[2] + o.z};
+        float near = 0.f, far = 0.f;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const float2 f = faces(c[k], x[k]);
+          const float dn = fmaxf(fmaxf(f.x, -f.y), 0.f), df = fmaxf(-f.x, f.y);
+          near = fmaf(dn, dn, near);
+          far = fmaf(df, df, far);
+        }
+        if (!(near < reach * reach)) continue;
+        cell[u] = c[0] * sx + c[1] * sy + c[2];
+        if (bury > 0.f && far <= bury * bury) atomicOr(&a.buried[cell[u]], 1);
       }
-      if (!(near_xy < reach * reach)) continue;
-      const long long row = c[0] * sx + c[1] * sy;
-      for (int cz = b[2] + lane % kColumnLanes; cz <= e[2]; cz += kColumnLanes) {
-        const float2 f = faces(cz, x[2]);
-        const float dn = fmaxf(fmaxf(f.x, -f.y), 0.f);
-        if (!(fmaf(dn, dn, near_xy) < reach * reach)) continue;
-        const long long cell = row + cz;
-        a.mem.put(cell, at);
-        const float df = fmaxf(-f.x, f.y);
-        if (bury > 0.f && fmaf(df, df, far_xy) <= bury * bury) atomicOr(&a.buried[cell], 1);
-      }
+      a.mem.put(cell, at);
     }
   }
 }
