@@ -51,8 +51,10 @@ __device__ __forceinline__ double half_sqrt3() { return ddiv(__dsqrt_rn(3.0), 2.
 // axis needs of them is done for a block's eight atoms together (24 threads;
 // three lanes of each atom's own warp: 78 -> 70 us of that table, and 37 + 49
 // -> 28 + 41 us of two passes over 10,001 atoms of the periodic form).
+// Five blocks per SM (48 registers): 6 spill; the compiler's own 56 registers
+// leave four (table stage of 10,001 GBMV-II atoms with 4, 5, 6: 117, 112, 129 us).
 template <int MODE>
-__global__ void table_members_grid_kernel(const float4* __restrict__ pos, const double* __restrict__ radius, int n,
+__global__ void __launch_bounds__(kMemberThreads, 5) table_members_grid_kernel(const float4* __restrict__ pos, const double* __restrict__ radius, int n,
                                           const TableGeom* __restrict__ gp, double h, double buffer, Members mem,
                                           long long cell_cap) {
   __shared__ double s_d[kMemberWarps][3][kMaxSamples];
@@ -152,7 +154,7 @@ __global__ void table_members_grid_kernel(const float4* __restrict__ pos, const 
 // FP32 value is clear of the decision's boundary by a margin that covers its
 // rounding, and in the reference's FP64 operations otherwise (FP64 runs at a
 // small fraction of the FP32 rate on this part).
-__global__ void table_members_periodic_kernel(const float4* __restrict__ pos, const double* __restrict__ radius,
+__global__ void __launch_bounds__(kMemberThreads, 5) table_members_periodic_kernel(const float4* __restrict__ pos, const double* __restrict__ radius,
                                               int n, const TableGeom* __restrict__ gp, double buffer, Members mem,
                                               long long cell_cap, unsigned* __restrict__ status) {
   // per warp and axis: the samples, their cell index (-1 outside) and the
@@ -357,7 +359,7 @@ __device__ __forceinline__ void sort_list(const int* src, int* entries, const In
 }
 
 template <bool GBSW>
-__global__ void __launch_bounds__(kSortWarps * kWarp) sort_cells_kernel(Members mem, const int* __restrict__ start,
+__global__ void __launch_bounds__(kSortWarps * kWarp, 12) sort_cells_kernel(Members mem, const int* __restrict__ start,
                                                                         int* entries, int2* __restrict__ cell,
                                                                         Inline in, const TableGeom* __restrict__ gp,
                                                                         int cap, long long cell_cap,

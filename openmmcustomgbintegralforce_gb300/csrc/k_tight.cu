@@ -132,7 +132,9 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
   };
   // after an odd list: the pair reads of the integral pass meet a sphere no point is near
   const float4 kPadEntry = make_float4(0.f, 0.f, 0.f, -1e6f);
-  __shared__ float4 s_e[kSortWarps][kSortBuf];
+  // keys and atoms only, the positions are read again in sorted order: with them
+  // here (24 KB a block) 9 blocks fitted an SM and the table stage took 207 us
+  // at 50,000 atoms, 183 without
   __shared__ int s_i[kSortWarps][kSortBuf];
   __shared__ float s_k[kSortWarps][kSortBuf];
   const int wib = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
@@ -204,13 +206,11 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
           if (r == 0) first[c].first = e;
         }
       } else {
-        float4* ge = s_e[wib] + grp * kSortSmall;
         int* gi = s_i[wib] + grp * kSortSmall;
         float* gk = s_k[wib] + grp * kSortSmall;
         for (int q = gl; q < cnt; q += kSortLanes) {
           const int i = src[q];
           const float4 e = __ldg(pos + i);
-          ge[q] = e;
           gi[q] = i;
           gk[q] = key(e);
         }
@@ -223,9 +223,10 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
             const float ko = gk[o];
             r += (ko < kq) || (ko == kq && gi[o] < iq);
           }
-          put(s + r, ge[q]);
+          const float4 e = __ldg(pos + iq);
+          put(s + r, e);
           index[s + r] = iq;
-          if (r == 0) first[c].first = ge[q];
+          if (r == 0) first[c].first = e;
         }
       }
       if ((cnt & 1) && gl == 0) put(s + cnt, kPadEntry);
@@ -244,7 +245,6 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
       for (int q = lane; q < ccnt; q += kWarp) {
         const int i = csrc[q];
         const float4 e = __ldg(pos + i);
-        s_e[wib][q] = e;
         s_i[wib][q] = i;
         const float dx = e.x - ctr[0], dy = e.y - ctr[1], dz = e.z - ctr[2];
         s_k[wib][q] = sqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz))) - (e.w - w);
@@ -258,9 +258,10 @@ __global__ void __launch_bounds__(kSortWarps * kWarp) tight_sort_kernel(const fl
           const float ko = s_k[wib][o];
           r += (ko < kq) || (ko == kq && s_i[wib][o] < iq);
         }
-        put(cs + r, s_e[wib][q]);
+        const float4 e = __ldg(pos + iq);
+        put(cs + r, e);
         index[cs + r] = iq;
-        if (r == 0) first[cc].first = s_e[wib][q];
+        if (r == 0) first[cc].first = e;
       }
       if ((ccnt & 1) && lane == 0) put(cs + ccnt, kPadEntry);
       __syncwarp();
