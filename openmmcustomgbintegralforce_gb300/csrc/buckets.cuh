@@ -5,7 +5,7 @@
 // (scan.cuh), and the sort reads bucket and chain and writes them there.
 // Enumerating the members twice, to count and to fill, had cost more than the
 // bucket's scattered slots do: table stage of 50,000 GBSW atoms 240 -> 220 us,
-// of 1,001 40 -> 37, of 6,001 on a grid table 78 -> 60.  (Slots of a number
+// of 1,000 40 -> 37, of 6,007 on a grid table 78 -> 60.  (Slots of a number
 // side by side, for neighbouring cells' sake, measured the same or worse;
 // starts taken inside the sort, by groups of 32 cells, saved the scan's 4 us
 // and cost 40 in the sort and 20 in the integrals of 50,000 atoms.)
@@ -54,8 +54,8 @@ struct Members {
   }
   // U cells at once (-1: none): the slots are all on their way before the first
   // is needed, where a warp would wait out an L2 round trip for each (table
-  // stage of 50,000 GBSW atoms 218 -> 204 us, of 1,001 36 -> 33.5; 2 or 8 in
-  // flight instead of 4: the same at 50,000, slower at 1,001 and 6,001).
+  // stage of 50,000 GBSW atoms 218 -> 204 us, of 1,000 36 -> 33.5; 2 or 8 in
+  // flight instead of 4: the same at 50,000, slower at 1,000 and 6,007).
   template <int U>
   __device__ __forceinline__ void put(const long long (&cell)[U], int atom) const {
     int slot[U];

@@ -223,8 +223,8 @@ gbx_status alloc_atom_buffers(Context* ctx) {
     GBX_TRY(dalloc(ctx, &ctx->d_sval, (size_t)n * Q));
     GBX_TRY(dalloc(ctx, &ctx->d_ptotal, 1));
   }
-  if (ctx->cfg.cutoff > 0) {
-    GBX_TRY(dalloc(ctx, &ctx->d_perm, n));
+  if (ctx->cfg.cutoff > 0) GBX_TRY(dalloc(ctx, &ctx->d_perm, n));
+  if (ctx->cfg.cutoff > 0 || gbx::items_in_order(ctx)) {
     GBX_TRY(dalloc(ctx, &ctx->d_perm_tmp, n));
     GBX_TRY(dalloc(ctx, &ctx->d_cell_of, n));
     GBX_TRY(dalloc(ctx, &ctx->d_scount, gbx::kMaxSortCells));
@@ -513,6 +513,7 @@ gbx_status run_pipeline(Context* ctx, const float4* posq, unsigned long long* fo
   GBX_TRY(mark());
   GBX_TRY(gbx::launch_binning(ctx, ctx->d_pos, count_work));
   GBX_TRY(mark());
+  GBX_TRY(gbx::launch_spatial_order(ctx, ctx->d_pos));
   GBX_TRY(gbx::launch_integrals(ctx, ctx->d_pos, count_work));
   GBX_TRY(mark());
   if (ctx->custom) {

@@ -15,7 +15,7 @@ namespace gbx {
 constexpr int kWarp = 32;
 constexpr double kFixedScale = 4294967296.0;  // 2^32, OpenMM's force fixed-point scale
 constexpr int kMaxSortSegment = 2048;         // longest cell list the sort handles
-constexpr int kMaxSortCells = 1 << 17;        // cells of the cutoff pair term's spatial order
+constexpr int kMaxSortCells = 1 << 17;        // cells of the spatial order
 
 // Device status bits (context->d_status).
 enum : unsigned {
@@ -55,7 +55,7 @@ struct TableGeom {
   unsigned chained;  // list members outside their cell's bucket
 };
 
-// Grid of the spatial order of the cutoff pair term (k_pair.cu).
+// Grid of the atoms' spatial order (k_pair.cu).
 struct SortGeom {
   float lo[3];
   float inv_cell;
@@ -189,13 +189,13 @@ struct Context {
   int energy_parts = 0;
   unsigned long long* d_energy_fx = nullptr;  // pair energy, fixed point (2^-32)
   float4* d_tile_box = nullptr;               // cutoff: bounding box of each 32-atom tile
-  int* d_perm = nullptr;                      // cutoff: atoms in spatial order [n]
-  int* d_perm_tmp = nullptr;                  // cutoff: the same before the per-cell sort [n]
-  int* d_cell_of = nullptr;                   // cutoff: spatial cell of each atom [n]
-  int* d_scount = nullptr;                    // cutoff: atoms per spatial cell [kMaxSortCells]
+  int* d_perm = nullptr;                      // cutoff: atoms in spatial order, ascending per cell [n]
+  int* d_perm_tmp = nullptr;                  // atoms in spatial order, any order within a cell [n]
+  int* d_cell_of = nullptr;                   // spatial cell of each atom [n]
+  int* d_scount = nullptr;                    // atoms per spatial cell [kMaxSortCells]
   int* d_sstart = nullptr;
   int* d_scursor = nullptr;
-  SortGeom* d_sgeom = nullptr;                  // cutoff: spatial grid geometry
+  SortGeom* d_sgeom = nullptr;                  // spatial grid geometry
   float* d_pstate = nullptr;                  // GBMV: per-point sums kept for the chain rule
   // GBMV points binned by lookup-table cell (k_gbmv.cu)
   int2* d_pat = nullptr;                      // [n Q] (the point's cell or -1, slot within the cell)
@@ -366,6 +366,22 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
 int pair_energy_parts(int n, int segments);
 int pair_segments(int n, int sms);
 ModelConst make_model_const(const Context* ctx);
+// The atoms in spatial order: for the cutoff pair term's tiles (d_perm, sorted
+// within a cell), and for the GBSW integrals and chain rule (d_perm_tmp, any
+// order within a cell), whose running warps then share a part of the table.
+// That pays once the table (some 2.6 KB an atom) crowds the 129 MB L2, or where
+// the pair term needs the order anyway.  Forming it takes 17 us; whole calls
+// without and with it, all pairs: 20,000 atoms, 32 x 110 points 1,385 and 1,400
+// us, 30,000 2,201 and 2,195, 40,000 3,160 and 3,084, 50,000 4,242 and 4,061 (24 x
+// 38 points 1,093 and 1,109 at 30,000, 1,629 and 1,630 at 40,000, 2,265 and 2,239
+// at 50,000); 1.5 nm cutoff, 10,000 atoms 342 and 338, 50,000 1,515 and 1,466.
+constexpr int kOrderAtoms = 40000;
+inline bool pair_in_order(const Context* ctx) { return ctx->cfg.cutoff > 0 && !ctx->cfg.periodic && !ctx->custom; }
+inline bool items_in_order(const Context* ctx) {
+  return ctx->cfg.model == GBX_MODEL_GBSW && (ctx->n >= kOrderAtoms || pair_in_order(ctx));
+}
+gbx_status launch_spatial_order(Context* ctx, const float4* pos);
+
 // The GBSW chain rule forms dE/dJ itself: no launch_chain_prep (compiled
 // expressions and the adjoint, which needs more from it, go through memory).
 bool chain_forms_dEdJ(const Context* ctx, bool adjoint);

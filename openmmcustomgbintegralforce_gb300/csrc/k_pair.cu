@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kSymThreads, ADJ ? 3 : 4) pair_sym_kernel(SymA
 }
 
 // ---------------------------------------------------------------------------
-// Spatial order for the cutoff pair term: atoms are binned into cubic cells
+// Spatial order: atoms are binned into cubic cells
 // (1 nm, grown so that the grid holds at most kMaxSortCells cells) and, within
 // a cell, kept in ascending atom order, so the permutation depends on the
 // input alone.  32 consecutive slots then form a compact tile whose bounding
@@ -700,6 +700,29 @@ cudaError_t launch_pair_raw(const float4* pos, const float* charge, const float2
   return cudaGetLastError();
 }
 
+gbx_status launch_spatial_order(Context* ctx, const float4* pos) {
+  const bool pair = pair_in_order(ctx);
+  if (!pair && !items_in_order(ctx)) return GBX_OK;
+  const int n = ctx->n, nb = (n + 255) / 256;
+  const SortGeom* sg = ctx->d_sgeom;  // written, and d_scount cleared, by the call's first kernel
+  cudaStream_t st = ctx->stream;
+  sort_count_kernel<<<nb, 256, 0, st>>>(pos, n, sg, ctx->d_cell_of, ctx->d_scount);
+  sort_scan_kernel<<<1, kBoxThreads, 0, st>>>(ctx->d_scount, sg, ctx->d_sstart, ctx->d_scursor);
+  sort_scatter_kernel<<<nb, 256, 0, st>>>(ctx->d_cell_of, n, ctx->d_sstart, ctx->d_scursor, ctx->d_perm_tmp);
+  ctx->launches += 3;
+  if (pair) {
+    sort_cells_by_atom_kernel<<<ctx->sms * 8, kSymThreads, 0, st>>>(ctx->d_scount, ctx->d_sstart, sg, ctx->d_perm_tmp,
+                                                                    ctx->d_perm);
+    ++ctx->launches;
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    ctx->last_error = std::string("spatial order launch: ") + cudaGetErrorString(e);
+    return GBX_ERR_CUDA;
+  }
+  return GBX_OK;
+}
+
 gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* force, int stride, bool adjoint) {
   SymArgs a = sym_args(ctx->n);
   a.pos = pos;
@@ -728,15 +751,7 @@ gbx_status launch_pair(Context* ctx, const float4* pos, unsigned long long* forc
     }
     ++ctx->launches;
   } else if (a.cutoff2 > 0) {
-    // spatial order, then tile boxes over it
-    const int n = a.n, nb = (n + 255) / 256;
-    const SortGeom* sg = ctx->d_sgeom;  // written, and d_scount cleared, by the call's first kernel
-    sort_count_kernel<<<nb, 256, 0, st>>>(pos, n, sg, ctx->d_cell_of, ctx->d_scount);
-    sort_scan_kernel<<<1, kBoxThreads, 0, st>>>(ctx->d_scount, sg, ctx->d_sstart, ctx->d_scursor);
-    sort_scatter_kernel<<<nb, 256, 0, st>>>(ctx->d_cell_of, n, ctx->d_sstart, ctx->d_scursor, ctx->d_perm_tmp);
-    sort_cells_by_atom_kernel<<<ctx->sms * 8, kSymThreads, 0, st>>>(ctx->d_scount, ctx->d_sstart, sg, ctx->d_perm_tmp,
-                                                               ctx->d_perm);
-    ctx->launches += 4;
+    // tile boxes over the spatial order
     a.perm = ctx->d_perm;
     tile_box_kernel<<<(a.ntiles + wpb - 1) / wpb, kSymThreads, 0, st>>>(pos, ctx->d_perm, a.n, a.ntiles,
                                                                         ctx->d_tile_box);

@@ -55,7 +55,7 @@ struct PrepareArgs {
   int mode;
   double h, buffer, box[3], reach;
   long long ref_cap;
-  SortGeom* sort;  // cutoff pair term: the grid of its spatial order
+  SortGeom* sort;  // the grid of the atoms' spatial order
 };
 
 // Internal positions: x, y, z and the model's main per-atom parameter in .w
@@ -173,7 +173,7 @@ __device__ __forceinline__ void ref_rest(const PrepareArgs& a, TableGeom& g, uns
   if (g.ncell > a.ref_cap) status |= kStatusTableCells;
 }
 
-// The grid of the cutoff pair term's spatial order: 1 nm cells, grown so that
+// The grid of the atoms' spatial order: 1 nm cells, grown so that
 // there are at most kMaxSortCells.  (One block that read every position for
 // its extents took 27 us of a 50,000-atom step.)
 __device__ __forceinline__ SortGeom sort_grid(const GeomPart& e) {
@@ -187,7 +187,11 @@ __device__ __forceinline__ SortGeom sort_grid(const GeomPart& e) {
       g.dims[d] = (span >= 0.0f && span < (float)kMaxSortCells) ? (int)span + 1 : 1;
       tot *= g.dims[d];
     }
-    if (tot <= kMaxSortCells || cell > 1e6f) {
+    if (tot > kMaxSortCells && cell > 1e6f) {  // absurd extents: one cell
+      g.dims[0] = g.dims[1] = g.dims[2] = 1;
+      tot = 1;
+    }
+    if (tot <= kMaxSortCells) {
       for (int d = 0; d < 3; ++d) g.lo[d] = e.mn[d];
       g.inv_cell = 1.0f / cell;
       g.ncell = (int)tot;
@@ -397,7 +401,7 @@ gbx_status launch_prepare(Context* ctx, const void* posq, bool tight, bool refer
     clear(ctx->d_next_item, 1);
     clear(ctx->d_rmax, 1);
   }
-  if (call && ctx->d_sgeom && !c.periodic && !ctx->custom) {
+  if (call && (pair_in_order(ctx) || items_in_order(ctx))) {
     a.sort = ctx->d_sgeom;
     clear(ctx->d_scount, kMaxSortCells);
   }

@@ -50,9 +50,9 @@ __device__ __forceinline__ double half_sqrt3() { return ddiv(__dsqrt_rn(3.0), 2.
 // the same for three lanes as for 32 and were what bound the pass, so what an
 // axis needs of them is done for a block's eight atoms together (24 threads;
 // three lanes of each atom's own warp: 78 -> 70 us of that table, and 37 + 49
-// -> 28 + 41 us of two passes over 10,001 atoms of the periodic form).
+// -> 28 + 41 us of two passes over 10,000 atoms of the periodic form).
 // Five blocks per SM (48 registers): 6 spill; the compiler's own 56 registers
-// leave four (table stage of 10,001 GBMV-II atoms with 4, 5, 6: 117, 112, 129 us).
+// leave four (table stage of 10,000 GBMV-II atoms with 4, 5, 6: 117, 112, 129 us).
 template <int MODE>
 __global__ void __launch_bounds__(kMemberThreads, 5) table_members_grid_kernel(const float4* __restrict__ pos, const double* __restrict__ radius, int n,
                                           const TableGeom* __restrict__ gp, double h, double buffer, Members mem,
@@ -278,7 +278,7 @@ constexpr int kSortWarps = 4;
 // Inline copies of GBMV lists (ascending, as the list) and GBSW lists (pairs,
 // field by field, the likeliest burying atom first: a point's V does not
 // depend on the order, and most listed points end at their first entry; the
-// integrals of 6,001 atoms: 262 us with ascending single entries, 244 so).
+// integrals of 6,007 atoms: 262 us with ascending single entries, 244 so).
 struct Inline {
   const float4* pos;
   const float2* par;

@@ -457,11 +457,13 @@ enum { kEmitNone = 0, kEmitOthers = 1, kEmitAll = 2 };
 // from `next_item` one at a time, so a warp that finishes a cheap item (a
 // buried or exposed atom) takes the next instead of idling until the slowest
 // warp of its block is done.  Each item's results depend on the item alone.
+// `order` (or nullptr): the atoms in the order to take them in.
 template <class Q, int EMIT>
 __global__ void __launch_bounds__(kThreads, 12) gbsw_integral_kernel(const float4* __restrict__ pos, int n, Entries tab,
                                                                  Quad quad, ModelConst m, int n_chunks,
                                                                  float* __restrict__ Jpart, ShellSink sink,
-                                                                 unsigned* __restrict__ next_item) {
+                                                                 unsigned* __restrict__ next_item,
+                                                                 const int* __restrict__ order) {
   __shared__ int2 s_queue[kThreads / kWarp][2][kQueue];  // (q | length << 16, list start): short and long lists
   // lists start at even entries and each cell's record sits beside its first
   // entry, so both are read 32 bytes at a time
@@ -475,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 12) gbsw_integral_kernel(const float
     if (warp >= n * n_chunks) return;
     int fill = 0;           // warp-uniform: points recorded so far (may exceed R)
     bool too_long = false;  // a shaping entry beyond list position 63
-    const int i = warp % n, c = warp / n;
+    const int c = warp / n, k = warp - c * n, i = order ? __ldg(order + k) : k;
     const float4 xi = pos[i];
     Q query;
     query.init(tab, xi, quad.qoff);
@@ -675,6 +677,7 @@ struct ChainRecords {
   const int* st;    // the point's list start
   const int* count;
   int R;
+  const int* order;  // the items' atoms, as the integral pass took them (nullptr: ascending)
 };
 
 // A component whose fixed-point value is 0 (|g| < 2^-33, common for distant
@@ -721,7 +724,7 @@ struct Shaping {
 };
 
 // dE/dJ of an atom: as a kernel before left it, or formed from dE/dB and dB/dJ
-// by the warp that needs it (a launch less: 98.6 -> 97.6 us at 1,001 atoms, and
+// by the warp that needs it (a launch less: 98.6 -> 97.6 us at 1,000 atoms, and
 // no difference from 6,000 up).
 struct DEdJ {
   const float2* value;  // nullptr: not formed
@@ -765,7 +768,7 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
   const int lane = threadIdx.x % kWarp, wib = threadIdx.x / kWarp;
   if (warp >= n * n_chunks) return;
-  const int i = warp % n, c = warp / n;
+  const int c = warp / n, nth = warp - c * n, i = rr.order ? __ldg(rr.order + nth) : nth;
   const float4 xi = pos[i];
   const float2 de = dEdJ.of(i, lane);
   const unsigned lt = (1u << lane) - 1u;
@@ -1111,7 +1114,7 @@ void launch_integrals_t(Context* ctx, const float4* pos, const ModelConst& m, bo
                   : ctx->records_self ? gbsw_integral_kernel<Q, kEmitAll>
                                       : gbsw_integral_kernel<Q, kEmitOthers>;
     kernel<<<grid, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, ctx->n_chunks, ctx->d_J, sink,
-                                               ctx->d_next_item);
+                                               ctx->d_next_item, items_in_order(ctx) ? ctx->d_perm_tmp : nullptr);
   }
   else if (count_work)
     integral_kernel<MODEL, Q, true><<<volume_blocks(ctx), kThreads, 0, ctx->stream>>>(
@@ -1134,7 +1137,8 @@ void launch_chain_t(Context* ctx, const float4* pos, const ModelConst& m) {
   const ChainOut o{ctx->d_f4, m.cutoff_chain_quirk && m.cutoff2 > 0.0f, m.cutoff2};
   const int blocks = volume_blocks(ctx);
   if constexpr (MODEL == GBX_MODEL_GBSW) {
-    const ChainRecords rr{ctx->d_srec, ctx->d_srec_st, ctx->records ? ctx->d_rcount : nullptr, ctx->srec_R};
+    const ChainRecords rr{ctx->d_srec, ctx->d_srec_st, ctx->records ? ctx->d_rcount : nullptr, ctx->srec_R,
+                          items_in_order(ctx) ? ctx->d_perm_tmp : nullptr};
     const DEdJ de{chain_forms_dEdJ(ctx, ADJ) ? nullptr : ctx->d_dEdJ, ctx->d_dEdB_fx, ctx->d_dBdJ};
     gbsw_chain_kernel<Q, ADJ><<<blocks, kThreads, 0, ctx->stream>>>(pos, ctx->n, t, qd, m, ctx->n_chunks, de, o, rr);
   } else {

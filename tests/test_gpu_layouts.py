@@ -274,3 +274,21 @@ def test_counted_work_is_the_reference_walk(name):
     for k in ("volume_evals", "shell_evals"):
         assert abs(got[k] / ref[k] - 1) < 1e-4, k
     ctx.close()
+
+
+# with a cutoff the integrals take the atoms in spatial order, without (below
+# 40,000 atoms) as they come; neither changes a volume
+@pytest.mark.parametrize("n", [1, 33, 700])
+@pytest.mark.parametrize("kw", [{}, dict(reference_table=True)], ids=["exact", "reference"])
+def test_integrals_do_not_depend_on_the_order(n, kw):
+    g = make_globule(n, seed=14)
+    a, b = context(GBModel.charmm_gbsw(**kw), g), context(GBModel.charmm_gbsw(cutoff=1.2, **kw), g)
+    for _ in range(2):
+        a.execute_host(g.positions)
+        b.execute_host(g.positions)
+        assert np.array_equal(a.integrals(), b.integrals()) and np.array_equal(a.born_radii(), b.born_radii())
+    a.adjoint(g.positions)
+    b.adjoint(g.positions)
+    assert np.array_equal(a.integrals(), b.integrals())
+    a.close()
+    b.close()
