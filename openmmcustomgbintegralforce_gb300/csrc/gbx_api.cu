@@ -342,10 +342,12 @@ gbx_status prepare_records(Context* ctx, bool wanted, bool adjoint) {
 }
 
 // Buckets of `want` slots per cell: at most 256 and, so that a sparse grid does
-// not pay for empty cells, four times the entries in all; list members past
-// them are chained.  Never shrinks.
+// not pay for empty cells, eight times the entries (or 2^24) in all; list
+// members past them are chained.  Never shrinks.  (Four times, or 2^22, cut the
+// buckets of a 2,513-atom GBMV table, most of whose box is empty, below its
+// longest lists.)
 gbx_status grow_buckets(Context* ctx, gbx::TableBuckets& b, long long want, long long cells, long long entries) {
-  const long long room = std::max(4 * entries, 1LL << 22) / std::max(cells, 1LL);
+  const long long room = std::max(8 * entries, 1LL << 24) / std::max(cells, 1LL);
   const int size = (int)std::min(std::min(want, 256LL), room);
   if (size <= b.size) return GBX_OK;
   b.size = 0;
@@ -356,7 +358,8 @@ gbx_status grow_buckets(Context* ctx, gbx::TableBuckets& b, long long want, long
 
 // Slots for the longest list seen and a quarter more.
 long long bucket_for(int longest) { return ((long long)longest * 5 / 4 + 7) / 8 * 8; }
-constexpr long long kFirstBucket = 32;  // before any list is known
+// before any list is known: above the longest lists of the usual radii and cells
+constexpr long long kFirstTightBucket = 32, kFirstBucket = 96;
 
 gbx_status grow_table(Context* ctx, long long cells, long long entries) {
   const long long slots = std::max(kFirstBucket, (long long)ctx->buckets.size);
@@ -436,7 +439,7 @@ gbx_status build_table_checked(Context* ctx, const void* posq, bool check, bool 
 }
 
 gbx_status grow_tight(Context* ctx, long long cells, long long entries) {
-  const long long slots = std::max(kFirstBucket, (long long)ctx->tbuckets.size);
+  const long long slots = std::max(kFirstTightBucket, (long long)ctx->tbuckets.size);
   if (cells > ctx->tcell_cap) {
     const long long cap = cells + cells / 4 + 1024;
     GBX_TRY(dalloc(ctx, &ctx->d_tcount, cap));
