@@ -78,12 +78,12 @@ FLOPS_PAIR = 39.0
 
 # DRAM bytes (read + write) per step of each stage's kernels, from one ncu
 # capture of the same workload and build (the files named in TRAFFIC_SOURCE).
-TRAFFIC = {"gbsw50k": {"integrals": 1689.1e6 + 715.5e6, "pair": 3.0e6 + 3.0e6, "chain_rule": 1107.7e6,
-                       "lookup_table": 180.0e6 + 146.6e6 + 5.5e6 + 9.6e6},
-           "gbmv10k": {"integrals": 404.7e6 + 48.0e6, "chain_rule": 291.8e6, "point_binning": 93.0e6 + 153.1e6,
-                       "pair": 0.63e6 + 0.63e6},
-           "gbmv1_10k": {"integrals": 211.0e6 + 48.0e6, "chain_rule": 127.1e6, "point_binning": 89.7e6 + 151.1e6,
-                         "pair": 0.63e6 + 0.62e6}}
+TRAFFIC = {"gbsw50k": {"integrals": 409.3e6 + 684.7e6, "pair": 3.1e6, "chain_rule": 762.1e6 + 1.1e6,
+                       "lookup_table": 176.1e6 + 59.9e6 + 4.8e6 + 1.0e6},
+           "gbmv10k": {"integrals": 106.4e6 + 134.9e6 + 48.0e6, "chain_rule": 163.6e6 + 3.4e6,
+                       "point_binning": 67.9e6 + 154.4e6, "pair": 0.7e6},
+           "gbmv1_10k": {"integrals": 91.6e6 + 62.4e6 + 48.0e6, "chain_rule": 94.1e6 + 2.8e6,
+                         "point_binning": 70.8e6 + 154.7e6, "pair": 0.7e6}}
 TRAFFIC_SOURCE = {"gbsw50k": "profiles/launches_gbsw50k.md", "gbmv10k": "profiles/launches_gbmv10k.md",
                   "gbmv1_10k": "profiles/launches_gbmv1_10k.md"}
 
