@@ -775,8 +775,10 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
   // F_i as fixed-point integers: every contribution is rounded on its own, so
   // the record and the list-walk paths give the same bits
   long long fix = 0, fiy = 0, fiz = 0;
+  // the records need no cell query, and setting one up is FP64 work in every
+  // warp: 43 -> 35 us at 6,007 atoms on a grid table, 258 -> 244 in a periodic box
   Q query;
-  query.init(tab, xi, quad.qoff);
+  query.init_images(tab);
   float4* sv = s_v[wib];
   float2* sc = s_c[wib];
   unsigned* items = s_item[wib];
@@ -869,6 +871,7 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
       if (carried > 0 && head == base) evaluate();
     }
   } else {
+    query.init(tab, xi, quad.qoff);
     Points pts{};
     pts.init<Q>(quad, m, xi, c, n_chunks, lane);
     for (int b = pts.t0; b < pts.t1; b += kWarp) {

@@ -83,6 +83,8 @@ struct RefQuery {
   bool box;      // box-sampled table: points are moved by whole boxes
   const TableGeom* g;
   const double* qoff;
+  // What distances need, without the cell query (images: the box).
+  __device__ __forceinline__ void init_images(const Entries&) {}
   // A coordinate t = v / step + rel in cell units carries the FP32 rounding of
   // rel, of v and 1 / step, of the sum and of a move by whole boxes: at most
   // 2^-24 (3 |rel| + 4 |v| / step).  The guard band is twice 4 (|rel| + reach /
@@ -205,6 +207,12 @@ struct BoxQuery : RefQuery {
 struct MinImageQuery : RefQuery {
   static constexpr bool kImages = true;
   float L[3], iL[3];
+  __device__ __forceinline__ void init_images(const Entries& t) {
+    for (int k = 0; k < 3; ++k) {
+      L[k] = (float)t.geom->box[k];
+      iL[k] = (float)t.geom->inv_box[k];
+    }
+  }
   __device__ __forceinline__ void init(const TableGeom& geom, const float4 xi, const double* qo, long long cap) {
     RefQuery::init(geom, xi, qo, cap);
     for (int k = 0; k < 3; ++k) {
@@ -259,6 +267,12 @@ struct PeriodicQuery {
   bool off;
   const TableGeom* g;
   const double* qoff;
+  __device__ __forceinline__ void init_images(const Entries& t) {
+    for (int k = 0; k < 3; ++k) {
+      L[k] = (float)t.geom->box[k];
+      iL[k] = (float)t.geom->inv_box[k];
+    }
+  }
   __device__ __forceinline__ void init(const TableGeom& geom, const float4 xi, const double* qo, long long cap) {
     g = &geom;
     qoff = qo;
@@ -320,6 +334,7 @@ struct TightQuery {
   float xr[3];
   float inv_h;
   int dims[3];
+  __device__ __forceinline__ void init_images(const Entries&) {}
   __device__ __forceinline__ void init(const TableGeom& g, const float4 xi, const double*, long long cap) {
     xr[0] = (float)((double)xi.x - g.min[0]);
     xr[1] = (float)((double)xi.y - g.min[1]);
@@ -395,6 +410,12 @@ struct PeriodicTightQuery : TightQuery {
   float eps;
   const TableGeom* wg;
   const double* qoff;
+  __device__ __forceinline__ void init_images(const Entries& t) {
+    for (int k = 0; k < 3; ++k) {
+      L[k] = (float)t.wrap->box[k];
+      iL[k] = (float)t.wrap->inv_box[k];
+    }
+  }
   __device__ __forceinline__ void init(const Entries& t, const float4 xi, const double* qo) {
     TightQuery::init(*t.geom, xi, qo, usable_cells(t));
     const TableGeom& W = *t.wrap;
