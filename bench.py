@@ -78,8 +78,8 @@ FLOPS_PAIR = 39.0
 
 # DRAM bytes (read + write) per step of each stage's kernels, from one ncu
 # capture of the same workload and build (the files named in TRAFFIC_SOURCE).
-TRAFFIC = {"gbsw50k": {"integrals": 409.3e6 + 684.7e6, "pair": 3.1e6, "chain_rule": 762.1e6 + 1.1e6,
-                       "lookup_table": 176.1e6 + 59.9e6 + 4.8e6 + 1.0e6},
+TRAFFIC = {"gbsw50k": {"integrals": 403.2e6 + 684.6e6, "pair": 3.2e6, "chain_rule": 762.1e6 + 1.4e6,
+                       "lookup_table": 199.5e6 + 47.8e6 + 4.8e6 + 1.0e6},
            "gbmv10k": {"integrals": 106.4e6 + 134.9e6 + 48.0e6, "chain_rule": 163.6e6 + 3.4e6,
                        "point_binning": 67.9e6 + 154.4e6, "pair": 0.7e6},
            "gbmv1_10k": {"integrals": 91.6e6 + 62.4e6 + 48.0e6, "chain_rule": 94.1e6 + 2.8e6,
