@@ -136,7 +136,7 @@ struct RefQuery {
   __device__ __forceinline__ int cell_at(const float* t, bool& unsafe) const {
     int id[3];
     float face = 0.0f;  // the largest distance from a cell's middle along an axis
-    bool in = true;
+    bool in = dims[0] > 0;  // the bound below wraps where there are no cells
     const int last = box ? 0 : 1;  // a grid's last index is a point, not a cell
 #pragma unroll
     for (int k = 0; k < 3; ++k) {

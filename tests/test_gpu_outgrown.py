@@ -1,0 +1,137 @@
+"""Calls whose lookup table outgrew its buffers, on the reference's tables:
+an unchecked call lacks the volume terms (every point is solvent) and the next
+one reports it, a host call and a checked adjoint evaluate again, and both then
+give a fresh context's bits."""
+import numpy as np
+import pytest
+
+from openmmcustomgbintegralforce_gb300._lib import EXEC_CHECK, EXEC_ENERGY, EXEC_FORCES, Context, CustomContext, GBXError
+from openmmcustomgbintegralforce_gb300.expression_sets import MODIFIED
+from openmmcustomgbintegralforce_gb300.globule import make_globule
+from openmmcustomgbintegralforce_gb300.spec import TABLE_GRID, GBModel
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+BOTH = EXEC_FORCES | EXEC_ENERGY
+STALE = 10
+MODELS = {"grid": GBModel.gbsw_integral(), "standalone": GBModel.charmm_gbsw(reference_table=True),
+          "gbmv1": GBModel.gbmv1(table_mode=TABLE_GRID), "gbmv2": GBModel.gbmv2(table_mode=TABLE_GRID)}
+
+
+def context(m, g):
+    ctx = Context(m, g.n)
+    ctx.set_particle_parameters(g.charge, g.radius)
+    return ctx
+
+
+def device_call(ctx, pos, flags=BOTH):
+    """(energy, forces, status) of a call on the current stream's buffers."""
+    n = ctx.n
+    posq = torch.zeros((n, 4), dtype=torch.float32, device="cuda:0")
+    posq[:, :3] = torch.from_numpy(pos).to(posq)
+    force = torch.zeros((3, n), dtype=torch.int64, device="cuda:0")
+    energy = torch.zeros(1, dtype=torch.float64, device="cuda:0")
+    torch.cuda.synchronize()
+    status = 0
+    try:
+        ctx.execute_device(posq.data_ptr(), force.data_ptr(), n, energy.data_ptr(), flags, 0)
+    except GBXError as e:
+        status = e.status
+    torch.cuda.synchronize()
+    return float(energy), force.T.cpu().numpy() / 2.0 ** 32, status
+
+
+def spread(g):
+    """The atoms 1.6 times as far apart: some four times the cells."""
+    c = g.positions.mean(axis=0)
+    return c + 1.6 * (g.positions - c)
+
+
+def far(g):
+    """One atom 60 nm away along z: few more atoms per cell, far longer an axis."""
+    x = g.positions.copy()
+    x[7, 2] += 60.0
+    return x
+
+
+@pytest.mark.parametrize("moved", [spread, far])
+@pytest.mark.parametrize("name", list(MODELS))
+def test_unchecked_call_lacks_the_volume_terms(name, moved):
+    g = make_globule(400, seed=13)
+    m = MODELS[name]
+    ctx, fresh = context(m, g), context(m, g)
+    assert device_call(ctx, g.positions, BOTH | EXEC_CHECK)[2] == 0
+    inside = ctx.integrals()
+    assert device_call(ctx, g.positions)[2] == 0
+    x = moved(g)
+    assert device_call(ctx, x)[2] == 0
+    # no cell: V = 0 at every point (GBMV-I: 1 / (1 + e^10), from its empty sum), so an
+    # integral is that fraction of the quadrature's own sum, to the rounding of
+    # 624 to 912 FP32 terms added 32 apart (30 additions of 2^-24: 2e-6 of it);
+    # the sums are 1/r0 - 1/r1 and (1/r0^4 - 1/r1^4) / 4, far above any error of the rule
+    got = ctx.integrals()
+    S = np.array([1 / m.r0 - 1 / m.r1, 0.25 * (m.r0 ** -4 - m.r1 ** -4)])
+    covered = 1 / (1 + np.exp(10.0)) if name == "gbmv1" else 0.0
+    assert (np.abs(got) < (2e-6 + 1.1 * covered) * S[:, None]).all()
+    assert (np.abs(inside).max(axis=1) > 100 * np.abs(got).max(axis=1)).all()
+    E, F, status = device_call(ctx, x)  # reported, evaluated checked
+    assert status == STALE
+    Ef, Ff, _ = device_call(fresh, x, BOTH | EXEC_CHECK)
+    assert E == Ef and np.array_equal(F, Ff)
+    E, F, status = device_call(ctx, x)
+    assert status == 0 and E == Ef and np.array_equal(F, Ff)
+    ctx.close()
+    fresh.close()
+
+
+@pytest.mark.parametrize("moved", [spread, far])
+@pytest.mark.parametrize("name", list(MODELS))
+def test_host_call_and_adjoint_evaluate_again(name, moved):
+    g = make_globule(400, seed=14)
+    a, b, fresh = (context(MODELS[name], g) for _ in range(3))
+    x = moved(g)
+    for _ in range(2):
+        a.execute_host(g.positions)
+        b.adjoint(g.positions)
+    n = g.n
+    posq = torch.zeros((n, 4), dtype=torch.float32, device="cuda:0")
+    posq[:, :3] = torch.from_numpy(x).to(posq)
+    out = torch.zeros(3 + 5 * n, dtype=torch.float64, device="cuda:0")
+    torch.cuda.synchronize()
+    at = out.data_ptr()
+    b.adjoint_device(posq.data_ptr(), at, at + 8, at + 8 * (1 + 3 * n), at + 8 * (1 + 4 * n), at + 8 * (1 + 5 * n),
+                     EXEC_CHECK, 0)
+    torch.cuda.synchronize()
+    want = fresh.adjoint(x)
+    got = out.cpu().numpy()
+    assert got[0] == want["energy"]
+    assert np.array_equal(got[1:], np.concatenate([want[k].reshape(-1) for k in ("forces", "dEdq", "dEdR", "dEdalpha")]))
+    E, F = a.execute_host(x)
+    Ef, Ff = fresh.execute_host(x)
+    assert E == Ef and np.array_equal(F, Ff)
+    for c in (a, b, fresh):
+        c.close()
+
+
+# the same table under a user's expressions
+def test_compiled_expressions_on_the_grid_table():
+    g = make_globule(400, seed=15)
+    params = np.stack([g.charge, g.radius, np.ones(g.n)], axis=1)
+    x = far(g)
+
+    def make():
+        c = CustomContext(MODELS["grid"], g.n, MODIFIED)
+        c.set_custom_parameters(params)
+        return c
+
+    ctx, fresh = make(), make()
+    assert device_call(ctx, g.positions, BOTH | EXEC_CHECK)[2] == 0
+    assert device_call(ctx, g.positions)[2] == 0
+    assert device_call(ctx, x)[2] == 0
+    E, F, status = device_call(ctx, x)
+    assert status == STALE
+    Ef, Ff, _ = device_call(fresh, x, BOTH | EXEC_CHECK)
+    assert E == Ef and np.array_equal(F, Ff)
+    ctx.close()
+    fresh.close()
