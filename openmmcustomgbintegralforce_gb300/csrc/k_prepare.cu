@@ -13,6 +13,7 @@
 #include <algorithm>
 
 #include "gbx_internal.cuh"
+#include "queries.cuh"
 
 namespace gbx {
 namespace {
@@ -96,8 +97,8 @@ __device__ __forceinline__ void tight_axis(const PrepareArgs& a, const GeomPart&
                                            unsigned& status) {
   const double h = a.tight_h, margin = (double)e.wmax + a.switch_width + h;
   g.min[k] = (double)e.mn[k] - margin;
-  g.dims[k] = (int)ceil(((double)e.mx[k] - (double)e.mn[k] + 2.0 * margin) / h) + 1;
-  if (!(g.dims[k] >= 1 && g.dims[k] <= 65536)) {
+  g.dims[k] = axis_cells(((double)e.mx[k] - (double)e.mn[k] + 2.0 * margin) / h, status);
+  if (g.dims[k] > 65536) {
     status |= kStatusTableCells;
     g.dims[k] = 1;
   }
@@ -121,7 +122,7 @@ __device__ __forceinline__ void tight_rest(const PrepareArgs& a, const GeomPart&
   g.total = 0;
   g.longest = 0;
   g.chained = 0u;
-  g.ncell = (long long)g.dims[0] * g.dims[1] * g.dims[2];
+  g.ncell = grid_cells(g.dims);
   if (g.ncell > a.tight_cap) status |= kStatusTableCells;
 }
 
@@ -135,7 +136,7 @@ __device__ __forceinline__ void ref_axis(const PrepareArgs& a, const GeomPart& e
     const double cog = __ddiv_rn(e.sum[k], (double)a.n), half = __ddiv_rn(box, 2.0);
     g.min[k] = __dsub_rn(cog, half);
     g.max[k] = __dadd_rn(cog, half);
-    g.dims[k] = (int)ceil(__ddiv_rn(box, a.h)) + 1;
+    g.dims[k] = axis_cells(__ddiv_rn(box, a.h), status);
     g.step[k] = __ddiv_rn(box, (double)g.dims[k]);
   } else {
     double pad;
@@ -150,7 +151,7 @@ __device__ __forceinline__ void ref_axis(const PrepareArgs& a, const GeomPart& e
       status |= kStatusTableCells;
       g.dims[k] = 1;
     } else {
-      g.dims[k] = (int)ceil(__ddiv_rn(length, a.h)) + 1;
+      g.dims[k] = axis_cells(__ddiv_rn(length, a.h), status);
     }
     g.min[k] = lo;
     g.max[k] = __dadd_rn(lo, __dmul_rn((double)(g.dims[k] - 1), a.h));
@@ -169,7 +170,7 @@ __device__ __forceinline__ void ref_rest(const PrepareArgs& a, TableGeom& g, uns
   g.chained = 0u;
   g.L = a.mode == GBX_TABLE_PERIODIC ? fmax(fmax(g.step[0], g.step[1]), g.step[2]) : a.h;
   if (a.mode == GBX_TABLE_PERIODIC) g.pad = 0.0;
-  g.ncell = (long long)g.dims[0] * g.dims[1] * g.dims[2];
+  g.ncell = grid_cells(g.dims);
   if (g.ncell > a.ref_cap) status |= kStatusTableCells;
 }
 

@@ -51,6 +51,27 @@ __device__ __forceinline__ long long usable_cells(const Entries& t) {
 }
 
 // ---------------------------------------------------------------------------
+// Grids
+// ---------------------------------------------------------------------------
+
+// Indices along a grid axis of `steps` steps: one more than that rounded up.
+// Non-finite or absurd extents (atoms blown apart, positions that are not
+// numbers) have no such number in an int: a single index then, and the status
+// that the table could not be built.
+__device__ __forceinline__ int axis_cells(double steps, unsigned& status) {
+  const double c = ceil(steps);
+  if (c >= 0.0 && c < 2147483647.0) return (int)c + 1;
+  status |= kStatusTableCells;
+  return 1;
+}
+
+// Cells of a grid, at most 2^62 (more than any table has room for).
+__device__ __forceinline__ long long grid_cells(const int dims[3]) {
+  const long long plane = (long long)dims[0] * dims[1];
+  return (double)plane * dims[2] < 4611686018427387904.0 ? plane * dims[2] : 1LL << 62;
+}
+
+// ---------------------------------------------------------------------------
 // Cell queries
 // ---------------------------------------------------------------------------
 

@@ -37,3 +37,10 @@ extern "C" void query_cells(int mode, const double* lo, const double* step, cons
     exact[q] = gbx::query_exact(g, xi, off, q);
   }
 }
+
+// The grid of three axes of `steps` grid steps: its dims, its cells, the status.
+extern "C" long long grid_of(const double* steps, int* dims, unsigned* status) {
+  *status = 0u;
+  for (int k = 0; k < 3; ++k) dims[k] = gbx::axis_cells(steps[k], *status);
+  return gbx::grid_cells(dims);
+}

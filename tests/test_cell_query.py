@@ -27,7 +27,9 @@ def lib(tmp_path_factory):
                     "-I", CUDA_INCLUDE, "-I", os.path.join(REPO, "include"),
                     "-I", os.path.join(REPO, "openmmcustomgbintegralforce_gb300", "csrc"),
                     os.path.join(HERE, "cell_query.cpp"), "-o", out], check=True)
-    return ctypes.CDLL(out)
+    lib = ctypes.CDLL(out)
+    lib.grid_of.restype = ctypes.c_longlong
+    return lib
 
 
 def query(lib, mode, lo, step, dims, x, off, cells=None, entries=0, total=0, reach=2.0):
@@ -81,3 +83,30 @@ def test_an_outgrown_table_gives_no_cell(lib, mode, short):
             got, _ = query(lib, MODES[mode], lo, step, dims, x, points(rng, 300), **room)
             assert (got < 0).all(), (dims, z)
 
+
+
+def grid_of(lib, steps):
+    dims, status = (ctypes.c_int * 3)(), ctypes.c_uint()
+    ncell = lib.grid_of((ctypes.c_double * 3)(*steps), dims, ctypes.byref(status))
+    return list(dims), ncell, status.value
+
+
+TABLE_CELLS = 1  # status: the grid has more cells than are allocated
+
+
+# lengths in grid steps, with the largest that an index still holds
+@pytest.mark.parametrize("steps", [(0.0, 0.4, 1.0), (19.99, 20.0, 20.01), (1.0, 2147483646.0, 3.5), (2.0 ** 30,) * 3])
+def test_grids_that_exist(lib, steps):
+    dims, ncell, status = grid_of(lib, steps)
+    assert dims == [int(np.ceil(s)) + 1 for s in steps] and status == 0
+    assert ncell == min(int(np.prod([int(d) for d in dims], dtype=object)), 2 ** 62)
+
+
+# no grid: atoms out of any range, or nowhere
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 2147483646.5, 1e20, 1e300, -1.0])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_grids_that_do_not_exist(lib, axis, bad):
+    steps = [20.0, 21.0, 22.0]
+    steps[axis] = bad
+    dims, ncell, status = grid_of(lib, steps)
+    assert status == TABLE_CELLS and min(dims) == 1 and ncell == np.prod(dims)

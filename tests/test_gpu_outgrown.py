@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 BOTH = EXEC_FORCES | EXEC_ENERGY
-STALE = 10
+NONFINITE, TOO_LARGE, STALE = 5, 6, 10
 MODELS = {"grid": GBModel.gbsw_integral(), "standalone": GBModel.charmm_gbsw(reference_table=True),
           "gbmv1": GBModel.gbmv1(table_mode=TABLE_GRID), "gbmv2": GBModel.gbmv2(table_mode=TABLE_GRID)}
 
@@ -135,3 +135,35 @@ def test_compiled_expressions_on_the_grid_table():
     assert E == Ef and np.array_equal(F, Ff)
     ctx.close()
     fresh.close()
+
+
+# atoms nowhere, or so far away that no grid has an index for them: an error,
+# no cell of such a grid is read, and the context goes on
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, 1e20, -1e20])
+@pytest.mark.parametrize("which", ["one", "all"])
+@pytest.mark.parametrize("name", ["grid", "standalone", "gbmv1", "gbmv2"])
+def test_positions_without_a_grid(name, which, bad):
+    g = make_globule(200, seed=16)
+    ctx = context(MODELS[name], g)
+    E, F, status = device_call(ctx, g.positions, BOTH | EXEC_CHECK)
+    assert status == 0
+    x = g.positions.copy()
+    if which == "one":
+        x[3, 1] = bad
+    else:
+        x[:] = bad
+    # the extents leave out one position that is not a number, and atoms all at
+    # one place have a grid wherever that is
+    grid = np.isnan(bad) if which == "one" else np.isfinite(bad)
+    for _ in range(2):
+        assert device_call(ctx, x, BOTH | EXEC_CHECK)[2] in ((0, NONFINITE) if grid else (TOO_LARGE,))
+        device_call(ctx, x)  # unchecked: reported by the next call
+    # nor may such atoms size a table (a grid of one cell is not taken for one then)
+    fresh = context(MODELS[name], g)
+    assert device_call(fresh, x)[2] in ((0, NONFINITE, TOO_LARGE) if grid else (TOO_LARGE,))
+    assert device_call(fresh, g.positions)[1].shape == F.shape
+    fresh.close()
+    device_call(ctx, g.positions, BOTH | EXEC_CHECK)
+    E2, F2, status = device_call(ctx, g.positions, BOTH | EXEC_CHECK)
+    assert status == 0 and E2 == E and np.array_equal(F2, F)
+    ctx.close()
