@@ -631,6 +631,12 @@ gbx_status pipeline(Context* ctx, const float4* posq, unsigned long long* force,
   return run_pipeline(ctx, posq, force, stride, energy, check, adjoint, count_work, forces);
 }
 
+void settle_published(Context* ctx, unsigned st) {
+  // a run publishes one of each at most (publish_status)
+  if (st & (kStatusTableCells | kStatusTableEntries | kStatusSegmentTooLong)) ++ctx->pub_seen_overflows;
+  if (st & kStatusNonFinite) ++ctx->pub_seen_nonfinite;
+}
+
 gbx_status set_chunks(Context* ctx, int chunks) {
   const int Q = ctx->cfg.n_radial * ctx->cfg.lebedev_order;
   chunks = std::max(1, std::min(chunks, std::max(1, Q / 32)));
@@ -1232,6 +1238,7 @@ gbx_status host_results(Context* ctx, double* forces, double* energy, bool optim
   GBX_CUDA(cudaStreamSynchronize(ctx->stream));
   const unsigned st = *ctx->h_status;
   if (optimistic && (st & (gbx::kStatusTableCells | gbx::kStatusTableEntries | gbx::kStatusSegmentTooLong))) {
+    gbx::settle_published(ctx, st);
     if (rerun) *rerun = true;
     return GBX_OK;
   }
@@ -1372,6 +1379,7 @@ gbx_status gbx_adjoint(gbx_context* handle, const void* posq, double* energy, do
     GBX_CUDA(cudaStreamSynchronize(ctx->stream));
     const unsigned st = *ctx->h_status;
     if (st & (gbx::kStatusTableCells | gbx::kStatusTableEntries | gbx::kStatusSegmentTooLong)) {
+      gbx::settle_published(ctx, st);
       GBX_TRY(evaluate(true));
     } else if (st & gbx::kStatusNonFinite) {
       ctx->last_error = "non-finite Born radius";

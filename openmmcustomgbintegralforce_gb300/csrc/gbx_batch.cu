@@ -170,6 +170,17 @@ gbx_status run_checked(gbx_batch* b, cudaStream_t main) {
   return GBX_OK;
 }
 
+// A replay or unchecked fan-out that is evaluated again (every stream has been
+// waited for): each molecule settles what it published there.
+gbx_status settle(gbx_batch* b) {
+  for (auto c : b->mols) {
+    unsigned st = 0;
+    BCUDA(b, cudaMemcpy(&st, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    settle_published(c, st);
+  }
+  return GBX_OK;
+}
+
 gbx_status run(gbx_batch* b, cudaStream_t main, bool force_check) {
   if (force_check || !b->sized) return run_checked(b, main);
   if (!b->graph || b->graph_stream != main || graph_stale(b)) BTRY(capture(b, main));
@@ -181,7 +192,10 @@ gbx_status run(gbx_batch* b, cudaStream_t main, bool force_check) {
     b->last_error = "non-finite Born radius in the batch";
     return GBX_ERR_NONFINITE;
   }
-  if (st & (kStatusTableCells | kStatusTableEntries | kStatusSegmentTooLong)) return run_checked(b, main);
+  if (st & (kStatusTableCells | kStatusTableEntries | kStatusSegmentTooLong)) {
+    BTRY(settle(b));
+    return run_checked(b, main);
+  }
   return GBX_OK;
 }
 
@@ -231,6 +245,7 @@ gbx_status run_adjoint(gbx_batch* b, cudaStream_t main, bool force_check, const 
   BCUDA(b, cudaStreamSynchronize(main));
   unsigned st = *b->h_status;
   if (!force_check && (st & (kStatusTableCells | kStatusTableEntries | kStatusSegmentTooLong))) {
+    BTRY(settle(b));
     BTRY(adjoint_fan_out(b, main, true, o));
     BCUDA(b, cudaMemcpyAsync(b->h_status, b->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, main));
     BCUDA(b, cudaStreamSynchronize(main));

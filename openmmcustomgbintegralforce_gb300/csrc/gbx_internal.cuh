@@ -340,6 +340,10 @@ __host__ __device__ __forceinline__ double fixed_to_double(unsigned long long v)
 gbx_status pipeline(Context* ctx, const float4* posq, unsigned long long* force, int stride, double* energy, bool check,
                     bool adjoint, bool count_work, bool forces);
 gbx_status set_chunks(Context* ctx, int chunks);
+// For a call whose first, unchecked run outgrew its table (status st, read back)
+// and that evaluates again: what that run published is settled within the call,
+// so that no later call reports it.  What calls before it published stays due.
+void settle_published(Context* ctx, unsigned st);
 gbx_status fix_chain_records(Context* ctx);
 // Whether the exact GBSW table serves this context's configuration and
 // parameters (a periodic one needs the standalone grid's reach below half

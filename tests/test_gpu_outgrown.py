@@ -5,7 +5,8 @@ give a fresh context's bits."""
 import numpy as np
 import pytest
 
-from openmmcustomgbintegralforce_gb300._lib import EXEC_CHECK, EXEC_ENERGY, EXEC_FORCES, Context, CustomContext, GBXError
+from openmmcustomgbintegralforce_gb300._lib import (EXEC_CHECK, EXEC_ENERGY, EXEC_FORCES, Batch, Context,
+                                                     CustomContext, GBXError)
 from openmmcustomgbintegralforce_gb300.expression_sets import MODIFIED
 from openmmcustomgbintegralforce_gb300.globule import make_globule
 from openmmcustomgbintegralforce_gb300.spec import TABLE_GRID, GBModel
@@ -167,3 +168,47 @@ def test_positions_without_a_grid(name, which, bad):
     E2, F2, status = device_call(ctx, g.positions, BOTH | EXEC_CHECK)
     assert status == 0 and E2 == E and np.array_equal(F2, F)
     ctx.close()
+
+
+# a call that evaluates again has dealt with its table: the next call has
+# nothing to report, unless an unchecked one before was not reported yet
+@pytest.mark.parametrize("due", [False, True])
+@pytest.mark.parametrize("entry", ["host", "adjoint", "batch", "batch_adjoint"])
+@pytest.mark.parametrize("name", ["exact", "grid", "gbmv2"])
+def test_a_call_that_evaluated_again_leaves_nothing_to_report(name, entry, due):
+    g = make_globule(400, seed=18)
+    m = MODELS.get(name, GBModel.charmm_gbsw())
+    fresh = context(m, g)
+    batch = Batch([m, m], [g.n, g.n]) if entry.startswith("batch") else None
+    ctx = batch.molecules[1] if batch else Context(m, g.n)
+    for c in batch.molecules if batch else [ctx]:
+        c.set_particle_parameters(g.charge, g.radius)
+
+    def call(pos):
+        if batch:
+            x = np.concatenate([g.positions, pos])
+            batch.adjoint_host(x) if entry == "batch_adjoint" else batch.execute_host(x)
+        elif entry == "host":
+            ctx.execute_host(pos)
+        else:
+            n = g.n
+            posq = torch.zeros((n, 4), dtype=torch.float32, device="cuda:0")
+            posq[:, :3] = torch.from_numpy(pos).to(posq)
+            out = torch.zeros(1, dtype=torch.float64, device="cuda:0")
+            torch.cuda.synchronize()
+            ctx.adjoint_device(posq.data_ptr(), out.data_ptr(), 0, 0, 0, 0, EXEC_CHECK, 0)
+
+    for _ in range(2):
+        call(g.positions)
+    assert device_call(ctx, g.positions)[2] == 0
+    if due:
+        # in between in size, so that the call below outgrows the same buffers
+        assert device_call(ctx, spread(g))[2] == 0
+    call(spread(g))
+    E, F, status = device_call(ctx, g.positions)
+    assert status == (STALE if due else 0)
+    Ef, Ff, _ = device_call(fresh, g.positions, BOTH | EXEC_CHECK)
+    assert E == Ef and np.array_equal(F, Ff)
+    assert device_call(ctx, spread(g))[2] == 0
+    (batch or ctx).close()
+    fresh.close()
