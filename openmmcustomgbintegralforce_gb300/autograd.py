@@ -34,8 +34,7 @@ class GBEnergyFunction(torch.autograd.Function):
         if positions.shape != (n, 3) or charges.shape != (n,) or radii.shape != (n,) or alpha.shape != (2,):
             raise ValueError("GBEnergyFunction: expected positions [n,3], charges [n], radii [n], alpha [2]")
         # one transfer for the three parameter tensors, one allocation for every
-        # output, one product for every gradient: the call's host work is
-        # torch operations, each of them 5 to 30 us
+        # output: the call's host work is torch operations, each of them 5 to 30 us
         parts = [t.detach() for t in (charges, radii, alpha)]
         if len({(t.dtype, t.device) for t in parts}) > 1:
             parts = [t.to(positions.device, torch.float64) for t in parts]
@@ -62,12 +61,11 @@ class GBEnergyFunction(torch.autograd.Function):
     def backward(ctx, grad):
         (out,) = ctx.saved_tensors
         n = ctx.n
-        g = out * grad.to(torch.float64)
-        tp, tq, tr, ta = ctx.dtypes
-        if tp == tq == tr == ta:
-            g = g.to(tp)
-        dx, dq, dR, da = g[1:].split((3 * n, n, n, 2))
-        return (-dx).view(n, 3).to(tp), dq.to(tq), dR.to(tr), da.to(ta), None, None
+        tp, *rest = ctx.dtypes
+        dx, *dp = (out[1:] * grad.to(torch.float64)).split((3 * n, n, n, 2))
+        # copies, none a view of the product: a caller may write to one, or keep
+        # it, whatever becomes of the others
+        return (dx.view(n, 3).neg().to(tp), *(d.to(t, copy=True) for d, t in zip(dp, rest)), None, None)
 
 
 class GBEnergy(torch.nn.Module):
