@@ -254,6 +254,7 @@ gbx_status alloc_atom_buffers(Context* ctx) {
   GBX_CUDA(cudaMallocHost((void**)&ctx->h_status, sizeof(unsigned)));
   GBX_CUDA(cudaMallocHost((void**)&ctx->h_energy, sizeof(double)));
   GBX_CUDA(cudaEventCreateWithFlags(&ctx->srec_ev, cudaEventDisableTiming));
+  GBX_CUDA(cudaEventCreateWithFlags(&ctx->last_ev, cudaEventDisableTiming));
   GBX_TRY(dalloc(ctx, &ctx->d_pub, 5));
   GBX_CUDA(cudaMemset(ctx->d_pub, 0, sizeof(unsigned long long) * 5));
   GBX_CUDA(cudaHostAlloc((void**)&ctx->h_pub, sizeof(gbx::StatusRecord), cudaHostAllocMapped));
@@ -592,6 +593,18 @@ void set_model_params(const Context* ctx, float* wpar, float2* par) {
   }
 }
 
+// Marks the end of a call that returns with its kernels pending, on its stream
+// (a caller's graph marks each replay), for what must wait for them: an event
+// of the context's own, since the caller's stream may be gone by then.
+gbx_status mark_enqueued(Context* ctx) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  GBX_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+  GBX_CUDA(cudaEventRecordWithFlags(ctx->last_ev, ctx->stream,
+                                    cap == cudaStreamCaptureStatusNone ? cudaEventRecordDefault
+                                                                       : cudaEventRecordExternal));
+  return GBX_OK;
+}
+
 // Reads the status the device published for earlier unchecked calls (no
 // synchronisation).  A call whose lookup table outgrew its buffers ran
 // without the volume terms: *stale tells the caller to run this call checked
@@ -839,6 +852,7 @@ gbx_status gbx_destroy(gbx_context* handle) {
   if (ctx->h_energy) cudaFreeHost(ctx->h_energy);
   if (ctx->h_pub) cudaFreeHost(ctx->h_pub);
   if (ctx->srec_ev) cudaEventDestroy(ctx->srec_ev);
+  if (ctx->last_ev) cudaEventDestroy(ctx->last_ev);
   if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
   delete ctx;
   return GBX_OK;
@@ -863,6 +877,10 @@ gbx_status gbx_set_particle_parameters(gbx_context* handle, const double* charge
       return GBX_ERR_INVALID_ARGUMENT;
     }
   }
+  // the copy must race neither a call in flight, whose kernels read the
+  // parameters until its pair term, nor the next one: a plain copy is ordered
+  // with no stream that is created non-blocking
+  GBX_CUDA(cudaEventSynchronize(ctx->last_ev));
   ctx->charge.assign(charge, charge + n);
   ctx->radius.assign(radius, radius + n);
   std::vector<unsigned char> block(kParamBytes * (size_t)n);
@@ -873,7 +891,8 @@ gbx_status gbx_set_particle_parameters(gbx_context* handle, const double* charge
   memcpy(r, radius, sizeof(double) * n);
   for (int i = 0; i < n; ++i) qf[i] = (float)charge[i];
   set_model_params(ctx, wpar, par);
-  GBX_CUDA(cudaMemcpy(ctx->d_params, block.data(), block.size(), cudaMemcpyHostToDevice));
+  GBX_CUDA(cudaMemcpyAsync(ctx->d_params, block.data(), block.size(), cudaMemcpyHostToDevice, ctx->own_stream));
+  GBX_CUDA(cudaStreamSynchronize(ctx->own_stream));
   gbx::choose_table(ctx);
   return GBX_OK;
 }
@@ -1041,6 +1060,7 @@ gbx_status gbx_set_custom_parameters(gbx_context* handle, const double* params) 
   if (!ctx || !params) return GBX_ERR_INVALID_ARGUMENT;
   if (!ctx->custom) return GBX_ERR_UNSUPPORTED;
   std::vector<double> radius;
+  GBX_CUDA(cudaEventSynchronize(ctx->last_ev));  // as gbx_set_particle_parameters
   GBX_TRY(gbx::custom_set_parameters(ctx, params, radius));
   std::vector<double> q(ctx->n, 0.0);  // the custom terms read their own parameters
   return gbx_set_particle_parameters(handle, q.data(), radius.data());
@@ -1102,7 +1122,11 @@ gbx_status gbx_execute(gbx_context* handle, const void* posq, unsigned long long
     }
     return GBX_OK;
   };
-  if (check || count || ctx->timing) return report(body());
+  auto direct = [&]() -> gbx_status {
+    GBX_TRY(body());
+    return check ? GBX_OK : mark_enqueued(ctx);  // a checked call has waited
+  };
+  if (check || count || ctx->timing) return report(direct());
   // unchecked: one CUDA graph of the whole call, captured on first use
   const Context::GraphKey key{posq, force_fixed, force_stride, energy, flags & ~GBX_EXEC_CHECK, ctx->stream};
   if (!ctx->graph || !(key == ctx->graph_key)) {
@@ -1110,7 +1134,7 @@ gbx_status gbx_execute(gbx_context* handle, const void* posq, unsigned long long
     GBX_TRY(fix_chain_records(ctx));
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       (void)cudaGetLastError();  // a stream that cannot be captured: launch directly
-      return report(body());
+      return report(direct());
     }
     const long long before = ctx->launches;
     gbx_status s = body();
@@ -1134,7 +1158,7 @@ gbx_status gbx_execute(gbx_context* handle, const void* posq, unsigned long long
   GBX_CUDA(cudaGraphLaunch(ctx->graph, ctx->stream));
   ctx->launches += ctx->graph_kernels;
   ctx->have_result = true;
-  return report(GBX_OK);
+  return report(mark_enqueued(ctx));
 }
 
 gbx_status gbx_set_atom_order(gbx_context* handle, const int* atom_index) {
@@ -1388,7 +1412,8 @@ gbx_status gbx_adjoint(gbx_context* handle, const void* posq, double* energy, do
   } else {
     GBX_TRY(evaluate((flags & GBX_EXEC_CHECK) || (ctx->use_tight ? ctx->tcell_cap == 0 : ctx->cell_cap == 0)));
   }
-  return gbx::launch_adjoint_out(ctx, energy, forces, dEdq, dEdR, dEdalpha);
+  GBX_TRY(gbx::launch_adjoint_out(ctx, energy, forces, dEdq, dEdR, dEdalpha));
+  return flags & GBX_EXEC_CHECK ? GBX_OK : mark_enqueued(ctx);
 }
 
 gbx_status gbx_get_born_radii(gbx_context* handle, double* born) {

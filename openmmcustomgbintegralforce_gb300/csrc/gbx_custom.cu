@@ -912,9 +912,12 @@ gbx_status custom_set_parameters(Context* ctx, const double* params, std::vector
       pf[(size_t)k * n + i] = (float)v;
     }
   for (int i = 0; i < n; ++i) radius[i] = p->params[(size_t)p->radius_index * n + i];
-  if (cudaMemcpy(p->d_params, p->params.data(), sizeof(double) * p->params.size(), cudaMemcpyHostToDevice) !=
+  // the caller has waited for calls in flight; ordered before the next as gbx_set_particle_parameters' copy
+  if (cudaMemcpyAsync(p->d_params, p->params.data(), sizeof(double) * p->params.size(), cudaMemcpyHostToDevice,
+                      ctx->own_stream) != cudaSuccess ||
+      cudaMemcpyAsync(p->d_paramsf, pf.data(), sizeof(float) * pf.size(), cudaMemcpyHostToDevice, ctx->own_stream) !=
           cudaSuccess ||
-      cudaMemcpy(p->d_paramsf, pf.data(), sizeof(float) * pf.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+      cudaStreamSynchronize(ctx->own_stream) != cudaSuccess)
     return GBX_ERR_CUDA;
   return GBX_OK;
 }

@@ -236,6 +236,7 @@ struct Context {
   double* h_energy = nullptr;    // pinned: energy of the last host-path call
   cudaEvent_t srec_ev = nullptr;
   bool srec_pending = false;     // srec_ev recorded and not yet read
+  cudaEvent_t last_ev = nullptr; // the last unchecked call's work (mark_enqueued)
   bool have_result = false;
 
   long long launches = 0;  // kernels this context has launched
