@@ -43,6 +43,8 @@
 // FP32 difference is within a few tenths of a nanometre of the cell.
 #include <math.h>
 
+#include <algorithm>
+
 #include "bitonic.cuh"
 #include "gbx_internal.cuh"
 #include "queries.cuh"
@@ -492,28 +494,25 @@ struct __align__(16) PointChain {
 // 28, 32 blocks per SM: GBMV-II 381, 360, 369 us; GBMV-I 453, 416, 406 us;
 // four-warp blocks 405 and 446 us).
 constexpr int kChainWarps = 1;
+struct ChainShared {
+  ChainPair list[kMaxList / 2];
+  PointChain pt[kWarp];
+  float3 own[kWarp];
+};
+
+// One cell: P points, first in its slots, of `binned`.  r: R_j of the pairs (adjoint).
 template <int MODEL, bool PER, bool ADJ>
-__global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MODEL_GBMV2 ? 28 : 32)
-    gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab, Quad quad, ModelConst m, CellPoints cp,
-                           const float2* __restrict__ dEdJ, CellChainOut out) {
-  __shared__ ChainPair s_list[kChainWarps][kMaxList / 2];
-  __shared__ float2 s_r[ADJ ? kChainWarps : 1][ADJ ? kMaxList / 2 : 1];  // R_j of the pairs
-  __shared__ PointChain s_pt[kChainWarps][kWarp];
-  __shared__ float3 s_own[kChainWarps][kWarp];
-  const int w = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-  const long long cell = (long long)blockIdx.x * kChainWarps + w;
+__device__ __forceinline__ void chain_cell(const float4* __restrict__ pos, const Entries& tab, const Quad& quad,
+                                           const ModelConst& m, const CellPoints& cp, const float2* __restrict__ dEdJ,
+                                           const CellChainOut& out, long long cell, int binned, int P, int lane,
+                                           ChainShared& sh, float2* r) {
   const TableGeom& G = *tab.geom;
-  if (cell >= G.ncell || cell >= tab.cell_cap) return;
-  const int binned = cp.count[cell];
-  if (binned == 0) return;
-  const int P = cp.live[cell];
-  if (P == 0) return;
   const int2 cs = __ldg(tab.cell + cell);
   const int cnt = min(cs.x, kMaxList);
   const float3 c0 = cell_corner(G, (int)cell);
   Image<PER> img;
   img.init(G);
-  ChainPair* L = s_list[w];
+  ChainPair* L = sh.list;
   for (int l = lane; l < ((cnt + 1) & ~1); l += kWarp) {
     float4 a = make_float4(c0.x, c0.y, c0.z, 0.0f);  // padding: every contribution exactly zero
     float2 pk = make_float2(1.0f, 1.0f);
@@ -531,7 +530,7 @@ __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MO
     // GBMV-I's adjoint: dS/dR_j = -4 gamma_j e_j r^4 / R_j (gamma ~ R^-4), the division once per entry
     f[8] = ADJ && MODEL == GBX_MODEL_GBMV1 ? -4.0f * a.w / pk.x : pk.x;
     f[10] = __int_as_float(k);
-    if (ADJ) reinterpret_cast<float*>(s_r[w] + l / 2)[l & 1] = pk.y;
+    if (ADJ) reinterpret_cast<float*>(r + l / 2)[l & 1] = pk.y;
   }
   __syncwarp();
   const int start = cp.start[cell];
@@ -551,7 +550,7 @@ __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MO
     acc[e][0] = acc[e][1] = acc[e][2] = bc2(0.f);
     accR[e] = bc2(0.f);
   }
-  PointChain* pts = s_pt[w];
+  PointChain* pts = sh.pt;
   const float Cp = 10.0f * m.p1;
   for (int base = 0; base < P; base += kWarp) {
     // lane t prepares point base + t
@@ -678,7 +677,7 @@ __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MO
           const int j = es + e * kChainEnt, l = 2 * j;
           if (l < cnt) {
             const ChainPair c = L[j];
-            pair(e, l, c.x, c.y, c.z, c.w, c.k, ADJ ? s_r[w][j] : bc2(0.f), c.idx);
+            pair(e, l, c.x, c.y, c.z, c.w, c.k, ADJ ? r[j] : bc2(0.f), c.idx);
           }
         }
       }
@@ -690,12 +689,12 @@ __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MO
         py_ += __shfl_xor_sync(0xffffffffu, py_, off);
         pz_ += __shfl_xor_sync(0xffffffffu, pz_, off);
       }
-      if (es == 0 && t < np) s_own[w][t] = make_float3(px_, py_, pz_);
+      if (es == 0 && t < np) sh.own[t] = make_float3(px_, py_, pz_);
     }
     __syncwarp();
     // owner forces of these points: runs of one atom summed, one reduction per run
     {
-      float3 o = lane < np ? s_own[w][lane] : make_float3(0.f, 0.f, 0.f);
+      float3 o = lane < np ? sh.own[lane] : make_float3(0.f, 0.f, 0.f);
       const int key = lane < np ? pts[lane].i : -1 - lane;
       if (sorted) {
 #pragma unroll
@@ -746,6 +745,55 @@ __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MO
       const int2 k = L[es + e * kChainEnt].idx;
       if (l < cnt) add_fixed_one(out, k.x, ps, sign * sum.x);
       if (l + 1 < cnt) add_fixed_one(out, k.y, ps, sign * sum.y);
+    }
+  }
+}
+
+// SPARSE: a grid of fewer blocks than cells, each warp taking every so manieth
+// cell.  A block costs its launch, half a nanosecond of the whole pass, also for
+// a cell without points; the loop costs registers (72 to 128 bytes of spills
+// where one cell takes 8 to 24).  A molecule in a wide box has mostly empty
+// cells: chain rule with a block per cell and with the loop, 300 atoms in 10 nm
+// (1,048 cells an atom) 205 and 35 us, 2,000 atoms in 30 nm (4,060) 5,114 and
+// 121.  The line, in allocated cells (a quarter more than the box has), 24 x 26
+// points, per atom: GBMV-II 10,000 atoms 18 238 and 242, 33 297 and 293, 52 371
+// and 252, 2,513 atoms 30 72 and 88, 52 96 and 92, 1,000 atoms 74 49 and 49;
+// GBMV-I 10,000 atoms 33 311 and 346, 52 385 and 303.  4,096 to 65,536 blocks:
+// the same within a tenth at those sizes, more for 40 atoms (39 us with 65,536, 27
+// with 32,768).
+constexpr long long kSparseCells = 40;     // allocated cells per atom above which the loop is taken
+constexpr long long kSparseBlocks = 32768; // its grid, and the fewest cells it is taken for
+template <int MODEL, bool PER, bool ADJ, bool SPARSE>
+__global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MODEL_GBMV2 ? 28 : 32)
+    gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab, Quad quad, ModelConst m, CellPoints cp,
+                           const float2* __restrict__ dEdJ, CellChainOut out) {
+  __shared__ ChainShared s_sh[kChainWarps];
+  __shared__ float2 s_r[ADJ ? kChainWarps : 1][ADJ ? kMaxList / 2 : 1];
+  const int w = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+  const long long warp = (long long)blockIdx.x * kChainWarps + w;
+  const long long ncell = min(tab.geom->ncell, tab.cell_cap);
+  if constexpr (!SPARSE) {
+    if (warp >= ncell) return;
+    const int binned = cp.count[warp];
+    if (binned == 0) return;
+    const int P = cp.live[warp];
+    if (P == 0) return;
+    chain_cell<MODEL, PER, ADJ>(pos, tab, quad, m, cp, dEdJ, out, warp, binned, P, lane, s_sh[w], s_r[ADJ ? w : 0]);
+  } else {
+    // a lane looks at a cell; the warp then does those with points one by one
+    const long long warps = (long long)gridDim.x * kChainWarps;
+    for (long long first = warp; first < ncell; first += kWarp * warps) {
+      const long long mine = first + lane * warps;
+      int binned = 0, P = 0;
+      if (mine < ncell) binned = cp.count[mine];
+      if (binned > 0) P = cp.live[mine];
+      for (unsigned todo = __ballot_sync(0xffffffffu, P > 0); todo != 0u; todo &= todo - 1u) {
+        const int from = __ffs((int)todo) - 1;
+        chain_cell<MODEL, PER, ADJ>(pos, tab, quad, m, cp, dEdJ, out, first + from * warps,
+                                    __shfl_sync(0xffffffffu, binned, from), __shfl_sync(0xffffffffu, P, from), lane,
+                                    s_sh[w], s_r[ADJ ? w : 0]);
+        __syncwarp();  // the next cell takes the same buffers
+      }
     }
   }
 }
@@ -827,19 +875,29 @@ gbx_status launch_gbmv_cells_chain(Context* ctx, const float4* pos, const ModelC
   const CellPoints cp{ctx->d_pcount, ctx->d_plive, ctx->d_pstart, ctx->d_porder, ctx->d_pat,
                       ctx->d_sval,   ctx->d_pstate, (size_t)npts};
   const CellChainOut o{ctx->d_f4};
-  const int cell_blocks = (int)((ctx->cell_cap + kChainWarps - 1) / kChainWarps);
+  const long long cell_blocks = (ctx->cell_cap + kChainWarps - 1) / kChainWarps;
+  const bool sparse = cell_blocks > kSparseBlocks && ctx->cell_cap > kSparseCells * ctx->n;
   const bool per = ctx->cfg.periodic != 0;
-  const int sel = (m.model == GBX_MODEL_GBMV1 ? 0 : 4) + (per ? 2 : 0) + (adjoint ? 1 : 0);
-  switch (sel) {
-    case 0: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 1: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 2: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 3: gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 4: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 5: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    case 6: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, false><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
-    default: gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, true><<<cell_blocks, kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o); break;
+  void (*kernel)(const float4*, Entries, Quad, ModelConst, CellPoints, const float2*, CellChainOut);
+  switch ((m.model == GBX_MODEL_GBMV1 ? 0 : 8) + (per ? 4 : 0) + (adjoint ? 2 : 0) + (sparse ? 1 : 0)) {
+    case 0: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, false, false>; break;
+    case 1: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, false, true>; break;
+    case 2: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, true, false>; break;
+    case 3: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, false, true, true>; break;
+    case 4: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, false, false>; break;
+    case 5: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, false, true>; break;
+    case 6: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, true, false>; break;
+    case 7: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV1, true, true, true>; break;
+    case 8: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, false, false>; break;
+    case 9: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, false, true>; break;
+    case 10: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, true, false>; break;
+    case 11: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, false, true, true>; break;
+    case 12: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, false, false>; break;
+    case 13: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, false, true>; break;
+    case 14: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, true, false>; break;
+    default: kernel = gbmv_cell_chain_kernel<GBX_MODEL_GBMV2, true, true, true>; break;
   }
+  kernel<<<(int)(sparse ? kSparseBlocks : cell_blocks), kChainWarps * kWarp, 0, st>>>(pos, t, qd, m, cp, ctx->d_dEdJ, o);
   ++ctx->launches;
   return GBX_OK;
 }
