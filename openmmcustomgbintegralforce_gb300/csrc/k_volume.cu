@@ -759,6 +759,7 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
                                                                  ChainOut out, ChainRecords rr) {
   constexpr int kComp = ADJ ? 4 : 3;  // integers pushed per item
   constexpr int kWarps = kThreads / kWarp;
+  constexpr int kWalkKeep = 4;        // shaping entries remembered by a list walk
   constexpr int kRing = 2 * kWarp;    // fewer than 32 items pending, plus one round of at most 32
   __shared__ float4 s_v[kWarps][kRing];   // (v, V) of two batches' records
   __shared__ float2 s_c[kWarps][kRing];   // (c, list start)
@@ -880,6 +881,7 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
       const int slot = ((b - pts.t0) & kWarp) + lane;
       const int q = pts.q(b + lane);
       int cnt = 0, st = 0;
+      int kept[kWalkKeep] = {}, shaping = 0;  // list positions of the first shaping entries, and how many there are
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       float V = 1.0f;
       if (b + lane < pts.t1) {
@@ -891,23 +893,39 @@ __global__ void __launch_bounds__(kThreads, 8) gbsw_chain_kernel(const float4* _
           cnt = cs.x;  // buried or empty: no atom shapes the point
           st = cs.y;
         }
-        for (int l = 0; l < cnt; ++l) {
-          const float4 a = entry_at(tab, st + l);
-          const float dr = sphere_gap(query.delta(a, xi, v), a.w);
-          if (dr <= -m.sw) {
-            V = 0.0f;
-            cnt = 0;
-          } else if (dr < m.sw) {
-            V *= fmaf(dr, fmaf(-m.c3 * dr, dr, m.c1), 0.5f);
+        for (int l = 0; l < cnt; l += 2) {  // an odd list ends in a padding entry no point is near
+          const EntryPair p = ldg_entries(tab.e, st + l);
+          const float g[2] = {sphere_gap(query.delta(make_float4(p.x.x, p.y.x, p.z.x, 0.f), xi, v), -p.nw.x),
+                              sphere_gap(query.delta(make_float4(p.x.y, p.y.y, p.z.y, 0.f), xi, v), -p.nw.y)};
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (g[h] <= -m.sw) {
+              V = 0.0f;
+              cnt = 0;
+            } else if (g[h] < m.sw) {
+              V *= fmaf(g[h], fmaf(-m.c3 * g[h], g[h], m.c1), 0.5f);
+#pragma unroll
+              for (int u = 0; u < kWalkKeep; ++u)
+                if (shaping == u) kept[u] = l + h;
+              ++shaping;
+            }
           }
         }
-        if (V == 0.0f) cnt = 0;
+        if (V == 0.0f) cnt = shaping = 0;
         sv[slot] = make_float4(v.x, v.y, v.z, V);
         sc[slot] = make_float2(fmaf(de.x, w.x, de.y * w.y), __int_as_float(st));
       }
-      for (int l = 0; __any_sync(0xffffffffu, l < cnt); ++l) {
-        bool in = false;
-        if (l < cnt) {
+      // the shaping entries: those kept, or where there were more, all looked at again
+      const bool few = shaping <= kWalkKeep;
+      const int looks = few ? shaping : cnt;
+      for (int t = 0; __any_sync(0xffffffffu, t < looks); ++t) {
+        bool in = t < looks;
+        int l = t;
+        if (in && few) {
+#pragma unroll
+          for (int u = 0; u < kWalkKeep; ++u)
+            if (t == u) l = kept[u];
+        } else if (in) {
           const float4 a = entry_at(tab, st + l);
           in = fabsf(sphere_gap(query.delta(a, xi, v), a.w)) < m.sw;
         }

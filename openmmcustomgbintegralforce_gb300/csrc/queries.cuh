@@ -509,8 +509,8 @@ struct IsTight<PeriodicTightQuery> {
 
 // Entry `at` of a GBSW list as (x, y, z, R').
 __device__ __forceinline__ float4 entry_at(const Entries& t, int at) {
-  const float* p = reinterpret_cast<const float*>(t.e) + 8 * (size_t)(at >> 1) + (at & 1);
-  return make_float4(__ldg(p), __ldg(p + 2), __ldg(p + 4), -__ldg(p + 6));
+  const EntryPair p = ldg_entries(t.e, at & ~1);  // one load, where its four fields took one each
+  return at & 1 ? make_float4(p.x.y, p.y.y, p.z.y, -p.nw.y) : make_float4(p.x.x, p.y.x, p.z.x, -p.nw.x);
 }
 
 // ds/dS of the logistic below, from its p
