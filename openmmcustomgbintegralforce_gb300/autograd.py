@@ -61,11 +61,14 @@ class GBEnergyFunction(torch.autograd.Function):
     def backward(ctx, grad):
         (out,) = ctx.saved_tensors
         n = ctx.n
-        tp, *rest = ctx.dtypes
-        dx, *dp = (out[1:] * grad.to(torch.float64)).split((3 * n, n, n, 2))
+        g = out[1:] * grad  # FP64, as the saved gradients: `grad` is one number
+        tp, tq, tr, ta = ctx.dtypes
+        if tp == tq == tr == ta:
+            g = g.to(tp)
         # copies, none a view of the product: a caller may write to one, or keep
         # it, whatever becomes of the others
-        return (dx.view(n, 3).neg().to(tp), *(d.to(t, copy=True) for d, t in zip(dp, rest)), None, None)
+        dx, dq, dR, da = torch.split_with_sizes_copy(g, (3 * n, n, n, 2))
+        return dx.view(n, 3).neg().to(tp), dq.to(tq), dR.to(tr), da.to(ta), None, None
 
 
 class GBEnergy(torch.nn.Module):
