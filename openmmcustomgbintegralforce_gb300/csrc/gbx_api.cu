@@ -1158,6 +1158,7 @@ gbx_status gbx_execute(gbx_context* handle, const void* posq, unsigned long long
   GBX_CUDA(cudaGraphLaunch(ctx->graph, ctx->stream));
   ctx->launches += ctx->graph_kernels;
   ctx->have_result = true;
+  ctx->table_valid = !ctx->use_tight;  // a replay leaves what the captured call did
   return report(mark_enqueued(ctx));
 }
 
@@ -1322,6 +1323,7 @@ gbx_status host_graph_launch(Context* ctx, bool forces) {
   GBX_CUDA(cudaGraphLaunch(ctx->host_graph, ctx->stream));
   ctx->launches += ctx->host_graph_kernels;
   ctx->have_result = true;
+  ctx->table_valid = !ctx->use_tight;
   return GBX_OK;
 }
 

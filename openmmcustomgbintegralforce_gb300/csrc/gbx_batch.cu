@@ -185,6 +185,7 @@ gbx_status run(gbx_batch* b, cudaStream_t main, bool force_check) {
   if (force_check || !b->sized) return run_checked(b, main);
   if (!b->graph || b->graph_stream != main || graph_stale(b)) BTRY(capture(b, main));
   BCUDA(b, cudaGraphLaunch(b->graph, main));
+  for (auto c : b->mols) c->table_valid = !c->use_tight;  // a replay leaves what the captured calls did
   BCUDA(b, cudaMemcpyAsync(b->h_status, b->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, main));
   BCUDA(b, cudaStreamSynchronize(main));
   const unsigned st = *b->h_status;
