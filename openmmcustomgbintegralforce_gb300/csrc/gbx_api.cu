@@ -1467,6 +1467,10 @@ gbx_status gbx_get_lookup_table(gbx_context* handle, int dims[3], double mn[3], 
   gbx::TableGeom g;
   GBX_CUDA(cudaStreamSynchronize(ctx->stream));
   GBX_CUDA(cudaMemcpy(&g, ctx->d_geom, sizeof(g), cudaMemcpyDeviceToHost));
+  if (g.ncell > ctx->cell_cap || g.total > ctx->entry_cap) {
+    ctx->last_error = "the last call was unchecked and its lookup table outgrew its buffers: it has no lists";
+    return GBX_ERR_STALE_RESULT;
+  }
   for (int k = 0; k < 3; ++k) {
     if (dims) dims[k] = g.dims[k];
     if (mn) mn[k] = g.min[k];

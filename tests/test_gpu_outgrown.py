@@ -212,3 +212,24 @@ def test_a_call_that_evaluated_again_leaves_nothing_to_report(name, entry, due):
     assert device_call(ctx, spread(g))[2] == 0
     (batch or ctx).close()
     fresh.close()
+
+
+def blown(g):
+    """Some 10^27 cells."""
+    return g.positions * 1e8
+
+
+# an outgrown table has no lists to return, however many cells it wanted
+@pytest.mark.parametrize("name,moved", [(k, f) for k in ("grid", "standalone", "gbmv2") for f in (spread, far, blown)
+                                        if k == "standalone" or f is not blown])
+def test_no_table_where_it_outgrew_its_buffers(name, moved):
+    g = make_globule(400, seed=20)
+    ctx = context(MODELS[name], g)
+    assert device_call(ctx, g.positions, BOTH | EXEC_CHECK)[2] == 0
+    assert device_call(ctx, moved(g))[2] == 0
+    with pytest.raises(GBXError) as e:
+        ctx.lookup_table()
+    assert e.value.status == STALE
+    assert device_call(ctx, g.positions)[2] == STALE
+    assert ctx.lookup_table()["counts"].sum() > 0
+    ctx.close()
