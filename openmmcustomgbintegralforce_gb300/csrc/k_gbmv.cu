@@ -761,8 +761,9 @@ __device__ __forceinline__ void chain_cell(const float4* __restrict__ pos, const
 // GBMV-I 10,000 atoms 33 311 and 346, 52 385 and 303.  4,096 to 65,536 blocks:
 // the same within a tenth at those sizes, more for 40 atoms (39 us with 65,536, 27
 // with 32,768).
-constexpr long long kSparseCells = 40;     // allocated cells per atom above which the loop is taken
-constexpr long long kSparseBlocks = 32768; // its grid, and the fewest cells it is taken for
+constexpr long long kSparseCells = 40;     // allocated cells per atom above which the loop is taken,
+constexpr long long kSparseFrom = 65536;   // and in all (41,000 of 1,000 atoms: 41 and 47 us)
+constexpr long long kSparseBlocks = 32768; // its grid
 template <int MODEL, bool PER, bool ADJ, bool SPARSE>
 __global__ void __launch_bounds__(kChainWarps* kWarp, ADJ ? 24 : MODEL == GBX_MODEL_GBMV2 ? 28 : 32)
     gbmv_cell_chain_kernel(const float4* __restrict__ pos, Entries tab, Quad quad, ModelConst m, CellPoints cp,
@@ -876,7 +877,7 @@ gbx_status launch_gbmv_cells_chain(Context* ctx, const float4* pos, const ModelC
                       ctx->d_sval,   ctx->d_pstate, (size_t)npts};
   const CellChainOut o{ctx->d_f4};
   const long long cell_blocks = (ctx->cell_cap + kChainWarps - 1) / kChainWarps;
-  const bool sparse = cell_blocks > kSparseBlocks && ctx->cell_cap > kSparseCells * ctx->n;
+  const bool sparse = ctx->cell_cap > kSparseFrom && ctx->cell_cap > kSparseCells * ctx->n;
   const bool per = ctx->cfg.periodic != 0;
   void (*kernel)(const float4*, Entries, Quad, ModelConst, CellPoints, const float2*, CellChainOut);
   switch ((m.model == GBX_MODEL_GBMV1 ? 0 : 8) + (per ? 4 : 0) + (adjoint ? 2 : 0) + (sparse ? 1 : 0)) {

@@ -26,8 +26,8 @@ def context(m, g):
     return ctx
 
 
-# 600 atoms: 40 allocated cells an atom are 24,000, fewer than the 32,768 that
-# the loop is taken for; 1,500 atoms: 60,000.  Boxes of 12 nm hold 531,441 cells.
+# the loop is taken above 65,536 allocated cells and 40 an atom; a box of 12 nm
+# has 531,441 cells
 @pytest.mark.parametrize("kw", [{}, dict(cutoff=1.0, periodic=True)], ids=["plain", "periodic"])
 @pytest.mark.parametrize("n", [2, 33, 600, 1500])
 @pytest.mark.parametrize("name", ["gbmv1", "gbmv2"])
