@@ -138,7 +138,9 @@ GBX_API gbx_status gbx_destroy(gbx_context* ctx);
 GBX_API gbx_status gbx_last_error(const gbx_context* ctx, char* buf, size_t len);
 
 /* Per-particle charge (e) and input radius (nm).  Replaces
- * copyParametersToContext (charmmKernels.h:88,128; CharmmReferenceKernels.cpp:439-458). */
+ * copyParametersToContext (charmmKernels.h:88,128; CharmmReferenceKernels.cpp:439-458).
+ * Waits for the context's unchecked calls (replays of a caller's graph of one
+ * too): their results are those of the parameters they were issued with. */
 GBX_API gbx_status gbx_set_particle_parameters(gbx_context* ctx, const double* charge, const double* radius);
 /* ------------------------------------------------------------------------
  * A CharmmGBMVForce with expressions outside the canonical CHARMM set
@@ -254,14 +256,17 @@ GBX_API gbx_status gbx_get_dEdB(gbx_context* ctx, double* dEdB);
 
 /* Lookup table of the last execute (or built by gbx_build_lookup_table):
  * dims, min corner, steps and the per-cell lists in ascending atom order.
- * Pass NULL arrays to query sizes first. */
+ * Pass NULL arrays to query sizes first.  GBX_ERR_STALE_RESULT after an
+ * unchecked execute whose table outgrew its buffers: it has no lists. */
 GBX_API gbx_status gbx_build_lookup_table(gbx_context* ctx, const void* posq, void* stream);
 GBX_API gbx_status gbx_get_lookup_table(gbx_context* ctx, int dims[3], double min[3], double step[3],
                                         int64_t* ncell, int32_t* counts, int64_t* total, int32_t* atoms);
 
-/* Adjoint: dE/dx (as forces), dE/dq [n], dE/dR_in [n], dE/dalpha [2].  The
- * per-point volumes are recomputed, not stored.  No counterpart in the
- * reference, which only returns forces; it carries the same chain rule
+/* Adjoint: dE/dx (as forces), dE/dq [n], dE/dR_in [n], dE/dalpha [2].  GBSW
+ * adjoints keep point records as force calls do (gbx_set_chain_records; none
+ * under a caller's stream capture) and walk the lists where those do not
+ * serve; GBMV ones keep the points' sums.  No counterpart in the reference,
+ * which only returns forces; it carries the same chain rule
  * (CharmmReferenceGBSW.cpp:597-674) to the parameters.  Host arrays. */
 GBX_API gbx_status gbx_adjoint_host(gbx_context* ctx, const double* positions, double* energy, double* forces,
                                     double* dEdq, double* dEdR, double* dEdalpha);

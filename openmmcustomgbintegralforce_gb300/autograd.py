@@ -5,8 +5,9 @@ One forward call runs the whole pipeline once in adjoint mode -- table,
 integrals, Born radii, pair term, chain rule with dE/dR and dE/dq -- and
 keeps the gradients with respect to positions, charges, input radii and the
 two Born-radius coefficients (alpha0, alpha1) for the backward, which only
-scales them by the incoming gradient.  Per-point volumes are recomputed
-inside the chain rule rather than stored, so memory stays O(N + table).
+scales them by the incoming gradient.  Beside the table the context holds a
+record per point that some atom's shell holds (GBSW) or the sums of every
+point (GBMV); none of them is kept for the backward.
 
 The reference exposes the same gradients through its reference platform
 (CharmmReferenceGBSW.cpp:597-674 for dB/dx, CharmmReferenceGBMV.cpp:349-443

@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(kMemberThreads, 5) table_members_grid_kernel(c
       sq[k][m] = (float)d * (float)d;
     }
     __syncwarp();
-    // FP32 squared distances carry a relative error below 4 2^-24
+    // FP32 squared distances carry a relative error below 5 2^-24 (three roundings of
+    // a square, two of the sums), the rounded bounds 2^-24 more: 1e-6 is 16.8 2^-24
     const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
     const int total = nn[0] * nn[1] * nn[2];
     const BoxIndex box(nn[1], nn[2]);
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(kMemberThreads, 5) table_members_periodic_kern
     }
     __syncwarp();
     const long long sy = g.dims[2], sx = (long long)g.dims[1] * g.dims[2];
-    // FP32 squared distances carry a relative error below 4 2^-24
+    // the margin of table_members_grid_kernel
     const float in2 = (float)(pad2 * (1.0 - 1e-6)), out2 = (float)(pad2 * (1.0 + 1e-6));
     const int total = cnt[0] * cnt[1] * cnt[2];
     const BoxIndex box(cnt[1], cnt[2]);

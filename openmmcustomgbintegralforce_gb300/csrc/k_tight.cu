@@ -15,7 +15,8 @@
 //   * the grid spans the atoms' bounding box plus max(R') + w + h, so a
 //     point outside it touches no shell (V = 1).
 //
-// eps (2e-5 nm plus 2 ulp of the largest coordinate) covers the FP32
+// eps (2e-5 nm plus 4 2^-23 of the largest coordinate, with the grid's margins
+// and a periodic system's longest box edge added to it) covers the FP32
 // rounding of both the build and the point-to-cell assignment, so every
 // atom a point needs is in the list of whichever neighbouring cell its FP32
 // coordinates select.  Entries are stored inline (x, y, z, R') and sorted by
